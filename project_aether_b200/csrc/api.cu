@@ -48,12 +48,7 @@ int run_sort(SortArgs& a, int path) {
   const bool roomy = a.workspace_bytes >= bucketed_workspace_bytes(a.n, a.num_cells);
   const bool bucketed = plan.usable && path != 1 && (roomy || path == 2);
   if (path == 2 && (!plan.usable || !roomy)) return cudaErrorInvalidValue;
-  if (!bucketed) return standard_sort(a, nullptr);
-  cudaError_t e = bucketed_sort(a, plan);
-  if (e != cudaSuccess) return e;
-  // Runs only if the device found a bucket the finish kernel cannot hold.
-  const Header* hdr = static_cast<const Header*>(a.workspace);
-  return standard_sort(a, &hdr->use_standard);
+  return bucketed ? bucketed_sort(a, plan) : standard_sort(a);
 }
 
 }  // namespace

@@ -27,6 +27,7 @@ constexpr uint32_t kValueMask = ~kFlagMask;
 constexpr int kErrLookbackTimeout = 1;
 constexpr int kErrBucketOverflow = 2;
 constexpr int kErrBulkCopyTimeout = 3;
+constexpr int kErrBarrierTimeout = 4;
 constexpr int kErrReceiveOverflow = 5;
 constexpr int kErrExchangeTimeout = 6;
 
@@ -52,12 +53,15 @@ struct SliceSegments {
 struct alignas(16) Header {
   int32_t error;              // first error code seen, 0 when clean
   int32_t use_standard;       // bucketed path: 1 when it handed over to the digit passes
+  uint32_t barrier;           // arrivals at the barriers of the cooperative launch
+  uint32_t unused;
   uint32_t tile_counter[kMaxPasses];  // ticket dispenser of each digit pass
   uint32_t aux_counter[8];
   uint32_t max_bucket;        // bucketed path: largest bucket seen
-  uint32_t pad[49];
+  uint32_t pad[47];
   uint32_t digit_hist[kMaxPasses][kRadix];  // global digit histograms (upsweep)
 };
+constexpr size_t kHeaderKept = 16;  // bytes the hand-over to the digit passes does not clear
 static_assert(sizeof(Header) % 256 == 0, "header must keep 256-byte alignment");
 
 __host__ __device__ inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
@@ -274,10 +278,12 @@ struct SortArgs {
 
 size_t standard_workspace_bytes(int64_t n, int64_t num_cells);
 size_t standard_workspace_bytes_with_records(int64_t n, int64_t num_cells);
-// `run_if`: device flag; when not null the kernels do nothing unless it is
-// nonzero (the hand-over from the bucketed path), and the first 8 bytes of the
-// workspace header (error code and that flag) are left as they are.
-cudaError_t standard_sort(const SortArgs& a, const int32_t* run_if);
+// The digit-pass sort, one launch per step.
+cudaError_t standard_sort(const SortArgs& a);
+// Arguments of the same sort inside one cooperative launch (the hand-over from the bucketed
+// path); refuses the workspaces that standard_sort refuses.
+struct DigitPassArgs;
+cudaError_t digit_pass_args(const SortArgs& a, DigitPassArgs* out);
 
 // One digit pass over three tiles of zero keys with the ticket dispenser started at 1: the
 // tile that would publish first is never processed, so every look-back runs out of polls,
@@ -327,10 +333,9 @@ cudaError_t launch_make_keys(const float* x, const float* y, const float* z, int
 cudaError_t launch_gather(const int32_t* index, int64_t n, const float* x, const float* y,
                           const float* z, const float* velocity, int64_t padded, float* xs,
                           float* ys, float* zs, float* vs, int64_t padded_sorted,
-                          cudaStream_t stream, const int32_t* run_if = nullptr);
+                          cudaStream_t stream);
 cudaError_t launch_cell_tables(const uint32_t* sorted_keys, int64_t n, int64_t num_cells,
-                               int32_t* cell_counts, int32_t* cell_start, cudaStream_t stream,
-                               const int32_t* run_if = nullptr);
+                               int32_t* cell_counts, int32_t* cell_start, cudaStream_t stream);
 
 cudaError_t slab_exchange_count(const float* x, const float* vx, const PushSpec& push, int64_t n,
                                 const AetherGrid& g, int world, int64_t* totals, void* workspace,

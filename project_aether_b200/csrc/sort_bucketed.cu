@@ -39,6 +39,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "digit_passes.cuh"
 
 namespace aether {
 
@@ -1241,8 +1242,24 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
 }
 
 // The buckets the kernel above skipped: those with more records than its shared
-// memory holds.  Usually there are none and every block returns after a look at
-// the largest bucket count.
+// memory holds.  `block` of `blocks` takes every blocks-th bucket; false if one of its
+// buckets cannot be finished at all.
+template <class Shape>
+__device__ bool finish_large_buckets(FinishSmem<Shape>& s, const RunTable& t, const FinishOut& out,
+                                     int64_t num_cells, uint32_t capacity, int block, int blocks) {
+  for (int b = block; b < t.buckets; b += blocks) {
+    const uint32_t begin = t.bucket_start[b], end = t.bucket_start[b + 1];
+    const int count = static_cast<int>(end - begin);
+    if (static_cast<uint32_t>(count) <= capacity) continue;
+    const int64_t first_cell = static_cast<int64_t>(b) << t.shift;
+    const int cells_here = static_cast<int>(
+        min(static_cast<long long>(1) << t.shift, static_cast<long long>(num_cells - first_cell)));
+    if (!finish_large_bucket<Shape>(s, out, t, b, begin, count, first_cell, cells_here)) return false;
+  }
+  return true;
+}
+
+// Behind the finish kernel of the multi-GPU form, which has no digit passes to hand over to.
 template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, 1)
 bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
@@ -1250,20 +1267,39 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
   chain_begin();
   if (hdr->use_standard || hdr->max_bucket <= capacity) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
-  for (int b = blockIdx.x; b < t.buckets; b += gridDim.x) {
-    const uint32_t begin = t.bucket_start[b], end = t.bucket_start[b + 1];
-    const int count = static_cast<int>(end - begin);
-    if (static_cast<uint32_t>(count) <= capacity) continue;
-    const int64_t first_cell = static_cast<int64_t>(b) << t.shift;
-    const int cells_here = static_cast<int>(
-        min(static_cast<long long>(1) << t.shift, static_cast<long long>(num_cells - first_cell)));
-    if (!finish_large_bucket<Shape>(s, out, t, b, begin, count, first_cell, cells_here)) {
-      if (threadIdx.x == 0) hdr->use_standard = 1;
-      return;
-    }
-  }
+  if (!finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
+                                   num_cells, capacity, blockIdx.x, gridDim.x) &&
+      threadIdx.x == 0)
+    hdr->use_standard = 1;
 }
+
+// Behind the finish kernel of an ordinary call, one cooperative launch: the oversized buckets,
+// then, when the call was handed over, the whole digit-pass sort.  Usually there is nothing
+// to do and every block returns after a look at the header.  What bounds it is then the launch
+// itself: as the separate kernels it replaces (the oversized buckets, a clear, the keys, up to
+// four digit passes, two table kernels and the payload gather, each returning at once) the same
+// look cost 13-17 us of every call on the device and 11 launches on the host.
+template <class Shape>
+__global__ void __launch_bounds__(Shape::kThreads, 1)
+bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
+                   DigitPassArgs digits) {
+  const bool handed_over = ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) != 0;
+  if (!handed_over && hdr->max_bucket <= capacity) return;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  // A block that comes late may already see another block's hand-over and skip its buckets:
+  // the digit passes then write everything.
+  if (!handed_over &&
+      !finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
+                                   num_cells, capacity, blockIdx.x, gridDim.x) &&
+      threadIdx.x == 0)
+    atomicExch(&hdr->use_standard, 1);
+  if (!grid_barrier(&hdr->barrier, 1, &hdr->error)) return;
+  if (ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) == 0) return;
+  digit_passes_in_grid<Shape::kThreads>(
+      digits, *reinterpret_cast<PassSmem<Shape::kThreads>*>(smem_raw), hdr, 1);
+}
+static_assert(sizeof(PassSmem<FinishLarge::kThreads>) <= sizeof(FinishSmem<FinishLarge>),
+              "the tail kernel's shared memory holds either");
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -1390,34 +1426,63 @@ namespace {
 
 template <class Shape>
 cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                          uint32_t group_capacity, const uint32_t* n_on_device = nullptr) {
+                          const uint32_t* n_on_device = nullptr) {
   const size_t table_bytes = 3 * 2 * static_cast<size_t>(t.row_words) * sizeof(uint32_t);
   if (Shape::kThreads <= 512 && table_bytes > kSmallShapeTableBytes) return cudaErrorInvalidValue;
   const int smem = static_cast<int>(sizeof(FinishSmem<Shape>) + table_bytes);
   cudaError_t e = cudaFuncSetAttribute(bucket_finish_kernel<Shape>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  // Buckets in no group (more records than a group may hold) go to the large shape whatever
-  // the shape of the groups: a single cell may then hold up to its 5120 records.
-  const int smem_large = static_cast<int>(sizeof(FinishSmem<FinishLarge>));
-  e = cudaFuncSetAttribute(bucket_finish_large_kernel<FinishLarge>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem_large);
-  if (e != cudaSuccess) return e;
   const int per_sm = Shape::kThreads <= 512 ? 2 : 1;
   e = launch_chained<true>(bucket_finish_kernel<Shape>, std::min(t.buckets, sm_count() * per_sm),
                      Shape::kThreads, smem, a.stream, t, a.n, n_on_device, a.num_cells, out, hdr);
   if (e != cudaSuccess) return e;
+  return e;
+}
+
+// Buckets in no group (more records than a group may hold) go to the large shape whatever
+// the shape of the groups: a single cell may then hold up to its 5120 records.
+constexpr int kTailSmem = static_cast<int>(sizeof(FinishSmem<FinishLarge>));
+
+cudaError_t launch_finish_large(const RunTable& t, const SortArgs& a, const FinishOut& out,
+                                Header* hdr, uint32_t group_capacity) {
+  cudaError_t e = cudaFuncSetAttribute(bucket_finish_large_kernel<FinishLarge>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+  if (e != cudaSuccess) return e;
   e = launch_chained<true>(bucket_finish_large_kernel<FinishLarge>, std::min(t.buckets, sm_count()),
-                     FinishLarge::kThreads, smem_large, a.stream, t, a.num_cells, out, hdr,
-                     group_capacity);
+                           FinishLarge::kThreads, kTailSmem, a.stream, t, a.num_cells, out, hdr,
+                           group_capacity);
   return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
+                        uint32_t group_capacity) {
+  DigitPassArgs digits;
+  cudaError_t e = digit_pass_args(a, &digits);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(bucket_tail_kernel<FinishLarge>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute cooperative{};
+  cooperative.id = cudaLaunchAttributeCooperative;
+  cooperative.val.cooperative = 1;
+  cudaLaunchConfig_t config{};
+  // One block per multiprocessor (all resident at once), fewer where there is little to do.
+  config.gridDim = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(sm_count(), a.n / 2048)));
+  config.blockDim = FinishLarge::kThreads;
+  config.dynamicSmemBytes = kTailSmem;
+  config.stream = a.stream;
+  config.attrs = &cooperative;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, bucket_tail_kernel<FinishLarge>, t, a.num_cells, out, hdr,
+                            group_capacity, digits);
 }
 
 }  // namespace
 
 // Enqueues the bucketed path.  When a bucket turns out too large for the finish
-// kernel the device sets Header::use_standard and the remaining kernels return
-// at once; the caller then enqueues the digit-pass path predicated on that flag.
+// kernel the device sets Header::use_standard, the kernels between return at once
+// and the tail kernel runs the digit passes.
 cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   const BucketLayout l = bucket_layout(a.n, p.buckets);
   if (a.workspace_bytes < l.total || l.chunks > kMaxChunks) return cudaErrorInvalidValue;
@@ -1543,8 +1608,9 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                       a.vs, a.padded_sorted};
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
                    table_row_words(l.chunks), l.chunks, buckets, p.shift};
-  e = p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, group_capacity)
-                     : launch_finish<FinishLarge>(t, a, out, hdr, group_capacity);
+  e = p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr)
+                     : launch_finish<FinishLarge>(t, a, out, hdr);
+  if (e == cudaSuccess) e = launch_tail(t, a, out, hdr, group_capacity);
   stage_end(kStageBucketFinish, a.stream);
   count_launches(2);
   return e;
@@ -1708,9 +1774,9 @@ cudaError_t sliced_sort_finish(const SortArgs& a, int64_t plan_n, const SliceSeg
                       a.vs, a.padded_sorted};
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
                    table_row_words(l.chunks), l.chunks, buckets, p.shift};
-  const cudaError_t e = p.small_blocks
-                            ? launch_finish<FinishSmall>(t, a, out, hdr, group_capacity, n_on_device)
-                            : launch_finish<FinishLarge>(t, a, out, hdr, group_capacity, n_on_device);
+  cudaError_t e = p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, n_on_device)
+                                 : launch_finish<FinishLarge>(t, a, out, hdr, n_on_device);
+  if (e == cudaSuccess) e = launch_finish_large(t, a, out, hdr, group_capacity);
   stage_end(kStageBucketFinish, a.stream);
   return e;
 }

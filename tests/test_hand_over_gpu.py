@@ -1,0 +1,57 @@
+"""Calls that the bucketed path hands over to the digit passes on the device: one cooperative
+launch then runs them all."""
+
+import numpy as np
+import pytest
+import torch
+
+import project_aether_b200 as pa
+from oracle import sort_oracle as so
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(n, device, seed):
+    gen = torch.Generator(device=device).manual_seed(seed)
+    pos = [torch.rand(n, device=device, generator=gen) for _ in range(3)]
+    vel = torch.zeros((3, -(-n // 4) * 4), device=device)
+    vel[:, :n] = torch.randn((3, n), device=device, generator=gen)
+    return pos, vel
+
+
+# One, two, three and four passes (key widths of 8, 10, 22 and 28 bits); tiles of 6144 keys cut
+# exactly, one short and one over, and more tiles than multiprocessors.
+@pytest.mark.parametrize('n,cells', [(12_288, (1, 1, 1)), (12_287, (7, 1, 1)), (40_001, (32, 32, 32)),
+                                     (6_145, (128, 128, 128)), (1_200_007, (64, 64, 128))])
+@pytest.mark.parametrize('moved', [False, True])
+def test_dense_cell_is_sorted_by_the_digit_passes(cuda, n, cells, moved):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), cells)
+    pos, vel = _state(n, cuda, n)
+    crowd = torch.arange(n, device=cuda) % 7 != 0  # most particles in one cell
+    for k in range(3):
+        pos[k][crowd] = 0.4
+        vel[k, :n][crowd] *= 1e-6
+    dt = 1e-3
+    push = (dt, grid.lo, grid.hi) if moved else None
+    seed = 0x1234567 + n
+    got = pa.sort_and_gather_particles(*pos, vel, grid, seed, push=push)
+    assert pa.last_sort_status(cuda) == 0
+    assert pa.last_sort_used_digit_passes(cuda)
+    p = [t.cpu().numpy() for t in pos]
+    v = vel.cpu().numpy()
+    if moved:
+        p, rows = so.push_particles(p, [v[k, :n] for k in range(3)], dt, grid.lo, grid.hi)
+        v[:, :n] = np.stack(rows)
+    want = so.sort_particles(*p, so.Grid(grid.lo, grid.hi, grid.cells), seed)
+    sorted_payload = so.gather_payload(want.particle_index, *p, v)
+    np.testing.assert_array_equal(got.order.keys.cpu().numpy().view(np.uint32), want.keys)
+    np.testing.assert_array_equal(got.order.particle_index.cpu().numpy(), want.particle_index)
+    np.testing.assert_array_equal(got.order.cell_counts.cpu().numpy(), want.cell_counts)
+    np.testing.assert_array_equal(got.order.cell_start.cpu().numpy(), want.cell_start)
+    for g, w in zip((*got.positions, got.velocity), sorted_payload):
+        np.testing.assert_array_equal(g.cpu().numpy(), w)
+    if not moved:  # the same call without payload
+        order = pa.sort_particles_by_cell(*pos, grid, seed)
+        assert pa.last_sort_status(cuda) == 0
+        np.testing.assert_array_equal(order.particle_index.cpu().numpy(), want.particle_index)
+        np.testing.assert_array_equal(order.cell_start.cpu().numpy(), want.cell_start)
