@@ -7,14 +7,13 @@
 // sum rounded on its own, as the reference's host replay computes them
 // (dsmc_collide_tma_test.cu:45-84).
 //
-// Layout of the work: a block owns a run of consecutive cells.  It packs as many
-// whole cells as fit into a shared-memory stage (4096 particles), reads their
-// velocities with coalesced 128-bit loads, draws every cell's number of candidate
-// pairs, and then hands the pairs of ALL staged cells out to its threads one pair
-// per thread, so that cells of ten particles keep a block as busy as cells of a
-// thousand.  Velocities are updated in shared memory and the stage is written
-// back with coalesced stores only when a pair in it collided.  A cell larger
-// than the stage is worked on in global memory by the whole block.
+// Layout of the work: a block owns a run of consecutive cells, one per thread.  It draws every
+// cell's number of candidate pairs, scans the numbers, and hands the pairs of ALL its cells out
+// to its threads one pair per thread, so that cells of ten particles keep a block as busy as
+// cells of a thousand.  A pair's velocities are read from and, if it collides, written to
+// global memory directly: pair p of a cell is its particles 2p and 2p + 1, so neighbouring
+// threads read neighbouring words, no two pairs share a particle, and the sectors of the many
+// particles that are in no candidate pair are neither read nor written.
 #include <algorithm>
 
 #include "common.cuh"
@@ -23,9 +22,6 @@ namespace aether {
 namespace {
 
 constexpr int kCollideThreads = 256;
-constexpr int kMaxCellsPerBlock = 256;
-constexpr int kStageParticles = 4096;
-constexpr int kStageRow = kStageParticles + 4;  // room for the aligned start of the first quad
 constexpr uint32_t kCellDraw = 0xFFFFFFFFu;     // pair id of a cell's selection draw
 
 struct CollideArgs {
@@ -35,8 +31,6 @@ struct CollideArgs {
   int* collisions;
   int padded;
   int num_cells;
-  int cells_per_block;
-  int aligned;  // velocity rows start on 16-byte boundaries
   float selection_factor, coefficient, exponent;
   uint32_t key0, key1, step_lo, step_hi;
 };
@@ -106,200 +100,72 @@ __device__ __forceinline__ bool collide_pair(float* a, float* b, float majorant,
   return true;
 }
 
-struct CollideSmem {
-  float stage[3][kStageRow];
-  int start[kMaxCellsPerBlock + 1];        // cell_start of the block's cells
-  int pair_first[kMaxCellsPerBlock + 1];   // exclusive prefix of candidate pairs of the staged cells
-  int accepted[kMaxCellsPerBlock];
-  uint32_t observed[kMaxCellsPerBlock];    // largest sigma*g seen, as float bits (non-negative)
-  float majorant[kMaxCellsPerBlock];       // sigma_g_max of the staged cells before this step
-  uint32_t warp_sum[32];
-  uint32_t total;
-  int any_accepted;
-};
-
-__global__ void __launch_bounds__(kCollideThreads)
+// Bound by the latency of a block's chain (starts, draw, scan, pairs, results) and by the sectors
+// that hold candidate pairs; so little shared memory, and five blocks of 256 threads (48
+// registers) per multiprocessor.  A first design staged every particle of the block's cells in
+// shared memory, four blocks per multiprocessor, and wrote the stage back: 16 M particles in 2 M
+// cells took it 123 us, this kernel 63 (436 MB if every velocity is read and written once).
+__global__ void __launch_bounds__(kCollideThreads, 5)
 collide_kernel(CollideArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  CollideSmem& s = *reinterpret_cast<CollideSmem*>(smem_raw);
+  __shared__ int start[kCollideThreads];
+  __shared__ int pair_first[kCollideThreads];      // exclusive prefix of the candidate pairs
+  __shared__ int accepted[kCollideThreads];
+  __shared__ uint32_t observed[kCollideThreads];   // largest sigma*g seen, as float bits (non-negative)
+  __shared__ float majorants[kCollideThreads];     // sigma_g_max before this step
+  __shared__ uint32_t warp_sum[32];
+  __shared__ uint32_t total;
   const int tid = threadIdx.x;
-  const int first_cell = blockIdx.x * a.cells_per_block;
-  const int cells_here = min(a.cells_per_block, a.num_cells - first_cell);
-  for (int i = tid; i <= cells_here; i += kCollideThreads) s.start[i] = a.cell_start[first_cell + i];
+  const int first_cell = blockIdx.x * kCollideThreads;
+  const int cells_here = min(kCollideThreads, a.num_cells - first_cell);
+  const int my_cell = first_cell + tid;
+  float majorant = 0.0f;
+  uint32_t selections = 0;
+  if (tid < cells_here) {
+    const int begin = a.cell_start[my_cell];
+    const int count = a.cell_start[my_cell + 1] - begin;
+    majorant = a.sigma_g_max[my_cell];
+    selections = static_cast<uint32_t>(max(
+        0, ntc_selections(count, majorant, a.selection_factor,
+                          unit_float(collision_words(my_cell, kCellDraw, a).x))));
+    start[tid] = begin;
+    accepted[tid] = 0;
+    observed[tid] = 0;
+    majorants[tid] = majorant;
+  }
+  const int before = static_cast<int>(block_exclusive_scan(selections, warp_sum, &total));
+  pair_first[tid] = before;
   __syncthreads();
-
-  int lo = 0;  // first cell of the block not yet done
-  while (lo < cells_here) {
-    const int origin = s.start[lo];
-    // Whole cells lo..hi-1 fit the stage: hi = last index with start[hi] <= origin + stage.
-    int hi;
-    {
-      int left = lo, right = cells_here;  // invariant: start[left] <= limit
-      const int limit = origin + kStageParticles;
-      while (left < right) {
-        const int mid = (left + right + 1) >> 1;
-        if (s.start[mid] <= limit) left = mid; else right = mid - 1;
-      }
-      hi = left;
-    }
-    if (hi == lo) {
-      // One cell larger than the stage: the block works on it in global memory.
-      const int cell = first_cell + lo;
-      const int count = s.start[lo + 1] - origin;
-      const float majorant = a.sigma_g_max[cell];
-      if (tid == 0) {
-        s.accepted[0] = 0;
-        s.observed[0] = 0;
-      }
-      __syncthreads();
-      const int selections = ntc_selections(count, majorant, a.selection_factor,
-                                            unit_float(collision_words(cell, kCellDraw, a).x));
-      int mine = 0;
-      float seen = 0.0f;
-      for (int pair = tid; pair < selections; pair += kCollideThreads) {
-        const size_t i = static_cast<size_t>(origin) + 2 * pair;
-        float v1[3], v2[3];
+  const int pairs = static_cast<int>(total);
+  for (int p = tid; p < pairs; p += kCollideThreads) {
+    // The cell of pair p: last t with pair_first[t] <= p (cells without pairs share a value).
+    int t = 0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          v1[c] = a.velocity[static_cast<size_t>(c) * a.padded + i];
-          v2[c] = a.velocity[static_cast<size_t>(c) * a.padded + i + 1];
-        }
-        float sigma_g = 0.0f;
-        if (collide_pair(v1, v2, majorant, a, collision_words(cell, static_cast<uint32_t>(pair), a),
-                         &sigma_g)) {
+    for (int step = kCollideThreads / 2; step > 0; step >>= 1)
+      if (pair_first[t + step] <= p) t += step;
+    const uint32_t pair = static_cast<uint32_t>(p - pair_first[t]);
+    const size_t i = static_cast<size_t>(start[t]) + 2 * pair;
+    float v1[3], v2[3];
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            a.velocity[static_cast<size_t>(c) * a.padded + i] = v1[c];
-            a.velocity[static_cast<size_t>(c) * a.padded + i + 1] = v2[c];
-          }
-          ++mine;
-        }
-        seen = fmaxf(seen, sigma_g);
-      }
-      if (mine) atomicAdd(&s.accepted[0], mine);
-      if (seen > 0.0f) atomicMax(&s.observed[0], __float_as_uint(seen));
-      __syncthreads();
-      if (tid == 0) {
-        a.sigma_g_max[cell] = fmaxf(majorant, __uint_as_float(s.observed[0]));
-        a.collisions[cell] = s.accepted[0];
-      }
-      __syncthreads();
-      lo += 1;
-      continue;
+    for (int c = 0; c < 3; ++c) {
+      v1[c] = a.velocity[static_cast<size_t>(c) * a.padded + i];
+      v2[c] = a.velocity[static_cast<size_t>(c) * a.padded + i + 1];
     }
-
-    const int staged_cells = hi - lo;
-    const int end = s.start[hi];
-    const int shift = a.aligned ? (origin & 3) : 0;  // stage index 0 holds particle origin - shift
-    const int base = origin - shift;
-    // Stage the velocities of particles [origin, end).
-    if (a.aligned) {
-      const int quads = (end - base + 3) >> 2;  // the rows are padded to a multiple of four
-      for (int q = tid; q < quads; q += kCollideThreads) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          *reinterpret_cast<float4*>(&s.stage[c][4 * q]) = *reinterpret_cast<const float4*>(
-              a.velocity + static_cast<size_t>(c) * a.padded + base + 4 * q);
-      }
-    } else {
-      for (int i = tid; i < end - origin; i += kCollideThreads) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          s.stage[c][i] = a.velocity[static_cast<size_t>(c) * a.padded + origin + i];
-      }
-    }
-    // Candidate pairs of every staged cell (one cell per thread; at most 256 cells).
-    float majorant = 0.0f;
-    uint32_t selections = 0;
-    if (tid < staged_cells) {
-      const int cell = first_cell + lo + tid;
-      const int count = s.start[lo + tid + 1] - s.start[lo + tid];
-      majorant = a.sigma_g_max[cell];
-      selections = static_cast<uint32_t>(max(
-          0, ntc_selections(count, majorant, a.selection_factor,
-                            unit_float(collision_words(cell, kCellDraw, a).x))));
-      s.accepted[tid] = 0;
-      s.observed[tid] = 0;
-      s.majorant[tid] = majorant;
-    }
-    if (tid == 0) s.any_accepted = 0;
-    const uint32_t before = block_exclusive_scan(selections, s.warp_sum, &s.total);
-    if (tid < staged_cells) s.pair_first[tid] = static_cast<int>(before);
-    __syncthreads();
-    const int pairs = static_cast<int>(s.total);
-    if (tid == 0) s.pair_first[staged_cells] = pairs;
-    __syncthreads();
-
-    for (int p = tid; p < pairs; p += kCollideThreads) {
-      // The cell of pair p: last t with pair_first[t] <= p (cells without pairs share a value).
-      int left = 0, right = staged_cells - 1;
-      while (left < right) {
-        const int mid = (left + right + 1) >> 1;
-        if (s.pair_first[mid] <= p) left = mid; else right = mid - 1;
-      }
-      const int t = left;
-      const int pair = p - s.pair_first[t];
-      const int cell = first_cell + lo + t;
-      const int k = s.start[lo + t] - base + 2 * pair;
-      float v1[3], v2[3];
+    float sigma_g = 0.0f;
+    if (collide_pair(v1, v2, majorants[t], a, collision_words(first_cell + t, pair, a), &sigma_g)) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        v1[c] = s.stage[c][k];
-        v2[c] = s.stage[c][k + 1];
+        a.velocity[static_cast<size_t>(c) * a.padded + i] = v1[c];
+        a.velocity[static_cast<size_t>(c) * a.padded + i + 1] = v2[c];
       }
-      const float cell_majorant = s.majorant[t];
-      float sigma_g = 0.0f;
-      if (collide_pair(v1, v2, cell_majorant, a,
-                       collision_words(cell, static_cast<uint32_t>(pair), a), &sigma_g)) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          s.stage[c][k] = v1[c];
-          s.stage[c][k + 1] = v2[c];
-        }
-        atomicAdd(&s.accepted[t], 1);
-        s.any_accepted = 1;
-      }
-      if (sigma_g > 0.0f) atomicMax(&s.observed[t], __float_as_uint(sigma_g));
+      atomicAdd(&accepted[t], 1);
     }
-    __syncthreads();
-    if (tid < staged_cells) {
-      const int cell = first_cell + lo + tid;
-      a.sigma_g_max[cell] = fmaxf(majorant, __uint_as_float(s.observed[tid]));
-      a.collisions[cell] = s.accepted[tid];
-    }
-    if (s.any_accepted) {
-      // Write the stage back: 128-bit stores over the quads that lie wholly inside
-      // [origin, end), single words at the ragged ends.
-      if (a.aligned) {
-        const int first_quad = (shift + 3) >> 2;          // first quad starting at or after origin
-        const int last_quad = (end - base) >> 2;           // quads below this end inside the range
-        for (int q = first_quad + tid; q < last_quad; q += kCollideThreads) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            *reinterpret_cast<float4*>(a.velocity + static_cast<size_t>(c) * a.padded + base +
-                                       4 * q) = *reinterpret_cast<const float4*>(&s.stage[c][4 * q]);
-        }
-        const int head_end = min(end - base, 4 * first_quad);
-        const int tail_begin = max(head_end, 4 * last_quad);
-        if (tid < 8) {
-          const int i = tid < 4 ? shift + tid : tail_begin + (tid - 4);
-          const bool ok = tid < 4 ? i < head_end : i < end - base;
-          if (ok) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-              a.velocity[static_cast<size_t>(c) * a.padded + base + i] = s.stage[c][i];
-          }
-        }
-      } else {
-        for (int i = tid; i < end - origin; i += kCollideThreads) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            a.velocity[static_cast<size_t>(c) * a.padded + origin + i] = s.stage[c][i];
-        }
-      }
-    }
-    __syncthreads();
-    lo = hi;
+    if (sigma_g > 0.0f) atomicMax(&observed[t], __float_as_uint(sigma_g));
+  }
+  __syncthreads();
+  if (tid < cells_here) {
+    const float raised = fmaxf(majorant, __uint_as_float(observed[tid]));
+    if (__float_as_uint(raised) != __float_as_uint(majorant)) a.sigma_g_max[my_cell] = raised;
+    a.collisions[my_cell] = accepted[tid];
   }
 }
 
@@ -323,13 +189,6 @@ cudaError_t collide_cells(float* velocity, const int* cell_start, float* sigma_g
   a.collisions = collisions;
   a.padded = padded;
   a.num_cells = num_cells;
-  // Cells per block: about three quarters of a stage at the average occupancy, so
-  // that most blocks fill the stage once.
-  const double per_cell = std::max(1.0, static_cast<double>(num_particles) / num_cells);
-  int cells = static_cast<int>(0.75 * kStageParticles / per_cell);
-  cells = std::max(32, std::min(kMaxCellsPerBlock, cells / 32 * 32));
-  a.cells_per_block = cells;
-  a.aligned = (reinterpret_cast<uintptr_t>(velocity) & 15) == 0;
   a.selection_factor = selection_factor;
   a.coefficient = coefficient;
   a.exponent = exponent;
@@ -337,12 +196,9 @@ cudaError_t collide_cells(float* velocity, const int* cell_start, float* sigma_g
   a.key1 = static_cast<uint32_t>(seed >> 32);
   a.step_lo = static_cast<uint32_t>(step);
   a.step_hi = static_cast<uint32_t>(step >> 32);
-  cudaError_t e = cudaFuncSetAttribute(collide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(sizeof(CollideSmem)));
-  if (e != cudaSuccess) return e;
-  const int blocks = (num_cells + cells - 1) / cells;
+  const int blocks = (num_cells + kCollideThreads - 1) / kCollideThreads;
   stage_begin(kStageCollide, stream);
-  collide_kernel<<<blocks, kCollideThreads, sizeof(CollideSmem), stream>>>(a);
+  collide_kernel<<<blocks, kCollideThreads, 0, stream>>>(a);
   stage_end(kStageCollide, stream);
   count_launches(1);
   return cudaGetLastError();

@@ -21,7 +21,7 @@ def _state(n, device, seed):
 
 # One, two, three and four passes (key widths of 8, 10, 22 and 28 bits); tiles of 6144 keys cut
 # exactly, one short and one over, and more tiles than multiprocessors.
-@pytest.mark.parametrize('n,cells', [(12_288, (1, 1, 1)), (12_287, (7, 1, 1)), (40_001, (32, 32, 32)),
+@pytest.mark.parametrize('n,cells', [(6_144, (2, 1, 1)), (12_287, (7, 1, 1)), (40_001, (32, 32, 32)),
                                      (6_145, (128, 128, 128)), (1_200_007, (64, 64, 128))])
 @pytest.mark.parametrize('moved', [False, True])
 def test_dense_cell_is_sorted_by_the_digit_passes(cuda, n, cells, moved):
