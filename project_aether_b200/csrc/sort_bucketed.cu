@@ -190,124 +190,74 @@ bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
   }
 }
 
-// Per bucket: particles in all chunks.
-__global__ void __launch_bounds__(256)
-bucket_total_kernel(const uint32_t* __restrict__ bucket_count, int buckets, int chunks,
-                    uint32_t* __restrict__ total) {
-  chain_begin();
-  const int b = blockIdx.x * 256 + threadIdx.x;
-  if (b >= buckets) return;
-  uint32_t sum = 0;
-  for (int c = 0; c < chunks; ++c) sum += bucket_count[static_cast<size_t>(c) * buckets + b];
-  total[b] = sum;
-}
-
-// Exclusive scan of the [chunk][bucket] counts in memory order: where every run
-// starts in the record array.  Two levels (1024 entries per block, then the
-// block totals), then one pass that writes the run starts twice: as the scatter's
-// cursors, which the scatter advances, and as the table run_begin[chunk * buckets + b]
-// (with the total behind its last entry) from which the finish kernel takes the run
-// of any range of buckets [b0, b1) in chunk c: run_begin[c*B + b0] .. run_begin[c*B + b1].
-constexpr int kFlatScanBlock = 1024;
-
-__global__ void __launch_bounds__(kFlatScanBlock)
-run_scan_local_kernel(const uint32_t* __restrict__ count, int64_t entries,
-                      uint32_t* __restrict__ local, uint32_t* __restrict__ block_sum) {
-  chain_begin();
-  __shared__ uint32_t warp_sum[32];
-  __shared__ uint32_t total;
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * kFlatScanBlock + threadIdx.x;
-  const uint32_t v = i < entries ? count[i] : 0u;
-  const uint32_t excl = block_exclusive_scan(v, warp_sum, &total);
-  if (i < entries) local[i] = excl;
-  if (threadIdx.x == 0) block_sum[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kFlatScanBlock)
-run_scan_blocks_kernel(uint32_t* __restrict__ block_sum, int blocks) {
-  chain_begin();
-  __shared__ uint32_t warp_sum[32];
-  __shared__ uint32_t total, carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < blocks; base += kFlatScanBlock) {
-    const int i = base + threadIdx.x;
-    const uint32_t v = i < blocks ? block_sum[i] : 0u;
-    const uint32_t excl = block_exclusive_scan(v, warp_sum, &total);
-    if (i < blocks) block_sum[i] = carry + excl;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += total;
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(256)
-run_table_kernel(const uint32_t* __restrict__ local, const uint32_t* __restrict__ block_sum,
-                 int64_t entries, uint32_t n, uint32_t* __restrict__ cursor,
-                 uint32_t* __restrict__ run_begin) {
-  chain_begin();
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
-  if (i > entries) return;
-  const uint32_t start = i < entries ? local[i] + block_sum[i / kFlatScanBlock] : n;
-  run_begin[i] = start;
-  if (i < entries) cursor[i] = start;
-}
-
 // ------------------------------------------------------------------------
-// Bucket starts.
+// Where the runs start.
 // ------------------------------------------------------------------------
-constexpr int kScanThreads = 1024;
+constexpr int kRunScanThreads = 1024;
+constexpr int kRunScanPart = kRunScanThreads * 4;  // entries of a row per block
 
-__global__ void __launch_bounds__(kScanThreads)
-bucket_scan_kernel(const uint32_t* __restrict__ bucket_count, int buckets, int64_t n,
-                   const uint32_t* __restrict__ n_on_device, uint32_t capacity,
-                   uint32_t* __restrict__ bucket_start, uint32_t* __restrict__ cursor,
-                   Header* __restrict__ hdr) {
+// Exclusive scan of every chunk's row of counts; block (part, chunk) writes kRunScanPart entries
+// of the row.  Chunk c's records begin at record c << chunk_log, because a chunk is that many
+// consecutive particles, so the rows do not wait for one another; and a block adds up the
+// entries before its own for itself (they lie in L2) instead of waiting for their blocks.  The
+// starts are written twice: as the scatter's cursors, which the scatter advances, and as the
+// table run_begin[chunk * buckets + b] (with n behind its last entry) from which the run of any
+// range of buckets [b0, b1) in chunk c is taken: run_begin[c*B + b0] .. run_begin[c*B + b1].
+// Bound by latency.  This kernel and group_kernel replace seven (bucket totals, two bucket scans,
+// three levels of run scan, two group kernels); from the count's end to the scatter's begin, before
+// and after: 4 M particles in 10,000 cells 75 / 10 us, 16 M in 2 M 33 / 15, 128 M in 16 M 89 / 36.
+__global__ void __launch_bounds__(kRunScanThreads)
+run_scan_kernel(const uint32_t* __restrict__ count, int buckets, int chunk_log, uint32_t n,
+                uint32_t* __restrict__ cursor, uint32_t* __restrict__ run_begin) {
   chain_begin();
   __shared__ uint32_t warp_sum[32];
-  __shared__ uint32_t biggest;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) biggest = 0;
-  __syncthreads();
-  const int per = (buckets + kScanThreads - 1) / kScanThreads;
-  const int first = min(buckets, tid * per), last = min(buckets, first + per);
-  uint32_t sum = 0, big = 0;
-  for (int b = first; b < last; ++b) {
-    const uint32_t c = bucket_count[b];
-    sum += c;
-    big = max(big, c);
-  }
-  uint32_t incl = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) warp_sum[warp] = incl;
-  if (big) atomicMax(&biggest, big);
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = warp_sum[lane], wi = w;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
-      if (lane >= o) wi += t;
+  __shared__ uint32_t total, before_part;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const size_t row = static_cast<size_t>(blockIdx.y) * buckets;
+  const int part = blockIdx.x * kRunScanPart;
+  const int i = part + tid * 4;
+  const bool vec = buckets % 4 == 0;  // rows then start on 16-byte boundaries
+  if (tid == 0) before_part = static_cast<uint32_t>(blockIdx.y) << chunk_log;
+  uint32_t c[4] = {0, 0, 0, 0}, before = 0;
+  if (vec) {
+    if (i < buckets) {
+      const uint4 q = *reinterpret_cast<const uint4*>(count + row + i);
+      c[0] = q.x; c[1] = q.y; c[2] = q.z; c[3] = q.w;
     }
-    warp_sum[lane] = wi - w;
+#pragma unroll 8
+    for (int k = tid * 4; k < part; k += kRunScanPart) {
+      const uint4 q = *reinterpret_cast<const uint4*>(count + row + k);
+      before += q.x + q.y + q.z + q.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = i + k < buckets ? count[row + i + k] : 0u;
+#pragma unroll 8
+    for (int k = tid; k < part; k += kRunScanThreads) before += count[row + k];
   }
+  before = __reduce_add_sync(0xffffffffu, before);
   __syncthreads();
-  uint32_t run = warp_sum[warp] + incl - sum;
-  for (int b = first; b < last; ++b) {
-    bucket_start[b] = run;
-    if (cursor) cursor[b] = run;
-    run += bucket_count[b];
+  if (lane == 0 && before) atomicAdd(&before_part, before);
+  uint32_t start = block_exclusive_scan(c[0] + c[1] + c[2] + c[3], warp_sum, &total);
+  start += before_part;  // complete: the scan has barriers
+  if (vec) {
+    if (i < buckets) {
+      const uint4 q = make_uint4(start, start + c[0], start + c[0] + c[1], start + c[0] + c[1] + c[2]);
+      *reinterpret_cast<uint4*>(cursor + row + i) = q;
+      *reinterpret_cast<uint4*>(run_begin + row + i) = q;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < buckets) {
+        cursor[row + i + k] = start;
+        run_begin[row + i + k] = start;
+      }
+      start += c[k];
+    }
   }
-  if (tid == 0) {
-    bucket_start[buckets] = n_on_device ? *n_on_device : static_cast<uint32_t>(n);
-    hdr->max_bucket = biggest;
-    // A bucket above `capacity` cannot be finished at all: hand over before the scatter runs.
-    if (biggest > capacity) hdr->use_standard = 1;
-  }
+  if (blockIdx.x == 0 && blockIdx.y == gridDim.y - 1 && tid == 0)
+    run_begin[static_cast<size_t>(gridDim.y) * buckets] = n;
 }
 
 // ------------------------------------------------------------------------
@@ -514,6 +464,7 @@ bucket_count_segments_kernel(const float* __restrict__ x, const float* __restric
 // STAGED: the row fits shared memory (padded against bank conflicts); it is read and written
 // once, coalesced, and every thread scans a contiguous piece of it.  Otherwise 1024 entries
 // at a time.
+constexpr int kFlatScanBlock = 1024;
 constexpr int kStagedScanMax = 48 * 1024;  // buckets whose row (plus padding) fits 200 KB
 
 template <bool STAGED>
@@ -622,96 +573,152 @@ bucket_scatter_segments_kernel(const float* __restrict__ x, const float* __restr
 // ------------------------------------------------------------------------
 // Groups: consecutive buckets that one block finishes together.
 // ------------------------------------------------------------------------
-// One thread per aligned block of 2^group_shift buckets cuts it, greedily from the bucket
-// totals, into groups of consecutive buckets with at most `capacity` records, and appends
-// them (first bucket, end bucket) to the group list; their order in the list is of no
-// consequence.  A bucket that exceeds the capacity on its own is not listed:
-// bucket_finish_large_kernel takes it.
-__global__ void __launch_bounds__(256)
-group_cut_kernel(const uint32_t* __restrict__ bucket_start, int buckets, int group_shift,
-                 uint32_t capacity, uint2* __restrict__ groups, uint32_t* __restrict__ group_count) {
-  chain_begin();
-  const int block_of_buckets = blockIdx.x * 256 + threadIdx.x;
-  const int b_first = block_of_buckets << group_shift;
-  if (b_first >= buckets) return;
-  const int b_last = min(buckets, b_first + (1 << group_shift));
-  uint32_t base = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    uint32_t found = 0;
-    int b0 = b_first;
-    uint32_t begin = bucket_start[b0];
-    while (b0 < b_last) {
-      int b1 = b0 + 1;
-      uint32_t end = bucket_start[b1];
-      const bool fits = end - begin <= capacity;
-      if (fits) {
-        while (b1 < b_last) {
-          const uint32_t further = bucket_start[b1 + 1];
-          if (further - begin > capacity) break;
-          end = further;
-          ++b1;
-        }
-        if (pass == 1) groups[base + found] = make_uint2(static_cast<uint32_t>(b0), static_cast<uint32_t>(b1));
-        ++found;
-      }
-      b0 = b1;
-      begin = end;
-    }
-    if (pass == 0) {
-      if (found == 0) return;
-      base = atomicAdd(group_count, found);
-    }
-  }
-}
-
 // Words of one row of a group's table: one entry per chunk and three more, rounded up to
 // whole 16-byte pieces (the finish kernel fetches the tables with 16-byte copies).
 __host__ __device__ inline int table_row_words(int chunks) { return (chunks + 3 + 3) / 4 * 4; }
 
-// Where the records of every group lie: per group two rows of table_row_words(chunks) words,
+constexpr int kGroupSpan = 256;        // buckets per block of group_kernel
+constexpr int kGroupStagedChunks = 32; // chunks whose run starts the block keeps
+
+// A block takes kGroupSpan consecutive buckets.  Bucket starts: the records before bucket b are
+// the records before it in every chunk, sum over c of run_begin[c][b] - (first record of c).
+// Every aligned block of 2^group_shift buckets is then cut greedily into groups of consecutive
+// buckets with at most `capacity` records (each bucket looks up where a group that began with
+// it would end, and those links are followed), and every group gets a table
+// of where its records lie, two rows of table_row_words(chunks) words,
 //   row 0: [c] first record of the group's run in chunk c; [chunks] first output slot of the
 //          group; [chunks + 1], [chunks + 2] its buckets b0, b1
 //   row 1: [c] records of the group in chunks before c; [chunks] records of the group.
-// One warp per group, a lane per chunk.
-__global__ void __launch_bounds__(256)
-group_table_kernel(const uint2* __restrict__ groups, const uint32_t* __restrict__ group_count,
-                   const uint32_t* __restrict__ bucket_start, const uint32_t* __restrict__ run_begin,
-                   int chunks, int buckets, uint32_t* __restrict__ tables) {
+// The order of the groups in the list is of no consequence.  A bucket that exceeds the capacity
+// on its own is not listed: finish_large_buckets takes it; one above `largest` cannot be
+// finished at all and hands the call over before the scatter runs.
+// Bound by latency: with a warp per group for its table and one thread following the links it
+// took 22 us at 4 M particles (1250 buckets), with a chunk's loads one after the other 35 us at
+// 64 M (16 chunks); now 6.5 and 19.
+// `segments`: the sliced form, whose chunks begin at chunk_base[c] instead of c << chunk_log.
+__global__ void __launch_bounds__(kGroupSpan)
+group_kernel(const uint32_t* __restrict__ run_begin, int buckets, int chunks, int chunk_log,
+             const SliceSegments* __restrict__ segments, int group_shift, uint32_t capacity,
+             uint32_t largest, uint32_t* __restrict__ bucket_start, uint32_t* __restrict__ tables,
+             uint32_t* __restrict__ group_count, Header* __restrict__ hdr) {
   chain_begin();
-  const int lane = threadIdx.x & 31;
-  const uint32_t total = *group_count;
+  // Up to kGroupStagedChunks chunks, [chunks][kGroupSpan + 1] each: the first record of every
+  // run, and the records before the bucket in the chunks before c.
+  extern __shared__ uint32_t staged[];
+  __shared__ uint32_t start[kGroupSpan + 1];
+  __shared__ uint16_t link[kGroupSpan], group_first[kGroupSpan], jumps[kGroupSpan + 1];
+  __shared__ unsigned char is_first[kGroupSpan + 1];
+  __shared__ uint32_t warp_sum[32], found, list_base;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int b0 = blockIdx.x * kGroupSpan;
+  const int here = min(kGroupSpan, buckets - b0);
+  const bool keep = chunks <= kGroupStagedChunks;
+  uint32_t* earlier = staged + chunks * (kGroupSpan + 1);
+  // Entry `here` (the end of the last bucket) is summed by the first thread as well.  The loads of
+  // eight chunks are under way together.
+  for (int i = tid; i <= here; i += kGroupSpan) {
+    uint32_t sum = 0;
+    for (int c0 = 0; c0 < chunks; c0 += 8) {
+      uint32_t s[8], base[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int c = min(c0 + k, chunks - 1);
+        s[k] = run_begin[static_cast<size_t>(c) * buckets + b0 + i];
+        base[k] = segments ? segments->chunk_base[c] : static_cast<uint32_t>(c) << chunk_log;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int c = c0 + k;
+        if (c >= chunks) break;
+        if (keep) {
+          staged[c * (kGroupSpan + 1) + i] = s[k];
+          earlier[c * (kGroupSpan + 1) + i] = sum;
+        }
+        sum += s[k] - base[k];
+      }
+    }
+    start[i] = sum;
+    bucket_start[b0 + i] = sum;
+  }
+  __syncthreads();
+  uint32_t load = 0;
+  const bool first_of_block = tid < here && (tid & ((1 << group_shift) - 1)) == 0;
+  int jump = kGroupSpan;
+  if (tid < here) {
+    load = start[tid + 1] - start[tid];
+    const int block_end = min(here, ((tid >> group_shift) + 1) << group_shift);
+    int lo = tid + 1, hi = block_end;  // the last end with start[end] - start[tid] <= capacity
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (start[mid] - start[tid] <= capacity) lo = mid; else hi = mid - 1;
+    }
+    link[tid] = static_cast<uint16_t>(lo);
+    jump = lo < block_end ? lo : kGroupSpan;  // leaves its aligned block: no link
+  }
+  is_first[tid] = first_of_block;
+  if (tid == 0) is_first[kGroupSpan] = 0;
+  const uint32_t biggest = __reduce_max_sync(0xffffffffu, load);
+  if (lane == 0 && biggest > 0) {
+    atomicMax(&hdr->max_bucket, biggest);
+    if (biggest > largest) hdr->use_standard = 1;
+  }
+  // The groups' first buckets: those reached from the aligned blocks' first buckets along the
+  // links, 2^k links at a time in round k.
+  for (int hops = 1; hops < (1 << group_shift) && hops < kGroupSpan; hops <<= 1) {
+    jumps[tid] = static_cast<uint16_t>(jump);
+    if (tid == 0) jumps[kGroupSpan] = kGroupSpan;
+    __syncthreads();
+    const bool pass_on = is_first[tid];
+    const int to = jump;
+    jump = jumps[jump];
+    __syncthreads();
+    if (pass_on) is_first[to] = 1;
+  }
+  __syncthreads();
+  if (tid < here && load > capacity) is_first[tid] = 0;  // too large for a group
+  if (tid >= here) is_first[tid] = 0;
+  const uint32_t mine = is_first[tid];
+  const uint32_t place = block_exclusive_scan(mine, warp_sum, &found);
+  if (mine) group_first[place] = static_cast<uint16_t>(tid);
+  if (tid == 0) list_base = found ? atomicAdd(group_count, found) : 0u;
+  __syncthreads();
+  // The block's tables are one piece of memory: written word by word in order, whatever group and
+  // chunk a word belongs to.
   const int row_words = table_row_words(chunks);
-  for (uint32_t g = blockIdx.x * 8 + (threadIdx.x >> 5); g < total; g += gridDim.x * 8) {
-    const uint2 group = groups[g];
-    uint32_t* row0 = tables + static_cast<size_t>(g) * 2 * row_words;
+  uint32_t* table = tables + static_cast<size_t>(list_base) * 2 * row_words;
+  if (keep) {
+    const uint32_t words = found * 2 * row_words;
+    for (uint32_t w = tid; w < words; w += kGroupSpan) {
+      const uint32_t row = w / row_words, g = row >> 1;
+      const int c = static_cast<int>(w - row * row_words);
+      const int first = group_first[g], end = link[first];
+      uint32_t value = 0;
+      if (row & 1) {
+        if (c < chunks) value = earlier[c * (kGroupSpan + 1) + end] - earlier[c * (kGroupSpan + 1) + first];
+        else if (c == chunks) value = start[end] - start[first];
+      } else {
+        if (c < chunks) value = staged[c * (kGroupSpan + 1) + first];
+        else if (c == chunks) value = start[first];
+        else if (c == chunks + 1) value = static_cast<uint32_t>(b0 + first);
+        else if (c == chunks + 2) value = static_cast<uint32_t>(b0 + end);
+      }
+      table[w] = value;
+    }
+  } else if (tid < static_cast<int>(found)) {
+    const int first = group_first[tid], end = link[first];
+    uint32_t* row0 = table + static_cast<size_t>(tid) * 2 * row_words;
     uint32_t* row1 = row0 + row_words;
     uint32_t offset = 0;
-    for (int c0 = 0; c0 < chunks; c0 += 32) {
-      const int c = c0 + lane;
-      uint32_t length = 0, start = 0;
-      if (c < chunks) {
-        const size_t row = static_cast<size_t>(c) * buckets;
-        start = run_begin[row + group.x];
-        length = run_begin[row + group.y] - start;
-      }
-      uint32_t incl = length;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      if (c < chunks) {
-        row0[c] = start;
-        row1[c] = offset + incl - length;
-      }
-      offset += __shfl_sync(0xffffffffu, incl, 31);
+    for (int c = 0; c < chunks; ++c) {
+      const uint32_t* row = run_begin + static_cast<size_t>(c) * buckets + b0;
+      row0[c] = row[first];
+      row1[c] = offset;
+      offset += row[end] - row[first];
     }
-    if (lane == 0) {
-      row0[chunks] = bucket_start[group.x];
-      row0[chunks + 1] = group.x;
-      row0[chunks + 2] = group.y;
-      row1[chunks] = offset;
-    }
+    row0[chunks] = start[first];
+    row0[chunks + 1] = static_cast<uint32_t>(b0 + first);
+    row0[chunks + 2] = static_cast<uint32_t>(b0 + end);
+    row1[chunks] = offset;
   }
 }
 
@@ -721,7 +728,7 @@ group_table_kernel(const uint2* __restrict__ groups, const uint32_t* __restrict_
 constexpr uint32_t kBulkChunkBytes = 32768;  // bytes per bulk copy
 constexpr uint32_t kBulkWaitLimit = 1u << 24;  // polls of the copy barrier
 constexpr int kMaxSegments = 32;  // runs of cells an oversized bucket is cut into
-constexpr int kMaxGroupBuckets = 512;  // buckets in the aligned block a group may not leave
+constexpr int kMaxGroupBuckets = kGroupSpan;  // buckets in the aligned block a group may not leave
 constexpr int kMaxChunks = 256;        // 2^30 particles in chunks of 2^22
 constexpr int kTableRowWords = (kMaxChunks + 3 + 3) / 4 * 4;
 
@@ -1324,9 +1331,7 @@ struct BucketLayout {
   int chunk_log;
   int chunks;
   int64_t entries;  // chunks * buckets runs
-  int scan_blocks;
-  size_t count_off, total_off, start_off, cursor_off, local_off, block_sum_off, run_begin_off,
-      groups_off, tables_off, records_off, total;
+  size_t count_off, start_off, cursor_off, run_begin_off, tables_off, records_off, total;
 };
 
 // Tables and records for `n` particles (or room for that many) in `chunks` chunks.
@@ -1335,17 +1340,12 @@ BucketLayout bucket_layout_of(int64_t n, int64_t buckets, int chunk_log, int chu
   l.chunk_log = chunk_log;
   l.chunks = chunks;
   l.entries = static_cast<int64_t>(l.chunks) * buckets;
-  l.scan_blocks = static_cast<int>((l.entries + kFlatScanBlock - 1) / kFlatScanBlock);
   const size_t words = sizeof(uint32_t);
   l.count_off = sizeof(Header);  // zeroed per call together with the header
-  l.total_off = align_up(l.count_off + l.entries * words, 256);
-  l.start_off = align_up(l.total_off + buckets * words, 256);
+  l.start_off = align_up(l.count_off + l.entries * words, 256);  // zeroed up to here
   l.cursor_off = align_up(l.start_off + (buckets + 1) * words, 256);
-  l.local_off = align_up(l.cursor_off + l.entries * words, 256);
-  l.block_sum_off = align_up(l.local_off + l.entries * words, 256);
-  l.run_begin_off = align_up(l.block_sum_off + l.scan_blocks * words, 256);
-  l.groups_off = align_up(l.run_begin_off + (l.entries + 1) * words, 256);
-  l.tables_off = align_up(l.groups_off + buckets * 2 * words, 256);
+  l.run_begin_off = align_up(l.cursor_off + l.entries * words, 256);
+  l.tables_off = align_up(l.run_begin_off + (l.entries + 1) * words, 256);
   l.records_off = align_up(l.tables_off + buckets * 2 * table_row_words(l.chunks) * words, 256);
   l.total = align_up(l.records_off + static_cast<size_t>(n) * kRecordWords * words, 256);
   return l;
@@ -1424,6 +1424,22 @@ size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells) {
 
 namespace {
 
+cudaError_t launch_groups(cudaStream_t stream, const uint32_t* run_begin, int buckets, int chunks,
+                          int chunk_log, const SliceSegments* segments, int group_shift,
+                          uint32_t capacity, uint32_t* start, uint32_t* tables, Header* hdr) {
+  const size_t staged = chunks <= kGroupStagedChunks
+                            ? 2 * static_cast<size_t>(chunks) * (kGroupSpan + 1) * sizeof(uint32_t) : 0;
+  if (staged > 40 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(staged));
+    if (e != cudaSuccess) return e;
+  }
+  return launch_chained(group_kernel, (buckets + kGroupSpan - 1) / kGroupSpan, kGroupSpan, staged,
+                        stream, run_begin, buckets, chunks, chunk_log, segments, group_shift,
+                        capacity, FinishLarge::kLargestBucket, start, tables,
+                        &hdr->aux_counter[1], hdr);
+}
+
 template <class Shape>
 cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
                           const uint32_t* n_on_device = nullptr) {
@@ -1490,16 +1506,12 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   auto words_at = [&](size_t off) { return reinterpret_cast<uint32_t*>(base + off); };
   Header* hdr = reinterpret_cast<Header*>(base);
   uint32_t* count = words_at(l.count_off);
-  uint32_t* total = words_at(l.total_off);
   uint32_t* start = words_at(l.start_off);
   uint32_t* cursor = words_at(l.cursor_off);
-  uint32_t* local = words_at(l.local_off);
-  uint32_t* block_sum = words_at(l.block_sum_off);
   uint32_t* run_begin = words_at(l.run_begin_off);
-  uint2* groups = reinterpret_cast<uint2*>(base + l.groups_off);
   uint32_t* tables = words_at(l.tables_off);
   uint32_t* records = words_at(l.records_off);
-  cudaError_t e = cudaMemsetAsync(base, 0, l.total_off, a.stream);  // header and run counts
+  cudaError_t e = cudaMemsetAsync(base, 0, l.start_off, a.stream);  // header and run counts
   if (e != cudaSuccess) return e;
   const int buckets = static_cast<int>(p.buckets);
   const uint32_t k0 = static_cast<uint32_t>(a.seed), k1 = static_cast<uint32_t>(a.seed >> 32);
@@ -1551,36 +1563,18 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   if (e != cudaSuccess) return e;
 
   stage_begin(kStageBucketScan, a.stream);
-  const uint32_t largest = FinishLarge::kLargestBucket;
   const int max_cells = p.small_blocks ? FinishSmall::kMaxCells : FinishLarge::kMaxCells;
   const uint32_t group_capacity = bucket_group_capacity(a.n, p);
   const int group_shift = std::min(log2_floor(kMaxGroupBuckets),
                                    std::max(0, log2_floor(max_cells) - p.shift));
-  const int blocks_of_buckets = (buckets + (1 << group_shift) - 1) >> group_shift;
-  e = launch_chained(bucket_total_kernel, (buckets + 255) / 256, 256, 0, a.stream, count, buckets,
-                     l.chunks, total);
+  const dim3 scan_grid((buckets + kRunScanPart - 1) / kRunScanPart, l.chunks);
+  e = launch_chained(run_scan_kernel, scan_grid, kRunScanThreads, 0, a.stream, count, buckets,
+                     l.chunk_log, static_cast<uint32_t>(a.n), cursor, run_begin);
   if (e == cudaSuccess)
-    e = launch_chained(bucket_scan_kernel, 1, kScanThreads, 0, a.stream, total, buckets, a.n,
-                       nullptr, largest, start, nullptr, hdr);
-  if (e == cudaSuccess)
-    e = launch_chained(group_cut_kernel, (blocks_of_buckets + 255) / 256, 256, 0, a.stream, start,
-                       buckets, group_shift, group_capacity, groups, &hdr->aux_counter[1]);
-  if (e == cudaSuccess)
-    e = launch_chained(run_scan_local_kernel, l.scan_blocks, kFlatScanBlock, 0, a.stream, count,
-                       l.entries, local, block_sum);
-  if (e == cudaSuccess)
-    e = launch_chained(run_scan_blocks_kernel, 1, kFlatScanBlock, 0, a.stream, block_sum,
-                       l.scan_blocks);
-  if (e == cudaSuccess)
-    e = launch_chained(run_table_kernel, static_cast<int>((l.entries + 1 + 255) / 256), 256, 0,
-                       a.stream, local, block_sum, l.entries, static_cast<uint32_t>(a.n), cursor,
-                       run_begin);
-  if (e == cudaSuccess)
-    e = launch_chained(group_table_kernel,
-                       std::max(1, std::min((buckets + 7) / 8, sm_count() * 8)), 256, 0, a.stream,
-                       groups, &hdr->aux_counter[1], start, run_begin, l.chunks, buckets, tables);
+    e = launch_groups(a.stream, run_begin, buckets, l.chunks, l.chunk_log, nullptr, group_shift,
+                      group_capacity, start, tables, hdr);
   if (e != cudaSuccess) return e;
-  count_launches(7);
+  count_launches(3);
   stage_end(kStageBucketScan, a.stream);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -1655,7 +1649,7 @@ cudaError_t sliced_sort_begin(const SortArgs& a, int64_t plan_n, int slices) {
   const SlicedState st = sliced_state(a, plan_n, slices);
   if (!st.ok) return cudaErrorInvalidValue;
   stage_reset();
-  return cudaMemsetAsync(st.base, 0, st.layout.total_off, a.stream);  // header and run counts
+  return cudaMemsetAsync(st.base, 0, st.layout.start_off, a.stream);  // header and run counts
 }
 
 cudaError_t sliced_sort_slice(const SortArgs& a, int64_t plan_n, const SliceSegments* segments,
@@ -1746,11 +1740,8 @@ cudaError_t sliced_sort_finish(const SortArgs& a, int64_t plan_n, const SliceSeg
   auto words_at = [&](size_t off) { return reinterpret_cast<uint32_t*>(st.base + off); };
   Header* hdr = reinterpret_cast<Header*>(st.base);
   const int buckets = static_cast<int>(p.buckets);
-  uint32_t* count = words_at(l.count_off);
-  uint32_t* total = words_at(l.total_off);
   uint32_t* start = words_at(l.start_off);
   uint32_t* run_begin = words_at(l.run_begin_off);
-  uint2* groups = reinterpret_cast<uint2*>(st.base + l.groups_off);
   uint32_t* tables = words_at(l.tables_off);
   uint32_t* records = words_at(l.records_off);
   const uint32_t* n_on_device = &segments->n;
@@ -1760,22 +1751,16 @@ cudaError_t sliced_sort_finish(const SortArgs& a, int64_t plan_n, const SliceSeg
   const uint32_t group_capacity = bucket_group_capacity(plan_n, p);
   const int group_shift = std::min(log2_floor(kMaxGroupBuckets),
                                    std::max(0, log2_floor(max_cells) - p.shift));
-  const int blocks_of_buckets = (buckets + (1 << group_shift) - 1) >> group_shift;
-  bucket_total_kernel<<<(buckets + 255) / 256, 256, 0, a.stream>>>(count, buckets, l.chunks, total);
-  bucket_scan_kernel<<<1, kScanThreads, 0, a.stream>>>(total, buckets, a.n, n_on_device,
-                                                       FinishLarge::kLargestBucket, start, nullptr,
-                                                       hdr);
-  group_cut_kernel<<<(blocks_of_buckets + 255) / 256, 256, 0, a.stream>>>(
-      start, buckets, group_shift, group_capacity, groups, &hdr->aux_counter[1]);
-  group_table_kernel<<<std::max(1, std::min((buckets + 7) / 8, sm_count() * 8)), 256, 0, a.stream>>>(
-      groups, &hdr->aux_counter[1], start, run_begin, l.chunks, buckets, tables);
-  count_launches(6);
+  cudaError_t e = launch_groups(a.stream, run_begin, buckets, l.chunks, 0, segments, group_shift,
+                                group_capacity, start, tables, hdr);
+  if (e != cudaSuccess) return e;
+  count_launches(3);
   const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
                       a.vs, a.padded_sorted};
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
                    table_row_words(l.chunks), l.chunks, buckets, p.shift};
-  cudaError_t e = p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, n_on_device)
-                                 : launch_finish<FinishLarge>(t, a, out, hdr, n_on_device);
+  e = p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, n_on_device)
+                     : launch_finish<FinishLarge>(t, a, out, hdr, n_on_device);
   if (e == cudaSuccess) e = launch_finish_large(t, a, out, hdr, group_capacity);
   stage_end(kStageBucketFinish, a.stream);
   return e;
