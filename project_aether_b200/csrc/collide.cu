@@ -101,11 +101,11 @@ __device__ __forceinline__ bool collide_pair(float* a, float* b, float majorant,
 }
 
 // Bound by the latency of a block's chain (starts, draw, scan, pairs, results) and by the sectors
-// that hold candidate pairs; so little shared memory, and five blocks of 256 threads (48
+// that hold candidate pairs; so little shared memory, and six blocks of 256 threads (40
 // registers) per multiprocessor.  A first design staged every particle of the block's cells in
 // shared memory, four blocks per multiprocessor, and wrote the stage back: 16 M particles in 2 M
-// cells took it 123 us, this kernel 63 (436 MB if every velocity is read and written once).
-__global__ void __launch_bounds__(kCollideThreads, 5)
+// cells took it 123 us, this kernel 61 (436 MB if every velocity is read and written once).
+__global__ void __launch_bounds__(kCollideThreads, 6)
 collide_kernel(CollideArgs a) {
   __shared__ int start[kCollideThreads];
   __shared__ int pair_first[kCollideThreads];      // exclusive prefix of the candidate pairs
