@@ -342,8 +342,8 @@ int AetherDsmcCollideTma(float* velocity, const int* cell_start, float* sigma_g_
  *     work overlaps on the GPU (different streams, no dependency) race on it:
  *     serialise them.
  *   - Which of the two sort paths runs follows from the size: calls whose
- *     bucketed record layout fits the array (up to a few hundred thousand
- *     particles) take the bucketed path, larger ones the digit passes.
+ *     bucketed layout (8 bytes per particle and 48 per bucket) fits the array
+ *     take the bucketed path, nearly all of them; the others the digit passes.
  *   - The device status of a call (a bounded wait that gave up) lives in that
  *     array too: read it with AetherSortStaticReadStatus, and the path that
  *     produced the result with AetherSortStaticReadUsedDigitPasses; both

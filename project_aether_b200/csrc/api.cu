@@ -44,8 +44,9 @@ int run_sort(SortArgs& a, int path) {
   // (with or without payload outputs) and the workspace is large enough for its records.  A
   // caller with a smaller workspace (the static-scratch entry point above a few hundred
   // thousand particles, or a workspace sized for the digit passes only) gets the digit passes.
-  const BucketPlan plan = plan_buckets(a.n, a.num_cells);
-  const bool roomy = a.workspace_bytes >= bucketed_workspace_bytes(a.n, a.num_cells);
+  const bool keys_only = a.xs == nullptr;
+  const BucketPlan plan = plan_buckets(a.n, a.num_cells, keys_only);
+  const bool roomy = a.workspace_bytes >= bucketed_workspace_bytes(a.n, a.num_cells, keys_only);
   const bool bucketed = plan.usable && path != 1 && (roomy || path == 2);
   if (path == 2 && (!plan.usable || !roomy)) return cudaErrorInvalidValue;
   return bucketed ? bucketed_sort(a, plan) : standard_sort(a);
@@ -207,13 +208,14 @@ extern "C" size_t AetherSortWorkspaceBytes(int64_t n, int64_t num_cells, int wit
   // The digit passes gather the payload through 32-byte records when there is room for them.
   const size_t standard = with_payload ? standard_workspace_bytes_with_records(n, num_cells)
                                        : standard_workspace_bytes(n, num_cells);
-  return std::max(standard, bucketed_workspace_bytes(n, num_cells));
+  return std::max({standard, bucketed_workspace_bytes(n, num_cells, false),
+                   bucketed_workspace_bytes(n, num_cells, true)});
 }
 
 extern "C" int AetherSortBucketPlan(int64_t n, int64_t num_cells, int32_t* cells_per_bucket_log2,
                                     int64_t* buckets, int32_t* group_capacity) {
   if (!count_ok(n) || num_cells <= 0 || key_bits_of(num_cells) > 32) return cudaErrorInvalidValue;
-  const BucketPlan plan = plan_buckets(n, num_cells);
+  const BucketPlan plan = plan_buckets(n, num_cells, false);
   if (cells_per_bucket_log2) *cells_per_bucket_log2 = plan.shift;
   if (buckets) *buckets = plan.buckets;
   if (group_capacity) *group_capacity = static_cast<int32_t>(bucket_group_capacity(n, plan));

@@ -299,13 +299,14 @@ struct BucketPlan {
   int64_t buckets;
   bool usable;        // false when even single-cell buckets would be too full on average
   bool small_blocks;  // finish kernel shape: two small blocks per multiprocessor, or one large
+  bool keys_only;     // no payload: 8-byte records and a shape of their own
 };
-BucketPlan plan_buckets(int64_t n, int64_t num_cells);
+BucketPlan plan_buckets(int64_t n, int64_t num_cells, bool keys_only);
 // Most buckets for which the small finish shape is planned (at most 32,768; 0: never).
 void set_small_shape_buckets(int64_t buckets);
 // Most records of a group of buckets (what one block of the finish kernel sorts at a time).
 uint32_t bucket_group_capacity(int64_t n, const BucketPlan& p);
-size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells);
+size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells, bool keys_only);
 cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p);
 
 // The bucketed sort of a segmented input, slice by slice (the local sort of the sliced
