@@ -54,6 +54,7 @@ constexpr int kKeyRecordWords = 2;  // 8-byte record {key, index} of calls witho
 // ------------------------------------------------------------------------
 constexpr int kCountThreads = 512;       // blocks that share an SM (table up to 96 KB)
 constexpr int kCountThreadsWide = 1024;  // one block per SM (table up to 200 KB)
+constexpr int kCountRounds = 1;          // fewest rounds of four particles per thread for a block
 
 #ifndef AETHER_TUNE_CHUNK_LOG
 #define AETHER_TUNE_CHUNK_LOG 22
@@ -61,19 +62,32 @@ constexpr int kCountThreadsWide = 1024;  // one block per SM (table up to 200 KB
 constexpr int kChunkLog = AETHER_TUNE_CHUNK_LOG;  // particles per chunk of the record layout at 64 M
                                                   // particles; see chunk_log_for
 
-// Where a block keeps its counts while it works through a slice.
+// Where a block keeps its counts while it works through its particles.
 enum CountTable {
   kTableGlobal = 0,    // no table: adds go straight to the chunk's row of counts
   kTableShared32 = 1,  // 32-bit counters in shared memory (up to 200 KB: 51,200 buckets)
-  kTableShared16 = 2,  // 16-bit counters, two per word (up to 102,400 buckets); a slice holds
-                       // fewer than 65,536 particles, so no counter can carry into its neighbour
+  kTableShared16 = 2,  // 16-bit counters, two per word (up to 102,400 buckets)
 };
-constexpr int kSlice16 = 61440;  // particles per slice with 16-bit counters (15 rounds of 4096)
+// A 16-bit counter that reaches 2^15 is emptied into the row of counts by the lane whose add took
+// it there.  Until that lane has subtracted, the others may add at most what a block counts
+// between two barriers (kRoundsPerBarrier rounds of 4096 particles, 2^14), so no counter carries
+// into its neighbour however many particles the block counts.
+constexpr uint32_t kEmptyAt = 1u << 15;
+constexpr int kRoundsPerBarrier = 4;
+static_assert(kCountThreadsWide * 4 * kRoundsPerBarrier <= (1 << 15) - 32, "16-bit counters");
 
 template <int TABLE>
-__device__ __forceinline__ void table_add(uint32_t* table, uint32_t bin, uint32_t count) {
-  if (TABLE == kTableShared16) atomicAdd(&table[bin >> 1], count << (16 * (bin & 1)));
-  else atomicAdd(&table[bin], count);
+__device__ __forceinline__ void table_add(uint32_t* table, uint32_t* row, uint32_t bin, uint32_t count) {
+  if (TABLE == kTableShared16) {
+    const int sh = 16 * (bin & 1);
+    const uint32_t before = (atomicAdd(&table[bin >> 1], count << sh) >> sh) & 0xffffu;
+    if (before < kEmptyAt && before + count >= kEmptyAt) {
+      atomicSub(&table[bin >> 1], kEmptyAt << sh);
+      atomicAdd(&row[bin], kEmptyAt);
+    }
+  } else {
+    atomicAdd(&table[bin], count);
+  }
 }
 
 // One count per lane into `table`; lanes that hit the same bin share one add when the whole
@@ -81,57 +95,59 @@ __device__ __forceinline__ void table_add(uint32_t* table, uint32_t bin, uint32_
 // Returns whether lanes shared an add (the same for all lanes): on input in random order
 // they never do, and the caller then skips the votes for the rest of its round.
 template <int TABLE>
-__device__ __forceinline__ bool count_add(uint32_t* table, uint32_t bin, bool valid) {
+__device__ __forceinline__ bool count_add(uint32_t* table, uint32_t* row, uint32_t bin, bool valid) {
   const uint32_t active = __ballot_sync(0xffffffffu, valid);
   if (active == 0) return true;
   const int first = __ffs(active) - 1;
   const uint32_t first_bin = __shfl_sync(0xffffffffu, bin, first);
   const bool uniform = __all_sync(0xffffffffu, !valid || bin == first_bin);
   if (uniform) {
-    if (static_cast<int>(lane_id()) == first) table_add<TABLE>(table, first_bin, __popc(active));
+    if (static_cast<int>(lane_id()) == first) table_add<TABLE>(table, row, first_bin, __popc(active));
     return true;
   }
   const uint32_t next_bin = __shfl_down_sync(0xffffffffu, bin, 1);
   const bool clustered = __any_sync(0xffffffffu, valid && lane_id() < 31 && next_bin == bin);
   if (clustered) {
     const uint32_t peers = __match_any_sync(0xffffffffu, valid ? bin : 0xffffffffu) & active;
-    if (valid && (peers & lanemask_lt()) == 0) table_add<TABLE>(table, bin, __popc(peers));
+    if (valid && (peers & lanemask_lt()) == 0) table_add<TABLE>(table, row, bin, __popc(peers));
   } else if (valid) {
-    table_add<TABLE>(table, bin, 1u);
+    table_add<TABLE>(table, row, bin, 1u);
   }
   return clustered;
 }
 
-// Work unit = one slice of one chunk; a block counts the slice into its table and adds the
-// table to the chunk's row of counts, count[chunk * buckets + b].
+// A block counts `per_block` consecutive particles into its table, and adds the table to the
+// chunk's row of counts, count[chunk * buckets + b], at the end and wherever its particles pass
+// into the next chunk.  One share per block keeps those adds few: with two slices of a chunk per
+// block they were more than half as many as the particles at 16 M (16,384 buckets) and more than
+// the particles at 256 M (65,536 buckets, whose 16-bit counters also kept the slices below 2^16).
 template <int TABLE, bool VEC, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, THREADS == kCountThreads ? 3 : 1)
 bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
-                    PushSpec push, int64_t n, AetherGrid g, int shift,
-                    int buckets, int chunks, int chunk_log, int parts, int64_t slice,
-                    uint32_t* __restrict__ bucket_count) {
+                    PushSpec push, int64_t n, AetherGrid g, int shift, int buckets, int chunk_log,
+                    int64_t per_block, uint32_t* __restrict__ bucket_count) {
   chain_begin();
   extern __shared__ uint32_t hist[];
-  const int table_words = TABLE == kTableShared16 ? (buckets + 1) / 2 : buckets;
-  for (int unit = blockIdx.x; unit < chunks * parts; unit += gridDim.x) {
-    const int chunk = unit / parts, part = unit % parts;
+  const int table_words = TABLE == kTableGlobal ? 0
+                          : TABLE == kTableShared16 ? (buckets + 1) / 2 : buckets;
+  for (int i = threadIdx.x; i < table_words; i += THREADS) hist[i] = 0;
+  __syncthreads();
+  // Particle numbers fit 30 bits: index arithmetic in 32.
+  int first = static_cast<int>(blockIdx.x * per_block);
+  const int block_last = static_cast<int>(min(static_cast<long long>(n), static_cast<long long>(first) + per_block));
+  while (first < block_last) {
+    const int chunk = first >> chunk_log;
+    const int last = static_cast<int>(min(static_cast<long long>(block_last),
+                                          static_cast<long long>(chunk + 1) << chunk_log));
     uint32_t* row = bucket_count + static_cast<size_t>(chunk) * buckets;
-    if (TABLE != kTableGlobal) {
-      for (int i = threadIdx.x; i < table_words; i += THREADS) hist[i] = 0;
-      __syncthreads();
-    }
     uint32_t* target = TABLE != kTableGlobal ? hist : row;
-    const int64_t chunk_first = static_cast<int64_t>(chunk) << chunk_log;
-    const int64_t chunk_last = min(static_cast<long long>(n),
-                                   static_cast<long long>(chunk_first + (int64_t{1} << chunk_log)));
-    const int64_t first = chunk_first + part * slice;
-    const int64_t last = min(static_cast<long long>(chunk_last), static_cast<long long>(first + slice));
-    const int64_t rounds = first < last ? (last - first + THREADS * 4 - 1) / (THREADS * 4) : 0;
-    for (int64_t r = 0; r < rounds; ++r) {
-      const int64_t i0 = first + (r * THREADS + threadIdx.x) * 4;
+    const int rounds = (last - first + THREADS * 4 - 1) / (THREADS * 4);
+    for (int r = 0; r < rounds; ++r) {
+      const bool whole = VEC && last - first - r * THREADS * 4 >= THREADS * 4;  // no particle missing
+      const int i0 = first + (r * THREADS + static_cast<int>(threadIdx.x)) * 4;
       float px[4], py[4], pz[4];
-      if (VEC && i0 + 4 <= last) {
+      if (whole) {
         const float4 a = ldcs4(x + i0), b = ldcs4(y + i0), c = ldcs4(z + i0);
         px[0] = a.x; px[1] = a.y; px[2] = a.z; px[3] = a.w;
         py[0] = b.x; py[1] = b.y; py[2] = b.z; py[3] = b.w;
@@ -147,7 +163,7 @@ bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
       }
       if (push.enabled) {  // count the particles where the fused move stage puts them
         float w[3][4];
-        if (VEC && i0 + 4 <= last) {
+        if (whole) {
           const float4 a = ldcs4(v + i0), b = ldcs4(v + padded + i0), c = ldcs4(v + 2 * padded + i0);
           w[0][0] = a.x; w[0][1] = a.y; w[0][2] = a.z; w[0][3] = a.w;
           w[1][0] = b.x; w[1][1] = b.y; w[1][2] = b.z; w[1][3] = b.w;
@@ -172,23 +188,29 @@ bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const uint32_t bin = cell_of(px[k], py[k], pz[k], g) >> shift;
-        if (sharing) sharing = count_add<TABLE>(target, bin, i0 + k < last);
-        else if (i0 + k < last) table_add<TABLE>(target, bin, 1u);
+        const bool valid = whole || i0 + k < last;
+        if (sharing) sharing = count_add<TABLE>(target, row, bin, valid);
+        else if (valid) table_add<TABLE>(target, row, bin, 1u);
       }
+      if (TABLE == kTableShared16 && (r + 1) % kRoundsPerBarrier == 0) __syncthreads();
     }
     if (TABLE != kTableGlobal) {
       __syncthreads();
       for (int i = threadIdx.x; i < table_words; i += THREADS) {
         const uint32_t w = hist[i];
-        if (TABLE == kTableShared16) {
-          if (w & 0xffffu) atomicAdd(&row[2 * i], w & 0xffffu);
-          if (w >> 16) atomicAdd(&row[2 * i + 1], w >> 16);
-        } else if (w) {
-          atomicAdd(&row[i], w);
+        if (w) {
+          if (TABLE == kTableShared16) {
+            if (w & 0xffffu) atomicAdd(&row[2 * i], w & 0xffffu);
+            if (w >> 16) atomicAdd(&row[2 * i + 1], w >> 16);
+          } else {
+            atomicAdd(&row[i], w);
+          }
+          hist[i] = 0;
         }
       }
       __syncthreads();
     }
+    first = last;
   }
 }
 
@@ -585,7 +607,7 @@ bucket_count_segments_kernel(const float* __restrict__ x, const float* __restric
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        count_add<TABLE>(target, cell_of(px[j], py[j], pz[j], g) >> shift,
+        count_add<TABLE>(target, row, cell_of(px[j], py[j], pz[j], g) >> shift,
                          i0 + j >= lo && i0 + j < last);
     }
   }
@@ -1755,18 +1777,13 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     const size_t table_bytes = table == kTableShared32 ? bytes32 : table == kTableShared16 ? bytes16 : 0;
     const bool wide = table_bytes > 96 * 1024;  // one 1024-thread block per SM holds the table
     const int threads = wide ? kCountThreadsWide : kCountThreads;
-    const int blocks_per_sm = table == kTableGlobal ? 4 : wide ? 1 : table_bytes <= 48 * 1024 ? 4 : 2;
-    const int64_t chunk_size = int64_t{1} << l.chunk_log;
-    const int64_t covered = std::min<int64_t>(a.n, chunk_size);
-    // Slices of a chunk: enough units to fill the GPU twice over, each a multiple of one
-    // block round (4 particles per thread) so that the 16-byte loads stay aligned.
-    const int want = std::max(1, sm_count() * blocks_per_sm * 2 / l.chunks);
+    const int blocks_per_sm = table == kTableGlobal ? 3 : wide ? 1 : table_bytes <= 64 * 1024 ? 3 : 2;
+    // Equal shares, each a multiple of one block round (4 particles per thread) so that the
+    // 16-byte loads stay aligned.
     const int64_t round = threads * 4;
-    int64_t slice = std::max<int64_t>(round, ((covered + want - 1) / want + round - 1) / round * round);
-    if (table == kTableShared16) slice = std::min<int64_t>(slice, kSlice16 / round * round);
-    const int parts = static_cast<int>((covered + slice - 1) / slice);
-    const int grid = static_cast<int>(std::max<int64_t>(
-        1, std::min<int64_t>(static_cast<int64_t>(l.chunks) * parts, sm_count() * blocks_per_sm)));
+    const int64_t most = static_cast<int64_t>(sm_count()) * blocks_per_sm;
+    const int64_t per_block = std::max<int64_t>(kCountRounds, ((a.n + most - 1) / most + round - 1) / round) * round;
+    const int grid = static_cast<int>((a.n + per_block - 1) / per_block);
 #define AETHER_COUNT_LAUNCH(TABLE, THREADS)                                                      \
   do {                                                                                            \
     auto kernel = vec ? bucket_count_kernel<TABLE, true, THREADS>                                 \
@@ -1777,8 +1794,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
       if (e != cudaSuccess) return e;                                                             \
     }                                                                                             \
     kernel<<<grid, THREADS, table_bytes, a.stream>>>(a.x, a.y, a.z, a.velocity, a.padded, a.push, \
-                                                     a.n, a.grid, p.shift, buckets, l.chunks,     \
-                                                     l.chunk_log, parts, slice, count);           \
+                                                     a.n, a.grid, p.shift, buckets,               \
+                                                     l.chunk_log, per_block, count);              \
   } while (0)
     if (table == kTableGlobal) AETHER_COUNT_LAUNCH(kTableGlobal, kCountThreads);
     else if (table == kTableShared16) AETHER_COUNT_LAUNCH(kTableShared16, kCountThreadsWide);
