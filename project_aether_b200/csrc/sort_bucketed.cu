@@ -409,6 +409,104 @@ bucket_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
   }
 }
 
+// Lanes of a warp that do not agree on a bucket skip the votes for the rest of a tile.
+__device__ __forceinline__ uint32_t rank_in_tile(uint32_t* table, uint32_t b, bool valid, bool& sharing) {
+  if (!sharing) return valid ? atomicAdd(&table[b], 1u) : 0u;
+  const uint32_t next_b = __shfl_down_sync(0xffffffffu, b, 1);
+  sharing = __any_sync(0xffffffffu, valid && lane_id() < 31 && next_b == b);
+  return reserve_slot(table, b, valid);
+}
+
+// ------------------------------------------------------------------------
+// Scatter of small inputs: slots reserved tile by tile.
+// ------------------------------------------------------------------------
+// With a thousand buckets or so the slot counters fill few L2 lines, and one returning add per
+// particle queues on them (1 M particles on 2048 counters: 47 us, of which the stores would need
+// 16).  Here a block ranks a tile's particles with adds in shared memory and reserves each
+// bucket's slots with one add per tile, consecutive threads on consecutive counters.  It pays
+// while a tile has about as many particles as there are buckets.
+template <bool VEC, int ITEMS>
+__global__ void __launch_bounds__(kScatterThreads, ITEMS <= 4 ? 2 : 1)
+tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
+                    const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
+                    PushSpec push, int64_t n, AetherGrid g, uint32_t k0, uint32_t k1, int shift,
+                    int buckets, int chunk_log, uint32_t* __restrict__ cursor,
+                    uint32_t* __restrict__ records, const Header* __restrict__ hdr) {
+  constexpr int kTile = kScatterThreads * ITEMS;
+  chain_begin();
+  if (hdr->use_standard) return;
+  extern __shared__ uint32_t slot_of[];  // a tile's counts, then its first slots
+  const int tid = threadIdx.x;
+  const int64_t tiles = (n + kTile - 1) / kTile;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t first = tile * kTile;
+    uint32_t* row = cursor + static_cast<size_t>(first >> chunk_log) * buckets;
+    for (int b = tid; b < buckets; b += kScatterThreads) slot_of[b] = 0;
+    __syncthreads();
+    float f[6][ITEMS];
+    uint32_t key[ITEMS], rank[ITEMS];
+    bool sharing = true;
+#pragma unroll
+    for (int q = 0; q < ITEMS; q += 4) {
+      const int64_t i0 = first + (q / 4 * kScatterThreads + tid) * 4;
+      if (VEC && i0 + 4 <= n) {
+        load_items<4>(x + i0, f[0] + q);
+        load_items<4>(y + i0, f[1] + q);
+        load_items<4>(z + i0, f[2] + q);
+        if (v) {
+          load_items<4>(v + i0, f[3] + q);
+          load_items<4>(v + padded + i0, f[4] + q);
+          load_items<4>(v + 2 * padded + i0, f[5] + q);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const bool ok = i0 + k < n;
+          f[0][q + k] = ok ? x[i0 + k] : 0.f;
+          f[1][q + k] = ok ? y[i0 + k] : 0.f;
+          f[2][q + k] = ok ? z[i0 + k] : 0.f;
+          f[3][q + k] = ok && v ? v[i0 + k] : 0.f;
+          f[4][q + k] = ok && v ? v[padded + i0 + k] : 0.f;
+          f[5][q + k] = ok && v ? v[2 * padded + i0 + k] : 0.f;
+        }
+      }
+      if (!v) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) f[3][q + k] = f[4][q + k] = f[5][q + k] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const int64_t i = first + (k / 4 * kScatterThreads + tid) * 4 + k % 4;
+      if (push.enabled) {  // the fused move stage: the record carries the moved particle
+        push_axis(f[0][k], f[3][k], push.dt, push.lo[0], push.hi[0]);
+        push_axis(f[1][k], f[4][k], push.dt, push.lo[1], push.hi[1]);
+        push_axis(f[2][k], f[5][k], push.dt, push.lo[2], push.hi[2]);
+      }
+      const uint32_t cell = cell_of(f[0][k], f[1][k], f[2][k], g);
+      key[k] = make_key(cell, static_cast<uint32_t>(i), k0, k1);
+      rank[k] = rank_in_tile(slot_of, cell >> shift, i < n, sharing);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int b = tid; b < buckets; b += kScatterThreads) {
+      const uint32_t c = slot_of[b];
+      if (c) slot_of[b] = atomicAdd(&row[b], c);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const int64_t i = first + (k / 4 * kScatterThreads + tid) * 4 + k % 4;
+      if (i < n)
+        store_record(records + static_cast<size_t>(slot_of[key[k] >> (kShuffleBits + shift)] + rank[k]) *
+                                   kRecordWords,
+                     key[k], static_cast<uint32_t>(i), f[0][k], f[1][k], f[2][k], f[3][k], f[4][k],
+                     f[5][k]);
+    }
+    __syncthreads();  // the table is reused by the next tile
+  }
+}
+
 // ------------------------------------------------------------------------
 // Calls without payload: 8-byte records, split tile by tile.
 // ------------------------------------------------------------------------
@@ -425,14 +523,6 @@ constexpr int kSplitMaxBuckets = 16384;  // 128 KB of tables beside the stage
 
 __host__ __device__ inline size_t split_smem_bytes(int tile, int buckets) {
   return static_cast<size_t>(tile) * 8 + 2 * (static_cast<size_t>(buckets + 3) / 4 * 4) * sizeof(uint32_t);
-}
-
-// Lanes of a warp that do not agree on a bucket skip the votes for the rest of a tile.
-__device__ __forceinline__ uint32_t rank_in_tile(uint32_t* table, uint32_t b, bool valid, bool& sharing) {
-  if (!sharing) return valid ? atomicAdd(&table[b], 1u) : 0u;
-  const uint32_t next_b = __shfl_down_sync(0xffffffffu, b, 1);
-  sharing = __any_sync(0xffffffffu, valid && lane_id() < 31 && next_b == b);
-  return reserve_slot(table, b, valid);
 }
 
 template <bool VEC, int ITEMS, int THREADS>
@@ -1568,8 +1658,8 @@ BucketLayout bucket_layout_of(int64_t n, int64_t buckets, int chunk_log, int chu
 BucketLayout bucket_layout(int64_t n, const BucketPlan& p) {
   const int64_t buckets = p.buckets;
   // Tiles split in shared memory write whole runs: no window has to be kept small for them.
-  const int chunk_log = p.keys_only && buckets <= kSplitMaxBuckets ? kKeyChunkLog
-                                                                   : chunk_log_for(buckets, n);
+  const int chunk_log = p.tiled || (p.keys_only && buckets <= kSplitMaxBuckets)
+                            ? kKeyChunkLog : chunk_log_for(buckets, n);
   const int chunks = static_cast<int>(
       std::max<int64_t>(1, (n + (int64_t{1} << chunk_log) - 1) >> chunk_log));
   return bucket_layout_of(n, buckets, chunk_log, chunks,
@@ -1581,6 +1671,10 @@ BucketLayout bucket_layout(int64_t n, const BucketPlan& p) {
 // (measured at 64 M particles: 65,536 buckets of 1,024 against 16,384 of 4,096).
 constexpr int64_t kMaxSmallShapeBuckets = 32 * 1024;
 int64_t g_small_shape_buckets = kMaxSmallShapeBuckets;  // tuning knob, see set_small_shape_buckets
+
+// Up to where slots are reserved tile by tile.
+constexpr int64_t kTiledMostParticles = 6 << 20;
+constexpr int64_t kTiledMostBuckets = 8192;
 
 // Largest bucket width 2^s, s <= max_shift, whose average load stays at or below `target`,
 // with at least 2048 buckets (fewer make the slot counters of the scatter contend: measured
@@ -1602,17 +1696,33 @@ int log2_floor(int v) {
 }  // namespace
 
 namespace {
-int64_t group_capacity_for(int64_t n, int capacity) {
-  return std::min<int64_t>(capacity, std::max<int64_t>(1024, n / (4 * static_cast<int64_t>(sm_count()))));
+// Records a group may hold: a finish block's capacity, or less where the groups would then not
+// fill the rounds the blocks make (up to four; beyond, the last round matters little).  A quarter
+// above an even share, so that whole buckets fit.
+int64_t group_capacity_for(int64_t n, int capacity, int blocks_per_sm) {
+  const int64_t blocks = static_cast<int64_t>(sm_count()) * blocks_per_sm;
+  const int64_t rounds = std::max<int64_t>(1, (n + blocks * capacity - 1) / (blocks * capacity));
+  if (rounds > 4) return capacity;
+  return std::min<int64_t>(capacity, std::max<int64_t>(256, n / (blocks * rounds) * 5 / 4));
 }
 
-BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small) {
+// `tiled`: the call may use tile_scatter_kernel, to which few buckets are no burden.
+BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small, bool tiled) {
   BucketPlan p;
-  p.keys_only = false;
+  p.keys_only = p.tiled = false;
   // The small finish shape (two blocks per multiprocessor) wants buckets well below its
   // capacity, so that the groups cut from them fill a block whatever the density does
   // inside a row of cells.
   p.small_blocks = true;
+  if (tiled && allow_small && n <= kTiledMostParticles) {
+    const int64_t target = std::min<int64_t>(1100, group_capacity_for(n, FinishSmall::kCapacity, 2) / 2);
+    p.shift = shift_for(n, num_cells, target, log2_floor(FinishSmall::kMaxCells), 1);
+    p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
+    p.tiled = p.buckets <= kTiledMostBuckets;
+    p.usable = p.tiled && n > 0 && n <= 1100 * p.buckets && p.buckets <= g_small_shape_buckets;
+    if (p.usable) return p;
+    p.tiled = false;
+  }
   p.shift = shift_for(n, num_cells, 1100, log2_floor(FinishSmall::kMaxCells));
   p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
   p.usable = allow_small && n > 0 && n <= 1100 * p.buckets && p.buckets <= g_small_shape_buckets;
@@ -1626,13 +1736,14 @@ BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small) {
 }  // namespace
 
 BucketPlan plan_buckets(int64_t n, int64_t num_cells, bool keys_only) {
-  if (!keys_only) return plan_buckets_shape(n, num_cells, true);
+  if (!keys_only) return plan_buckets_shape(n, num_cells, true, true);
   // Groups of a call without payload: a finish block's capacity, or less on small inputs so that
   // every block gets some; buckets of at most four fifths of that.
   BucketPlan p;
   p.keys_only = true;
+  p.tiled = false;
   p.small_blocks = false;
-  const int64_t capacity = group_capacity_for(n, FinishKeys::kCapacity);
+  const int64_t capacity = group_capacity_for(n, FinishKeys::kCapacity, 2);
   p.shift = shift_for(n, num_cells, capacity * 4 / 5 + 64, log2_floor(FinishKeys::kMaxCells), 1);
   p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
   p.usable = n > 0 && n <= 4160 * p.buckets && p.buckets <= (int64_t{1} << 24);
@@ -1647,7 +1758,8 @@ uint32_t bucket_group_capacity(int64_t n, const BucketPlan& p) {
   // A block's capacity, or less on small inputs so that every multiprocessor gets several groups.
   return static_cast<uint32_t>(group_capacity_for(
       n, p.keys_only ? FinishKeys::kCapacity : p.small_blocks ? FinishSmall::kCapacity
-                                                              : FinishLarge::kCapacity));
+                                                              : FinishLarge::kCapacity,
+      p.keys_only || p.small_blocks ? 2 : 1));
 }
 
 size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells, bool keys_only) {
@@ -1726,6 +1838,19 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
   config.numAttrs = 1;
   return cudaLaunchKernelEx(&config, bucket_tail_kernel<Shape>, t, a.num_cells, out, hdr,
                             group_capacity, digits);
+}
+
+template <int ITEMS>
+cudaError_t launch_tile_scatter(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, int shift,
+                                int buckets, int chunk_log, uint32_t* cursor, uint32_t* records,
+                                Header* hdr) {
+  constexpr int kTile = kScatterThreads * ITEMS;
+  auto kernel = vec ? tile_scatter_kernel<true, ITEMS> : tile_scatter_kernel<false, ITEMS>;
+  const int64_t blocks = std::min<int64_t>((a.n + kTile - 1) / kTile, 2 * sm_count());
+  return launch_chained<true>(kernel, static_cast<int>(blocks), kScatterThreads,
+                              static_cast<size_t>(buckets) * sizeof(uint32_t), a.stream, a.x, a.y,
+                              a.z, a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, shift, buckets,
+                              chunk_log, cursor, records, hdr);
 }
 
 template <int ITEMS, int THREADS>
@@ -1840,6 +1965,11 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                                                               : launch_split<4, kSplitThreads>;
     e = launch(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr);
     if (e != cudaSuccess) return e;
+  } else if (p.tiled) {
+    e = a.n >= static_cast<int64_t>(sm_count()) * kScatterThreads * 16
+            ? launch_tile_scatter<8>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr)
+            : launch_tile_scatter<4>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr);
+    if (e != cudaSuccess) return e;
   } else {
     constexpr int kItems = 2;
     const int64_t groups = (a.n + kItems - 1) / kItems;
@@ -1883,7 +2013,7 @@ namespace {
 BucketPlan sliced_plan(int64_t plan_n, int64_t num_cells, int slices) {
   const bool tables_fit =
       3 * 2 * static_cast<size_t>(table_row_words(slices)) * sizeof(uint32_t) <= kSmallShapeTableBytes;
-  return plan_buckets_shape(plan_n, num_cells, tables_fit);
+  return plan_buckets_shape(plan_n, num_cells, tables_fit, false);
 }
 }  // namespace
 
