@@ -1703,7 +1703,7 @@ int64_t group_capacity_for(int64_t n, int capacity, int blocks_per_sm) {
   const int64_t blocks = static_cast<int64_t>(sm_count()) * blocks_per_sm;
   const int64_t rounds = std::max<int64_t>(1, (n + blocks * capacity - 1) / (blocks * capacity));
   if (rounds > 4) return capacity;
-  return std::min<int64_t>(capacity, std::max<int64_t>(256, n / (blocks * rounds) * 5 / 4));
+  return std::min<int64_t>(capacity, std::max<int64_t>(1024, n / (blocks * rounds) * 5 / 4));
 }
 
 // `tiled`: the call may use tile_scatter_kernel, to which few buckets are no burden.
@@ -1716,7 +1716,7 @@ BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small, bo
   p.small_blocks = true;
   if (tiled && allow_small && n <= kTiledMostParticles) {
     const int64_t target = std::min<int64_t>(1100, group_capacity_for(n, FinishSmall::kCapacity, 2) / 2);
-    p.shift = shift_for(n, num_cells, target, log2_floor(FinishSmall::kMaxCells), 1);
+    p.shift = shift_for(n, num_cells, target, log2_floor(FinishSmall::kMaxCells));
     p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
     p.tiled = p.buckets <= kTiledMostBuckets;
     p.usable = p.tiled && n > 0 && n <= 1100 * p.buckets && p.buckets <= g_small_shape_buckets;
@@ -1945,7 +1945,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     e = launch_groups(a.stream, run_begin, buckets, l.chunks, l.chunk_log, nullptr, group_shift,
                       group_capacity, start, tables, hdr);
   if (e != cudaSuccess) return e;
-  count_launches(3);
+  count_launches(2);
   stage_end(kStageBucketScan, a.stream);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
