@@ -299,6 +299,7 @@ struct BucketPlan {
   int64_t buckets;
   bool usable;        // false when even single-cell buckets would be too full on average
   bool small_blocks;  // finish kernel shape: two small blocks per multiprocessor, or one large
+  bool one_launch;    // small call: one cooperative launch
   bool tiled;         // scatter: slots reserved tile by tile
   bool keys_only;     // no payload: 8-byte records and a shape of their own
 };

@@ -1329,7 +1329,7 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
     const size_t entry = static_cast<size_t>(c) * t.buckets + b;
     const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
     for (uint32_t i = tid; i < length; i += kThreads) {
-      const uint32_t key = __ldg(t.records + static_cast<size_t>(start + i) * Shape::kRecordWords);
+      const uint32_t key = __ldcg(t.records + static_cast<size_t>(start + i) * Shape::kRecordWords);
       atomicAdd(&cell_count[(key >> kShuffleBits) - static_cast<uint32_t>(first_cell)], 1u);
     }
   }
@@ -1381,7 +1381,7 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
       const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
       for (uint32_t i = tid; i < length; i += kThreads) {
         const uint32_t* rec = t.records + static_cast<size_t>(start + i) * Shape::kRecordWords;
-        const uint2 lo = __ldg(reinterpret_cast<const uint2*>(rec));
+        const uint2 lo = __ldcg(reinterpret_cast<const uint2*>(rec));
         const int cell = static_cast<int>((lo.x >> kShuffleBits) - static_cast<uint32_t>(first_cell));
         if (cell >= c0 && cell < c1) {
           const uint32_t slot = atomicAdd(&s.fill, 1u);
@@ -1390,7 +1390,7 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
             to[0] = lo;
 #pragma unroll
             for (int k = 1; k < Shape::kRecordWords / 2; ++k)
-              to[k] = __ldg(reinterpret_cast<const uint2*>(rec) + k);
+              to[k] = __ldcg(reinterpret_cast<const uint2*>(rec) + k);
           }
         }
       }
@@ -1609,6 +1609,175 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
   digit_passes_in_grid<Shape::kThreads>(
       digits, *reinterpret_cast<PassSmem<Shape::kThreads>*>(smem_raw), hdr, 1);
 }
+// ------------------------------------------------------------------------
+// Small calls: the whole sort in one cooperative launch.
+// ------------------------------------------------------------------------
+// Up to here a call's time is the host's enqueueing of kernels and the latency of each; the work
+// itself is a few microseconds.  A block takes one tile of at most kSmallItems particles per
+// thread and keeps it in registers: it ranks the particles in their buckets (shared memory),
+// reserves each bucket's places with one add per tile, and, behind a grid barrier, scans the
+// bucket totals for itself and stores the records.  Behind a second barrier the blocks finish
+// the groups, behind a third the few calls that need it run the digit passes.
+// Per call, as a memset and seven launches / as a memset and this one: sort of 5000 particles 47 /
+// 34 us, step of 200 K particles 82 / 72; the rest of that is the host's.
+constexpr int kSmallThreads = 512;
+constexpr int kSmallItems = 4;
+constexpr int kSmallMostBuckets = 2048;
+
+struct SmallArgs {
+  const float *x, *y, *z, *v;
+  int64_t padded, n, num_cells;
+  PushSpec push;
+  AetherGrid grid;
+  uint32_t k0, k1;
+  int shift, buckets, group_shift, items;
+  uint32_t window;     // output slots per group, about
+  uint32_t* count;     // [buckets], zero
+  uint32_t* start;     // [buckets + 1]
+  uint2* groups;       // [buckets]
+  uint32_t* records;
+};
+
+template <class Shape>
+__global__ void __launch_bounds__(kSmallThreads, 2)
+small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr) {
+  static_assert(Shape::kThreads == kSmallThreads, "one block size for all phases");
+  static_assert(sizeof(FinishSmem<Shape>::raw) >= 2 * (kSmallMostBuckets + 4) * sizeof(uint32_t),
+                "the bucket tables lie over the records");
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
+  uint32_t* place = s.raw;                        // tile's counts, then its places in the buckets
+  uint32_t* start = s.raw + kSmallMostBuckets;    // bucket starts
+  constexpr uint32_t kHalf = Shape::kCapacity / 2;
+  const int tid = threadIdx.x;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * a.items * kSmallThreads + tid;
+
+  for (int b = tid; b < a.buckets; b += kSmallThreads) place[b] = 0;
+  __syncthreads();
+  float f[kSmallItems][6];
+  uint32_t key[kSmallItems], rank[kSmallItems];
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    const int64_t i = first + k * kSmallThreads;
+    const bool ok = k < a.items && i < a.n;
+    f[k][0] = ok ? a.x[i] : 0.f;
+    f[k][1] = ok ? a.y[i] : 0.f;
+    f[k][2] = ok ? a.z[i] : 0.f;
+    f[k][3] = ok && a.v ? a.v[i] : 0.f;
+    f[k][4] = ok && a.v ? a.v[a.padded + i] : 0.f;
+    f[k][5] = ok && a.v ? a.v[2 * a.padded + i] : 0.f;
+  }
+  bool sharing = true;
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    const int64_t i = first + k * kSmallThreads;
+    if (a.push.enabled) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) push_axis(f[k][c], f[k][3 + c], a.push.dt, a.push.lo[c], a.push.hi[c]);
+    }
+    const uint32_t cell = cell_of(f[k][0], f[k][1], f[k][2], a.grid);
+    key[k] = make_key(cell, static_cast<uint32_t>(i), a.k0, a.k1);
+    rank[k] = rank_in_tile(place, cell >> a.shift, k < a.items && i < a.n, sharing);
+  }
+  __syncthreads();
+  for (int b = tid; b < a.buckets; b += kSmallThreads) {
+    const uint32_t c = place[b];
+    if (c) place[b] = atomicAdd(&a.count[b], c);
+  }
+  if (!grid_barrier(&hdr->barrier, 1, &hdr->error)) return;
+
+  uint32_t carry = 0, biggest = 0;
+  for (int base = 0; base < a.buckets; base += kSmallThreads * 4) {
+    uint32_t c[4], sum = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int b = base + tid * 4 + k;
+      c[k] = b < a.buckets ? __ldcg(a.count + b) : 0u;
+      sum += c[k];
+      biggest = max(biggest, c[k]);
+    }
+    uint32_t before = carry + block_exclusive_scan(sum, s.warp_sum, &s.total);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int b = base + tid * 4 + k;
+      if (b < a.buckets) start[b] = before;
+      before += c[k];
+    }
+    carry += s.total;
+    __syncthreads();  // the scan's scratch is used again
+  }
+  if (tid == 0) start[a.buckets] = static_cast<uint32_t>(a.n);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    const int64_t i = first + k * kSmallThreads;
+    if (k >= a.items || i >= a.n) continue;
+    const uint32_t b = key[k] >> (kShuffleBits + a.shift);
+    uint32_t* record = a.records + static_cast<size_t>(start[b] + place[b] + rank[k]) * Shape::kRecordWords;
+    if constexpr (Shape::kRecordWords == kKeyRecordWords)
+      *reinterpret_cast<uint2*>(record) = make_uint2(key[k], static_cast<uint32_t>(i));
+    else
+      store_record(record, key[k], static_cast<uint32_t>(i), f[k][0], f[k][1], f[k][2], f[k][3],
+                   f[k][4], f[k][5]);
+  }
+  // Groups: a bucket begins one where an aligned block of buckets begins, where it or the bucket
+  // before it has more than half a block's records, and where its start passes into the next
+  // window (at most half the capacity) of output slots; so a group never has more than the
+  // capacity.  Every block takes a share of the buckets.
+  auto begins = [&](int b) {
+    return (b & ((1 << a.group_shift) - 1)) == 0 || start[b + 1] - start[b] > kHalf ||
+           start[b] - start[b - 1] > kHalf || start[b] / a.window != start[b - 1] / a.window;
+  };
+  const int share = (a.buckets + gridDim.x - 1) / gridDim.x;
+  const int share_end = min(a.buckets, static_cast<int>(blockIdx.x + 1) * share);
+  for (int b = blockIdx.x * share + tid; b < share_end; b += kSmallThreads) {
+    if (!begins(b) || start[b + 1] - start[b] > static_cast<uint32_t>(Shape::kCapacity)) continue;
+    int end = b + 1;
+    while (end < a.buckets && !begins(end)) ++end;
+    a.groups[atomicAdd(&hdr->aux_counter[1], 1u)] = make_uint2(static_cast<uint32_t>(b), static_cast<uint32_t>(end));
+  }
+  if (blockIdx.x == 0) {
+    for (int b = tid; b <= a.buckets; b += kSmallThreads) a.start[b] = start[b];
+    biggest = __reduce_max_sync(0xffffffffu, biggest);
+    if ((tid & 31) == 0) {
+      atomicMax(&hdr->max_bucket, biggest);
+      if (biggest > Shape::kLargestBucket) atomicExch(&hdr->use_standard, 1);
+    }
+    if (tid == 0) out.cell_start[a.num_cells] = static_cast<int32_t>(a.n);
+  }
+  if (!grid_barrier(&hdr->barrier, 2, &hdr->error)) return;
+
+  if (ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) == 0) {
+    bool held = true;
+    const uint32_t groups = ld_relaxed(&hdr->aux_counter[1]);
+    for (uint32_t g = blockIdx.x; g < groups; g += gridDim.x) {
+      const uint2 group = __ldcg(a.groups + g);
+      const uint32_t begin = __ldcg(a.start + group.x);
+      const int count = static_cast<int>(__ldcg(a.start + group.y) - begin);
+      const int64_t first_cell = static_cast<int64_t>(group.x) << a.shift;
+      const int cells_here = static_cast<int>(
+          min(static_cast<long long>(group.y - group.x) << a.shift, static_cast<long long>(a.num_cells - first_cell)));
+      const int drop = drop_for<Shape>(cells_here);
+      const int hist_words = max(8, cells_here * (32 >> drop));
+      const uint2* from = reinterpret_cast<const uint2*>(a.records + static_cast<size_t>(begin) * Shape::kRecordWords);
+      uint2* to = reinterpret_cast<uint2*>(s.raw);
+#pragma unroll 8
+      for (int i = tid; i < count * (Shape::kRecordWords / 2); i += kSmallThreads) to[i] = __ldcg(from + i);
+      for (int i = tid; i < hist_words; i += kSmallThreads) s.hist[i] = 0;
+      __syncthreads();
+      held = sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop) && held;
+    }
+    if (held && ld_relaxed(&hdr->max_bucket) > static_cast<uint32_t>(Shape::kCapacity)) {
+      const RunTable t{a.records, a.start, a.start, nullptr, nullptr, 0, 1, a.buckets, a.shift};
+      held = finish_large_buckets<Shape>(s, t, out, a.num_cells, Shape::kCapacity, blockIdx.x, gridDim.x);
+    }
+    if (!held && tid == 0) atomicExch(&hdr->use_standard, 1);
+  }
+  if (!grid_barrier(&hdr->barrier, 3, &hdr->error)) return;
+  if (ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) == 0) return;
+  digit_passes_in_grid<kSmallThreads>(digits, *reinterpret_cast<PassSmem<kSmallThreads>*>(smem_raw), hdr, 3);
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // The chunk-major record layout: while a chunk is scattered its stores stay inside the
@@ -1658,7 +1827,7 @@ BucketLayout bucket_layout_of(int64_t n, int64_t buckets, int chunk_log, int chu
 BucketLayout bucket_layout(int64_t n, const BucketPlan& p) {
   const int64_t buckets = p.buckets;
   // Tiles split in shared memory write whole runs: no window has to be kept small for them.
-  const int chunk_log = p.tiled || (p.keys_only && buckets <= kSplitMaxBuckets)
+  const int chunk_log = p.one_launch || p.tiled || (p.keys_only && buckets <= kSplitMaxBuckets)
                             ? kKeyChunkLog : chunk_log_for(buckets, n);
   const int chunks = static_cast<int>(
       std::max<int64_t>(1, (n + (int64_t{1} << chunk_log) - 1) >> chunk_log));
@@ -1671,6 +1840,13 @@ BucketLayout bucket_layout(int64_t n, const BucketPlan& p) {
 // (measured at 64 M particles: 65,536 buckets of 1,024 against 16,384 of 4,096).
 constexpr int64_t kMaxSmallShapeBuckets = 32 * 1024;
 int64_t g_small_shape_buckets = kMaxSmallShapeBuckets;  // tuning knob, see set_small_shape_buckets
+
+// Blocks of the one-launch sort, and what it takes: a tile per resident block.
+int64_t small_call_particles() { return 2 * static_cast<int64_t>(sm_count()) * kSmallThreads * kSmallItems; }
+int small_call_blocks(int64_t n, int64_t buckets) {
+  return static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(2 * sm_count(), std::max((n + kSmallThreads - 1) / kSmallThreads, buckets / 8))));
+}
 
 // Up to where slots are reserved tile by tile.
 constexpr int64_t kTiledMostParticles = 6 << 20;
@@ -1706,10 +1882,37 @@ int64_t group_capacity_for(int64_t n, int capacity, int blocks_per_sm) {
   return std::min<int64_t>(capacity, std::max<int64_t>(1024, n / (blocks * rounds) * 5 / 4));
 }
 
-// `tiled`: the call may use tile_scatter_kernel, to which few buckets are no burden.
+// Output slots per group of the one-launch sort: an even share of a block, at most half of what
+// a block holds.
+uint32_t small_call_window(int64_t n, int64_t buckets, int capacity) {
+  const int64_t blocks = small_call_blocks(n, buckets);
+  return static_cast<uint32_t>(std::min<int64_t>(capacity / 2, std::max<int64_t>(64, (n + blocks - 1) / blocks)));
+}
+
+template <class Shape>
+bool plan_one_launch(int64_t n, int64_t num_cells, BucketPlan* p) {
+  if (n <= 0 || n > small_call_particles()) return false;
+  // Buckets of half a window, so that groups are even.
+  const int64_t target = small_call_window(n, 0, Shape::kCapacity) / 2;
+  const int shift = shift_for(n, num_cells, target, log2_floor(Shape::kMaxCells), 1);
+  const int64_t buckets = (num_cells + (int64_t{1} << shift) - 1) >> shift;
+  if (buckets > kSmallMostBuckets || n > Shape::kCapacity * 2 / 5 * buckets) return false;
+  p->shift = shift;
+  p->buckets = buckets;
+  p->usable = p->one_launch = true;
+  return true;
+}
+
+// `tiled`: the call may use the one-launch sort or tile_scatter_kernel, to which few buckets are
+// no burden.
 BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small, bool tiled) {
   BucketPlan p;
-  p.keys_only = p.tiled = false;
+  p.keys_only = p.tiled = p.one_launch = false;
+  if (tiled && allow_small && plan_one_launch<FinishSmall>(n, num_cells, &p)) {
+    p.small_blocks = true;
+    if (p.buckets <= g_small_shape_buckets) return p;
+    p.one_launch = false;
+  }
   // The small finish shape (two blocks per multiprocessor) wants buckets well below its
   // capacity, so that the groups cut from them fill a block whatever the density does
   // inside a row of cells.
@@ -1741,8 +1944,9 @@ BucketPlan plan_buckets(int64_t n, int64_t num_cells, bool keys_only) {
   // every block gets some; buckets of at most four fifths of that.
   BucketPlan p;
   p.keys_only = true;
-  p.tiled = false;
+  p.tiled = p.one_launch = false;
   p.small_blocks = false;
+  if (plan_one_launch<FinishKeys>(n, num_cells, &p)) return p;
   const int64_t capacity = group_capacity_for(n, FinishKeys::kCapacity, 2);
   p.shift = shift_for(n, num_cells, capacity * 4 / 5 + 64, log2_floor(FinishKeys::kMaxCells), 1);
   p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
@@ -1871,6 +2075,53 @@ cudaError_t launch_split(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, 
 
 }  // namespace
 
+namespace {
+template <class Shape>
+cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLayout& l) {
+  constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<kSmallThreads>)));
+  static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two blocks must share a multiprocessor");
+  auto* base = static_cast<unsigned char*>(a.workspace);
+  DigitPassArgs digits;
+  cudaError_t e = digit_pass_args(a, &digits);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(small_sort_kernel<Shape>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (e != cudaSuccess) return e;
+  const int blocks = small_call_blocks(a.n, p.buckets);
+  SmallArgs s{};
+  s.x = a.x; s.y = a.y; s.z = a.z; s.v = a.velocity;
+  s.padded = a.padded; s.n = a.n; s.num_cells = a.num_cells;
+  s.push = a.push;
+  s.grid = a.grid;
+  s.k0 = static_cast<uint32_t>(a.seed);
+  s.k1 = static_cast<uint32_t>(a.seed >> 32);
+  s.shift = p.shift;
+  s.buckets = static_cast<int>(p.buckets);
+  s.group_shift = std::max(0, log2_floor(Shape::kMaxCells) - p.shift);
+  s.items = static_cast<int>((a.n + static_cast<int64_t>(blocks) * kSmallThreads - 1) /
+                             (static_cast<int64_t>(blocks) * kSmallThreads));
+  s.window = small_call_window(a.n, p.buckets, Shape::kCapacity);
+  s.count = reinterpret_cast<uint32_t*>(base + l.count_off);
+  s.start = reinterpret_cast<uint32_t*>(base + l.start_off);
+  s.groups = reinterpret_cast<uint2*>(base + l.tables_off);
+  s.records = reinterpret_cast<uint32_t*>(base + l.records_off);
+  const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
+                      a.vs, a.padded_sorted};
+  cudaLaunchAttribute cooperative{};
+  cooperative.id = cudaLaunchAttributeCooperative;
+  cooperative.val.cooperative = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = static_cast<unsigned>(blocks);
+  config.blockDim = kSmallThreads;
+  config.dynamicSmemBytes = kSmem;
+  config.stream = a.stream;
+  config.attrs = &cooperative;
+  config.numAttrs = 1;
+  count_launches(1);
+  return cudaLaunchKernelEx(&config, small_sort_kernel<Shape>, s, out, digits,
+                            reinterpret_cast<Header*>(base));
+}
+}  // namespace
+
 // Enqueues the bucketed path.  When a bucket turns out too large for the finish
 // kernel the device sets Header::use_standard, the kernels between return at once
 // and the tail kernel runs the digit passes.
@@ -1888,6 +2139,12 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   uint32_t* records = words_at(l.records_off);
   cudaError_t e = cudaMemsetAsync(base, 0, l.start_off, a.stream);  // header and run counts
   if (e != cudaSuccess) return e;
+  if (p.one_launch) {
+    stage_begin(kStageBucketFinish, a.stream);
+    e = p.keys_only ? launch_small<FinishKeys>(a, p, l) : launch_small<FinishSmall>(a, p, l);
+    stage_end(kStageBucketFinish, a.stream);
+    return e;
+  }
   const int buckets = static_cast<int>(p.buckets);
   const uint32_t k0 = static_cast<uint32_t>(a.seed), k1 = static_cast<uint32_t>(a.seed >> 32);
   const bool vec = aligned16(a.x) && aligned16(a.y) && aligned16(a.z) &&

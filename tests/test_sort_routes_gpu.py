@@ -118,3 +118,51 @@ def test_counters_of_sixteen_bits_are_emptied_in_time(cuda):
     step = keys[1:] - keys[:-1]
     assert bool(((step > 0) | ((step == 0) & (index[1:] > index[:-1]))).all())
     assert torch.equal(got.positions[0], x[index])
+
+
+# One launch; middling; large enough for the plain scatter.
+@pytest.mark.parametrize('n', [40_000, 1_500_000, 7_000_000])
+def test_capture_and_replay(cuda, n):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (64, 64, 32))
+    pos, vel = _state(n, cuda, 8)
+    other, other_vel = _state(n, cuda, 9)
+    stream = torch.cuda.Stream(cuda)
+    with torch.cuda.stream(stream):  # the stream's workspace exists before the capture
+        pa.sort_and_gather_particles(*pos, vel, grid, 5)
+        pa.sort_particles_by_cell(*pos, grid, 5)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        got = pa.sort_and_gather_particles(*pos, vel, grid, 5)
+        order = pa.sort_particles_by_cell(*pos, grid, 5)
+    for a, b in ((pos, vel), (other, other_vel)):
+        for to, source in zip(pos, a):
+            to.copy_(source)
+        vel.copy_(b)
+        graph.replay()
+        torch.cuda.synchronize()
+        want = pa.sort_and_gather_particles(*pos, vel, grid, 5)
+        for g, w in zip((*got.order, *got.positions, got.velocity),
+                        (*want.order, *want.positions, want.velocity)):
+            assert torch.equal(g, w)
+        for g, w in zip(order, want.order):
+            assert torch.equal(g, w)
+
+
+def test_two_streams_side_by_side(cuda):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (64, 64, 32))
+    sizes = (50_000, 300_000, 1_500_000)
+    states = [_state(n, cuda, n) for n in sizes]
+    want = [pa.sort_and_gather_particles(*pos, vel, grid, 3) for pos, vel in states]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(cuda) for _ in range(2)]
+    results = []
+    for _ in range(4):
+        for k, (pos, vel) in enumerate(states):
+            for s in streams:
+                with torch.cuda.stream(s):
+                    results.append((k, pa.sort_and_gather_particles(*pos, vel, grid, 3)))
+    torch.cuda.synchronize()
+    for k, got in results:
+        for g, w in zip((*got.order, *got.positions), (*want[k].order, *want[k].positions)):
+            assert torch.equal(g, w)
