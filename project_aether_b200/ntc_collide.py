@@ -18,6 +18,7 @@ from typing import NamedTuple, Optional
 import torch
 
 from . import _native
+from ._launch import on_device, raw_stream
 
 BOLTZMANN = 1.380649e-23
 
@@ -80,8 +81,8 @@ def collide(library: ctypes.CDLL, velocity: torch.Tensor, cell_start: torch.Tens
             velocity.shape[1] > 0 and (velocity.stride(1) != 1
                                        or velocity.stride(0) != velocity.shape[1])):
         raise ValueError('Velocity must be a contiguous (3, padded) tensor.')
-    with torch.cuda.device(velocity.device):
-        stream = torch.cuda.current_stream().cuda_stream
+    with on_device(velocity.device):
+        stream = raw_stream(velocity.device)
         status = library.AetherDsmcCollideTma(
             velocity.data_ptr(), cell_start.data_ptr(), sigma_g_max.data_ptr(),
             collisions.data_ptr(), int(num_particles), velocity.shape[1], sigma_g_max.numel(),

@@ -12,6 +12,7 @@ from collections.abc import Sequence
 import torch
 
 from . import _native
+from ._launch import on_device, raw_stream
 
 
 def fused_particle_push(positions: Sequence[torch.Tensor], velocities: Sequence[torch.Tensor],
@@ -37,8 +38,8 @@ def fused_particle_push(positions: Sequence[torch.Tensor], velocities: Sequence[
     device = tensors[0].device
     lo_c = (ctypes.c_float * 3)(*[float(v) for v in lo])
     hi_c = (ctypes.c_float * 3)(*[float(v) for v in hi])
-    with torch.cuda.device(device):
-        stream = torch.cuda.current_stream(device).cuda_stream
+    with on_device(device):
+        stream = raw_stream(device)
         _native.check(lib.AetherParticlePush(
-            *(ctypes.c_void_p(t.data_ptr()) for t in tensors), n, float(dt), lo_c, hi_c,
-            ctypes.c_void_p(stream)), 'AetherParticlePush')
+            *(t.data_ptr() for t in tensors), n, float(dt), lo_c, hi_c,
+            stream), 'AetherParticlePush')

@@ -23,6 +23,7 @@ from typing import NamedTuple, Optional, Tuple
 import torch
 
 from . import _native
+from ._launch import on_device, raw_stream
 from .cell_grid import CellGrid, MAX_PARTICLES, key_bits, num_passes  # noqa: F401
 
 PATH_AUTO, PATH_DIGIT_PASSES, PATH_BUCKETED = 0, 1, 2
@@ -60,7 +61,7 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """One cached scratch buffer per device and stream, grown on demand (with an eighth
     of headroom, so that a particle count that creeps up from call to call does not
     reallocate gigabytes every time)."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, raw_stream(device))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = None
@@ -83,18 +84,20 @@ def native_grid(grid: CellGrid, ix_offset: int = 0,
 
 
 def _check_positions(x, y, z):
+    n = x.numel() if isinstance(x, torch.Tensor) else -1
     for t in (x, y, z):
         if (not isinstance(t, torch.Tensor) or not t.is_cuda or t.dtype != torch.float32
-                or t.numel() != x.numel()):
+                or t.numel() != n):
             raise ValueError('Positions must be float32 CUDA tensors of the '
                              'same length.')
-    if x.numel() > MAX_PARTICLES:
+    if n > MAX_PARTICLES:
         raise ValueError(f'At most {MAX_PARTICLES} particles per sort.')
-    return tuple(t.contiguous().view(-1) for t in (x, y, z))
+    return tuple(t if t.dim() == 1 and t.is_contiguous() else t.contiguous().view(-1)
+                 for t in (x, y, z))
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def sort_particles_by_cell(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
@@ -128,18 +131,18 @@ def sort_particles_by_cell(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
     cells = g.nx_local * g.ny * g.nz
     num_passes(cells)  # raises ValueError when the key does not fit
     n, device = x.numel(), x.device
-    with torch.cuda.device(device):
+    with on_device(device):
         keys = torch.empty(n, dtype=torch.int32, device=device)
         index = torch.empty(n, dtype=torch.int32, device=device)
         counts = torch.empty(cells, dtype=torch.int32, device=device)
         start = torch.empty(cells + 1, dtype=torch.int32, device=device)
         nbytes = lib.AetherSortWorkspaceBytes(n, cells, 0)
         ws = _workspace(device, nbytes)
-        stream = torch.cuda.current_stream(device).cuda_stream
+        stream = raw_stream(device)
         _native.check(lib.AetherSortParticlesByCell(
             _ptr(x), _ptr(y), _ptr(z), n, ctypes.byref(g), int(seed) & 0xFFFFFFFFFFFFFFFF,
             _ptr(keys), _ptr(index), _ptr(counts), _ptr(start), _ptr(ws), ws.numel(),
-            ctypes.c_void_p(stream)), 'AetherSortParticlesByCell')
+            stream), 'AetherSortParticlesByCell')
     return SortResult(keys, index, counts, start)
 
 
@@ -189,7 +192,7 @@ def sort_and_gather_particles(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
     g = native_grid(grid, ix_offset, nx_local)
     cells = g.nx_local * g.ny * g.nz
     num_passes(cells)
-    with torch.cuda.device(device):
+    with on_device(device):
         padded_sorted = padded if padded_out is None else int(padded_out)
         if padded_sorted < n:
             raise ValueError('padded_out must be at least the number of particles.')
@@ -207,16 +210,16 @@ def sort_and_gather_particles(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
             xs, ys, zs = (torch.empty(n, dtype=torch.float32, device=device) for _ in range(3))
             vs = torch.empty((3, padded_sorted), dtype=torch.float32, device=device)
         if padded_sorted > n:
-            vs[:, n:].zero_()
+            vs.narrow(1, n, padded_sorted - n).zero_()
         nbytes = lib.AetherSortWorkspaceBytes(n, cells, 1)
         ws = _workspace(device, nbytes)
-        stream = torch.cuda.current_stream(device).cuda_stream
+        stream = raw_stream(device)
         if push is None:
             _native.check(lib.AetherSortAndGatherParticles(
                 _ptr(x), _ptr(y), _ptr(z), _ptr(velocity), padded, n, ctypes.byref(g),
                 int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(keys), _ptr(index), _ptr(counts),
                 _ptr(start), _ptr(xs), _ptr(ys), _ptr(zs), _ptr(vs), padded_sorted, int(path),
-                _ptr(ws), ws.numel(), ctypes.c_void_p(stream)), 'AetherSortAndGatherParticles')
+                _ptr(ws), ws.numel(), stream), 'AetherSortAndGatherParticles')
         else:
             dt, lo, hi = push
             _native.check(lib.AetherPushSortAndGatherParticles(
@@ -225,7 +228,7 @@ def sort_and_gather_particles(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
                 (ctypes.c_float * 3)(*[float(v) for v in hi]), ctypes.byref(g),
                 int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(keys), _ptr(index), _ptr(counts),
                 _ptr(start), _ptr(xs), _ptr(ys), _ptr(zs), _ptr(vs), padded_sorted, int(path),
-                _ptr(ws), ws.numel(), ctypes.c_void_p(stream)),
+                _ptr(ws), ws.numel(), stream),
                 'AetherPushSortAndGatherParticles')
     return SortedParticles(SortResult(keys, index, counts, start), (xs, ys, zs), vs)
 
@@ -235,14 +238,14 @@ def last_sort_status(device=None) -> int:
     current stream of `device`: 0 when clean, nonzero when a bounded device
     wait gave up (the results of that call are then invalid)."""
     device = torch.device('cuda', torch.cuda.current_device()) if device is None else device
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, raw_stream(device))
     ws = _workspaces.get(key)
     if ws is None:
         return 0
     lib = _native.load_library()
     status = ctypes.c_int32(0)
-    with torch.cuda.device(device):
-        _native.check(lib.AetherSortReadStatus(_ptr(ws), ctypes.c_void_p(key[1]),
+    with on_device(device):
+        _native.check(lib.AetherSortReadStatus(_ptr(ws), key[1],
                                                ctypes.byref(status)), 'AetherSortReadStatus')
     return status.value
 
@@ -252,14 +255,14 @@ def last_sort_used_digit_passes(device=None) -> bool:
     `device` was handed from the bucketed path to the digit passes on the device
     (same results, slower)."""
     device = torch.device('cuda', torch.cuda.current_device()) if device is None else device
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, raw_stream(device))
     ws = _workspaces.get(key)
     if ws is None:
         return False
     lib = _native.load_library()
     used = ctypes.c_int32(0)
-    with torch.cuda.device(device):
-        _native.check(lib.AetherSortReadUsedDigitPasses(_ptr(ws), ctypes.c_void_p(key[1]),
+    with on_device(device):
+        _native.check(lib.AetherSortReadUsedDigitPasses(_ptr(ws), key[1],
                                                         ctypes.byref(used)),
                       'AetherSortReadUsedDigitPasses')
     return bool(used.value)
