@@ -985,9 +985,11 @@ constexpr int kTableRowWords = (kMaxChunks + 3 + 3) / 4 * 4;
 // one block's bulk copy and output stores overlap the other's ranking; it wants buckets of
 // about a thousand records, which the count kernel's table can only offer up to about a
 // hundred million particles.  Above that the large shape (one block per multiprocessor) runs.
-template <int THREADS, int CAPACITY, int LOW_BITS, int RECORD_WORDS>
+template <int THREADS, int CAPACITY, int LOW_BITS, int RECORD_WORDS, int BLOCKS, int MAX_DROP>
 struct FinishShape {
   static constexpr int kRecordWords = RECORD_WORDS;
+  static constexpr int kBlocks = BLOCKS;                    // per multiprocessor
+  static constexpr int kMaxDrop = MAX_DROP;                 // key bits left to the tie step, at most
   static constexpr int kThreads = THREADS;
   static constexpr int kCapacity = CAPACITY;                // records a block holds
   static constexpr int kItems = (CAPACITY + THREADS - 1) / THREADS;
@@ -995,22 +997,31 @@ struct FinishShape {
   static constexpr int kHistWords = (1 << LOW_BITS) / 4;    // byte counters, 4 per word
   static constexpr int kWordsPerThread = kHistWords / THREADS;
   // A group spans at most this many cells: its low key (cell in group, shuffle bits) then has
-  // at most LOW_BITS + 2 bits, two of which the tie step may take.
-  static constexpr int kMaxCells = 1 << (LOW_BITS + 2 - kShuffleBits);
+  // at most LOW_BITS + MAX_DROP bits, of which the tie step may take MAX_DROP.
+  static constexpr int kMaxCells = 1 << (LOW_BITS + MAX_DROP - kShuffleBits);
   static constexpr uint32_t kLargestBucket = static_cast<uint32_t>(kMaxSegments) * CAPACITY;
   static_assert(kWordsPerThread % 8 == 0, "the counter scan reads eight words at a time");
-  static_assert(kHistWords >= CAPACITY, "the tie step lays one word per record over the counters");
+  static_assert(kHistWords * 3 / 2 >= CAPACITY, "the tie step lays a word per record over the counters");
 };
-using FinishSmall = FinishShape<512, 2560, 14, kRecordWords>;
-using FinishLarge = FinishShape<1024, 5120, 15, kRecordWords>;
-// Calls without payload: 8-byte records leave room for two blocks of the large shape's capacity.
-using FinishKeys = FinishShape<512, 5120, 15, kKeyRecordWords>;
+using FinishSmall = FinishShape<512, 2560, 14, kRecordWords, 2, 2>;
+using FinishLarge = FinishShape<1024, 5120, 15, kRecordWords, 1, 2>;
+// Calls without payload: 8-byte records and counters for half as many key bits leave room for
+// three blocks of the large shape's capacity (with 2^15 counters, two blocks: 16 M particles 371
+// us per call against 347, 4 M 116 against 111).  Three key bits may go to the tie step, so that
+// sparse grids still have few buckets; indices must then stay below 2^29.
+using FinishKeys = FinishShape<512, 5120, 14, kKeyRecordWords, 3, 3>;
+constexpr int64_t kKeysMostParticles = int64_t{1} << 29;
 
 template <class Shape>
 struct __align__(128) FinishSmem {
   uint32_t raw[Shape::kCapacity * Shape::kRecordWords];  // the group's records as they lie in HBM
-  uint32_t hist[Shape::kHistWords];     // byte counter per low-key value
-  uint16_t word_prefix[Shape::kHistWords];  // exclusive prefix of each counter word
+  union {
+    struct {
+      uint32_t hist[Shape::kHistWords];         // byte counter per low-key value
+      uint16_t word_prefix[Shape::kHistWords];  // exclusive prefix of each counter word
+    };
+    uint32_t tie[Shape::kCapacity];  // what the tie step compares, when the counters are done with
+  };
   uint16_t order[Shape::kCapacity];     // record held by each sorted slot
   uint32_t warp_sum[32];
   uint32_t total;
@@ -1027,8 +1038,9 @@ static_assert(sizeof(FinishSmem<FinishLarge>) + 3 * 2 * kTableRowWords * sizeof(
                   227 * 1024, "finish kernel shared memory");
 static_assert(2 * (sizeof(FinishSmem<FinishSmall>) + kSmallShapeTableBytes + 1024) <= 228 * 1024,
               "two small finish blocks must share a multiprocessor");
-static_assert(2 * (sizeof(FinishSmem<FinishKeys>) + 3 * 2 * kTableRowWords * sizeof(uint32_t) + 1024) <=
-                  228 * 1024, "two finish blocks of a call without payload must share one");
+constexpr size_t kKeysShapeTableBytes = 3 * 2 * 20 * sizeof(uint32_t);  // up to 17 chunks
+static_assert(3 * (sizeof(FinishSmem<FinishKeys>) + kKeysShapeTableBytes + 1024) <= 228 * 1024,
+              "three finish blocks of a call without payload must share one");
 
 template <class Shape>
 __device__ __forceinline__ uint32_t* group_table(FinishSmem<Shape>& s, int q, int row_words) {
@@ -1127,7 +1139,9 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
   // staged record where that is free of bank conflicts, kept in a register otherwise.)
   constexpr bool kKeep = Shape::kRecordWords != kKeyRecordWords;
   uint32_t mine[kKeep ? kItems : 1] = {};
-  auto tie_word = [&](uint2 key_index) { return ((key_index.x & drop_mask) << 30) | key_index.y; };
+  auto tie_word = [&](uint2 key_index) {
+    return ((key_index.x & drop_mask) << (32 - Shape::kMaxDrop)) | key_index.y;
+  };
   auto tie_word_of = [&](int k) {
     return kKeep ? mine[kKeep ? k : 0]
                  : tie_word(*reinterpret_cast<const uint2*>(
@@ -1232,11 +1246,11 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
 
   // Records that share a counter must appear in ascending (dropped key bits,
   // original index): a record inside such a run goes to (run start + number of
-  // smaller records in the run).  Indices stay below 2^30, so the dropped bits
+  // smaller records in the run).  Indices stay below 2^(32 - kMaxDrop), so the dropped bits
   // ride above them in one word.  The words to compare are laid out run by run
   // over the counters, which nobody reads any more: a run is then a few
   // neighbouring words instead of as many records scattered over s.raw.
-  uint32_t* tie = s.hist;
+  uint32_t* tie = s.tie;
 #pragma unroll
   for (int k = 0; k < kItems; ++k)
     if (run[k]) tie[(run[k] & 0xffffu) + (packed[k] >> 16)] = tie_word_of(k);
@@ -1474,7 +1488,7 @@ __device__ __forceinline__ void touch_runs(FinishSmem<Shape>& s, int q, const Ru
 // asynchronous copies; a group's records are asked into L2 while the group before it is
 // sorted, and copied into shared memory as soon as that one's output is written.
 template <class Shape>
-__global__ void __launch_bounds__(Shape::kThreads, Shape::kThreads <= 512 ? 2 : 1)
+__global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_device,
                      int64_t num_cells, FinishOut out, Header* __restrict__ hdr) {
   chain_begin();
@@ -1918,7 +1932,8 @@ BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small, bo
   // inside a row of cells.
   p.small_blocks = true;
   if (tiled && allow_small && n <= kTiledMostParticles) {
-    const int64_t target = std::min<int64_t>(1100, group_capacity_for(n, FinishSmall::kCapacity, 2) / 2);
+    const int64_t target = std::min<int64_t>(
+        1100, group_capacity_for(n, FinishSmall::kCapacity, FinishSmall::kBlocks) / 2);
     p.shift = shift_for(n, num_cells, target, log2_floor(FinishSmall::kMaxCells));
     p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
     p.tiled = p.buckets <= kTiledMostBuckets;
@@ -1939,7 +1954,7 @@ BucketPlan plan_buckets_shape(int64_t n, int64_t num_cells, bool allow_small, bo
 }  // namespace
 
 BucketPlan plan_buckets(int64_t n, int64_t num_cells, bool keys_only) {
-  if (!keys_only) return plan_buckets_shape(n, num_cells, true, true);
+  if (!keys_only || n >= kKeysMostParticles) return plan_buckets_shape(n, num_cells, true, true);
   // Groups of a call without payload: a finish block's capacity, or less on small inputs so that
   // every block gets some; buckets of at most four fifths of that.
   BucketPlan p;
@@ -1947,7 +1962,7 @@ BucketPlan plan_buckets(int64_t n, int64_t num_cells, bool keys_only) {
   p.tiled = p.one_launch = false;
   p.small_blocks = false;
   if (plan_one_launch<FinishKeys>(n, num_cells, &p)) return p;
-  const int64_t capacity = group_capacity_for(n, FinishKeys::kCapacity, 2);
+  const int64_t capacity = group_capacity_for(n, FinishKeys::kCapacity, FinishKeys::kBlocks);
   p.shift = shift_for(n, num_cells, capacity * 4 / 5 + 64, log2_floor(FinishKeys::kMaxCells), 1);
   p.buckets = (num_cells + (int64_t{1} << p.shift) - 1) >> p.shift;
   p.usable = n > 0 && n <= 4160 * p.buckets && p.buckets <= (int64_t{1} << 24);
@@ -1963,7 +1978,7 @@ uint32_t bucket_group_capacity(int64_t n, const BucketPlan& p) {
   return static_cast<uint32_t>(group_capacity_for(
       n, p.keys_only ? FinishKeys::kCapacity : p.small_blocks ? FinishSmall::kCapacity
                                                               : FinishLarge::kCapacity,
-      p.keys_only || p.small_blocks ? 2 : 1));
+      p.keys_only ? FinishKeys::kBlocks : p.small_blocks ? FinishSmall::kBlocks : FinishLarge::kBlocks));
 }
 
 size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells, bool keys_only) {
@@ -1998,8 +2013,7 @@ cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut&
   cudaError_t e = cudaFuncSetAttribute(bucket_finish_kernel<Shape>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  const int per_sm = Shape::kThreads <= 512 ? 2 : 1;
-  e = launch_chained<true>(bucket_finish_kernel<Shape>, std::min(t.buckets, sm_count() * per_sm),
+  e = launch_chained<true>(bucket_finish_kernel<Shape>, std::min(t.buckets, sm_count() * Shape::kBlocks),
                      Shape::kThreads, smem, a.stream, t, a.n, n_on_device, a.num_cells, out, hdr);
   if (e != cudaSuccess) return e;
   return e;
