@@ -5,13 +5,19 @@
 //                          bucket being 2^s consecutive cell ids (the upsweep;
 //                          replaces the histogram half of _bin_keys_kernel,
 //                          fused_radix_sort.py:106-113)
-//   bucket_scan_kernel     exclusive scan of the bucket counts -> bucket starts
-//                          and write cursors; decides whether every bucket fits
-//                          one thread block's shared memory
+//   run_scan_kernel        where every (chunk, bucket) run of records starts: the
+//                          scatter's write cursors and the finish kernel's table
+//   group_kernel           bucket starts, groups of buckets that one block
+//                          finishes, where their records lie; decides whether
+//                          every bucket can be finished
 //   bucket_scatter_kernel  reads x,y,z,v once, builds the key (cell id + Philox
 //                          shuffle bits, fused_radix_sort.py:93-103) and writes
 //                          one 32-byte record {key, index, x, y, z, vx, vy, vz}
 //                          into the particle's bucket
+//   tile_scatter_kernel    the same for middling calls, with few buckets: slots
+//                          are reserved tile by tile
+//   key_split_kernel       calls without payload: 8-byte records {key, index},
+//                          put in bucket order tile by tile in shared memory
 //   bucket_finish_kernel   a thread block takes a GROUP of consecutive buckets
 //                          that fits its shared memory (cut on the device from
 //                          the bucket totals, so dense and thin regions both
@@ -23,12 +29,16 @@
 //                          count atomics, torch.cumsum and the payload gather:
 //                          fused_radix_sort.py:116-203,277-279,
 //                          dsmc_gpu_pipeline.py:107-109)
+//   bucket_tail_kernel     buckets too large for a group, and the whole digit-pass
+//                          sort for calls the bucketed path cannot hold
+//   small_sort_kernel      all of the above in one launch, for small calls
 //
 // The result equals the stable sort by key: the records of a bucket arrive in
 // no particular order, and the finish kernel orders them by (low key bits,
 // original index), which is the order a stable sort produces.
 //
-// Record layout in HBM: chunk-major.  The particles are taken in chunks of 2^22
+// Record layout of bucket_scatter_kernel: chunk-major (the other scatter kernels write whole
+// runs and use one chunk).  The particles are taken in chunks of 2^22
 // consecutive indices; the records of chunk c and bucket b form one run, and the
 // runs are laid out [chunk][bucket].  While chunk c is being scattered all
 // stores fall into its 128 MB region instead of the whole record array: B200
@@ -418,13 +428,14 @@ __device__ __forceinline__ uint32_t rank_in_tile(uint32_t* table, uint32_t b, bo
 }
 
 // ------------------------------------------------------------------------
-// Scatter of small inputs: slots reserved tile by tile.
+// Scatter of middling inputs: slots reserved tile by tile.
 // ------------------------------------------------------------------------
 // With a thousand buckets or so the slot counters fill few L2 lines, and one returning add per
-// particle queues on them (1 M particles on 2048 counters: 47 us, of which the stores would need
-// 16).  Here a block ranks a tile's particles with adds in shared memory and reserves each
-// bucket's slots with one add per tile, consecutive threads on consecutive counters.  It pays
-// while a tile has about as many particles as there are buckets.
+// particle queues on them (1 M particles on 2048 counters: 47 us).  Here a block ranks a tile's
+// particles with adds in shared memory and reserves each bucket's slots with one add per tile,
+// consecutive threads on consecutive counters: 17 us, the rate of scattered 32-byte stores
+// (62 G/s).  It pays while a tile has about as many particles as there are buckets.  Staging the
+// tile in shared memory, so that a bucket's records leave side by side, took 23 us.
 template <bool VEC, int ITEMS>
 __global__ void __launch_bounds__(kScatterThreads, ITEMS <= 4 ? 2 : 1)
 tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
@@ -517,6 +528,8 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
 // counters), places from a scan while those are under way, records staged by place, then
 // written out with neighbouring lanes at neighbouring addresses.  The scatter kernel above
 // instead pays one returning L2 add and one store request per particle (64 G/s at best).
+// Bound by instructions and latency (32 warps per multiprocessor between barriers): 4 M particles
+// on 1250 buckets 37 us, 16 M on 4096 155, where the 32-byte records took 93 and 241.
 constexpr int kSplitThreads = 512;       // two blocks per multiprocessor
 constexpr int kSplitThreadsWide = 1024;  // one block, twice the tile
 constexpr int kSplitMaxBuckets = 16384;  // 128 KB of tables beside the stage
