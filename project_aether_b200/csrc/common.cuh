@@ -126,6 +126,13 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
 __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// Whether the call was handed over to the digit passes, one answer for the whole block (a
+// barrier).  Other blocks may set the word while a kernel runs: threads that read it for
+// themselves could disagree and meet different barriers.
+__device__ __forceinline__ bool handed_over(const Header* hdr) {
+  return __syncthreads_or(threadIdx.x == 0 &&
+                          ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) != 0);
+}
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;

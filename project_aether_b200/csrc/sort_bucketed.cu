@@ -1505,7 +1505,7 @@ __global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_device,
                      int64_t num_cells, FinishOut out, Header* __restrict__ hdr) {
   chain_begin();
-  if (hdr->use_standard) return;
+  if (handed_over(hdr)) return;
   constexpr int kThreads = Shape::kThreads;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
@@ -1603,7 +1603,7 @@ __global__ void __launch_bounds__(Shape::kThreads, 1)
 bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
                            Header* __restrict__ hdr, uint32_t capacity) {
   chain_begin();
-  if (hdr->use_standard || hdr->max_bucket <= capacity) return;
+  if (handed_over(hdr) || hdr->max_bucket <= capacity) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   if (!finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
                                    num_cells, capacity, blockIdx.x, gridDim.x) &&
@@ -1621,18 +1621,18 @@ template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, 1)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
                    DigitPassArgs digits) {
-  const bool handed_over = ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) != 0;
-  if (!handed_over && hdr->max_bucket <= capacity) return;
+  const bool skip_buckets = handed_over(hdr);
+  if (!skip_buckets && hdr->max_bucket <= capacity) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   // A block that comes late may already see another block's hand-over and skip its buckets:
   // the digit passes then write everything.
-  if (!handed_over &&
+  if (!skip_buckets &&
       !finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
                                    num_cells, capacity, blockIdx.x, gridDim.x) &&
       threadIdx.x == 0)
     atomicExch(&hdr->use_standard, 1);
   if (!grid_barrier(&hdr->barrier, 1, &hdr->error)) return;
-  if (ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) == 0) return;
+  if (!handed_over(hdr)) return;
   digit_passes_in_grid<Shape::kThreads>(
       digits, *reinterpret_cast<PassSmem<Shape::kThreads>*>(smem_raw), hdr, 1);
 }
@@ -1774,7 +1774,7 @@ small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr)
   }
   if (!grid_barrier(&hdr->barrier, 2, &hdr->error)) return;
 
-  if (ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) == 0) {
+  if (!handed_over(hdr)) {
     bool held = true;
     const uint32_t groups = ld_relaxed(&hdr->aux_counter[1]);
     for (uint32_t g = blockIdx.x; g < groups; g += gridDim.x) {
@@ -1801,7 +1801,7 @@ small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr)
     if (!held && tid == 0) atomicExch(&hdr->use_standard, 1);
   }
   if (!grid_barrier(&hdr->barrier, 3, &hdr->error)) return;
-  if (ld_relaxed(reinterpret_cast<const uint32_t*>(&hdr->use_standard)) == 0) return;
+  if (!handed_over(hdr)) return;
   digit_passes_in_grid<kSmallThreads>(digits, *reinterpret_cast<PassSmem<kSmallThreads>*>(smem_raw), hdr, 3);
 }
 

@@ -50,8 +50,60 @@ def test_dense_cell_is_sorted_by_the_digit_passes(cuda, n, cells, moved):
     np.testing.assert_array_equal(got.order.cell_start.cpu().numpy(), want.cell_start)
     for g, w in zip((*got.positions, got.velocity), sorted_payload):
         np.testing.assert_array_equal(g.cpu().numpy(), w)
-    if not moved:  # the same call without payload
-        order = pa.sort_particles_by_cell(*pos, grid, seed)
-        assert pa.last_sort_status(cuda) == 0
-        np.testing.assert_array_equal(order.particle_index.cpu().numpy(), want.particle_index)
-        np.testing.assert_array_equal(order.cell_start.cpu().numpy(), want.cell_start)
+    # The same particles without payload.
+    order = pa.sort_particles_by_cell(*(torch.from_numpy(np.ascontiguousarray(a)).to(cuda) for a in p),
+                                      grid, seed)
+    assert pa.last_sort_status(cuda) == 0
+    assert pa.last_sort_used_digit_passes(cuda)
+    np.testing.assert_array_equal(order.keys.cpu().numpy().view(np.uint32), want.keys)
+    np.testing.assert_array_equal(order.particle_index.cpu().numpy(), want.particle_index)
+    np.testing.assert_array_equal(order.cell_counts.cpu().numpy(), want.cell_counts)
+    np.testing.assert_array_equal(order.cell_start.cpu().numpy(), want.cell_start)
+
+
+def _sorted_as_by_the_oracle(pos, vel, grid, seed, cuda):
+    got = pa.sort_and_gather_particles(*pos, vel, grid, seed)
+    assert pa.last_sort_status(cuda) == 0
+    handed_over = pa.last_sort_used_digit_passes(cuda)
+    want, *payload = so.c_sort_particles(*(t.cpu().numpy() for t in pos), vel.cpu().numpy(),
+                                         so.Grid(grid.lo, grid.hi, grid.cells), seed)
+    order = pa.sort_particles_by_cell(*pos, grid, seed)
+    assert pa.last_sort_status(cuda) == 0
+    for result in (got.order, order):
+        np.testing.assert_array_equal(result.keys.cpu().numpy().view(np.uint32), want.keys)
+        np.testing.assert_array_equal(result.particle_index.cpu().numpy(), want.particle_index)
+        np.testing.assert_array_equal(result.cell_counts.cpu().numpy(), want.cell_counts)
+        np.testing.assert_array_equal(result.cell_start.cpu().numpy(), want.cell_start)
+    n = pos[0].numel()
+    for g, w in zip(got.positions, payload):
+        np.testing.assert_array_equal(g.cpu().numpy(), w)
+    np.testing.assert_array_equal(got.velocity.cpu().numpy()[:, :n], payload[3][:, :n])
+    return handed_over, pa.last_sort_used_digit_passes(cuda)
+
+
+def _crowd(pos, chosen, cells, edge, device):
+    """Puts the chosen particles, in equal parts, into the middle of `cells` cells of a cubic
+    grid with `edge` cells along an axis, spread over the whole grid."""
+    k = int(chosen.sum())
+    cell = (torch.arange(k, device=device) % cells) * (edge ** 3 // cells)
+    for axis, stride in enumerate((1, edge, edge * edge)):
+        pos[axis][chosen] = ((cell // stride % edge).float() + 0.5) / edge
+
+
+# Every block of a full grid finds cells that its shared memory cannot hold, or byte counters
+# that wrap, at about the same time: the hand-over is decided while other blocks start, sort and
+# wait.  One launch; behind the finish kernel of middling calls.
+@pytest.mark.parametrize('n,edge,cells', [(500_009, 64, 60), (2_400_011, 64, 250)])
+def test_many_blocks_decide_on_the_hand_over_together(cuda, n, edge, cells):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (edge,) * 3)
+    for repeat in range(3):
+        # Cells of 6,700 particles, more than any block holds.
+        pos, vel = _state(n, cuda, n + repeat)
+        _crowd(pos, torch.arange(n, device=cuda) % 6 != 0, cells, edge, cuda)
+        assert _sorted_as_by_the_oracle(pos, vel, grid, 5 + repeat, cuda) == (True, True)
+        # Cells of 600 particles, all of them with the same shuffle value.
+        pos, vel = _state(n, cuda, n + repeat)
+        seed = 77 + repeat
+        same = torch.from_numpy(so.shuffle_bits(n, seed) == 9).to(cuda)
+        _crowd(pos, same, int(same.sum()) // 600, edge, cuda)
+        assert _sorted_as_by_the_oracle(pos, vel, grid, seed, cuda) == (True, True)
