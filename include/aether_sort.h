@@ -368,6 +368,19 @@ size_t AetherSortProbeLookbackWorkspaceBytes(void);
 int AetherSortProbeLookbackGiveUp(void* workspace, size_t workspace_bytes, uint32_t poll_limit,
                                   void* stream);
 
+/* Test hook (no counterpart in the reference): AetherSortAndGatherParticles, or without sorted
+ * outputs AetherSortParticlesByCell, with at most `most_blocks` thread blocks in the kernels whose
+ * blocks share work in phases (the sort of small calls in one launch, and the kernel behind the
+ * finish of larger ones).  A block there waits only for work that running blocks have taken on, so
+ * any number of blocks finishes the call, as when something else keeps most multiprocessors. */
+int AetherSortProbeFewBlocks(const float* x, const float* y, const float* z,
+                             const float* velocity, int64_t padded, int64_t n,
+                             const AetherGrid* grid, uint64_t seed, uint32_t* keys_out,
+                             int32_t* index_out, int32_t* cell_counts, int32_t* cell_start,
+                             float* x_sorted, float* y_sorted, float* z_sorted,
+                             float* velocity_sorted, int64_t padded_sorted, int most_blocks,
+                             void* workspace, size_t workspace_bytes, void* stream);
+
 /* Measurement hooks.  The reference times whole calls with CUDA events around
  * the Python entry point (project_aether/scripts/phase2_triton_sort_benchmark.py:
  * 73-84); these give the same kind of event timing per stage of one call.

@@ -264,9 +264,9 @@ int sort_and_gather(const float* x, const float* y, const float* z, const float*
                     uint32_t* keys_out, int32_t* index_out, int32_t* cell_counts,
                     int32_t* cell_start, float* x_sorted, float* y_sorted, float* z_sorted,
                     float* velocity_sorted, int64_t padded_sorted, int path, void* workspace,
-                    size_t workspace_bytes, void* stream, const PushSpec& push) {
+                    size_t workspace_bytes, void* stream, const PushSpec& push, int most_blocks = 0) {
   if (!grid) return cudaErrorInvalidValue;
-  if (n > 0 && (!x_sorted || !y_sorted || !z_sorted)) return cudaErrorInvalidValue;
+  if (n > 0 && !most_blocks && (!x_sorted || !y_sorted || !z_sorted)) return cudaErrorInvalidValue;
   if ((velocity == nullptr) != (velocity_sorted == nullptr)) return cudaErrorInvalidValue;
   if (velocity && (padded < n || padded_sorted < n)) return cudaErrorInvalidValue;
   if (path < 0 || path > 2) return cudaErrorInvalidValue;
@@ -281,6 +281,7 @@ int sort_and_gather(const float* x, const float* y, const float* z, const float*
   a.workspace = workspace; a.workspace_bytes = workspace_bytes;
   a.stream = static_cast<cudaStream_t>(stream);
   a.push = push;
+  a.most_blocks = most_blocks;
   return run_sort(a, path);
 }
 }  // namespace
@@ -295,6 +296,22 @@ extern "C" int AetherSortAndGatherParticles(
   return sort_and_gather(x, y, z, velocity, padded, n, grid, seed, keys_out, index_out,
                          cell_counts, cell_start, x_sorted, y_sorted, z_sorted, velocity_sorted,
                          padded_sorted, path, workspace, workspace_bytes, stream, PushSpec{});
+}
+
+extern "C" int AetherSortProbeFewBlocks(
+    const float* x, const float* y, const float* z, const float* velocity, int64_t padded,
+    int64_t n, const AetherGrid* grid, uint64_t seed, uint32_t* keys_out, int32_t* index_out,
+    int32_t* cell_counts, int32_t* cell_start, float* x_sorted, float* y_sorted, float* z_sorted,
+    float* velocity_sorted, int64_t padded_sorted, int most_blocks, void* workspace,
+    size_t workspace_bytes, void* stream) {
+  if (most_blocks < 1) return cudaErrorInvalidValue;
+  const bool payload = x_sorted != nullptr;  // all of it or none
+  if ((y_sorted != nullptr) != payload || (z_sorted != nullptr) != payload || (velocity && !payload))
+    return cudaErrorInvalidValue;
+  return sort_and_gather(x, y, z, velocity, padded, n, grid, seed, keys_out, index_out,
+                         cell_counts, cell_start, x_sorted, y_sorted, z_sorted, velocity_sorted,
+                         padded_sorted, 0, workspace, workspace_bytes, stream, PushSpec{},
+                         most_blocks);
 }
 
 extern "C" int AetherPushSortAndGatherParticles(

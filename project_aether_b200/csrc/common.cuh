@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "../../include/aether_sort.h"
@@ -49,19 +50,27 @@ struct SliceSegments {
   uint32_t length[kMaxSlices][kMaxWorld];
 };
 
-// Workspace header (first 1 KiB of the workspace, zeroed by every call).
+constexpr int kMaxTiles = 512;  // tiles of the one-launch sort
+
+// Workspace header (first 5 KiB of the workspace, zeroed by every call).
 struct alignas(16) Header {
   int32_t error;              // first error code seen, 0 when clean
   int32_t use_standard;       // bucketed path: 1 when it handed over to the digit passes
-  uint32_t barrier;           // arrivals at the barriers of the cooperative launch
-  uint32_t unused;
+  uint32_t phase_ticket, phase_done;  // run_phases: pieces handed out, pieces done
+  uint32_t max_bucket;        // bucketed path: largest bucket seen
+  // One-launch sort: tiles counted and stored, next tile to look at for a block that helps,
+  // groups cut, next task and tasks done of the finish.
+  uint32_t tiles_counted, tiles_stored, help_next, groups, task_next, tasks_done;
+  uint32_t kept_pad[5];
+  uint32_t tile_claimed[kMaxTiles / 32], tile_loose[kMaxTiles / 32];  // one bit per tile
   uint32_t tile_counter[kMaxPasses];  // ticket dispenser of each digit pass
   uint32_t aux_counter[8];
-  uint32_t max_bucket;        // bucketed path: largest bucket seen
-  uint32_t pad[47];
+  uint32_t pad[4];
   uint32_t digit_hist[kMaxPasses][kRadix];  // global digit histograms (upsweep)
 };
-constexpr size_t kHeaderKept = 16;  // bytes the hand-over to the digit passes does not clear
+// Bytes the hand-over to the digit passes does not clear: blocks that start late still look there.
+constexpr size_t kHeaderKept = 192;
+static_assert(offsetof(Header, tile_counter) == kHeaderKept && offsetof(Header, digit_hist) == 256, "header");
 static_assert(sizeof(Header) % 256 == 0, "header must keep 256-byte alignment");
 
 __host__ __device__ inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
@@ -284,14 +293,14 @@ struct SortArgs {
   size_t workspace_bytes;
   cudaStream_t stream;
   PushSpec push;
+  int most_blocks;  // 0, or a limit on the blocks of the kernels that work in phases (probe)
 };
 
 size_t standard_workspace_bytes(int64_t n, int64_t num_cells);
 size_t standard_workspace_bytes_with_records(int64_t n, int64_t num_cells);
 // The digit-pass sort, one launch per step.
 cudaError_t standard_sort(const SortArgs& a);
-// Arguments of the same sort inside one cooperative launch (the hand-over from the bucketed
-// path); refuses the workspaces that standard_sort refuses.
+// Arguments of the same sort inside one launch (the hand-over from the bucketed path); refuses the workspaces that standard_sort refuses.
 struct DigitPassArgs;
 cudaError_t digit_pass_args(const SortArgs& a, DigitPassArgs* out);
 
@@ -309,7 +318,7 @@ struct BucketPlan {
   int64_t buckets;
   bool usable;        // false when even single-cell buckets would be too full on average
   bool small_blocks;  // finish kernel shape: two small blocks per multiprocessor, or one large
-  bool one_launch;    // small call: one cooperative launch
+  bool one_launch;    // small call: one launch
   bool tiled;         // scatter: slots reserved tile by tile
   bool keys_only;     // no payload: 8-byte records and a shape of their own
 };

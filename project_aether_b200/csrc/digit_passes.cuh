@@ -1,6 +1,6 @@
 // Device bodies of the digit passes, used by the kernels of the digit-pass path
 // (sort_standard.cu: one launch per pass) and by the kernel behind the bucketed path
-// (sort_bucketed.cu: all passes in one cooperative launch, for the calls the bucketed
+// (sort_bucketed.cu: all passes in one launch, for the calls the bucketed
 // path hands over).  Buffers that one pass writes and the next one reads are plain
 // pointers (no __restrict__): inside one launch they must not be read through the
 // non-coherent cache.
@@ -199,12 +199,12 @@ __device__ __forceinline__ bool digit_pass(PassSmem<THREADS>& s, const uint32_t*
 // long runs of empty cells are filled by the whole warp.
 template <int THREADS>
 __device__ __forceinline__ void cell_bounds(const uint32_t* keys, int64_t n, int64_t num_cells,
-                                            int32_t* cell_start) {
+                                            int32_t* cell_start, uint32_t block, uint32_t blocks) {
   const int lane = threadIdx.x & 31;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * THREADS;
+  const int64_t stride = static_cast<int64_t>(blocks) * THREADS;
   const int64_t rounds = (n + 1 + stride - 1) / stride;
   for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t i = r * stride + static_cast<int64_t>(blockIdx.x) * THREADS + threadIdx.x;
+    const int64_t i = r * stride + static_cast<int64_t>(block) * THREADS + threadIdx.x;
     int64_t first = 0, last = -1;  // cells [first, last] start at i
     if (i <= n) {
       const int64_t cur = i < n ? static_cast<int64_t>(keys[i] >> kShuffleBits) : num_cells;
@@ -228,41 +228,76 @@ __device__ __forceinline__ void cell_bounds(const uint32_t* keys, int64_t n, int
 }
 
 // ------------------------------------------------------------------------
-// Barrier over all blocks of a cooperative launch.
+// Work in phases by the blocks of an ordinary launch.
 // ------------------------------------------------------------------------
-// `arrivals` starts at zero; barrier number k (1, 2, ...) of a launch waits for k * gridDim.x
-// arrivals.  Bounded: about two seconds on the global timer; a block that gives up records the
-// error, and the others leave when they see one.  Returns false in every thread of a block
-// that must stop.
-__device__ __forceinline__ bool grid_barrier(uint32_t* arrivals, uint32_t number, int32_t* error) {
+// A block may only wait for work that a running block has taken on: then it does not matter how
+// many blocks of the launch run at the same time (a cooperative launch, which makes all of them
+// resident, cannot start while another stream's kernel keeps one multiprocessor).
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;
+
+// Counts pieces of work as done, with all that the block has written.
+__device__ __forceinline__ void arrive(uint32_t* done, uint32_t pieces = 1) {
   __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(done, pieces);
+  }
+}
+
+// Waits until `*done & mask` reaches `target`; false, in every thread of the block, when that
+// takes longer than `limit_ns` on the global timer or when some block has recorded an error.
+// `last`: in thread 0, the whole word as it was then.
+__device__ __forceinline__ bool wait_reaches(const uint32_t* done, uint32_t target,
+                                             const int32_t* error, unsigned long long limit_ns,
+                                             uint32_t mask = 0xffffffffu, uint32_t* last = nullptr) {
   bool stop = false;
   if (threadIdx.x == 0) {
-    const uint32_t target = number * gridDim.x;
     unsigned long long started = 0;
-    __threadfence();
-    atomicAdd(arrivals, 1u);
     for (;;) {
       uint32_t seen;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrivals) : "memory");
-      if (seen >= target) break;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(done) : "memory");
+      if (last) *last = seen;
+      if ((seen & mask) >= target) break;
       if (ld_relaxed(reinterpret_cast<const uint32_t*>(error)) != 0) { stop = true; break; }
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (started == 0) started = now;
-      else if (now - started > 2000000000ull) {
-        atomicCAS(error, 0, kErrBarrierTimeout);
-        stop = true;
-        break;
-      }
+      else if (now - started > limit_ns) { stop = true; break; }
     }
     __threadfence();
   }
   return __syncthreads_or(stop) == 0;
 }
 
+// The same; a block that gives up records the error, and the others leave when they see it.
+__device__ __forceinline__ bool wait_for(const uint32_t* done, uint32_t target, int32_t* error,
+                                         unsigned long long limit_ns = kWaitLimitNs,
+                                         uint32_t mask = 0xffffffffu, uint32_t* last = nullptr) {
+  if (wait_reaches(done, target, error, limit_ns, mask, last)) return true;
+  if (threadIdx.x == 0) atomicCAS(error, 0, kErrBarrierTimeout);
+  return false;
+}
+
+// `phases` phases of `items` pieces of work each, whatever the number of blocks: piece k of the
+// whole is item k % items of phase k / items.  Pieces are handed out in that order, and a block
+// does one at a time, so all pieces of the phase it waits for belong to blocks that run.
+// body(phase, item) returns false when the block must stop.
+template <class Body>
+__device__ __forceinline__ void run_phases(Header* hdr, uint32_t items, uint32_t phases, Body body) {
+  __shared__ uint32_t turn;
+  for (;;) {
+    if (threadIdx.x == 0) turn = atomicAdd(&hdr->phase_ticket, 1u);
+    __syncthreads();
+    const uint32_t phase = turn / items, item = turn % items;
+    if (phase >= phases) return;
+    if (!wait_for(&hdr->phase_done, phase * items, &hdr->error)) return;
+    if (!body(phase, item)) return;
+    arrive(&hdr->phase_done);
+  }
+}
+
 // ------------------------------------------------------------------------
-// The whole digit-pass sort inside one cooperative launch.
+// The whole digit-pass sort inside one launch.
 // ------------------------------------------------------------------------
 struct DigitPassArgs {
   const float *x, *y, *z, *v;
@@ -285,94 +320,95 @@ struct DigitPassArgs {
   float4* records;        // room for one 32-byte payload record per particle, or null
 };
 
-// `barriers`: barriers of this launch already used.  The speed of this function matters
-// little: it runs for calls whose density the bucketed path cannot hold.
-template <int THREADS>
-__device__ __forceinline__ void digit_passes_in_grid(const DigitPassArgs& a, PassSmem<THREADS>& s,
-                                                     Header* hdr, uint32_t barriers) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * THREADS;
-  const int64_t first = static_cast<int64_t>(blockIdx.x) * THREADS + threadIdx.x;
-  for (int64_t i = first; i < a.clear_words; i += stride) a.clear_from[i] = 0;
-  if (!grid_barrier(&hdr->barrier, ++barriers, &hdr->error)) return;
+__device__ __forceinline__ uint32_t digit_phases(const DigitPassArgs& a) { return a.passes + 4; }
 
+// Item `item` of `items` of phase `phase` of the sort; false when a look-back gave up.  The speed
+// of this function matters little: it runs for calls whose density the bucketed path cannot hold.
+template <int THREADS>
+__device__ __forceinline__ bool digit_phase(const DigitPassArgs& a, PassSmem<THREADS>& s, Header* hdr,
+                                            uint32_t phase, uint32_t item, uint32_t items) {
+  const int64_t stride = static_cast<int64_t>(items) * THREADS;
+  const int64_t first = static_cast<int64_t>(item) * THREADS + threadIdx.x;
   const bool odd = a.passes % 2 != 0;
   uint32_t* out_v = reinterpret_cast<uint32_t*>(a.index_out);
   uint32_t *cur_k = odd ? a.keys_alt : a.keys_out, *cur_v = odd ? a.index_alt : out_v;
   uint32_t *nxt_k = odd ? a.keys_out : a.keys_alt, *nxt_v = odd ? out_v : a.index_alt;
 
-  // Keys, digit histograms and payload records (with the move stage, if it is fused).
-  uint32_t* hist = &s.warp_count[0][0];
-  for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += THREADS) hist[i] = 0;
-  __syncthreads();
-  const int64_t rounds = (a.n + stride - 1) / stride;
-  for (int64_t r = 0; r < rounds; ++r) {  // the same number for every thread: warp votes below
-    const int64_t i = r * stride + first;
-    const bool ok = i < a.n;
-    uint32_t key = 0;
-    if (ok) {
-      float px = a.x[i], py = a.y[i], pz = a.z[i];
-      if (a.records) {
-        float vx = a.v ? a.v[i] : 0.f, vy = a.v ? a.v[a.padded + i] : 0.f;
-        float vz = a.v ? a.v[2 * a.padded + i] : 0.f;
-        if (a.push.enabled) {
-          push_axis(px, vx, a.push.dt, a.push.lo[0], a.push.hi[0]);
-          push_axis(py, vy, a.push.dt, a.push.lo[1], a.push.hi[1]);
-          push_axis(pz, vz, a.push.dt, a.push.lo[2], a.push.hi[2]);
+  if (phase == 0) {
+    for (int64_t i = first; i < a.clear_words; i += stride) a.clear_from[i] = 0;
+  } else if (phase == 1) {
+    // Keys, digit histograms and payload records (with the move stage, if it is fused).
+    uint32_t* hist = &s.warp_count[0][0];
+    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += THREADS) hist[i] = 0;
+    __syncthreads();
+    const int64_t rounds = (a.n + stride - 1) / stride;
+    for (int64_t r = 0; r < rounds; ++r) {  // the same number for every thread: warp votes below
+      const int64_t i = r * stride + first;
+      const bool ok = i < a.n;
+      uint32_t key = 0;
+      if (ok) {
+        float px = a.x[i], py = a.y[i], pz = a.z[i];
+        if (a.records) {
+          float vx = a.v ? a.v[i] : 0.f, vy = a.v ? a.v[a.padded + i] : 0.f;
+          float vz = a.v ? a.v[2 * a.padded + i] : 0.f;
+          if (a.push.enabled) {
+            push_axis(px, vx, a.push.dt, a.push.lo[0], a.push.hi[0]);
+            push_axis(py, vy, a.push.dt, a.push.lo[1], a.push.hi[1]);
+            push_axis(pz, vz, a.push.dt, a.push.lo[2], a.push.hi[2]);
+          }
+          a.records[2 * i] = make_float4(px, py, pz, vx);
+          a.records[2 * i + 1] = make_float4(vy, vz, 0.f, 0.f);
         }
-        a.records[2 * i] = make_float4(px, py, pz, vx);
-        a.records[2 * i + 1] = make_float4(vy, vz, 0.f, 0.f);
+        key = make_key(cell_of(px, py, pz, a.grid), static_cast<uint32_t>(i), a.k0, a.k1);
+        cur_k[i] = key;
       }
-      key = make_key(cell_of(px, py, pz, a.grid), static_cast<uint32_t>(i), a.k0, a.k1);
-      cur_k[i] = key;
+      for (int p = 0; p < a.passes; ++p)
+        bin_add(hist + p * kRadix, (key >> (kRadixBits * p)) & (kRadix - 1), ok);
     }
-    for (int p = 0; p < a.passes; ++p)
-      bin_add(hist + p * kRadix, (key >> (kRadixBits * p)) & (kRadix - 1), ok);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < a.passes * kRadix; i += THREADS)
-    if (hist[i]) atomicAdd(&hdr->digit_hist[0][0] + i, hist[i]);
-  if (!grid_barrier(&hdr->barrier, ++barriers, &hdr->error)) return;
-
-  for (int p = 0; p < a.passes; ++p) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.passes * kRadix; i += THREADS)
+      if (hist[i]) atomicAdd(&hdr->digit_hist[0][0] + i, hist[i]);
+  } else if (phase < static_cast<uint32_t>(a.passes) + 2) {
+    const int p = static_cast<int>(phase) - 2;
+    if (p % 2 != 0) {
+      uint32_t* t = cur_k; cur_k = nxt_k; nxt_k = t;
+      t = cur_v; cur_v = nxt_v; nxt_v = t;
+    }
     uint32_t* st = a.status + static_cast<size_t>(p) * a.tiles * kRadix;
-    const bool good =
-        p == 0 ? digit_pass<true, THREADS>(s, cur_k, nullptr, nxt_k, nxt_v, a.n, 0,
-                                           hdr->digit_hist[0], st, &hdr->tile_counter[0], a.tiles,
-                                           &hdr->error, kPollLimit)
-               : digit_pass<false, THREADS>(s, cur_k, cur_v, nxt_k, nxt_v, a.n, kRadixBits * p,
-                                            hdr->digit_hist[p], st, &hdr->tile_counter[p], a.tiles,
-                                            &hdr->error, kPollLimit);
-    if (!good) return;  // the error is recorded: the other blocks leave at the barrier
-    if (!grid_barrier(&hdr->barrier, ++barriers, &hdr->error)) return;
-    uint32_t* t = cur_k; cur_k = nxt_k; nxt_k = t;
-    t = cur_v; cur_v = nxt_v; nxt_v = t;
-  }
-
-  if (a.xs) {
-    for (int64_t r = first; r < a.n; r += stride) {
-      const int64_t i = a.index_out[r];
-      float4 lo, hi;
-      if (a.records) {
-        lo = a.records[2 * i];
-        hi = a.records[2 * i + 1];
-      } else {
-        lo = make_float4(a.x[i], a.y[i], a.z[i], a.v ? a.v[i] : 0.f);
-        hi = make_float4(a.v ? a.v[a.padded + i] : 0.f, a.v ? a.v[2 * a.padded + i] : 0.f, 0.f, 0.f);
-      }
-      a.xs[r] = lo.x;
-      a.ys[r] = lo.y;
-      a.zs[r] = lo.z;
-      if (a.vs) {
-        a.vs[r] = lo.w;
-        a.vs[a.padded_sorted + r] = hi.x;
-        a.vs[2 * a.padded_sorted + r] = hi.y;
+    return p == 0 ? digit_pass<true, THREADS>(s, cur_k, nullptr, nxt_k, nxt_v, a.n, 0,
+                                              hdr->digit_hist[0], st, &hdr->tile_counter[0], a.tiles,
+                                              &hdr->error, kPollLimit)
+                  : digit_pass<false, THREADS>(s, cur_k, cur_v, nxt_k, nxt_v, a.n, kRadixBits * p,
+                                               hdr->digit_hist[p], st, &hdr->tile_counter[p], a.tiles,
+                                               &hdr->error, kPollLimit);
+  } else if (phase == static_cast<uint32_t>(a.passes) + 2) {
+    if (a.xs) {
+      for (int64_t r = first; r < a.n; r += stride) {
+        const int64_t i = __ldcg(a.index_out + r);
+        float4 lo, hi;
+        if (a.records) {
+          lo = __ldcg(a.records + 2 * i);
+          hi = __ldcg(a.records + 2 * i + 1);
+        } else {
+          lo = make_float4(a.x[i], a.y[i], a.z[i], a.v ? a.v[i] : 0.f);
+          hi = make_float4(a.v ? a.v[a.padded + i] : 0.f, a.v ? a.v[2 * a.padded + i] : 0.f, 0.f, 0.f);
+        }
+        a.xs[r] = lo.x;
+        a.ys[r] = lo.y;
+        a.zs[r] = lo.z;
+        if (a.vs) {
+          a.vs[r] = lo.w;
+          a.vs[a.padded_sorted + r] = hi.x;
+          a.vs[2 * a.padded_sorted + r] = hi.y;
+        }
       }
     }
+    cell_bounds<THREADS>(a.keys_out, a.n, a.num_cells, a.cell_start, item, items);
+  } else {
+    for (int64_t c = first; c < a.num_cells; c += stride)
+      a.cell_counts[c] = __ldcg(a.cell_start + c + 1) - __ldcg(a.cell_start + c);
   }
-  cell_bounds<THREADS>(a.keys_out, a.n, a.num_cells, a.cell_start);
-  if (!grid_barrier(&hdr->barrier, ++barriers, &hdr->error)) return;
-  for (int64_t c = first; c < a.num_cells; c += stride)
-    a.cell_counts[c] = a.cell_start[c + 1] - a.cell_start[c];
+  return true;
 }
 
 }  // namespace aether

@@ -1039,6 +1039,7 @@ struct __align__(128) FinishSmem {
   uint32_t warp_sum[32];
   uint32_t total;
   uint32_t gave_up;
+  uint32_t turn, groups, tasks;  // one-launch sort: what the block works on next; of how many
   unsigned long long barrier;    // mbarrier of the bulk copy
   uint32_t seg_begin[kMaxSegments + 1];  // oversized bucket: records before each run of cells
   uint16_t seg_first[kMaxSegments + 1];  // ... and the first cell of each run
@@ -1611,45 +1612,55 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
     hdr->use_standard = 1;
 }
 
-// Behind the finish kernel of an ordinary call, one cooperative launch: the oversized buckets,
-// then, when the call was handed over, the whole digit-pass sort.  Usually there is nothing
-// to do and every block returns after a look at the header.  What bounds it is then the launch
-// itself: as the separate kernels it replaces (the oversized buckets, a clear, the keys, up to
-// four digit passes, two table kernels and the payload gather, each returning at once) the same
-// look cost 13-17 us of every call on the device and 11 launches on the host.
+// Behind the finish kernel of an ordinary call: the oversized buckets, then, when the call was
+// handed over, the whole digit-pass sort.  Usually there is nothing to do and every block returns
+// after a look at the header.  What bounds it is then the launch itself: as the separate kernels
+// it replaces (the oversized buckets, a clear, the keys, up to four digit passes, two table
+// kernels and the payload gather, each returning at once) the same look cost 13-17 us of every
+// call on the device and 11 launches on the host.
 template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, 1)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
                    DigitPassArgs digits) {
-  const bool skip_buckets = handed_over(hdr);
-  if (!skip_buckets && hdr->max_bucket <= capacity) return;
+  chain_begin();
+  if (!handed_over(hdr) && hdr->max_bucket <= capacity) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  // A block that comes late may already see another block's hand-over and skip its buckets:
-  // the digit passes then write everything.
-  if (!skip_buckets &&
-      !finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
-                                   num_cells, capacity, blockIdx.x, gridDim.x) &&
-      threadIdx.x == 0)
-    atomicExch(&hdr->use_standard, 1);
-  if (!grid_barrier(&hdr->barrier, 1, &hdr->error)) return;
-  if (!handed_over(hdr)) return;
-  digit_passes_in_grid<Shape::kThreads>(
-      digits, *reinterpret_cast<PassSmem<Shape::kThreads>*>(smem_raw), hdr, 1);
+  const uint32_t items = gridDim.x;
+  run_phases(hdr, items, 1 + digit_phases(digits), [&](uint32_t phase, uint32_t item) {
+    const bool standard = handed_over(hdr);
+    if (phase > 0)
+      return standard && digit_phase<Shape::kThreads>(
+                             digits, *reinterpret_cast<PassSmem<Shape::kThreads>*>(smem_raw), hdr,
+                             phase - 1, item, items);
+    // A block that comes late may see another block's hand-over and skip its buckets: the digit
+    // passes then write everything.
+    if (!standard &&
+        !finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
+                                     num_cells, capacity, item, items) &&
+        threadIdx.x == 0)
+      atomicExch(&hdr->use_standard, 1);
+    return true;
+  });
 }
+
 // ------------------------------------------------------------------------
-// Small calls: the whole sort in one cooperative launch.
+// Small calls: the whole sort in one launch.
 // ------------------------------------------------------------------------
 // Up to here a call's time is the host's enqueueing of kernels and the latency of each; the work
 // itself is a few microseconds.  A block takes one tile of at most kSmallItems particles per
 // thread and keeps it in registers: it ranks the particles in their buckets (shared memory),
-// reserves each bucket's places with one add per tile, and, behind a grid barrier, scans the
-// bucket totals for itself and stores the records.  Behind a second barrier the blocks finish
-// the groups, behind a third the few calls that need it run the digit passes.
-// Per call, as a memset and seven launches / as a memset and this one: sort of 5000 particles 47 /
-// 34 us, step of 200 K particles 82 / 72; the rest of that is the host's.
+// reserves each bucket's places with one add per tile, and, when all tiles are counted, scans the
+// bucket totals for itself and stores the records.  When all are stored the blocks finish the
+// groups, and behind that the few calls that need it run the digit passes.
+// Usually all blocks run at once.  When they do not (something else holds multiprocessors), those
+// that run count the tiles of those that don't, after kHelpAfterNs: a block waits for work that
+// running blocks have taken on, and for nothing else.
 constexpr int kSmallThreads = 512;
 constexpr int kSmallItems = 4;
 constexpr int kSmallMostBuckets = 2048;
+constexpr uint32_t kFailedTask = 1u << 16;  // in tasks_done, above the number of tasks
+static_assert(2 * (kSmallMostBuckets + kMaxTiles) < kFailedTask, "two counts in a word");
+constexpr unsigned long long kHelpAfterNs = 50000;  // launch skew of a full grid: a few us
 
 struct SmallArgs {
   const float *x, *y, *z, *v;
@@ -1658,6 +1669,7 @@ struct SmallArgs {
   AetherGrid grid;
   uint32_t k0, k1;
   int shift, buckets, group_shift, items;
+  int tiles;           // of items * kSmallThreads particles; the last ones may be empty
   uint32_t window;     // output slots per group, about
   uint32_t* count;     // [buckets], zero
   uint32_t* start;     // [buckets + 1]
@@ -1666,53 +1678,60 @@ struct SmallArgs {
 };
 
 template <class Shape>
-__global__ void __launch_bounds__(kSmallThreads, 2)
-small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr) {
-  static_assert(Shape::kThreads == kSmallThreads, "one block size for all phases");
-  static_assert(sizeof(FinishSmem<Shape>::raw) >= 2 * (kSmallMostBuckets + 4) * sizeof(uint32_t),
-                "the bucket tables lie over the records");
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
-  uint32_t* place = s.raw;                        // tile's counts, then its places in the buckets
-  uint32_t* start = s.raw + kSmallMostBuckets;    // bucket starts
-  constexpr uint32_t kHalf = Shape::kCapacity / 2;
-  const int tid = threadIdx.x;
-  const int64_t first = static_cast<int64_t>(blockIdx.x) * a.items * kSmallThreads + tid;
+struct SmallTables {  // over the records of the finish
+  uint32_t *place, *start;
+  __device__ __forceinline__ explicit SmallTables(FinishSmem<Shape>& s)
+      : place(s.raw), start(s.raw + kSmallMostBuckets) {
+    static_assert(sizeof(s.raw) >= 2 * (kSmallMostBuckets + 4) * sizeof(uint32_t), "room for both");
+  }
+};
 
-  for (int b = tid; b < a.buckets; b += kSmallThreads) place[b] = 0;
-  __syncthreads();
-  float f[kSmallItems][6];
-  uint32_t key[kSmallItems], rank[kSmallItems];
+__device__ __forceinline__ bool claim_tile(Header* hdr, int tile) {
+  const uint32_t bit = 1u << (tile & 31);
+  return (atomicOr(&hdr->tile_claimed[tile >> 5], bit) & bit) == 0;
+}
+
+template <int RECORD_WORDS>
+__device__ __forceinline__ void store_small_record(const SmallArgs& a, uint32_t slot, uint32_t key,
+                                                   int64_t i, const float* f) {
+  uint32_t* record = a.records + static_cast<size_t>(slot) * RECORD_WORDS;
+  if constexpr (RECORD_WORDS == kKeyRecordWords)
+    *reinterpret_cast<uint2*>(record) = make_uint2(key, static_cast<uint32_t>(i));
+  else
+    store_record(record, key, static_cast<uint32_t>(i), f[0], f[1], f[2], f[3], f[4], f[5]);
+}
+
+// Particle i's values behind the fused move stage, and its cell.
+__device__ __forceinline__ uint32_t small_cell(const SmallArgs& a, float* f) {
+  if (a.push.enabled) {
 #pragma unroll
-  for (int k = 0; k < kSmallItems; ++k) {
-    const int64_t i = first + k * kSmallThreads;
-    const bool ok = k < a.items && i < a.n;
-    f[k][0] = ok ? a.x[i] : 0.f;
-    f[k][1] = ok ? a.y[i] : 0.f;
-    f[k][2] = ok ? a.z[i] : 0.f;
-    f[k][3] = ok && a.v ? a.v[i] : 0.f;
-    f[k][4] = ok && a.v ? a.v[a.padded + i] : 0.f;
-    f[k][5] = ok && a.v ? a.v[2 * a.padded + i] : 0.f;
+    for (int c = 0; c < 3; ++c) push_axis(f[c], f[3 + c], a.push.dt, a.push.lo[c], a.push.hi[c]);
   }
-  bool sharing = true;
-#pragma unroll
-  for (int k = 0; k < kSmallItems; ++k) {
-    const int64_t i = first + k * kSmallThreads;
-    if (a.push.enabled) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) push_axis(f[k][c], f[k][3 + c], a.push.dt, a.push.lo[c], a.push.hi[c]);
-    }
-    const uint32_t cell = cell_of(f[k][0], f[k][1], f[k][2], a.grid);
-    key[k] = make_key(cell, static_cast<uint32_t>(i), a.k0, a.k1);
-    rank[k] = rank_in_tile(place, cell >> a.shift, k < a.items && i < a.n, sharing);
-  }
-  __syncthreads();
-  for (int b = tid; b < a.buckets; b += kSmallThreads) {
+  return cell_of(f[0], f[1], f[2], a.grid);
+}
+__device__ __forceinline__ void load_small(const SmallArgs& a, int64_t i, bool ok, float* f) {
+  f[0] = ok ? a.x[i] : 0.f;
+  f[1] = ok ? a.y[i] : 0.f;
+  f[2] = ok ? a.z[i] : 0.f;
+  f[3] = ok && a.v ? a.v[i] : 0.f;
+  f[4] = ok && a.v ? a.v[a.padded + i] : 0.f;
+  f[5] = ok && a.v ? a.v[2 * a.padded + i] : 0.f;
+}
+
+// One add per bucket and tile: a tile's counts become its first places in the buckets.
+__device__ __forceinline__ void reserve_places(const SmallArgs& a, uint32_t* place) {
+  for (int b = threadIdx.x; b < a.buckets; b += kSmallThreads) {
     const uint32_t c = place[b];
     if (c) place[b] = atomicAdd(&a.count[b], c);
   }
-  if (!grid_barrier(&hdr->barrier, 1, &hdr->error)) return;
+  __syncthreads();
+}
 
+// Bucket starts from the bucket totals; returns the largest total this thread has seen.
+template <class Shape>
+__device__ __forceinline__ uint32_t scan_totals(const SmallArgs& a, FinishSmem<Shape>& s) {
+  uint32_t* start = SmallTables<Shape>(s).start;
+  const int tid = threadIdx.x;
   uint32_t carry = 0, biggest = 0;
   for (int base = 0; base < a.buckets; base += kSmallThreads * 4) {
     uint32_t c[4], sum = 0;
@@ -1735,35 +1754,31 @@ small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr)
   }
   if (tid == 0) start[a.buckets] = static_cast<uint32_t>(a.n);
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kSmallItems; ++k) {
-    const int64_t i = first + k * kSmallThreads;
-    if (k >= a.items || i >= a.n) continue;
-    const uint32_t b = key[k] >> (kShuffleBits + a.shift);
-    uint32_t* record = a.records + static_cast<size_t>(start[b] + place[b] + rank[k]) * Shape::kRecordWords;
-    if constexpr (Shape::kRecordWords == kKeyRecordWords)
-      *reinterpret_cast<uint2*>(record) = make_uint2(key[k], static_cast<uint32_t>(i));
-    else
-      store_record(record, key[k], static_cast<uint32_t>(i), f[k][0], f[k][1], f[k][2], f[k][3],
-                   f[k][4], f[k][5]);
-  }
-  // Groups: a bucket begins one where an aligned block of buckets begins, where it or the bucket
-  // before it has more than half a block's records, and where its start passes into the next
-  // window (at most half the capacity) of output slots; so a group never has more than the
-  // capacity.  Every block takes a share of the buckets.
+  return biggest;
+}
+
+// Groups: a bucket begins one where an aligned block of buckets begins, where it or the bucket
+// before it has more than half a block's records, and where its start passes into the next
+// window (at most half the capacity) of output slots; so a group never has more than the
+// capacity.  With every tile goes a share of the buckets, with the first what is written once.
+template <class Shape>
+__device__ __forceinline__ void cut_groups(const SmallArgs& a, const FinishOut& out, Header* hdr,
+                                           const uint32_t* start, uint32_t biggest, int tile) {
+  constexpr uint32_t kHalf = Shape::kCapacity / 2;
+  const int tid = threadIdx.x;
   auto begins = [&](int b) {
     return (b & ((1 << a.group_shift) - 1)) == 0 || start[b + 1] - start[b] > kHalf ||
            start[b] - start[b - 1] > kHalf || start[b] / a.window != start[b - 1] / a.window;
   };
-  const int share = (a.buckets + gridDim.x - 1) / gridDim.x;
-  const int share_end = min(a.buckets, static_cast<int>(blockIdx.x + 1) * share);
-  for (int b = blockIdx.x * share + tid; b < share_end; b += kSmallThreads) {
+  const int share = (a.buckets + a.tiles - 1) / a.tiles;
+  const int share_end = min(a.buckets, (tile + 1) * share);
+  for (int b = tile * share + tid; b < share_end; b += kSmallThreads) {
     if (!begins(b) || start[b + 1] - start[b] > static_cast<uint32_t>(Shape::kCapacity)) continue;
     int end = b + 1;
     while (end < a.buckets && !begins(end)) ++end;
-    a.groups[atomicAdd(&hdr->aux_counter[1], 1u)] = make_uint2(static_cast<uint32_t>(b), static_cast<uint32_t>(end));
+    a.groups[atomicAdd(&hdr->groups, 1u)] = make_uint2(static_cast<uint32_t>(b), static_cast<uint32_t>(end));
   }
-  if (blockIdx.x == 0) {
+  if (tile == 0) {
     for (int b = tid; b <= a.buckets; b += kSmallThreads) a.start[b] = start[b];
     biggest = __reduce_max_sync(0xffffffffu, biggest);
     if ((tid & 31) == 0) {
@@ -1772,13 +1787,179 @@ small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr)
     }
     if (tid == 0) out.cell_start[a.num_cells] = static_cast<int32_t>(a.n);
   }
-  if (!grid_barrier(&hdr->barrier, 2, &hdr->error)) return;
+}
 
-  if (!handed_over(hdr)) {
-    bool held = true;
-    const uint32_t groups = ld_relaxed(&hdr->aux_counter[1]);
-    for (uint32_t g = blockIdx.x; g < groups; g += gridDim.x) {
-      const uint2 group = __ldcg(a.groups + g);
+// A block that waits for blocks which do not run: it counts their tiles.  A tile counted here is
+// loose: nobody holds it in registers.  Its particles' places in their buckets are left in the
+// array of indices, which the finish overwrites, and when all tiles are counted any block that
+// comes this way stores it.
+template <class Shape>
+__device__ __noinline__ bool place_loose_tiles(const SmallArgs& a, const FinishOut& out, Header* hdr,
+                                               FinishSmem<Shape>& s) {
+  constexpr uint32_t kNone = 0xffffffffu, kTaken = 0xfffffffeu;
+  const SmallTables<Shape> table(s);
+  const int tid = threadIdx.x;
+  for (;;) {
+    if (tid == 0) {
+      const int left = a.tiles - 1 - static_cast<int>(atomicAdd(&hdr->help_next, 1u));
+      s.turn = left < 0 ? kNone : claim_tile(hdr, left) ? static_cast<uint32_t>(left) : kTaken;
+    }
+    for (int b = tid; b < a.buckets; b += kSmallThreads) table.place[b] = 0;
+    __syncthreads();
+    const uint32_t tile = s.turn;
+    __syncthreads();
+    if (tile == kNone) break;
+    if (tile == kTaken) continue;
+    const int64_t first = static_cast<int64_t>(tile) * a.items * kSmallThreads + tid;
+    for (int k = 0; k < a.items; ++k) {
+      const int64_t i = first + k * kSmallThreads;
+      if (i >= a.n) break;
+      float f[6];
+      load_small(a, i, true, f);
+      const uint32_t b = small_cell(a, f) >> a.shift;
+      out.keys[i] = b;
+      out.index[i] = static_cast<int32_t>(atomicAdd(&table.place[b], 1u));
+    }
+    __syncthreads();
+    reserve_places(a, table.place);
+    for (int k = 0; k < a.items; ++k) {
+      const int64_t i = first + k * kSmallThreads;
+      if (i < a.n) out.index[i] += static_cast<int32_t>(table.place[out.keys[i]]);
+    }
+    if (tid == 0) atomicOr(&hdr->tile_loose[tile >> 5], 1u << (tile & 31));
+    arrive(&hdr->tiles_counted);
+  }
+  if (!wait_for(&hdr->tiles_counted, a.tiles, &hdr->error)) return false;
+  bool scanned = false;
+  uint32_t biggest = 0;
+  for (int w = 0; w * 32 < a.tiles;) {
+    if (tid == 0) {
+      uint32_t got = kNone;
+      for (uint32_t bits; got == kNone && (bits = ld_relaxed(&hdr->tile_loose[w])) != 0;) {
+        const uint32_t bit = bits & (0u - bits);
+        if (atomicAnd(&hdr->tile_loose[w], ~bit) & bit) got = w * 32 + __ffs(bit) - 1;
+      }
+      __threadfence();  // the tile's places were written before its bit
+      s.turn = got;
+    }
+    __syncthreads();
+    const uint32_t tile = s.turn;
+    __syncthreads();
+    if (tile == kNone) {
+      ++w;
+      continue;
+    }
+    if (!scanned) biggest = scan_totals<Shape>(a, s);
+    scanned = true;
+    const int64_t first = static_cast<int64_t>(tile) * a.items * kSmallThreads + tid;
+    for (int k = 0; k < a.items; ++k) {
+      const int64_t i = first + k * kSmallThreads;
+      if (i >= a.n) break;
+      float f[6];
+      load_small(a, i, true, f);
+      const uint32_t cell = small_cell(a, f);
+      store_small_record<Shape::kRecordWords>(
+          a, table.start[cell >> a.shift] + static_cast<uint32_t>(__ldcg(out.index + i)),
+          make_key(cell, static_cast<uint32_t>(i), a.k0, a.k1), i, f);
+    }
+    cut_groups<Shape>(a, out, hdr, table.start, biggest, static_cast<int>(tile));
+    arrive(&hdr->tiles_stored);
+  }
+  return true;
+}
+
+template <class Shape>
+__global__ void __launch_bounds__(kSmallThreads, 2)
+small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ FinishOut out,
+                  DigitPassArgs digits, Header* hdr) {
+  static_assert(Shape::kThreads == kSmallThreads, "one block size for all phases");
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
+  const SmallTables<Shape> table(s);
+  const int tid = threadIdx.x;
+  const int tile = blockIdx.x;
+  const int64_t first = static_cast<int64_t>(tile) * a.items * kSmallThreads + tid;
+
+  for (int b = tid; b < a.buckets; b += kSmallThreads) table.place[b] = 0;
+  __syncthreads();
+  float f[kSmallItems][6];
+  uint32_t key[kSmallItems], rank[kSmallItems];
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    const int64_t i = first + k * kSmallThreads;
+    load_small(a, i, k < a.items && i < a.n, f[k]);
+  }
+  // A block that starts late finds its tile claimed by another and goes on without one.  The
+  // block's first task of the finish is asked for here, long before it is needed.
+  uint32_t claimed = 0xffffffffu, next = 0;
+  if (tid == 0) {
+    claimed = atomicOr(&hdr->tile_claimed[tile >> 5], 1u << (tile & 31));
+    next = atomicAdd(&hdr->task_next, 1u);
+  }
+  bool sharing = true;
+#pragma unroll
+  for (int k = 0; k < kSmallItems; ++k) {
+    const int64_t i = first + k * kSmallThreads;
+    const uint32_t cell = small_cell(a, f[k]);
+    key[k] = make_key(cell, static_cast<uint32_t>(i), a.k0, a.k1);
+    rank[k] = rank_in_tile(table.place, cell >> a.shift, k < a.items && i < a.n, sharing);
+  }
+  const bool holds = __syncthreads_or((claimed >> (tile & 31) & 1) == 0);
+  if (holds) {
+    reserve_places(a, table.place);
+#pragma unroll
+    for (int k = 0; k < kSmallItems; ++k) rank[k] += table.place[key[k] >> (kShuffleBits + a.shift)];
+    arrive(&hdr->tiles_counted);
+  }
+  if (holds && wait_reaches(&hdr->tiles_counted, a.tiles, &hdr->error, kHelpAfterNs)) {
+    const uint32_t biggest = scan_totals<Shape>(a, s);
+#pragma unroll
+    for (int k = 0; k < kSmallItems; ++k) {
+      const int64_t i = first + k * kSmallThreads;
+      if (k < a.items && i < a.n)
+        store_small_record<Shape::kRecordWords>(
+            a, table.start[key[k] >> (kShuffleBits + a.shift)] + rank[k], key[k], i, f[k]);
+    }
+    cut_groups<Shape>(a, out, hdr, table.start, biggest, tile);
+    arrive(&hdr->tiles_stored);
+  } else {
+    if (holds) {  // lets its tile go before it helps
+#pragma unroll
+      for (int k = 0; k < kSmallItems; ++k) {
+        const int64_t i = first + k * kSmallThreads;
+        if (k < a.items && i < a.n) out.index[i] = static_cast<int32_t>(rank[k]);
+      }
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        atomicOr(&hdr->tile_loose[tile >> 5], 1u << (tile & 31));
+      }
+    }
+    if (!place_loose_tiles<Shape>(a, out, hdr, s)) return;
+  }
+
+  // The finish: tasks are the groups, and, where a bucket exceeds what a block holds, shares of
+  // the buckets.  A block's next task is asked for while it works on one.
+  if (tid == 0) s.turn = next;
+  if (!wait_for(&hdr->tiles_stored, a.tiles, &hdr->error)) return;
+  // One thread asks: thousands of warps that ask for one line queue there (606,208 particles: 2 us).
+  if (tid == 0) {
+    const uint32_t groups = ld_relaxed(&hdr->groups), max_bucket = ld_relaxed(&hdr->max_bucket);
+    s.groups = groups;
+    // No task at all where a bucket is beyond any block: the digit passes will write everything.
+    s.tasks = max_bucket > Shape::kLargestBucket ? 0
+              : max_bucket > static_cast<uint32_t>(Shape::kCapacity) ? groups + a.tiles : groups;
+  }
+  // Where there is no such group this reads what nobody uses.
+  uint2 group = __ldcg(a.groups + min(s.turn, static_cast<uint32_t>(a.buckets) - 1));
+  __syncthreads();
+  const uint32_t groups = s.groups, tasks = s.tasks;
+  uint32_t done = 0;  // tasks done here; failed ones count kFailedTask more
+  for (;; ++done) {
+    const uint32_t task = s.turn;
+    if (task >= tasks) break;
+    if (done > 0 && task < groups) group = __ldcg(a.groups + task);
+    if (task < groups) {
       const uint32_t begin = __ldcg(a.start + group.x);
       const int count = static_cast<int>(__ldcg(a.start + group.y) - begin);
       const int64_t first_cell = static_cast<int64_t>(group.x) << a.shift;
@@ -1792,17 +1973,28 @@ small_sort_kernel(SmallArgs a, FinishOut out, DigitPassArgs digits, Header* hdr)
       for (int i = tid; i < count * (Shape::kRecordWords / 2); i += kSmallThreads) to[i] = __ldcg(from + i);
       for (int i = tid; i < hist_words; i += kSmallThreads) s.hist[i] = 0;
       __syncthreads();
-      held = sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop) && held;
-    }
-    if (held && ld_relaxed(&hdr->max_bucket) > static_cast<uint32_t>(Shape::kCapacity)) {
+      if (tid == 0) next = atomicAdd(&hdr->task_next, 1u);
+      if (!sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop)) done += kFailedTask;
+    } else {
+      if (tid == 0) next = atomicAdd(&hdr->task_next, 1u);
       const RunTable t{a.records, a.start, a.start, nullptr, nullptr, 0, 1, a.buckets, a.shift};
-      held = finish_large_buckets<Shape>(s, t, out, a.num_cells, Shape::kCapacity, blockIdx.x, gridDim.x);
+      if (!finish_large_buckets<Shape>(s, t, out, a.num_cells, Shape::kCapacity, task - groups, a.tiles))
+        done += kFailedTask;
     }
-    if (!held && tid == 0) atomicExch(&hdr->use_standard, 1);
+    __syncthreads();
+    if (tid == 0) s.turn = next;
+    __syncthreads();
   }
-  if (!grid_barrier(&hdr->barrier, 3, &hdr->error)) return;
-  if (!handed_over(hdr)) return;
-  digit_passes_in_grid<kSmallThreads>(digits, *reinterpret_cast<PassSmem<kSmallThreads>*>(smem_raw), hdr, 3);
+  if (done >= kFailedTask && tid == 0) atomicExch(&hdr->use_standard, 1);
+  arrive(&hdr->tasks_done, done);
+  uint32_t seen = 0;
+  if (!wait_for(&hdr->tasks_done, tasks, &hdr->error, kWaitLimitNs, kFailedTask - 1, &seen)) return;
+  if (!__syncthreads_or(tid == 0 && seen >= kFailedTask) && tasks > 0) return;
+  const uint32_t items = a.tiles;
+  run_phases(hdr, items, digit_phases(digits), [&](uint32_t phase, uint32_t item) {
+    return digit_phase<kSmallThreads>(digits, *reinterpret_cast<PassSmem<kSmallThreads>*>(smem_raw),
+                                      hdr, phase, item, items);
+  });
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -1869,10 +2061,13 @@ constexpr int64_t kMaxSmallShapeBuckets = 32 * 1024;
 int64_t g_small_shape_buckets = kMaxSmallShapeBuckets;  // tuning knob, see set_small_shape_buckets
 
 // Blocks of the one-launch sort, and what it takes: a tile per resident block.
-int64_t small_call_particles() { return 2 * static_cast<int64_t>(sm_count()) * kSmallThreads * kSmallItems; }
+int small_call_most_blocks() { return std::min(2 * sm_count(), kMaxTiles); }
+int64_t small_call_particles() {
+  return static_cast<int64_t>(small_call_most_blocks()) * kSmallThreads * kSmallItems;
+}
 int small_call_blocks(int64_t n, int64_t buckets) {
   return static_cast<int>(std::max<int64_t>(
-      1, std::min<int64_t>(2 * sm_count(), std::max((n + kSmallThreads - 1) / kSmallThreads, buckets / 8))));
+      1, std::min<int64_t>(small_call_most_blocks(), std::max((n + kSmallThreads - 1) / kSmallThreads, buckets / 8))));
 }
 
 // Up to where slots are reserved tile by tile.
@@ -2046,6 +2241,8 @@ cudaError_t launch_finish_large(const RunTable& t, const SortArgs& a, const Fini
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+int limited(int blocks, int most) { return most > 0 ? std::min(blocks, most) : blocks; }
+
 template <class Shape>
 cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
                         uint32_t group_capacity) {
@@ -2056,19 +2253,10 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
   e = cudaFuncSetAttribute(bucket_tail_kernel<Shape>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return e;
-  cudaLaunchAttribute cooperative{};
-  cooperative.id = cudaLaunchAttributeCooperative;
-  cooperative.val.cooperative = 1;
-  cudaLaunchConfig_t config{};
-  // One block per multiprocessor (all resident at once), fewer where there is little to do.
-  config.gridDim = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(sm_count(), a.n / 2048)));
-  config.blockDim = Shape::kThreads;
-  config.dynamicSmemBytes = kSmem;
-  config.stream = a.stream;
-  config.attrs = &cooperative;
-  config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, bucket_tail_kernel<Shape>, t, a.num_cells, out, hdr,
-                            group_capacity, digits);
+  // One block per multiprocessor, fewer where there is little to do.
+  const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sm_count(), a.n / 2048)));
+  return launch_chained<true>(bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks), Shape::kThreads,
+                              kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity, digits);
 }
 
 template <int ITEMS>
@@ -2106,7 +2294,7 @@ namespace {
 template <class Shape>
 cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLayout& l) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<kSmallThreads>)));
-  static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two blocks must share a multiprocessor");
+  static_assert(2 * (kSmem + 1024 + 64) <= 228 * 1024, "two blocks must share a multiprocessor");
   auto* base = static_cast<unsigned char*>(a.workspace);
   DigitPassArgs digits;
   cudaError_t e = digit_pass_args(a, &digits);
@@ -2126,6 +2314,7 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
   s.group_shift = std::max(0, log2_floor(Shape::kMaxCells) - p.shift);
   s.items = static_cast<int>((a.n + static_cast<int64_t>(blocks) * kSmallThreads - 1) /
                              (static_cast<int64_t>(blocks) * kSmallThreads));
+  s.tiles = blocks;
   s.window = small_call_window(a.n, p.buckets, Shape::kCapacity);
   s.count = reinterpret_cast<uint32_t*>(base + l.count_off);
   s.start = reinterpret_cast<uint32_t*>(base + l.start_off);
@@ -2133,19 +2322,10 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
   s.records = reinterpret_cast<uint32_t*>(base + l.records_off);
   const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
                       a.vs, a.padded_sorted};
-  cudaLaunchAttribute cooperative{};
-  cooperative.id = cudaLaunchAttributeCooperative;
-  cooperative.val.cooperative = 1;
-  cudaLaunchConfig_t config{};
-  config.gridDim = static_cast<unsigned>(blocks);
-  config.blockDim = kSmallThreads;
-  config.dynamicSmemBytes = kSmem;
-  config.stream = a.stream;
-  config.attrs = &cooperative;
-  config.numAttrs = 1;
+  small_sort_kernel<Shape><<<limited(blocks, a.most_blocks), kSmallThreads, kSmem, a.stream>>>(
+      s, out, digits, reinterpret_cast<Header*>(base));
   count_launches(1);
-  return cudaLaunchKernelEx(&config, small_sort_kernel<Shape>, s, out, digits,
-                            reinterpret_cast<Header*>(base));
+  return cudaGetLastError();
 }
 }  // namespace
 

@@ -128,7 +128,7 @@ constexpr int kBoundsThreads = 256;
 __global__ void __launch_bounds__(kBoundsThreads)
 cell_bounds_kernel(const uint32_t* keys, int64_t n, int64_t num_cells, int32_t* cell_start) {
   chain_begin();
-  cell_bounds<kBoundsThreads>(keys, n, num_cells, cell_start);
+  cell_bounds<kBoundsThreads>(keys, n, num_cells, cell_start, blockIdx.x, gridDim.x);
 }
 
 __global__ void __launch_bounds__(kBoundsThreads)
@@ -389,7 +389,7 @@ cudaError_t digit_pass_args(const SortArgs& a, DigitPassArgs* out) {
   d.padded_sorted = a.padded_sorted;
   d.passes = l.passes;
   d.tiles = static_cast<uint32_t>(l.tiles);
-  // The first words of the header (error, hand-over flag, barrier) stay as they are.
+  // The first words of the header (error, hand-over flag, phases) stay as they are.
   d.clear_from = reinterpret_cast<uint32_t*>(base + kHeaderKept);
   d.clear_words = static_cast<int64_t>((l.keys_alt_off - kHeaderKept) / sizeof(uint32_t));
   d.status = reinterpret_cast<uint32_t*>(base + l.status_off);
