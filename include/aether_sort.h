@@ -368,6 +368,16 @@ size_t AetherSortProbeLookbackWorkspaceBytes(void);
 int AetherSortProbeLookbackGiveUp(void* workspace, size_t workspace_bytes, uint32_t poll_limit,
                                   void* stream);
 
+/* Test hook for the waits between the phases of a kernel (one-launch sort, and the kernel behind
+ * the finish of larger calls): each of `blocks` blocks, at most two per multiprocessor, waits for
+ * one block more than there are, gives up after `limit_ns` nanoseconds (at most two seconds, the
+ * limit of those kernels), records code 4 in the workspace header (at least 5 KiB) and adds one to
+ * *returned (device memory).  `shared_bytes` (at most 200 KiB): shared memory each block keeps
+ * meanwhile. */
+int AetherSortProbeWaitGiveUp(void* workspace, size_t workspace_bytes, int blocks,
+                              size_t shared_bytes, uint64_t limit_ns, int32_t* returned,
+                              void* stream);
+
 /* Test hook (no counterpart in the reference): AetherSortAndGatherParticles, or without sorted
  * outputs AetherSortParticlesByCell, with at most `most_blocks` thread blocks in the kernels whose
  * blocks share work in phases (the sort of small calls in one launch, and the kernel behind the

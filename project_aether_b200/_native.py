@@ -121,6 +121,8 @@ _SIGNATURES = {
                                                 ctypes.c_size_t, _P]),
     'AetherSortProbeLookbackWorkspaceBytes': (ctypes.c_size_t, []),
     'AetherSortProbeLookbackGiveUp': (ctypes.c_int, [_P, ctypes.c_size_t, ctypes.c_uint32, _P]),
+    'AetherSortProbeWaitGiveUp': (ctypes.c_int, [_P, ctypes.c_size_t, ctypes.c_int, ctypes.c_size_t,
+                                                 ctypes.c_uint64, _P, _P]),
     'AetherSortSetStageTiming': (ctypes.c_int, [ctypes.c_int]),
     'AetherSortStageCount': (ctypes.c_int, []),
     'AetherSortStageName': (ctypes.c_char_p, [ctypes.c_int]),

@@ -201,6 +201,15 @@ extern "C" int AetherSortProbeLookbackGiveUp(void* workspace, size_t workspace_b
                                 static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int AetherSortProbeWaitGiveUp(void* workspace, size_t workspace_bytes, int blocks,
+                                         size_t shared_bytes, uint64_t limit_ns, int32_t* returned,
+                                         void* stream) {
+  if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || !returned)
+    return cudaErrorInvalidValue;
+  return wait_give_up_probe(workspace, workspace_bytes, blocks, shared_bytes, limit_ns, returned,
+                            static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int AetherSortAbiVersion(void) { return 1; }
 
 extern "C" size_t AetherSortWorkspaceBytes(int64_t n, int64_t num_cells, int with_payload) {

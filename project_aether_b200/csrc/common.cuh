@@ -310,6 +310,13 @@ cudaError_t digit_pass_args(const SortArgs& a, DigitPassArgs* out);
 // path; `workspace` needs lookback_probe_workspace_bytes() bytes.
 cudaError_t lookback_give_up_probe(void* workspace, size_t workspace_bytes, uint32_t poll_limit,
                                    cudaStream_t stream);
+// `blocks` blocks of which each waits, at most `limit_ns`, for one block more; each that gives up
+// adds one to *returned.  For tests of the give-up path of the waits between phases, and, with
+// `shared_bytes` of shared memory per block, of what runs beside a kernel that stays a while.
+constexpr int kProbeMostShared = 200 * 1024;
+cudaError_t wait_give_up_probe(void* workspace, size_t workspace_bytes, int blocks,
+                               size_t shared_bytes, uint64_t limit_ns, int32_t* returned,
+                               cudaStream_t stream);
 int64_t lookback_probe_particles();
 size_t lookback_probe_workspace_bytes();
 

@@ -367,6 +367,30 @@ cudaError_t lookback_give_up_probe(void* workspace, size_t workspace_bytes, uint
   return cudaGetLastError();
 }
 
+// A wait that runs out: every block counts itself in and waits for one more block than there are.
+__global__ void wait_give_up_kernel(Header* hdr, unsigned long long limit_ns, int32_t* returned) {
+  arrive(&hdr->phase_done);
+  if (!wait_for(&hdr->phase_done, gridDim.x + 1, &hdr->error, limit_ns) && threadIdx.x == 0)
+    atomicAdd(returned, 1);
+}
+
+cudaError_t wait_give_up_probe(void* workspace, size_t workspace_bytes, int blocks,
+                               size_t shared_bytes, uint64_t limit_ns, int32_t* returned,
+                               cudaStream_t stream) {
+  if (workspace_bytes < sizeof(Header) || blocks < 1 || blocks > 2 * sm_count() ||
+      shared_bytes > kProbeMostShared || limit_ns > kWaitLimitNs)
+    return cudaErrorInvalidValue;
+  cudaError_t e = cudaMemsetAsync(workspace, 0, sizeof(Header), stream);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(wait_give_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kProbeMostShared);
+  if (e != cudaSuccess) return e;
+  wait_give_up_kernel<<<blocks, 64, shared_bytes, stream>>>(static_cast<Header*>(workspace),
+                                                            limit_ns, returned);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t digit_pass_args(const SortArgs& a, DigitPassArgs* out) {
   const StandardLayout l = standard_layout(a.n, a.key_bits);
   if (a.workspace_bytes < l.total) return cudaErrorInvalidValue;

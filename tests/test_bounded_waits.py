@@ -20,7 +20,7 @@ from project_aether_b200.particle_sort import native_grid
 
 pytestmark = pytest.mark.gpu
 
-ERR_LOOKBACK_TIMEOUT, ERR_RECEIVE_OVERFLOW = 1, 5
+ERR_LOOKBACK_TIMEOUT, ERR_PHASE_TIMEOUT, ERR_RECEIVE_OVERFLOW = 1, 4, 5
 
 
 def test_lookback_gives_up_after_its_poll_limit_and_reports(cuda):
@@ -48,6 +48,37 @@ def test_lookback_gives_up_after_its_poll_limit_and_reports(cuda):
         assert int(r.cell_counts.sum()) == 50_000
         # A workspace that is too small is refused before any launch.
         assert lib.AetherSortProbeLookbackGiveUp(ws.data_ptr(), 1024, 8, stream) == 1
+
+
+@pytest.mark.parametrize('blocks', [1, 40])
+def test_wait_between_phases_gives_up_after_its_limit_and_reports(cuda, blocks):
+    lib = _native.load_library()
+    with torch.cuda.device(cuda):
+        ws = torch.empty(8192, dtype=torch.uint8, device=cuda)
+        returned = torch.zeros(1, dtype=torch.int32, device=cuda)
+        stream = ctypes.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+        status = ctypes.c_int32(-1)
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        _native.check(lib.AetherSortProbeWaitGiveUp(ws.data_ptr(), ws.numel(), blocks, 0, 1_000_000,
+                                                    returned.data_ptr(), stream),
+                      'AetherSortProbeWaitGiveUp')
+        _native.check(lib.AetherSortReadStatus(ws.data_ptr(), stream, ctypes.byref(status)),
+                      'AetherSortReadStatus')
+        elapsed = time.perf_counter() - t0
+        assert status.value == ERR_PHASE_TIMEOUT
+        assert int(returned) == blocks, 'every block must leave'
+        assert elapsed < 0.5, 'the wait must run out within milliseconds'
+        # An ordinary sort afterwards is clean.
+        grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (16, 16, 16))
+        x, y, z = (torch.rand(50_000, device=cuda) for _ in range(3))
+        r = pa.sort_particles_by_cell(x, y, z, grid, 1)
+        assert pa.last_sort_status(cuda) == 0
+        assert int(r.cell_counts.sum()) == 50_000
+        # Too small a workspace, too many blocks, too long a wait: refused before any launch.
+        for bad in ((1024, 1, 0, 1000), (8192, 0, 0, 1000), (8192, 10_000, 0, 1000),
+                    (8192, 1, 1 << 20, 1000), (8192, 1, 0, 3_000_000_000)):
+            assert lib.AetherSortProbeWaitGiveUp(ws.data_ptr(), *bad, returned.data_ptr(), stream) == 1
 
 
 def test_exchange_refuses_to_overflow_a_receive_buffer(cuda):

@@ -60,3 +60,33 @@ def test_any_number_of_blocks_finishes_the_call(cuda, n, edge, density, most_blo
         assert handed_over == (density == 'cell' and n > 100_000)
         for g, w in zip(got, (*want.order, *want.positions, want.velocity)):
             assert torch.equal(g, w)
+
+
+# One launch, and the kernel behind the finish of a middling call.
+@pytest.mark.parametrize('n', [5_000, 600_000, 1_200_000])
+def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
+    """A kernel of another stream keeps one multiprocessor's shared memory for 200 ms."""
+    lib = _native.load_library()
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (32, 32, 32))
+    pos = [torch.rand(n, device=cuda) for _ in range(3)]
+    vel = torch.randn((3, n), device=cuda)
+    beside, stream = torch.cuda.Stream(cuda), torch.cuda.Stream(cuda)
+    scratch = torch.empty(8192, dtype=torch.uint8, device=cuda)
+    returned = torch.zeros(1, dtype=torch.int32, device=cuda)
+    with torch.cuda.stream(stream):  # the stream's workspace exists
+        want = pa.sort_and_gather_particles(*pos, vel, grid, 3)
+    torch.cuda.synchronize()
+    _native.check(lib.AetherSortProbeWaitGiveUp(scratch.data_ptr(), scratch.numel(), 1, 200 * 1024,
+                                                200_000_000, returned.data_ptr(), beside.cuda_stream),
+                  'AetherSortProbeWaitGiveUp')
+    ended = torch.cuda.Event()
+    ended.record(beside)
+    with torch.cuda.stream(stream):
+        got = pa.sort_and_gather_particles(*pos, vel, grid, 3)
+        stream.synchronize()
+    assert not ended.query(), 'the call waited for the kernel beside it'
+    torch.cuda.synchronize()
+    assert int(returned) == 1
+    for g, w in zip((*got.order, *got.positions, got.velocity),
+                    (*want.order, *want.positions, want.velocity)):
+        assert torch.equal(g, w)
