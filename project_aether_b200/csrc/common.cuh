@@ -58,10 +58,11 @@ struct alignas(16) Header {
   int32_t use_standard;       // bucketed path: 1 when it handed over to the digit passes
   uint32_t phase_ticket, phase_done;  // run_phases: pieces handed out, pieces done
   uint32_t max_bucket;        // bucketed path: largest bucket seen
+  uint32_t redo_groups;       // groups whose counters wrapped, to be finished bucket by bucket
   // One-launch sort: tiles counted and stored, next tile to look at for a block that helps,
   // groups cut, next task and tasks done of the finish.
   uint32_t tiles_counted, tiles_stored, help_next, groups, task_next, tasks_done;
-  uint32_t kept_pad[5];
+  uint32_t kept_pad[4];
   uint32_t tile_claimed[kMaxTiles / 32], tile_loose[kMaxTiles / 32];  // one bit per tile
   uint32_t tile_counter[kMaxPasses];  // ticket dispenser of each digit pass
   uint32_t aux_counter[8];

@@ -1012,6 +1012,9 @@ struct FinishShape {
   // A group spans at most this many cells: its low key (cell in group, shuffle bits) then has
   // at most LOW_BITS + MAX_DROP bits, of which the tie step may take MAX_DROP.
   static constexpr int kMaxCells = 1 << (LOW_BITS + MAX_DROP - kShuffleBits);
+  // A run of cells cut from a bucket: few enough that every cell keeps 32 counters (5120 records on
+  // 32 counters are 160 each; 16 wrap from some 3500 records on).
+  static constexpr int kRunCells = 1 << (LOW_BITS + (MAX_DROP < 2 ? MAX_DROP : 2) - kShuffleBits);
   static constexpr uint32_t kLargestBucket = static_cast<uint32_t>(kMaxSegments) * CAPACITY;
   static_assert(kWordsPerThread % 8 == 0, "the counter scan reads eight words at a time");
   static_assert(kHistWords * 3 / 2 >= CAPACITY, "the tie step lays a word per record over the counters");
@@ -1334,6 +1337,7 @@ struct RunTable {
   int chunks;
   int buckets;
   int shift;                     // a bucket is 2^shift cells
+  uint32_t* redo;                // room for the groups whose counters wrapped, or null
 };
 
 // A bucket with more records than shared memory holds (a dense region: the
@@ -1372,7 +1376,8 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
     for (int c = 0; c < cells_here && ok; ++c) {
       const uint32_t here = cell_count[c];
       if (here > static_cast<uint32_t>(kCapacity)) ok = false;
-      if (load + here > static_cast<uint32_t>(kCapacity)) {  // close the run before cell c
+      if (load + here > static_cast<uint32_t>(kCapacity) ||
+          c - s.seg_first[segments] >= Shape::kRunCells) {  // close the run before cell c
         before += load;
         load = 0;
         ++segments;
@@ -1506,12 +1511,12 @@ __global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_device,
                      int64_t num_cells, FinishOut out, Header* __restrict__ hdr) {
   chain_begin();
+  const uint32_t groups = *t.group_count;
   if (handed_over(hdr)) return;
   constexpr int kThreads = Shape::kThreads;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t groups = *t.group_count;
   if (blockIdx.x == 0 && tid == 0)
     out.cell_start[num_cells] = n_on_device ? static_cast<int32_t>(*n_on_device) : static_cast<int32_t>(n);
   const uint32_t stride = gridDim.x;
@@ -1563,8 +1568,9 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
       copy_wait_all();
       return;
     }
-    if (!sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop)) {
-      if (tid == 0) hdr->use_standard = 1;
+    if (!sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop) && tid == 0) {
+      if (t.redo) t.redo[atomicAdd(&hdr->redo_groups, 1u)] = g;
+      else hdr->use_standard = 1;
     }
     // s.raw is free (sort_staged ended with a barrier): the next group's records, which L2
     // holds by now, can come in, and the group after it is asked into L2.
@@ -1580,16 +1586,16 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
   }
 }
 
-// The buckets the kernel above skipped: those with more records than its shared
-// memory holds.  `block` of `blocks` takes every blocks-th bucket; false if one of its
-// buckets cannot be finished at all.
+// Buckets first, first + step, ... below `last` that hold at least `at_least` records, one by one:
+// those the kernel above skipped, with more records than its shared memory holds, and those of a
+// group whose counters wrapped.  False if one of them cannot be finished at all.
 template <class Shape>
-__device__ bool finish_large_buckets(FinishSmem<Shape>& s, const RunTable& t, const FinishOut& out,
-                                     int64_t num_cells, uint32_t capacity, int block, int blocks) {
-  for (int b = block; b < t.buckets; b += blocks) {
+__device__ bool finish_buckets(FinishSmem<Shape>& s, const RunTable& t, const FinishOut& out,
+                               int64_t num_cells, int first, int last, int step, int at_least) {
+  for (int b = first; b < last; b += step) {
     const uint32_t begin = t.bucket_start[b], end = t.bucket_start[b + 1];
     const int count = static_cast<int>(end - begin);
-    if (static_cast<uint32_t>(count) <= capacity) continue;
+    if (count < at_least) continue;
     const int64_t first_cell = static_cast<int64_t>(b) << t.shift;
     const int cells_here = static_cast<int>(
         min(static_cast<long long>(1) << t.shift, static_cast<long long>(num_cells - first_cell)));
@@ -1606,13 +1612,14 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
   chain_begin();
   if (handed_over(hdr) || hdr->max_bucket <= capacity) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  if (!finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
-                                   num_cells, capacity, blockIdx.x, gridDim.x) &&
+  if (!finish_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out, num_cells,
+                             blockIdx.x, t.buckets, gridDim.x, capacity + 1) &&
       threadIdx.x == 0)
     hdr->use_standard = 1;
 }
 
-// Behind the finish kernel of an ordinary call: the oversized buckets, then, when the call was
+// Behind the finish kernel of an ordinary call: the oversized buckets and the groups whose counters
+// wrapped (calls without payload, whose sparse groups have 16 counters per cell), then, when the call was
 // handed over, the whole digit-pass sort.  Usually there is nothing to do and every block returns
 // after a look at the header.  What bounds it is then the launch itself: as the separate kernels
 // it replaces (the oversized buckets, a clear, the keys, up to four digit passes, two table
@@ -1623,7 +1630,8 @@ __global__ void __launch_bounds__(Shape::kThreads, 1)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
                    DigitPassArgs digits) {
   chain_begin();
-  if (!handed_over(hdr) && hdr->max_bucket <= capacity) return;
+  const bool all_done = hdr->max_bucket <= capacity && hdr->redo_groups == 0;
+  if (!handed_over(hdr) && all_done) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const uint32_t items = gridDim.x;
   run_phases(hdr, items, 1 + digit_phases(digits), [&](uint32_t phase, uint32_t item) {
@@ -1634,11 +1642,13 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
                              phase - 1, item, items);
     // A block that comes late may see another block's hand-over and skip its buckets: the digit
     // passes then write everything.
-    if (!standard &&
-        !finish_large_buckets<Shape>(*reinterpret_cast<FinishSmem<Shape>*>(smem_raw), t, out,
-                                     num_cells, capacity, item, items) &&
-        threadIdx.x == 0)
-      atomicExch(&hdr->use_standard, 1);
+    FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
+    bool good = standard || finish_buckets<Shape>(s, t, out, num_cells, item, t.buckets, items, capacity + 1);
+    for (uint32_t r = item; !standard && good && r < hdr->redo_groups; r += items) {
+      const uint32_t* row0 = t.tables + static_cast<size_t>(t.redo[r]) * 2 * t.row_words;
+      good = finish_buckets<Shape>(s, t, out, num_cells, row0[t.chunks + 1], row0[t.chunks + 2], 1, 0);
+    }
+    if (!good && threadIdx.x == 0) atomicExch(&hdr->use_standard, 1);
     return true;
   });
 }
@@ -1958,8 +1968,11 @@ small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ F
   for (;; ++done) {
     const uint32_t task = s.turn;
     if (task >= tasks) break;
-    if (done > 0 && task < groups) group = __ldcg(a.groups + task);
-    if (task < groups) {
+    const RunTable t{a.records, a.start, a.start, nullptr, nullptr, 0, 1, a.buckets, a.shift, nullptr};
+    int bucket = static_cast<int>(task - groups), last = a.buckets, step = a.tiles, at_least = Shape::kCapacity + 1;
+    bool one_by_one = task >= groups;
+    if (!one_by_one) {
+      if (done > 0) group = __ldcg(a.groups + task);
       const uint32_t begin = __ldcg(a.start + group.x);
       const int count = static_cast<int>(__ldcg(a.start + group.y) - begin);
       const int64_t first_cell = static_cast<int64_t>(group.x) << a.shift;
@@ -1974,13 +1987,13 @@ small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ F
       for (int i = tid; i < hist_words; i += kSmallThreads) s.hist[i] = 0;
       __syncthreads();
       if (tid == 0) next = atomicAdd(&hdr->task_next, 1u);
-      if (!sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop)) done += kFailedTask;
-    } else {
-      if (tid == 0) next = atomicAdd(&hdr->task_next, 1u);
-      const RunTable t{a.records, a.start, a.start, nullptr, nullptr, 0, 1, a.buckets, a.shift};
-      if (!finish_large_buckets<Shape>(s, t, out, a.num_cells, Shape::kCapacity, task - groups, a.tiles))
-        done += kFailedTask;
+      one_by_one = !sort_staged<Shape>(s, out, count, begin, first_cell, cells_here, drop);
+      bucket = group.x; last = group.y; step = 1; at_least = 0;
+    } else if (tid == 0) {
+      next = atomicAdd(&hdr->task_next, 1u);
     }
+    if (one_by_one && !finish_buckets<Shape>(s, t, out, a.num_cells, bucket, last, step, at_least))
+      done += kFailedTask;
     __syncthreads();
     if (tid == 0) s.turn = next;
     __syncthreads();
@@ -2458,7 +2471,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
                       a.vs, a.padded_sorted};
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
-                   table_row_words(l.chunks), l.chunks, buckets, p.shift};
+                   table_row_words(l.chunks), l.chunks, buckets, p.shift, p.keys_only ? cursor : nullptr};
   e = p.keys_only      ? launch_finish<FinishKeys>(t, a, out, hdr)
       : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr)
                        : launch_finish<FinishLarge>(t, a, out, hdr);
@@ -2618,7 +2631,7 @@ cudaError_t sliced_sort_finish(const SortArgs& a, int64_t plan_n, const SliceSeg
   const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
                       a.vs, a.padded_sorted};
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
-                   table_row_words(l.chunks), l.chunks, buckets, p.shift};
+                   table_row_words(l.chunks), l.chunks, buckets, p.shift, nullptr};
   e = p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, n_on_device)
                      : launch_finish<FinishLarge>(t, a, out, hdr, n_on_device);
   if (e == cudaSuccess) e = launch_finish_large(t, a, out, hdr, group_capacity);

@@ -107,3 +107,31 @@ def test_many_blocks_decide_on_the_hand_over_together(cuda, n, edge, cells):
         same = torch.from_numpy(so.shuffle_bits(n, seed) == 9).to(cuda)
         _crowd(pos, same, int(same.sum()) // 600, edge, cuda)
         assert _sorted_as_by_the_oracle(pos, vel, grid, seed, cuda) == (True, True)
+
+
+# In a grid of one particle per cell a bucket of a call without payload spans 1024 cells, on 16
+# byte counters each: one cell of some 3500 records or more wraps one of them.  One launch; a
+# bucket too large for a group; a group.  The bucket is then finished in runs of fewer cells.
+@pytest.mark.parametrize('n,edge,crowd', [(200_003, 96, 4_600), (900_001, 128, 5_120), (2_400_011, 128, 3_900)])
+def test_dense_cells_of_a_sparse_grid_stay_off_the_digit_passes(cuda, n, edge, crowd):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (edge,) * 3)
+    pos, vel = _state(n, cuda, n)
+    # Three cells in different buckets; the particles that fell into them before move one cell on.
+    middle = (torch.floor(torch.tensor([0.2, 0.5, 0.8], device=cuda) * edge) + 0.5) / edge
+    chosen = torch.arange(n, device=cuda) < 3 * crowd
+    there = torch.zeros(n, dtype=torch.bool, device=cuda)
+    for m in middle:
+        there |= sum(((p * edge).long() == (m * edge).long()).long() for p in pos) == 3
+    pos[0][there] += 1.0 / edge
+    for p in pos:
+        p[chosen] = middle[torch.arange(3 * crowd, device=cuda) % 3]
+    order = pa.sort_particles_by_cell(*pos, grid, 11)
+    assert pa.last_sort_status(cuda) == 0
+    assert not pa.last_sort_used_digit_passes(cuda)
+    assert int(order.cell_counts.max()) == crowd
+    want = so.c_sort_particles(*(t.cpu().numpy() for t in pos), vel.cpu().numpy(),
+                               so.Grid(grid.lo, grid.hi, grid.cells), 11)[0]
+    np.testing.assert_array_equal(order.keys.cpu().numpy().view(np.uint32), want.keys)
+    np.testing.assert_array_equal(order.particle_index.cpu().numpy(), want.particle_index)
+    np.testing.assert_array_equal(order.cell_counts.cpu().numpy(), want.cell_counts)
+    np.testing.assert_array_equal(order.cell_start.cpu().numpy(), want.cell_start)
