@@ -1347,10 +1347,12 @@ struct RunTable {
 // reads from global memory once per run) and sorts them like a small group.
 // Returns false if it cannot (a single cell larger than shared memory, too many
 // runs, or a wrapped byte counter): the call then goes to the digit passes.
-template <class Shape>
+// `record_words`: from one record to the next; Shape's words of a record are its first.
+// `after(first, count)`: what is left to do for these output slots when keys and indices stand.
+template <class Shape, class After>
 __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, const RunTable& t,
                                     int b, uint32_t begin, int count, int64_t first_cell,
-                                    int cells_here) {
+                                    int cells_here, int record_words, After after) {
   constexpr int kThreads = Shape::kThreads, kCapacity = Shape::kCapacity;
   const int tid = threadIdx.x;
   uint32_t* cell_count = s.hist;  // one word per cell; s.hist is free until a run is sorted
@@ -1361,7 +1363,7 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
     const size_t entry = static_cast<size_t>(c) * t.buckets + b;
     const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
     for (uint32_t i = tid; i < length; i += kThreads) {
-      const uint32_t key = __ldcg(t.records + static_cast<size_t>(start + i) * Shape::kRecordWords);
+      const uint32_t key = __ldcg(t.records + static_cast<size_t>(start + i) * record_words);
       atomicAdd(&cell_count[(key >> kShuffleBits) - static_cast<uint32_t>(first_cell)], 1u);
     }
   }
@@ -1413,7 +1415,7 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
       const size_t entry = static_cast<size_t>(c) * t.buckets + b;
       const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
       for (uint32_t i = tid; i < length; i += kThreads) {
-        const uint32_t* rec = t.records + static_cast<size_t>(start + i) * Shape::kRecordWords;
+        const uint32_t* rec = t.records + static_cast<size_t>(start + i) * record_words;
         const uint2 lo = __ldcg(reinterpret_cast<const uint2*>(rec));
         const int cell = static_cast<int>((lo.x >> kShuffleBits) - static_cast<uint32_t>(first_cell));
         if (cell >= c0 && cell < c1) {
@@ -1434,6 +1436,7 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
     if (!consistent) return false;
     if (!sort_staged<Shape>(s, out, seg_count, begin + seg_begin, first_cell + c0, c1 - c0, drop))
       return false;
+    after(begin + seg_begin, seg_count);
   }
   return true;
 }
@@ -1589,9 +1592,10 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
 // Buckets first, first + step, ... below `last` that hold at least `at_least` records, one by one:
 // those the kernel above skipped, with more records than its shared memory holds, and those of a
 // group whose counters wrapped.  False if one of them cannot be finished at all.
-template <class Shape>
+template <class Shape, class After>
 __device__ bool finish_buckets(FinishSmem<Shape>& s, const RunTable& t, const FinishOut& out,
-                               int64_t num_cells, int first, int last, int step, int at_least) {
+                               int64_t num_cells, int first, int last, int step, int at_least,
+                               int record_words, After after) {
   for (int b = first; b < last; b += step) {
     const uint32_t begin = t.bucket_start[b], end = t.bucket_start[b + 1];
     const int count = static_cast<int>(end - begin);
@@ -1599,9 +1603,16 @@ __device__ bool finish_buckets(FinishSmem<Shape>& s, const RunTable& t, const Fi
     const int64_t first_cell = static_cast<int64_t>(b) << t.shift;
     const int cells_here = static_cast<int>(
         min(static_cast<long long>(1) << t.shift, static_cast<long long>(num_cells - first_cell)));
-    if (!finish_large_bucket<Shape>(s, out, t, b, begin, count, first_cell, cells_here)) return false;
+    if (!finish_large_bucket<Shape>(s, out, t, b, begin, count, first_cell, cells_here, record_words, after))
+      return false;
   }
   return true;
+}
+template <class Shape>
+__device__ bool finish_buckets(FinishSmem<Shape>& s, const RunTable& t, const FinishOut& out,
+                               int64_t num_cells, int first, int last, int step, int at_least) {
+  return finish_buckets<Shape>(s, t, out, num_cells, first, last, step, at_least, Shape::kRecordWords,
+                               [](uint32_t, int) {});
 }
 
 // Behind the finish kernel of the multi-GPU form, which has no digit passes to hand over to.
@@ -1668,6 +1679,10 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
 constexpr int kSmallThreads = 512;
 constexpr int kSmallItems = 4;
 constexpr int kSmallMostBuckets = 2048;
+// Buckets that are finished one by one are sorted by key and index only, whatever the call: the
+// shape of calls without payload holds 5120 such records where the small shape holds 2560 with
+// payload.  A cell with more than 2560 particles would otherwise take the call to the digit passes.
+using FinishApart = FinishKeys;
 constexpr uint32_t kFailedTask = 1u << 16;  // in tasks_done, above the number of tasks
 static_assert(2 * (kSmallMostBuckets + kMaxTiles) < kFailedTask, "two counts in a word");
 constexpr unsigned long long kHelpAfterNs = 50000;  // launch skew of a full grid: a few us
@@ -1726,6 +1741,25 @@ __device__ __forceinline__ void load_small(const SmallArgs& a, int64_t i, bool o
   f[3] = ok && a.v ? a.v[i] : 0.f;
   f[4] = ok && a.v ? a.v[a.padded + i] : 0.f;
   f[5] = ok && a.v ? a.v[2 * a.padded + i] : 0.f;
+}
+
+// The payload of output slots whose indices this very thread has written (sort_staged deals the
+// slots out alike), from the inputs.
+__device__ __forceinline__ void gather_small(const SmallArgs& a, const FinishOut& out, uint32_t from, int count) {
+  for (int d = threadIdx.x; d < count; d += kSmallThreads) {
+    const size_t o = static_cast<size_t>(from) + d;
+    float f[6];
+    load_small(a, out.index[o], true, f);
+    small_cell(a, f);
+    out.xs[o] = f[0];
+    out.ys[o] = f[1];
+    out.zs[o] = f[2];
+    if (out.vs) {
+      out.vs[o] = f[3];
+      out.vs[out.padded_sorted + o] = f[4];
+      out.vs[2 * out.padded_sorted + o] = f[5];
+    }
+  }
 }
 
 // One add per bucket and tile: a tile's counts become its first places in the buckets.
@@ -1793,7 +1827,7 @@ __device__ __forceinline__ void cut_groups(const SmallArgs& a, const FinishOut& 
     biggest = __reduce_max_sync(0xffffffffu, biggest);
     if ((tid & 31) == 0) {
       atomicMax(&hdr->max_bucket, biggest);
-      if (biggest > Shape::kLargestBucket) atomicExch(&hdr->use_standard, 1);
+      if (biggest > FinishApart::kLargestBucket) atomicExch(&hdr->use_standard, 1);
     }
     if (tid == 0) out.cell_start[a.num_cells] = static_cast<int32_t>(a.n);
   }
@@ -1882,7 +1916,9 @@ template <class Shape>
 __global__ void __launch_bounds__(kSmallThreads, 2)
 small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ FinishOut out,
                   DigitPassArgs digits, Header* hdr) {
-  static_assert(Shape::kThreads == kSmallThreads, "one block size for all phases");
+  static_assert(Shape::kThreads == kSmallThreads && FinishApart::kThreads == kSmallThreads,
+                "one block size for all phases");
+  static_assert(sizeof(FinishSmem<FinishApart>) <= sizeof(FinishSmem<Shape>), "shared memory");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
   const SmallTables<Shape> table(s);
@@ -1957,7 +1993,7 @@ small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ F
     const uint32_t groups = ld_relaxed(&hdr->groups), max_bucket = ld_relaxed(&hdr->max_bucket);
     s.groups = groups;
     // No task at all where a bucket is beyond any block: the digit passes will write everything.
-    s.tasks = max_bucket > Shape::kLargestBucket ? 0
+    s.tasks = max_bucket > FinishApart::kLargestBucket ? 0
               : max_bucket > static_cast<uint32_t>(Shape::kCapacity) ? groups + a.tiles : groups;
   }
   // Where there is no such group this reads what nobody uses.
@@ -1992,7 +2028,12 @@ small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ F
     } else if (tid == 0) {
       next = atomicAdd(&hdr->task_next, 1u);
     }
-    if (one_by_one && !finish_buckets<Shape>(s, t, out, a.num_cells, bucket, last, step, at_least))
+    if (one_by_one &&
+        !finish_buckets<FinishApart>(
+            *reinterpret_cast<FinishSmem<FinishApart>*>(smem_raw), t, out, a.num_cells, bucket, last, step,
+            at_least, Shape::kRecordWords, [&](uint32_t from, int count) {
+              if (Shape::kRecordWords != kKeyRecordWords) gather_small(a, out, from, count);
+            }))
       done += kFailedTask;
     __syncthreads();
     if (tid == 0) s.turn = next;

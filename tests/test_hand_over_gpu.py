@@ -135,3 +135,46 @@ def test_dense_cells_of_a_sparse_grid_stay_off_the_digit_passes(cuda, n, edge, c
     np.testing.assert_array_equal(order.particle_index.cpu().numpy(), want.particle_index)
     np.testing.assert_array_equal(order.cell_counts.cpu().numpy(), want.cell_counts)
     np.testing.assert_array_equal(order.cell_start.cpu().numpy(), want.cell_start)
+
+
+# The one-launch sort with payload: cells between what a block holds with payload (2560) and what
+# the bucketed path takes (5120), and a row of cells, one bucket, of 100,000 particles.
+@pytest.mark.parametrize('n', [60_000, 300_000, 606_208])
+@pytest.mark.parametrize('crowd', [2_561, 5_120, 'row'])
+@pytest.mark.parametrize('moved', [False, True])
+def test_small_calls_take_what_larger_calls_take(cuda, n, crowd, moved):
+    if crowd == 'row' and n < 300_000:
+        pytest.skip('fewer particles than the row has')
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (64, 32, 32))
+    pos, vel = _state(n, cuda, n)
+    pos[2] *= 30 / 32  # the topmost layers hold the crowd alone
+    if crowd == 'row':
+        chosen = torch.arange(n, device=cuda) % (n // 100_000) == 0
+        chosen &= torch.cumsum(chosen, 0) <= 100_000
+    else:
+        chosen = torch.arange(n, device=cuda) < crowd
+        pos[0][chosen] = 32.5 / 64
+    pos[1][chosen] = 16.5 / 32
+    pos[2][chosen] = 31.5 / 32
+    for k in range(3):
+        vel[k, :n][chosen] *= 1e-7
+    seed, dt = 31, 1e-3
+    got = pa.sort_and_gather_particles(*pos, vel, grid, seed,
+                                       push=(dt, grid.lo, grid.hi) if moved else None)
+    assert pa.last_sort_status(cuda) == 0
+    assert not pa.last_sort_used_digit_passes(cuda)
+    p, v = [t.cpu().numpy() for t in pos], vel.cpu().numpy()
+    if moved:
+        p, rows = so.push_particles(p, [v[k, :n] for k in range(3)], dt, grid.lo, grid.hi)
+        v[:, :n] = np.stack(rows)
+        p = [np.ascontiguousarray(a) for a in p]
+    want, *payload = so.c_sort_particles(*p, v, so.Grid(grid.lo, grid.hi, grid.cells), seed)
+    np.testing.assert_array_equal(got.order.keys.cpu().numpy().view(np.uint32), want.keys)
+    np.testing.assert_array_equal(got.order.particle_index.cpu().numpy(), want.particle_index)
+    np.testing.assert_array_equal(got.order.cell_counts.cpu().numpy(), want.cell_counts)
+    np.testing.assert_array_equal(got.order.cell_start.cpu().numpy(), want.cell_start)
+    for g, w in zip(got.positions, payload):
+        np.testing.assert_array_equal(g.cpu().numpy(), w)
+    np.testing.assert_array_equal(got.velocity.cpu().numpy()[:, :n], payload[3][:, :n])
+    if crowd != 'row':
+        assert int(got.order.cell_counts.max()) == crowd
