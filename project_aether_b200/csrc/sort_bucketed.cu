@@ -1355,46 +1355,51 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
                                     int cells_here, int record_words, After after) {
   constexpr int kThreads = Shape::kThreads, kCapacity = Shape::kCapacity;
   const int tid = threadIdx.x;
+  static_assert(Shape::kMaxCells < Shape::kHistWords && Shape::kMaxCells <= 2 * kThreads, "cell counts");
   uint32_t* cell_count = s.hist;  // one word per cell; s.hist is free until a run is sorted
   for (int c = tid; c < cells_here; c += kThreads) cell_count[c] = 0;
   __syncthreads();
-  // Per-cell counts: one pass over the keys of the bucket's records.
+  // Per-cell counts: one pass over the keys of the bucket's records (lanes that agree share an
+  // add: a bucket that comes here is crowded).
   for (int c = 0; c < t.chunks; ++c) {
     const size_t entry = static_cast<size_t>(c) * t.buckets + b;
     const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
-    for (uint32_t i = tid; i < length; i += kThreads) {
-      const uint32_t key = __ldcg(t.records + static_cast<size_t>(start + i) * record_words);
-      atomicAdd(&cell_count[(key >> kShuffleBits) - static_cast<uint32_t>(first_cell)], 1u);
+    for (uint32_t base = 0; base < length; base += kThreads) {
+      const bool valid = base + tid < length;
+      const uint32_t key = valid ? __ldcg(t.records + static_cast<size_t>(start + base + tid) * record_words) : 0u;
+      bin_add(cell_count, (key >> kShuffleBits) - static_cast<uint32_t>(first_cell), valid);
     }
   }
   __syncthreads();
-  // Cut into runs of cells that fit (one thread; at most Shape::kMaxCells cells).
+  // Exclusive scan of the counts, two cells per thread, then one thread cuts the cells into runs
+  // that fit, each as long as can be.  (Walking through the counts one by one took it as long as
+  // all the rest.)
+  {
+    const int c0 = 2 * tid;
+    const uint32_t n0 = c0 < cells_here ? cell_count[c0] : 0u, n1 = c0 + 1 < cells_here ? cell_count[c0 + 1] : 0u;
+    const uint32_t before = block_exclusive_scan(n0 + n1, s.warp_sum, &s.total);
+    if (c0 <= cells_here) cell_count[c0] = before;
+    if (c0 + 1 <= cells_here) cell_count[c0 + 1] = before + n0;
+    if (c0 + 2 == cells_here) cell_count[cells_here] = before + n0 + n1;
+  }
+  __syncthreads();
   if (tid == 0) {
-    int segments = 0;
-    uint32_t load = 0, before = 0;
-    bool ok = true;
+    int segments = 0, c = 0;
     s.seg_first[0] = 0;
     s.seg_begin[0] = 0;
-    for (int c = 0; c < cells_here && ok; ++c) {
-      const uint32_t here = cell_count[c];
-      if (here > static_cast<uint32_t>(kCapacity)) ok = false;
-      if (load + here > static_cast<uint32_t>(kCapacity) ||
-          c - s.seg_first[segments] >= Shape::kRunCells) {  // close the run before cell c
-        before += load;
-        load = 0;
-        ++segments;
-        if (segments >= kMaxSegments) { ok = false; break; }
-        s.seg_first[segments] = static_cast<uint16_t>(c);
-        s.seg_begin[segments] = before;
+    while (c < cells_here && segments < kMaxSegments) {
+      int lo = c, hi = min(cells_here, c + Shape::kRunCells);
+      while (lo < hi) {  // the last end whose run still fits
+        const int mid = (lo + hi + 1) >> 1;
+        if (cell_count[mid] - cell_count[c] <= static_cast<uint32_t>(kCapacity)) lo = mid; else hi = mid - 1;
       }
-      load += here;
-    }
-    if (ok) {
+      if (lo == c) break;  // a cell of its own does not fit
+      c = lo;
       ++segments;
-      s.seg_first[segments] = static_cast<uint16_t>(cells_here);
-      s.seg_begin[segments] = before + load;
+      s.seg_first[segments] = static_cast<uint16_t>(c);
+      s.seg_begin[segments] = cell_count[c];
     }
-    s.total = ok ? static_cast<uint32_t>(segments) : 0u;
+    s.total = c == cells_here ? static_cast<uint32_t>(segments) : 0u;
   }
   __syncthreads();
   const int segments = static_cast<int>(s.total);
