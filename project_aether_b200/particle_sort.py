@@ -23,7 +23,7 @@ from typing import NamedTuple, Optional, Tuple
 import torch
 
 from . import _native
-from ._launch import on_device, raw_stream
+from ._launch import device_index, on_device, raw_stream
 from .cell_grid import CellGrid, MAX_PARTICLES, key_bits, num_passes  # noqa: F401
 
 PATH_AUTO, PATH_DIGIT_PASSES, PATH_BUCKETED = 0, 1, 2
@@ -61,7 +61,7 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """One cached scratch buffer per device and stream, grown on demand (with an eighth
     of headroom, so that a particle count that creeps up from call to call does not
     reallocate gigabytes every time)."""
-    key = (device.index, raw_stream(device))
+    key = (device_index(device), raw_stream(device))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = None
@@ -238,7 +238,7 @@ def last_sort_status(device=None) -> int:
     current stream of `device`: 0 when clean, nonzero when a bounded device
     wait gave up (the results of that call are then invalid)."""
     device = torch.device('cuda', torch.cuda.current_device()) if device is None else device
-    key = (device.index, raw_stream(device))
+    key = (device_index(device), raw_stream(device))
     ws = _workspaces.get(key)
     if ws is None:
         return 0
@@ -255,7 +255,7 @@ def last_sort_used_digit_passes(device=None) -> bool:
     `device` was handed from the bucketed path to the digit passes on the device
     (same results, slower)."""
     device = torch.device('cuda', torch.cuda.current_device()) if device is None else device
-    key = (device.index, raw_stream(device))
+    key = (device_index(device), raw_stream(device))
     ws = _workspaces.get(key)
     if ws is None:
         return False
