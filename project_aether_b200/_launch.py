@@ -10,7 +10,7 @@ _SAME_DEVICE = contextlib.nullcontext()
 
 def on_device(device: torch.device):
     """Context in which `device` is the current CUDA device."""
-    if torch.cuda.current_device() == device_index(device):
+    if device.index is None or torch.cuda.current_device() == device.index:
         return _SAME_DEVICE
     return torch.cuda.device(device)
 
@@ -22,4 +22,5 @@ def device_index(device: torch.device) -> int:
 
 def raw_stream(device: torch.device) -> int:
     """Handle of PyTorch's current stream on `device`."""
-    return torch._C._cuda_getCurrentRawStream(device_index(device))
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)

@@ -7,7 +7,7 @@
 // sum rounded on its own, as the reference's host replay computes them
 // (dsmc_collide_tma_test.cu:45-84).
 //
-// Layout of the work: a block owns a run of consecutive cells, one per thread.  It draws every
+// Layout of the work: a block owns a run of consecutive cells, at most one per thread.  It draws every
 // cell's number of candidate pairs, scans the numbers, and hands the pairs of ALL its cells out
 // to its threads one pair per thread, so that cells of ten particles keep a block as busy as
 // cells of a thousand.  A pair's velocities are read from and, if it collides, written to
@@ -22,6 +22,7 @@ namespace aether {
 namespace {
 
 constexpr int kCollideThreads = 256;
+constexpr int kCollideBlocks = 6;               // per multiprocessor
 constexpr uint32_t kCellDraw = 0xFFFFFFFFu;     // pair id of a cell's selection draw
 
 struct CollideArgs {
@@ -31,6 +32,7 @@ struct CollideArgs {
   int* collisions;
   int padded;
   int num_cells;
+  int cells_per_block;  // at most kCollideThreads
   float selection_factor, coefficient, exponent;
   uint32_t key0, key1, step_lo, step_hi;
 };
@@ -106,7 +108,7 @@ __device__ __forceinline__ bool collide_pair(float* a, float* b, float majorant,
 // registers) per multiprocessor.  A first design staged every particle of the block's cells in
 // shared memory, four blocks per multiprocessor, and wrote the stage back: 16 M particles in 2 M
 // cells took it 123 us, this kernel 61 (436 MB if every velocity is read and written once).
-__global__ void __launch_bounds__(kCollideThreads, 6)
+__global__ void __launch_bounds__(kCollideThreads, kCollideBlocks)
 collide_kernel(CollideArgs a) {
   __shared__ int start[kCollideThreads];
   __shared__ int pair_first[kCollideThreads];      // exclusive prefix of the candidate pairs
@@ -116,8 +118,8 @@ collide_kernel(CollideArgs a) {
   __shared__ uint32_t warp_sum[32];
   __shared__ uint32_t total;
   const int tid = threadIdx.x;
-  const int first_cell = blockIdx.x * kCollideThreads;
-  const int cells_here = min(kCollideThreads, a.num_cells - first_cell);
+  const int first_cell = blockIdx.x * a.cells_per_block;
+  const int cells_here = min(a.cells_per_block, a.num_cells - first_cell);
   const int my_cell = first_cell + tid;
   float majorant = 0.0f;
   uint32_t selections = 0;
@@ -170,6 +172,20 @@ collide_kernel(CollideArgs a) {
   }
 }
 
+// Cells per block: as many as a block has threads, fewer (halved, at least 16) until there is a
+// block for every place on the multiprocessors, six each; a block's threads share the pairs of
+// its cells whatever their number, but a block with few cells wastes threads on the cells' own
+// work.  0.075 pairs per particle, 256 cells per block / this rule: 10,000 cells of 400 particles
+// 46 / 13 us, 1000 cells of 400 45 / 10, 65,536 cells of 61 12.8 / 12.3; 128 cells per block at
+// 2 M cells of 8 take 76 us against 62.
+constexpr int kFewestCells = 16;
+int cells_per_block_for(int num_cells) {
+  const int places = kCollideBlocks * sm_count();
+  int cells = kCollideThreads;
+  while (cells > kFewestCells && (num_cells + cells - 1) / cells < places) cells /= 2;
+  return cells;
+}
+
 }  // namespace
 
 // Enqueues one collision step.  velocity (3, padded) is updated in place,
@@ -197,7 +213,8 @@ cudaError_t collide_cells(float* velocity, const int* cell_start, float* sigma_g
   a.key1 = static_cast<uint32_t>(seed >> 32);
   a.step_lo = static_cast<uint32_t>(step);
   a.step_hi = static_cast<uint32_t>(step >> 32);
-  const int blocks = (num_cells + kCollideThreads - 1) / kCollideThreads;
+  a.cells_per_block = cells_per_block_for(num_cells);
+  const int blocks = (num_cells + a.cells_per_block - 1) / a.cells_per_block;
   stage_begin(kStageCollide, stream);
   collide_kernel<<<blocks, kCollideThreads, 0, stream>>>(a);
   stage_end(kStageCollide, stream);

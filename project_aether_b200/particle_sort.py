@@ -61,7 +61,7 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """One cached scratch buffer per device and stream, grown on demand (with an eighth
     of headroom, so that a particle count that creeps up from call to call does not
     reallocate gigabytes every time)."""
-    key = (device_index(device), raw_stream(device))
+    key = (device.index, raw_stream(device))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = None
