@@ -2254,14 +2254,25 @@ size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells, bool keys_only) {
 
 namespace {
 
+// Lets a kernel have `most` bytes of dynamic shared memory: the most that any call asks for, so
+// that calls of different sizes from several threads set the same limit (with each call's own
+// need as the limit, one thread could lower it between another's setting and launch).
+template <class Kernel>
+cudaError_t allow_shared(Kernel kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
+}
+constexpr size_t kMostCountTable = 200 * 1024;
+constexpr size_t kMostGroupStage = 2 * kGroupStagedChunks * (kGroupSpan + 1) * sizeof(uint32_t);
+constexpr size_t kMostSplitShared = 192 * 1024;
+constexpr size_t kMostScanStage = (kStagedScanMax + 2 * (kFlatScanBlock + 1)) * sizeof(uint32_t);
+
 cudaError_t launch_groups(cudaStream_t stream, const uint32_t* run_begin, int buckets, int chunks,
                           int chunk_log, const SliceSegments* segments, int group_shift,
                           uint32_t capacity, uint32_t* start, uint32_t* tables, Header* hdr) {
   const size_t staged = chunks <= kGroupStagedChunks
                             ? 2 * static_cast<size_t>(chunks) * (kGroupSpan + 1) * sizeof(uint32_t) : 0;
   if (staged > 40 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(staged));
+    const cudaError_t e = allow_shared(group_kernel, kMostGroupStage);
     if (e != cudaSuccess) return e;
   }
   return launch_chained(group_kernel, (buckets + kGroupSpan - 1) / kGroupSpan, kGroupSpan, staged,
@@ -2277,8 +2288,8 @@ cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut&
   if (std::is_same_v<Shape, FinishSmall> && table_bytes > kSmallShapeTableBytes)
     return cudaErrorInvalidValue;
   const int smem = static_cast<int>(sizeof(FinishSmem<Shape>) + table_bytes);
-  cudaError_t e = cudaFuncSetAttribute(bucket_finish_kernel<Shape>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = allow_shared(bucket_finish_kernel<Shape>,
+                               sizeof(FinishSmem<Shape>) + 3 * 2 * kTableRowWords * sizeof(uint32_t));
   if (e != cudaSuccess) return e;
   e = launch_chained<true>(bucket_finish_kernel<Shape>, std::min(t.buckets, sm_count() * Shape::kBlocks),
                      Shape::kThreads, smem, a.stream, t, a.n, n_on_device, a.num_cells, out, hdr);
@@ -2291,8 +2302,7 @@ cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut&
 cudaError_t launch_finish_large(const RunTable& t, const SortArgs& a, const FinishOut& out,
                                 Header* hdr, uint32_t group_capacity) {
   constexpr int kSmem = static_cast<int>(sizeof(FinishSmem<FinishLarge>));
-  cudaError_t e = cudaFuncSetAttribute(bucket_finish_large_kernel<FinishLarge>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  cudaError_t e = allow_shared(bucket_finish_large_kernel<FinishLarge>, kSmem);
   if (e != cudaSuccess) return e;
   e = launch_chained<true>(bucket_finish_large_kernel<FinishLarge>, std::min(t.buckets, sm_count()),
                            FinishLarge::kThreads, kSmem, a.stream, t, a.num_cells, out, hdr,
@@ -2309,8 +2319,7 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
   DigitPassArgs digits;
   cudaError_t e = digit_pass_args(a, &digits);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(bucket_tail_kernel<Shape>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
   // One block per multiprocessor, fewer where there is little to do.
   const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sm_count(), a.n / 2048)));
@@ -2337,8 +2346,9 @@ cudaError_t launch_split(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, 
   constexpr int kTile = THREADS * ITEMS;
   const size_t bytes = split_smem_bytes(kTile, buckets);
   auto kernel = vec ? key_split_kernel<true, ITEMS, THREADS> : key_split_kernel<false, ITEMS, THREADS>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(bytes));
+  static_assert(kTile * 8 + 2 * sizeof(uint32_t) * (kTile > 8192 ? kTile / 2 : kSplitMaxBuckets) <= kMostSplitShared,
+                "shared memory");
+  const cudaError_t e = allow_shared(kernel, kMostSplitShared);
   if (e != cudaSuccess) return e;
   const int64_t blocks = std::min<int64_t>((a.n + kTile - 1) / kTile,
                                            (THREADS <= 512 ? 2 : 1) * sm_count());
@@ -2358,7 +2368,7 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
   DigitPassArgs digits;
   cudaError_t e = digit_pass_args(a, &digits);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(small_sort_kernel<Shape>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  e = allow_shared(small_sort_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
   const int blocks = small_call_blocks(a.n, p.buckets);
   SmallArgs s{};
@@ -2420,8 +2430,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   {
     const size_t bytes32 = static_cast<size_t>(buckets) * sizeof(uint32_t);
     const size_t bytes16 = (static_cast<size_t>(buckets) + 1) / 2 * sizeof(uint32_t);
-    const int table = bytes32 <= 200 * 1024 ? kTableShared32
-                      : bytes16 <= 200 * 1024 ? kTableShared16 : kTableGlobal;
+    const int table = bytes32 <= kMostCountTable ? kTableShared32
+                      : bytes16 <= kMostCountTable ? kTableShared16 : kTableGlobal;
     const size_t table_bytes = table == kTableShared32 ? bytes32 : table == kTableShared16 ? bytes16 : 0;
     const bool wide = table_bytes > 96 * 1024;  // one 1024-thread block per SM holds the table
     const int threads = wide ? kCountThreadsWide : kCountThreads;
@@ -2437,8 +2447,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     auto kernel = vec ? bucket_count_kernel<TABLE, true, THREADS>                                 \
                       : bucket_count_kernel<TABLE, false, THREADS>;                               \
     if (table_bytes > 48 * 1024) {                                                                \
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
-                               static_cast<int>(table_bytes));                                    \
+      e = allow_shared(kernel, kMostCountTable);                                                  \
       if (e != cudaSuccess) return e;                                                             \
     }                                                                                             \
     kernel<<<grid, THREADS, table_bytes, a.stream>>>(a.x, a.y, a.z, a.velocity, a.padded, a.push, \
@@ -2592,7 +2601,7 @@ cudaError_t sliced_sort_slice(const SortArgs& a, int64_t plan_n, const SliceSegm
   stage_begin(kStageBucketCount, a.stream);
   {
     const size_t table_bytes = static_cast<size_t>(buckets) * sizeof(uint32_t);
-    const bool shared = table_bytes <= 200 * 1024;
+    const bool shared = table_bytes <= kMostCountTable;
     const bool wide = shared && table_bytes > 96 * 1024;
     const int per_sm = !shared ? 4 : wide ? 1 : table_bytes <= 48 * 1024 ? 4 : 2;
     const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(units, sm_count() * per_sm)));
@@ -2601,16 +2610,14 @@ cudaError_t sliced_sort_slice(const SortArgs& a, int64_t plan_n, const SliceSegm
           a.x, a.y, a.z, a.n, vec, segments, slice, a.grid, st.plan.shift, buckets, row);
     } else if (wide) {
       auto kernel = bucket_count_segments_kernel<kTableShared32, kCountThreadsWide>;
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(table_bytes));
+      e = allow_shared(kernel, kMostCountTable);
       if (e != cudaSuccess) return e;
       kernel<<<grid, kCountThreadsWide, table_bytes, a.stream>>>(
           a.x, a.y, a.z, a.n, vec, segments, slice, a.grid, st.plan.shift, buckets, row);
     } else {
       auto kernel = bucket_count_segments_kernel<kTableShared32, kCountThreads>;
       if (table_bytes > 48 * 1024) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(table_bytes));
+        e = allow_shared(kernel, kMostCountTable);
         if (e != cudaSuccess) return e;
       }
       kernel<<<grid, kCountThreads, table_bytes, a.stream>>>(
@@ -2623,8 +2630,7 @@ cudaError_t sliced_sort_slice(const SortArgs& a, int64_t plan_n, const SliceSegm
     const int per = (buckets + kFlatScanBlock - 1) / kFlatScanBlock;
     const size_t bytes = (static_cast<size_t>(buckets) + 2 * (buckets / per + 1)) * sizeof(uint32_t);
     if (bytes > 48 * 1024) {
-      e = cudaFuncSetAttribute(chunk_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(bytes));
+      e = allow_shared(chunk_scan_kernel<true>, kMostScanStage);
       if (e != cudaSuccess) return e;
     }
     chunk_scan_kernel<true><<<1, kFlatScanBlock, bytes, a.stream>>>(row, buckets, segments, slice,

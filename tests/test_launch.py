@@ -1,5 +1,7 @@
 """Device and stream of a call (project_aether_b200/_launch.py)."""
 
+import threading
+
 import pytest
 import torch
 
@@ -28,3 +30,38 @@ def test_status_of_a_device_without_a_number(cuda):
     assert pa.last_sort_status(torch.device('cuda')) == 0
     assert pa.last_sort_used_digit_passes(torch.device('cuda')) == pa.last_sort_used_digit_passes(cuda)
     assert pa.last_sort_used_digit_passes(torch.device('cuda')) is True
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('sizes', [((2_500_000, (25, 25, 16)), (2_600_000, (16, 16, 11))),
+                                   ((16_500_000, (128, 128, 128)), (17_500_000, (128, 128, 128)))])
+def test_threads_with_calls_of_different_sizes(cuda, sizes):
+    """Kernels whose shared memory depends on the call, launched by two threads at a time: no
+    call's setting may take the other's launch its memory away."""
+    failures, results = [], [None, None]
+    inputs = [[torch.rand(n, device=cuda) for _ in range(3)] for n, _ in sizes]
+    grids = [pa.CellGrid((0., 0., 0.), (1., 1., 1.), cells) for _, cells in sizes]
+    want = [pa.sort_particles_by_cell(*x, g, 5) for x, g in zip(inputs, grids)]
+    torch.cuda.synchronize()
+    calls = 4000 if sizes[0][0] < 10**7 else 400
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream(cuda)):
+                for i in range(calls):
+                    results[k] = pa.sort_particles_by_cell(*inputs[k], grids[k], 5)
+                    if i % 50 == 49:
+                        torch.cuda.current_stream().synchronize()
+        except RuntimeError as error:
+            failures.append(str(error))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failures
+    for got, w in zip(results, want):
+        for a, b in zip(got, w):
+            assert torch.equal(a, b)
