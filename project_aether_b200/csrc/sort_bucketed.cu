@@ -2314,12 +2314,9 @@ int limited(int blocks, int most) { return most > 0 ? std::min(blocks, most) : b
 
 template <class Shape>
 cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                        uint32_t group_capacity) {
+                        uint32_t group_capacity, const DigitPassArgs& digits) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
-  DigitPassArgs digits;
-  cudaError_t e = digit_pass_args(a, &digits);
-  if (e != cudaSuccess) return e;
-  e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
+  const cudaError_t e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
   // One block per multiprocessor, fewer where there is little to do.
   const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sm_count(), a.n / 2048)));
@@ -2361,14 +2358,12 @@ cudaError_t launch_split(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, 
 
 namespace {
 template <class Shape>
-cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLayout& l) {
+cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLayout& l,
+                         const DigitPassArgs& digits) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<kSmallThreads>)));
   static_assert(2 * (kSmem + 1024 + 64) <= 228 * 1024, "two blocks must share a multiprocessor");
   auto* base = static_cast<unsigned char*>(a.workspace);
-  DigitPassArgs digits;
-  cudaError_t e = digit_pass_args(a, &digits);
-  if (e != cudaSuccess) return e;
-  e = allow_shared(small_sort_kernel<Shape>, kSmem);
+  const cudaError_t e = allow_shared(small_sort_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
   const int blocks = small_call_blocks(a.n, p.buckets);
   SmallArgs s{};
@@ -2413,11 +2408,14 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   uint32_t* run_begin = words_at(l.run_begin_off);
   uint32_t* tables = words_at(l.tables_off);
   uint32_t* records = words_at(l.records_off);
-  cudaError_t e = cudaMemsetAsync(base, 0, l.start_off, a.stream);  // header and run counts
+  DigitPassArgs digits;  // a workspace too small for them is refused before anything is enqueued
+  cudaError_t e = digit_pass_args(a, &digits);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(base, 0, l.start_off, a.stream);  // header and run counts
   if (e != cudaSuccess) return e;
   if (p.one_launch) {
     stage_begin(kStageBucketFinish, a.stream);
-    e = p.keys_only ? launch_small<FinishKeys>(a, p, l) : launch_small<FinishSmall>(a, p, l);
+    e = p.keys_only ? launch_small<FinishKeys>(a, p, l, digits) : launch_small<FinishSmall>(a, p, l, digits);
     stage_end(kStageBucketFinish, a.stream);
     return e;
   }
@@ -2531,8 +2529,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
       : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr)
                        : launch_finish<FinishLarge>(t, a, out, hdr);
   if (e == cudaSuccess)
-    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity)
-                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity);
+    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits)
+                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits);
   stage_end(kStageBucketFinish, a.stream);
   count_launches(2);
   return e;

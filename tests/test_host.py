@@ -75,6 +75,18 @@ def test_bad_arguments_are_rejected_before_any_launch(lib):
     assert rc == CUDA_ERROR_INVALID_VALUE
 
 
+def test_workspace_too_small_for_the_digit_passes_is_refused_before_any_launch(lib):
+    """Calls without payload: their 8-byte records fit a workspace that the digit passes, which
+    any such call may be handed over to, do not.  (Without a GPU a launch or a memset would
+    answer with another error.)"""
+    g = pa.particle_sort.native_grid(pa.CellGrid((0, 0, 0), (1, 1, 1), (25, 25, 16)))
+    fake = ctypes.c_void_p(1 << 20)  # never dereferenced
+    for n in (300_000, 2_500_000):
+        rc = lib.AetherSortParticlesByCell(fake, fake, fake, n, ctypes.byref(g), 0, fake, fake, fake,
+                                           fake, fake, int(8.4 * n), None)
+        assert rc == CUDA_ERROR_INVALID_VALUE
+
+
 def test_entry_point_rejects_cpu_tensors_like_the_reference():
     # fused_radix_sort.py:238-241
     grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (4, 4, 4))
