@@ -341,29 +341,42 @@ __device__ __forceinline__ bool digit_phase(const DigitPassArgs& a, PassSmem<THR
     uint32_t* hist = &s.warp_count[0][0];
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += THREADS) hist[i] = 0;
     __syncthreads();
-    const int64_t rounds = (a.n + stride - 1) / stride;
+    constexpr int kBatch = 2;  // particles whose loads are under way together
+    const int64_t rounds = (a.n + kBatch * stride - 1) / (kBatch * stride);
     for (int64_t r = 0; r < rounds; ++r) {  // the same number for every thread: warp votes below
-      const int64_t i = r * stride + first;
-      const bool ok = i < a.n;
-      uint32_t key = 0;
-      if (ok) {
-        float px = a.x[i], py = a.y[i], pz = a.z[i];
-        if (a.records) {
-          float vx = a.v ? a.v[i] : 0.f, vy = a.v ? a.v[a.padded + i] : 0.f;
-          float vz = a.v ? a.v[2 * a.padded + i] : 0.f;
-          if (a.push.enabled) {
-            push_axis(px, vx, a.push.dt, a.push.lo[0], a.push.hi[0]);
-            push_axis(py, vy, a.push.dt, a.push.lo[1], a.push.hi[1]);
-            push_axis(pz, vz, a.push.dt, a.push.lo[2], a.push.hi[2]);
-          }
-          a.records[2 * i] = make_float4(px, py, pz, vx);
-          a.records[2 * i + 1] = make_float4(vy, vz, 0.f, 0.f);
-        }
-        key = make_key(cell_of(px, py, pz, a.grid), static_cast<uint32_t>(i), a.k0, a.k1);
-        cur_k[i] = key;
+      float q[kBatch][6];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        const int64_t i = (r * kBatch + k) * stride + first;
+        const bool ok = i < a.n, moved = ok && a.records && a.v;
+        q[k][0] = ok ? a.x[i] : 0.f;
+        q[k][1] = ok ? a.y[i] : 0.f;
+        q[k][2] = ok ? a.z[i] : 0.f;
+        q[k][3] = moved ? a.v[i] : 0.f;
+        q[k][4] = moved ? a.v[a.padded + i] : 0.f;
+        q[k][5] = moved ? a.v[2 * a.padded + i] : 0.f;
       }
-      for (int p = 0; p < a.passes; ++p)
-        bin_add(hist + p * kRadix, (key >> (kRadixBits * p)) & (kRadix - 1), ok);
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        const int64_t i = (r * kBatch + k) * stride + first;
+        const bool ok = i < a.n;
+        uint32_t key = 0;
+        if (ok) {
+          if (a.records) {
+            if (a.push.enabled) {
+#pragma unroll
+              for (int c = 0; c < 3; ++c)
+                push_axis(q[k][c], q[k][3 + c], a.push.dt, a.push.lo[c], a.push.hi[c]);
+            }
+            a.records[2 * i] = make_float4(q[k][0], q[k][1], q[k][2], q[k][3]);
+            a.records[2 * i + 1] = make_float4(q[k][4], q[k][5], 0.f, 0.f);
+          }
+          key = make_key(cell_of(q[k][0], q[k][1], q[k][2], a.grid), static_cast<uint32_t>(i), a.k0, a.k1);
+          cur_k[i] = key;
+        }
+        for (int p = 0; p < a.passes; ++p)
+          bin_add(hist + p * kRadix, (key >> (kRadixBits * p)) & (kRadix - 1), ok);
+      }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < a.passes * kRadix; i += THREADS)
@@ -383,23 +396,38 @@ __device__ __forceinline__ bool digit_phase(const DigitPassArgs& a, PassSmem<THR
                                                &hdr->error, kPollLimit);
   } else if (phase == static_cast<uint32_t>(a.passes) + 2) {
     if (a.xs) {
-      for (int64_t r = first; r < a.n; r += stride) {
-        const int64_t i = __ldcg(a.index_out + r);
-        float4 lo, hi;
-        if (a.records) {
-          lo = __ldcg(a.records + 2 * i);
-          hi = __ldcg(a.records + 2 * i + 1);
-        } else {
-          lo = make_float4(a.x[i], a.y[i], a.z[i], a.v ? a.v[i] : 0.f);
-          hi = make_float4(a.v ? a.v[a.padded + i] : 0.f, a.v ? a.v[2 * a.padded + i] : 0.f, 0.f, 0.f);
+      constexpr int kBatch = 4;  // particles whose loads are under way together
+      for (int64_t r0 = first; r0 < a.n; r0 += kBatch * stride) {
+        float4 lo[kBatch], hi[kBatch];
+        int32_t index[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          const int64_t r = r0 + k * stride;
+          index[k] = r < a.n ? __ldcg(a.index_out + r) : 0;
         }
-        a.xs[r] = lo.x;
-        a.ys[r] = lo.y;
-        a.zs[r] = lo.z;
-        if (a.vs) {
-          a.vs[r] = lo.w;
-          a.vs[a.padded_sorted + r] = hi.x;
-          a.vs[2 * a.padded_sorted + r] = hi.y;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          const int64_t i = index[k];
+          if (a.records) {
+            lo[k] = __ldcg(a.records + 2 * i);
+            hi[k] = __ldcg(a.records + 2 * i + 1);
+          } else {
+            lo[k] = make_float4(a.x[i], a.y[i], a.z[i], a.v ? a.v[i] : 0.f);
+            hi[k] = make_float4(a.v ? a.v[a.padded + i] : 0.f, a.v ? a.v[2 * a.padded + i] : 0.f, 0.f, 0.f);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          const int64_t r = r0 + k * stride;
+          if (r >= a.n) break;
+          a.xs[r] = lo[k].x;
+          a.ys[r] = lo[k].y;
+          a.zs[r] = lo[k].z;
+          if (a.vs) {
+            a.vs[r] = lo[k].w;
+            a.vs[a.padded_sorted + r] = hi[k].x;
+            a.vs[2 * a.padded_sorted + r] = hi[k].y;
+          }
         }
       }
     }

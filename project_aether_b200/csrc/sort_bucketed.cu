@@ -1641,8 +1641,11 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
 // it replaces (the oversized buckets, a clear, the keys, up to four digit passes, two table
 // kernels and the payload gather, each returning at once) the same look cost 13-17 us of every
 // call on the device and 11 launches on the host.
+// Blocks per multiprocessor, fewer of them where there is little to do.
 template <class Shape>
-__global__ void __launch_bounds__(Shape::kThreads, 1)
+constexpr int kTailBlocks = Shape::kThreads <= 512 ? 2 : 1;
+template <class Shape>
+__global__ void __launch_bounds__(Shape::kThreads, kTailBlocks<Shape>)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
                    DigitPassArgs digits) {
   chain_begin();
@@ -2318,8 +2321,8 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
   const cudaError_t e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
-  // One block per multiprocessor, fewer where there is little to do.
-  const int blocks = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sm_count(), a.n / 2048)));
+  const int blocks = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(sm_count() * kTailBlocks<Shape>, a.n / 2048)));
   return launch_chained<true>(bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks), Shape::kThreads,
                               kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity, digits);
 }
