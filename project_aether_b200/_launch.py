@@ -10,17 +10,16 @@ _SAME_DEVICE = contextlib.nullcontext()
 
 def on_device(device: torch.device):
     """Context in which `device` is the current CUDA device."""
-    if device.index is None or torch.cuda.current_device() == device.index:
+    if torch.cuda.current_device() == device.index:
         return _SAME_DEVICE
     return torch.cuda.device(device)
 
 
-def device_index(device: torch.device) -> int:
-    """Number of a CUDA device; `cuda` without one is the current device."""
-    return torch.cuda.current_device() if device.index is None else device.index
+def numbered(device: torch.device) -> torch.device:
+    """The device by its number; `cuda` without one is the current device."""
+    return torch.device('cuda', torch.cuda.current_device()) if device.index is None else device
 
 
 def raw_stream(device: torch.device) -> int:
-    """Handle of PyTorch's current stream on `device`."""
-    index = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    """Handle of PyTorch's current stream on `device`, which has a number."""
+    return torch._C._cuda_getCurrentRawStream(device.index)

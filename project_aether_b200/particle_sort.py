@@ -23,7 +23,7 @@ from typing import NamedTuple, Optional, Tuple
 import torch
 
 from . import _native
-from ._launch import device_index, on_device, raw_stream
+from ._launch import numbered, on_device, raw_stream
 from .cell_grid import CellGrid, MAX_PARTICLES, key_bits, num_passes  # noqa: F401
 
 PATH_AUTO, PATH_DIGIT_PASSES, PATH_BUCKETED = 0, 1, 2
@@ -237,8 +237,8 @@ def last_sort_status(device=None) -> int:
     """Synchronises and returns the device status of the last sort on the
     current stream of `device`: 0 when clean, nonzero when a bounded device
     wait gave up (the results of that call are then invalid)."""
-    device = torch.device('cuda', torch.cuda.current_device()) if device is None else device
-    key = (device_index(device), raw_stream(device))
+    device = numbered(torch.device('cuda') if device is None else device)
+    key = (device.index, raw_stream(device))
     ws = _workspaces.get(key)
     if ws is None:
         return 0
@@ -254,8 +254,8 @@ def last_sort_used_digit_passes(device=None) -> bool:
     """Synchronises and tells whether the last sort on the current stream of
     `device` was handed from the bucketed path to the digit passes on the device
     (same results, slower)."""
-    device = torch.device('cuda', torch.cuda.current_device()) if device is None else device
-    key = (device_index(device), raw_stream(device))
+    device = numbered(torch.device('cuda') if device is None else device)
+    key = (device.index, raw_stream(device))
     ws = _workspaces.get(key)
     if ws is None:
         return False

@@ -13,11 +13,12 @@ def test_a_device_without_a_number_is_the_current_one(monkeypatch):
     monkeypatch.setattr(torch.cuda, 'current_device', lambda: 3)
     monkeypatch.setattr(torch._C, '_cuda_getCurrentRawStream', lambda index: 100 + int(index),
                         raising=False)
-    assert _launch.raw_stream(torch.device('cuda')) == 103
+    assert _launch.numbered(torch.device('cuda')) == torch.device('cuda', 3)
+    assert _launch.numbered(torch.device('cuda', 1)) == torch.device('cuda', 1)
     assert _launch.raw_stream(torch.device('cuda', 1)) == 101
-    assert _launch.on_device(torch.device('cuda')) is _launch.on_device(torch.device('cuda', 3))
     # Nothing was sorted on that device and stream.
     monkeypatch.setattr(particle_sort, '_workspaces', {})
+    assert pa.last_sort_status() == 0
     assert pa.last_sort_status(torch.device('cuda')) == 0
     assert pa.last_sort_used_digit_passes(torch.device('cuda')) is False
 
