@@ -42,8 +42,8 @@ int run_sort(SortArgs& a, int path) {
   stage_reset();
   // path 1 asks for the digit passes; otherwise the bucketed path runs whenever its plan fits
   // (with or without payload outputs) and the workspace is large enough for its records.  A
-  // caller with a smaller workspace (the static-scratch entry point above a few hundred
-  // thousand particles, or a workspace sized for the digit passes only) gets the digit passes.
+  // caller with a smaller workspace (the static-scratch entry point with a million particles in
+  // many buckets, or a workspace sized for the digit passes only) gets the digit passes.
   const bool keys_only = a.xs == nullptr;
   const BucketPlan plan = plan_buckets(a.n, a.num_cells, keys_only);
   const bool roomy = a.workspace_bytes >= bucketed_workspace_bytes(a.n, a.num_cells, keys_only);

@@ -219,17 +219,17 @@ void stage_end(Stage s, cudaStream_t stream);
 void stage_reset();
 void count_launches(int kernels);
 
-// Chained launches.  The kernels of one sort call run one after the other on one stream, two
-// dozen of them, and the gaps between them (the next kernel's launch begins when the previous
-// grid has drained) are most of what a small call costs.  A kernel launched with
+// Chained launches.  The kernels of a larger sort call (count, run scan, groups, scatter, finish,
+// tail; or the digit passes') run one after the other on one stream, and in the gaps between them
+// the next kernel's launch begins when the previous grid has drained.  A kernel launched with
 // launch_chained may be set up while its predecessor still runs: every kernel of the chain
 // begins with chain_begin(), which lets the kernel behind it start its launch
 // (griddepcontrol.launch_dependents) and then waits until the grids before it are complete
 // and their memory visible (griddepcontrol.wait).  Nothing of a kernel's work moves ahead of
 // that wait, so the order of the work is that of the stream.  Launched in the ordinary way
-// the same kernels find nothing to wait for.  Measured per sort, ordinary launches / short
-// kernels chained / all chained: 1 M particles 0.161 / 0.137 / 0.141 ms, 16 M 0.641 / 0.601 /
-// 0.613, 64 M 2.312 / 2.273 / 2.378, 128 M (steady state) 3.745 / 3.706 / 3.724.
+// the same kernels find nothing to wait for.  Measured per call with payload, ordinary launches /
+// short kernels chained / all chained: 1 M particles 66 / 61 / 56 us, 16 M 553 / 551 / 561, 64 M
+// 2225 / 2258 / 2369; without payload 1 M 57 / 53 / 52, 16 M 356 / 351 / 356, 64 M 1888 / 1884 / 1883.
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

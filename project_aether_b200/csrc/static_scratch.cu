@@ -1,8 +1,8 @@
 // AetherSortParticlesByCellStatic: the sort with its scratch memory in a fixed
 // array that is part of the library image, for callers that are not allowed to
-// allocate device memory.  Small calls (the bucketed layout of their records fits
-// the array: up to a few hundred thousand particles) take the bucketed path, larger
-// ones the digit passes; the results are the same.
+// allocate device memory.  Calls whose bucketed layout (8 bytes per particle and 48
+// per bucket) fits the array, nearly all of them, take the bucketed path, the others
+// the digit passes; the results are the same.
 #include "common.cuh"
 
 namespace aether {

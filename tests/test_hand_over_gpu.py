@@ -1,5 +1,5 @@
-"""Calls that the bucketed path hands over to the digit passes on the device: one cooperative
-launch then runs them all."""
+"""Calls that the bucketed path hands over to the digit passes on the device, where one kernel
+then runs them all, and calls that it keeps although they are crowded."""
 
 import numpy as np
 import pytest

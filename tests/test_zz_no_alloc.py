@@ -84,8 +84,8 @@ def test_static_scratch_entry_matches_workspace_entry_twice_in_a_row(cuda):
 
 
 def test_static_scratch_small_call_takes_the_bucketed_path_and_equals_the_oracle(cuda):
-    """Below a few hundred thousand particles the bucketed record layout fits the library's
-    array and that path runs; whichever path runs, the result is the CPU oracle's."""
+    """The bucketed layout of calls without payload fits the library's array and that path runs;
+    whichever path runs, the result is the CPU oracle's."""
     from oracle import sort_oracle as so
     lib = _native.load_library()
     grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (32, 32, 16))
