@@ -62,6 +62,24 @@ def test_any_number_of_blocks_finishes_the_call(cuda, n, edge, density, most_blo
             assert torch.equal(g, w)
 
 
+# Groups without payload whose byte counters wrap, finished again bucket by bucket.
+@pytest.mark.parametrize('most_blocks', [1, 7])
+@pytest.mark.parametrize('n,edge,crowd', [(200_003, 96, 4_600), (2_400_011, 128, 3_000)])
+def test_any_number_of_blocks_finishes_wrapped_groups(cuda, n, edge, crowd, most_blocks):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (edge,) * 3)
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    pos = [torch.rand(n, device=cuda, generator=gen) for _ in range(3)]
+    for p in pos:
+        p[:crowd] = 0.251
+        p[crowd:2 * crowd] = 0.751
+    vel = torch.zeros((3, n), device=cuda)
+    want = pa.sort_particles_by_cell(*pos, grid, 99)
+    status, handed_over, got = _few_blocks(pos, vel, grid, 99, most_blocks, False, cuda)
+    assert (status, handed_over) == (0, False)
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
+
+
 # One launch, and the kernel behind the finish of a middling call.
 @pytest.mark.parametrize('n', [5_000, 600_000, 1_200_000])
 def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
@@ -73,8 +91,9 @@ def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
     beside, stream = torch.cuda.Stream(cuda), torch.cuda.Stream(cuda)
     scratch = torch.empty(8192, dtype=torch.uint8, device=cuda)
     returned = torch.zeros(1, dtype=torch.int32, device=cuda)
-    with torch.cuda.stream(stream):  # the stream's workspace exists
+    with torch.cuda.stream(stream):  # the workspace and the arrays of the call below exist
         want = pa.sort_and_gather_particles(*pos, vel, grid, 3)
+        arrays = pa.sort_and_gather_particles(*pos, vel, grid, 4)
     torch.cuda.synchronize()
     _native.check(lib.AetherSortProbeWaitGiveUp(scratch.data_ptr(), scratch.numel(), 1, 200 * 1024,
                                                 200_000_000, returned.data_ptr(), beside.cuda_stream),
@@ -82,7 +101,7 @@ def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
     ended = torch.cuda.Event()
     ended.record(beside)
     with torch.cuda.stream(stream):
-        got = pa.sort_and_gather_particles(*pos, vel, grid, 3)
+        got = pa.sort_and_gather_particles(*pos, vel, grid, 3, out=arrays)
         stream.synchronize()
     assert not ended.query(), 'the call waited for the kernel beside it'
     torch.cuda.synchronize()
