@@ -82,8 +82,10 @@ def test_any_number_of_blocks_finishes_wrapped_groups(cuda, n, edge, crowd, most
 
 # One launch, and the kernel behind the finish of a middling call.
 @pytest.mark.parametrize('n', [5_000, 600_000, 1_200_000])
-def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
-    """A kernel of another stream keeps one multiprocessor's shared memory for 200 ms."""
+@pytest.mark.parametrize('kept', [1, 120])
+def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n, kept):
+    """A kernel of another stream keeps the shared memory of one multiprocessor, or of most, for
+    200 ms: a part of the call's blocks runs, and does the work of the others."""
     lib = _native.load_library()
     grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (32, 32, 32))
     pos = [torch.rand(n, device=cuda) for _ in range(3)]
@@ -95,7 +97,7 @@ def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
         want = pa.sort_and_gather_particles(*pos, vel, grid, 3)
         arrays = pa.sort_and_gather_particles(*pos, vel, grid, 4)
     torch.cuda.synchronize()
-    _native.check(lib.AetherSortProbeWaitGiveUp(scratch.data_ptr(), scratch.numel(), 1, 200 * 1024,
+    _native.check(lib.AetherSortProbeWaitGiveUp(scratch.data_ptr(), scratch.numel(), kept, 200 * 1024,
                                                 200_000_000, returned.data_ptr(), beside.cuda_stream),
                   'AetherSortProbeWaitGiveUp')
     ended = torch.cuda.Event()
@@ -105,7 +107,7 @@ def test_a_call_does_not_wait_for_a_kernel_beside_it(cuda, n):
         stream.synchronize()
     assert not ended.query(), 'the call waited for the kernel beside it'
     torch.cuda.synchronize()
-    assert int(returned) == 1
+    assert int(returned) == kept
     for g, w in zip((*got.order, *got.positions, got.velocity),
                     (*want.order, *want.positions, want.velocity)):
         assert torch.equal(g, w)
