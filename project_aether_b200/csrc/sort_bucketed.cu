@@ -1188,12 +1188,13 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
   {
 #pragma unroll
     for (int j = 0; j < kWordsPerThread; j += 4) {
-      const uint4 a = *reinterpret_cast<const uint4*>(&s.hist[tid * kWordsPerThread + j]);
+      uint4 a = make_uint4(0u, 0u, 0u, 0u);  // hist_words is a multiple of 8
+      if (tid * kWordsPerThread + j < hist_words) a = *reinterpret_cast<const uint4*>(&s.hist[tid * kWordsPerThread + j]);
       const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         local[j + q] = sum;
-        sum += tid * kWordsPerThread + j + q < hist_words ? byte_sum(w[q]) : 0u;
+        sum += byte_sum(w[q]);
       }
     }
   }
@@ -1298,28 +1299,36 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
     __syncthreads();
     return true;
   }
-  // Two neighbouring lanes pull one record out of shared memory, a half
-  // each (a quarter warp then reads four whole records: fewer bank conflicts than eight
-  // halves of eight records), and write their four words to four of the eight output arrays.
+  // A lane writes whole records, one word to each of the eight output arrays, so that a warp's store is
+  // 128 bytes side by side and its address the same offset for all arrays.  Of every two
+  // neighbouring lanes one reads its record's first half first and the other its second, so that a
+  // quarter warp's eight halves fall on all banks.  Bound by instructions and the shared-memory pipe: with
+  // two lanes to a record (half as many conflicts, twice the addresses, stores of two times 64 bytes) a call
+  // took 2271 us at 64 M hypersonic, now 2234, and 3932 / 3844 at 128 M moved; 16 M and 1 M alike.
   {
-    const int half = tid & 1;
-    uint32_t* const o0 = half ? reinterpret_cast<uint32_t*>(out.zs) : out.keys;
-    uint32_t* const o1 = half ? reinterpret_cast<uint32_t*>(out.vs)
-                              : reinterpret_cast<uint32_t*>(out.index);
-    uint32_t* const o2 = half ? (out.vs ? reinterpret_cast<uint32_t*>(out.vs + out.padded_sorted) : nullptr)
-                              : reinterpret_cast<uint32_t*>(out.xs);
-    uint32_t* const o3 = half ? (out.vs ? reinterpret_cast<uint32_t*>(out.vs + 2 * out.padded_sorted) : nullptr)
-                              : reinterpret_cast<uint32_t*>(out.ys);
-    int next = tid >> 1 < count ? s.order[tid >> 1] : 0;  // one round ahead of its use
-    for (int d = tid >> 1; d < count; d += kThreads / 2) {
-      const int rec = next;
-      if (d + kThreads / 2 < count) next = s.order[d + kThreads / 2];
-      const uint4 a = *reinterpret_cast<const uint4*>(&s.raw[rec * kRecordWords + 4 * half]);
-      const size_t o = static_cast<size_t>(begin) + d;
-      if (o0) __stcs(o0 + o, a.x);
-      if (o1) __stcs(o1 + o, a.y);
-      if (o2) __stcs(o2 + o, a.z);
-      if (o3) __stcs(o3 + o, a.w);
+    const bool odd = tid & 1;
+    const uint32_t* const half = s.raw + (odd ? 4 : 0);
+    const uint32_t* const other = s.raw + (odd ? 0 : 4);
+    const bool positions = out.xs != nullptr, velocity = out.vs != nullptr;
+    int next = tid < count ? s.order[tid] : 0;  // one round ahead of its use
+    for (int d = tid; d < count; d += kThreads) {
+      const int rec = next * kRecordWords;
+      if (d + kThreads < count) next = s.order[d + kThreads];
+      const uint4 a = *reinterpret_cast<const uint4*>(half + rec);
+      const uint4 b = *reinterpret_cast<const uint4*>(other + rec);
+      const uint32_t o = begin + d;
+      __stcs(out.keys + o, odd ? b.x : a.x);
+      __stcs(reinterpret_cast<uint32_t*>(out.index) + o, odd ? b.y : a.y);
+      if (positions) {
+        __stcs(reinterpret_cast<uint32_t*>(out.xs) + o, odd ? b.z : a.z);
+        __stcs(reinterpret_cast<uint32_t*>(out.ys) + o, odd ? b.w : a.w);
+        __stcs(reinterpret_cast<uint32_t*>(out.zs) + o, odd ? a.x : b.x);
+      }
+      if (velocity) {
+        __stcs(reinterpret_cast<uint32_t*>(out.vs) + o, odd ? a.y : b.y);
+        __stcs(reinterpret_cast<uint32_t*>(out.vs + out.padded_sorted) + o, odd ? a.z : b.z);
+        __stcs(reinterpret_cast<uint32_t*>(out.vs + 2 * out.padded_sorted) + o, odd ? a.w : b.w);
+      }
     }
   }
   __syncthreads();
