@@ -62,7 +62,8 @@ struct alignas(16) Header {
   // One-launch sort: tiles counted and stored, next tile to look at for a block that helps,
   // groups cut, next task and tasks done of the finish.
   uint32_t tiles_counted, tiles_stored, help_next, groups, task_next, tasks_done;
-  uint32_t kept_pad[4];
+  uint32_t settle_failed;     // the sort of a settled state gave the call to the general path
+  uint32_t kept_pad[3];
   uint32_t tile_claimed[kMaxTiles / 32], tile_loose[kMaxTiles / 32];  // one bit per tile
   uint32_t tile_counter[kMaxPasses];  // ticket dispenser of each digit pass
   uint32_t aux_counter[8];
@@ -240,9 +241,9 @@ void set_chained_launches(int mode);
 
 // `heavy`: a kernel that fills the multiprocessors for a long time (scatter, finish); chained
 // only in mode 2.
-template <bool HEAVY = false, class... Params, class... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes,
-                           cudaStream_t stream, Args&&... args) {
+template <class... Params, class... Args>
+cudaError_t launch_chained_if(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block,
+                              size_t shared_bytes, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
@@ -252,8 +253,14 @@ cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
-  config.numAttrs = chained_launches() >= (HEAVY ? 2 : 1) ? 1 : 0;
+  config.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+template <bool HEAVY = false, class... Params, class... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes,
+                           cudaStream_t stream, Args&&... args) {
+  return launch_chained_if(chained_launches() >= (HEAVY ? 2 : 1), kernel, grid, block, shared_bytes,
+                           stream, static_cast<Args&&>(args)...);
 }
 
 // ---- host-side launchers of the kernels (one translation unit each) ----

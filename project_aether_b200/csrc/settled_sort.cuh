@@ -1,0 +1,457 @@
+// The sort of a moved state that starts cell-sorted (included by sort_bucketed.cu).
+//
+// A time-stepping loop sorts the particles, moves them a little, and sorts them again: the input is
+// in the order of the cells its particles were in, and most of them are still there.  The buckets
+// of the general path take every particle through a record in HBM; here only those that left their
+// bucket (movers) travel so, and the others are read from the input where they lie:
+//
+//   settled_scan_kernel    reads the input once and moves the particles: their keys; where every
+//                          bucket's particles lie in the input (its home run; the input must be in
+//                          bucket order, before the move); who leaves which bucket, and the movers'
+//                          records into lists, one per block
+//   settled_sums_kernel,   where every bucket's arrivals and its output begin; groups of buckets
+//   settled_groups_kernel
+//   settled_movers_kernel  the lists' records to their buckets' arrivals
+//   settled_finish_kernel  a block takes a group: reads its home run and keys, moves the particles once
+//                          more, leaves out those that left, adds the arrivals, and sorts and
+//                          writes the group as the general finish kernel does
+//
+// It moves 24 + 4 + 28 + 32 bytes per particle, and some 130 more per mover, where the general path moves
+// 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
+// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3281 (941, 2157).
+//
+// Whether the input is in order is only known on the device.  Whatever speaks against it (a bucket
+// out of order, too many movers, a bucket that no block holds, a counter that wraps) sets
+// Header::settle_failed; the kernels above then stop, and the general path's kernels, which are
+// enqueued behind them and otherwise return at once, do the call from the start.
+
+constexpr int kSettledThreads = 512;
+constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round
+constexpr int kMoverShare = 4;                      // room for one mover in four particles
+constexpr int kSettledPart = 4096;                  // buckets per entry of the coarse sums
+constexpr uint32_t kGone = 0xffffffffu;             // no key: grids of 2^25 cells are left to the general path
+constexpr int kSettledRowWords = 8;                 // words of a group's table
+using FinishSettled = FinishSmall;
+// Records per bucket, on average at most.  Buckets cost this path little (a few words each), and with
+// eight or more to a group the groups fill a block whatever the density.
+constexpr int64_t kSettledTarget = 320;
+// Where single cells hold more than this on average, the buckets of the path would not fit a block.
+constexpr int64_t kSettledMostMean = 1024;
+
+struct SettledArgs {
+  const float *x, *y, *z, *v;
+  int64_t padded, num_cells;
+  int n;
+  PushSpec push;
+  AetherGrid grid;
+  uint32_t k0, k1;
+  int shift, buckets;
+  int per_block;          // particles per block of the scan, a multiple of kSettledRound
+  int scan_blocks;
+  uint32_t capacity;      // places of a group
+  uint32_t *first, *end;            // [buckets] home run in the input; both zero if it is empty
+  uint32_t *leavers, *arrivals;     // [buckets]
+  uint32_t* keys;                   // [n] key of every particle after the move, kGone of those that left
+  uint32_t* list_count;             // [scan_blocks] movers found by each block of the scan
+  uint32_t* cursor;                 // [buckets] next free place of each bucket's arrivals
+  uint32_t* sums;                   // [parts][4] particles at home, arrivals, output of kSettledPart buckets
+  uint32_t* tables;                 // [groups][kSettledRowWords]
+  uint32_t *list, *arrived;         // records: the movers block by block, and bucket by bucket
+  Header* hdr;
+};
+
+__device__ __forceinline__ bool settle_failed(const Header* hdr) {
+  return ld_relaxed(&hdr->settle_failed) != 0;
+}
+__device__ __forceinline__ void fail_settle(Header* hdr) { atomicExch(&hdr->settle_failed, 1u); }
+
+// The move and the cell of a particle with little arithmetic: walls are looked at together, and
+// the reflection is done by the few that hit one.  WHOLE: the slab is the whole grid.
+__device__ __forceinline__ void push_particle(const PushSpec& push, float* f) {
+  bool hit = false;
+  float moved[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    moved[c] = __fadd_rn(f[c], __fmul_rn(f[3 + c], push.dt));
+    hit |= moved[c] < push.lo[c] || moved[c] > push.hi[c];
+  }
+  if (hit) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) push_axis(f[c], f[3 + c], push.dt, push.lo[c], push.hi[c]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c] = moved[c];
+  }
+}
+template <bool WHOLE>
+__device__ __forceinline__ uint32_t settled_cell(float x, float y, float z, const AetherGrid& g) {
+  if (!WHOLE) return cell_of(x, y, z, g);
+  const int ix = axis_index(x, g.x0, g.inv_dx, g.nx);
+  const int iy = axis_index(y, g.y0, g.inv_dy, g.ny);
+  const int iz = axis_index(z, g.z0, g.inv_dz, g.nz);
+  return static_cast<uint32_t>((iz * g.ny + iy) * g.nx + ix);
+}
+
+// What a warp of the scan keeps in shared memory: the movers it has found and not yet stored.  A
+// round adds at most 128 to fewer than 32.
+struct MoverQueue {
+  uint4 record[160][2];  // {cell, index, x, y}, {z, vx, vy, vz}
+};
+
+// Stores 32 (or, at the end, the last `count`) of a warp's movers in the block's list; false if
+// there is no room.
+__device__ __forceinline__ bool flush_movers(const SettledArgs& a, const MoverQueue& queue, int from, int count,
+                                             uint32_t* fill, uint32_t allowed, uint32_t* list) {
+  const int lane = lane_id();
+  uint32_t place = 0;
+  if (lane == 0) place = atomicAdd(fill, static_cast<uint32_t>(count));
+  place = __shfl_sync(0xffffffffu, place, 0);
+  if (place + count > allowed) return false;
+  if (lane < count) {
+    const uint4 lo = queue.record[from + lane][0], hi = queue.record[from + lane][1];
+    atomicAdd(&a.arrivals[lo.x >> a.shift], 1u);
+    store_record(list + static_cast<size_t>(place + lane) * kRecordWords, lo.x, lo.y, __uint_as_float(lo.z),
+                 __uint_as_float(lo.w), __uint_as_float(hi.x), __uint_as_float(hi.y), __uint_as_float(hi.z),
+                 __uint_as_float(hi.w));
+  }
+  __syncwarp();  // the queue is written again
+  return true;
+}
+
+// One round of a block: four particles per thread, from i0 = this thread's first.  FULL: none of the
+// block's round is missing.  Returns what a lane found against the input's order.
+template <bool VEC, bool WHOLE, bool FULL>
+__device__ __forceinline__ bool scan_round(const SettledArgs& a, int i0, int last, MoverQueue& queue, int& queued) {
+  const int lane = lane_id();
+  float f[6][4];
+  if (FULL && VEC) {
+    load_items<4>(a.x + i0, f[0]);
+    load_items<4>(a.y + i0, f[1]);
+    load_items<4>(a.z + i0, f[2]);
+    load_items<4>(a.v + i0, f[3]);
+    load_items<4>(a.v + a.padded + i0, f[4]);
+    load_items<4>(a.v + 2 * a.padded + i0, f[5]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool ok = FULL || last - i0 > k;
+      f[0][k] = ok ? a.x[i0 + k] : 0.f;
+      f[1][k] = ok ? a.y[i0 + k] : 0.f;
+      f[2][k] = ok ? a.z[i0 + k] : 0.f;
+      f[3][k] = ok ? a.v[i0 + k] : 0.f;
+      f[4][k] = ok ? a.v[a.padded + i0 + k] : 0.f;
+      f[5][k] = ok ? a.v[2 * a.padded + i0 + k] : 0.f;
+    }
+  }
+  // The bucket of the particle before a warp's first one.
+  uint32_t before = 0;
+  if (lane == 0 && i0 > 0 && (FULL || i0 < last))
+    before = settled_cell<WHOLE>(a.x[i0 - 1], a.y[i0 - 1], a.z[i0 - 1], a.grid) >> a.shift;
+  uint32_t home[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) home[k] = settled_cell<WHOLE>(f[0][k], f[1][k], f[2][k], a.grid) >> a.shift;
+  const uint32_t left = __shfl_up_sync(0xffffffffu, home[3], 1);
+  if (lane > 0) before = left;
+  bool bad = false;
+  uint32_t found[4], key[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const bool valid = FULL || last - i0 > k;
+    if (valid && home[k] != before && i0 + k > 0) {
+      bad |= home[k] < before;
+      a.first[home[k]] = static_cast<uint32_t>(i0 + k);
+      a.end[before] = static_cast<uint32_t>(i0 + k);
+    }
+    before = home[k];
+    float q[6] = {f[0][k], f[1][k], f[2][k], f[3][k], f[4][k], f[5][k]};
+    push_particle(a.push, q);
+    const uint32_t cell = settled_cell<WHOLE>(q[0], q[1], q[2], a.grid);
+    const bool moved = valid && cell >> a.shift != home[k];
+    found[k] = __ballot_sync(0xffffffffu, moved);
+    key[k] = moved ? kGone : make_key(cell, static_cast<uint32_t>(i0 + k), a.k0, a.k1);
+    if (moved) {
+      atomicAdd(&a.leavers[home[k]], 1u);
+      uint4* to = queue.record[queued + __popc(found[k] & lanemask_lt())];
+      to[0] = make_uint4(cell, static_cast<uint32_t>(i0 + k), __float_as_uint(q[0]), __float_as_uint(q[1]));
+      to[1] = make_uint4(__float_as_uint(q[2]), __float_as_uint(q[3]), __float_as_uint(q[4]), __float_as_uint(q[5]));
+    }
+    queued += __popc(found[k]);
+  }
+  if (FULL) {
+    *reinterpret_cast<uint4*>(a.keys + i0) = make_uint4(key[0], key[1], key[2], key[3]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (last - i0 > k) a.keys[i0 + k] = key[k];
+  }
+  return bad;
+}
+
+// Bound by instructions (73 % of the issue slots; HBM would take half the time).  The home runs are
+// written where a bucket begins and where the bucket before it ends.  A mover costs two adds and a record
+// of {cell, index, moved state}, which goes through the warp's queue so that 32 of them are
+// stored at a time: stored one by one, under a branch per particle, 128 M took 761 us without keys, now 684.  Movers are counted as they are stored, so
+// that an input with too many of them, or one that is in no order at all, is given up within the first rounds.
+template <bool VEC, bool WHOLE>
+__global__ void __launch_bounds__(kSettledThreads, 2)
+settled_scan_kernel(const __grid_constant__ SettledArgs a) {
+  chain_begin();
+  __shared__ uint32_t fill, stop;
+  extern __shared__ MoverQueue queues[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  MoverQueue& queue = queues[tid >> 5];
+  if (tid == 0) fill = stop = 0;
+  __syncthreads();
+  const int block_first = blockIdx.x * a.per_block;
+  const int last = min(a.n - block_first, a.per_block) + block_first;
+  const uint32_t room = static_cast<uint32_t>(a.per_block / kMoverShare);
+  uint32_t* list = a.list + static_cast<size_t>(blockIdx.x) * room * kRecordWords;
+  // The two ends of the input; the places between are the rounds' business.
+  if (tid == 0 && blockIdx.x == 0) a.first[settled_cell<WHOLE>(a.x[0], a.y[0], a.z[0], a.grid) >> a.shift] = 0;
+  if (tid == 0 && last == a.n)
+    a.end[settled_cell<WHOLE>(a.x[last - 1], a.y[last - 1], a.z[last - 1], a.grid) >> a.shift] = static_cast<uint32_t>(a.n);
+  int queued = 0;
+  bool going = true;
+  for (int i = block_first, r = 0; going && i < last; i += kSettledRound, ++r) {
+    const int i0 = i + tid * 4;
+    const bool seen = last - i >= kSettledRound ? scan_round<VEC, WHOLE, true>(a, i0, last, queue, queued)
+                                                : scan_round<VEC, WHOLE, false>(a, i0, last, queue, queued);
+    bool bad = __any_sync(0xffffffffu, seen);  // one answer for the warp, as all below
+    // What the warps of a block may have stored up to their round r, with a few rounds of slack.
+    const uint32_t allowed = min(room, static_cast<uint32_t>(r + 3) * (kSettledRound / kMoverShare));
+    __syncwarp();
+    while (queued >= 32 && !bad) {
+      queued -= 32;
+      bad = !flush_movers(a, queue, queued, 32, &fill, allowed, list);
+    }
+    if (bad) {
+      if (lane == 0) {
+        *static_cast<volatile uint32_t*>(&stop) = 1;
+        fail_settle(a.hdr);
+      }
+      going = false;
+    } else {
+      if (tid == 0 && r % 4 == 3 && settle_failed(a.hdr)) *static_cast<volatile uint32_t*>(&stop) = 1;
+      going = !__any_sync(0xffffffffu, *static_cast<volatile uint32_t*>(&stop));
+    }
+  }
+  if (going && queued > 0 && !flush_movers(a, queue, 0, queued, &fill, room, list) && lane == 0) fail_settle(a.hdr);
+  __syncthreads();
+  if (tid == 0) a.list_count[blockIdx.x] = min(fill, room);
+}
+
+// Particles at home before the move, arrivals and output of every kSettledPart buckets.
+__global__ void __launch_bounds__(1024)
+settled_sums_kernel(const __grid_constant__ SettledArgs a) {
+  chain_begin();
+  if (settle_failed(a.hdr)) return;
+  __shared__ uint32_t sum[3];
+  if (threadIdx.x < 3) sum[threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t home = 0, arrivals = 0, left = 0;
+  const int b0 = blockIdx.x * kSettledPart;
+#pragma unroll
+  for (int k = 0; k < kSettledPart / 1024; ++k) {
+    const int b = b0 + k * 1024 + threadIdx.x;
+    if (b < a.buckets) {
+      home += a.end[b] - a.first[b];
+      arrivals += a.arrivals[b];
+      left += a.leavers[b];
+    }
+  }
+  home = __reduce_add_sync(0xffffffffu, home);
+  arrivals = __reduce_add_sync(0xffffffffu, arrivals);
+  left = __reduce_add_sync(0xffffffffu, left);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&sum[0], home);
+    atomicAdd(&sum[1], arrivals);
+    atomicAdd(&sum[2], home + arrivals - left);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) a.sums[blockIdx.x * 4 + threadIdx.x] = sum[threadIdx.x];
+}
+
+// A block takes kGroupSpan consecutive buckets; it adds up what lies before them for itself (the
+// coarse sums, and the buckets between the last of those and its own).  Groups as in group_kernel; a
+// bucket needs a place for each of its particles at home and each of its arrivals.  A group's
+// table: first particle of its home run, particles in it, first of its arrivals, arrivals, first
+// output slot, records, its buckets b0, b1.
+__global__ void __launch_bounds__(kGroupSpan)
+settled_groups_kernel(const __grid_constant__ SettledArgs a) {
+  chain_begin();
+  // One answer for the block: others may set the word meanwhile.
+  if (__syncthreads_or(threadIdx.x == 0 && settle_failed(a.hdr))) return;
+  __shared__ GroupCut cut;
+  __shared__ uint32_t base[3];  // at home, arrivals, output before the block's buckets
+  __shared__ uint32_t arrived[kGroupSpan + 1], output[kGroupSpan + 1];
+  const int tid = threadIdx.x;
+  const int b0 = blockIdx.x * kGroupSpan;
+  const int here = min(kGroupSpan, a.buckets - b0);
+  if (tid < 3) base[tid] = 0;
+  __syncthreads();
+  uint32_t before[3] = {0, 0, 0};
+  const int part = b0 / kSettledPart;
+  for (int p = tid; p < part; p += kGroupSpan) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) before[c] += a.sums[p * 4 + c];
+  }
+#pragma unroll 4
+  for (int b = part * kSettledPart + tid; b < b0; b += kGroupSpan) {
+    const uint32_t home = a.end[b] - a.first[b], in = a.arrivals[b];
+    before[0] += home;
+    before[1] += in;
+    before[2] += home + in - a.leavers[b];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, before[c]);
+    if ((tid & 31) == 0 && sum) atomicAdd(&base[c], sum);
+  }
+  uint32_t home = 0, in = 0, left = 0;
+  if (tid < here) {
+    home = a.end[b0 + tid] - a.first[b0 + tid];
+    in = a.arrivals[b0 + tid];
+    left = a.leavers[b0 + tid];
+  }
+  // Places (home + arrivals), arrivals and output before each bucket.
+  const uint32_t places = block_exclusive_scan(home + in, cut.warp_sum, &cut.found);
+  cut.start[tid] = places;
+  if (tid == here - 1) cut.start[here] = cut.found;
+  __syncthreads();
+  const uint32_t arrivals = block_exclusive_scan(in, cut.warp_sum, &cut.found);
+  arrived[tid] = arrivals;
+  if (tid == here - 1) arrived[here] = cut.found;
+  __syncthreads();
+  const uint32_t written = block_exclusive_scan(home + in - left, cut.warp_sum, &cut.found);
+  output[tid] = written;
+  if (tid == here - 1) output[here] = cut.found;
+  if (tid < here) a.cursor[b0 + tid] = base[1] + arrivals;
+  __syncthreads();
+  const int most = max(1, FinishSettled::kMaxCells >> a.shift);
+  const uint32_t biggest = cut_groups_of_block(cut, here, kGroupSpanLog, most, a.capacity, &a.hdr->aux_counter[2]);
+  if ((tid & 31) == 0 && biggest > a.capacity) fail_settle(a.hdr);
+  if (tid < static_cast<int>(cut.found)) {
+    const int first = cut.group_first[tid], end = cut.link[first];
+    uint4* table = reinterpret_cast<uint4*>(a.tables + (static_cast<size_t>(cut.list_base) + tid) * kSettledRowWords);
+    const uint32_t in_group = arrived[end] - arrived[first];
+    table[0] = make_uint4(base[0] + cut.start[first] - arrived[first],
+                          cut.start[end] - cut.start[first] - in_group, base[1] + arrived[first], in_group);
+    table[1] = make_uint4(base[2] + output[first], output[end] - output[first],
+                          static_cast<uint32_t>(b0 + first), static_cast<uint32_t>(b0 + end));
+  }
+}
+
+// The movers' records to their buckets, with their keys.
+__global__ void __launch_bounds__(kSettledThreads)
+settled_movers_kernel(const __grid_constant__ SettledArgs a) {
+  chain_begin();
+  if (settle_failed(a.hdr)) return;
+  const uint32_t room = static_cast<uint32_t>(a.per_block / kMoverShare);
+  const uint4* list = reinterpret_cast<const uint4*>(a.list + static_cast<size_t>(blockIdx.x) * room * kRecordWords);
+  const uint32_t count = a.list_count[blockIdx.x];
+#pragma unroll 2
+  for (uint32_t j = threadIdx.x; j < count; j += kSettledThreads) {
+    const uint4 lo = __ldcs(list + 2 * j), hi = __ldcs(list + 2 * j + 1);
+    const uint32_t slot = atomicAdd(&a.cursor[lo.x >> a.shift], 1u);
+    store_record(a.arrived + static_cast<size_t>(slot) * kRecordWords, make_key(lo.x, lo.y, a.k0, a.k1), lo.y,
+                 __uint_as_float(lo.z), __uint_as_float(lo.w), __uint_as_float(hi.x), __uint_as_float(hi.y),
+                 __uint_as_float(hi.z), __uint_as_float(hi.w));
+  }
+}
+
+// Asks for the whole 16-byte pieces of [from, from + bytes) in L2.
+__device__ __forceinline__ void prefetch_range(const void* from, uint32_t bytes) {
+  const uintptr_t p0 = (reinterpret_cast<uintptr_t>(from) + 15) & ~uintptr_t{15};
+  const uintptr_t p1 = (reinterpret_cast<uintptr_t>(from) + bytes) & ~uintptr_t{15};
+  if (p1 > p0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p0), "r"(static_cast<uint32_t>(p1 - p0)) : "memory");
+}
+
+// Bound by instructions: 2157 us for 128 M particles, two blocks per multiprocessor.
+// The finish: groups blockIdx.x, blockIdx.x + gridDim.x, ... of the list.  A thread loads all its
+// particles of a group before the first is used; the group behind is asked into L2 meanwhile.
+__global__ void __launch_bounds__(kSettledThreads, FinishSettled::kBlocks)
+settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_constant__ FinishOut out) {
+  chain_begin();
+  using Shape = FinishSettled;
+  constexpr int kItems = Shape::kItems;
+  const uint32_t groups = a.hdr->aux_counter[2];
+  const int tid = threadIdx.x;
+  // One answer for the block: others may set the word meanwhile.
+  if (__syncthreads_or(tid == 0 && settle_failed(a.hdr))) return;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
+  if (blockIdx.x == 0 && tid == 0) out.cell_start[a.num_cells] = a.n;
+  const uint4* tables = reinterpret_cast<const uint4*>(a.tables);
+  uint32_t g = blockIdx.x;
+  uint4 where{}, what{};
+  if (g < groups) {
+    where = tables[2 * g];
+    what = tables[2 * g + 1];
+  }
+  for (; g < groups; g += gridDim.x) {
+    const int home_first = static_cast<int>(where.x), home = static_cast<int>(where.y);
+    const int places = home + static_cast<int>(where.w);
+    const uint4* arrived = reinterpret_cast<const uint4*>(a.arrived) + 2 * static_cast<size_t>(where.z);
+    const uint32_t begin = what.x;
+    const int count = static_cast<int>(what.y);
+    const int64_t first_cell = static_cast<int64_t>(what.z) << a.shift;
+    const int cells_here = static_cast<int>(
+        min(static_cast<long long>(what.w - what.z) << a.shift, static_cast<long long>(a.num_cells - first_cell)));
+    float f[kItems][6];
+    uint32_t key[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const int r = tid + k * kSettledThreads;
+      if (r < home) {
+        const int i = home_first + r;
+        key[k] = __ldcs(a.keys + i);
+        f[k][0] = __ldcs(a.x + i);
+        f[k][1] = __ldcs(a.y + i);
+        f[k][2] = __ldcs(a.z + i);
+        f[k][3] = __ldcs(a.v + i);
+        f[k][4] = __ldcs(a.v + a.padded + i);
+        f[k][5] = __ldcs(a.v + 2 * a.padded + i);
+      } else if (r < places) {
+        const uint4 lo = __ldcg(arrived + 2 * (r - home)), hi = __ldcg(arrived + 2 * (r - home) + 1);
+        *reinterpret_cast<uint2*>(&s.raw[r * kRecordWords]) = make_uint2(lo.x, lo.y);
+        f[k][0] = __uint_as_float(lo.z);
+        f[k][1] = __uint_as_float(lo.w);
+        f[k][2] = __uint_as_float(hi.x);
+        f[k][3] = __uint_as_float(hi.y);
+        f[k][4] = __uint_as_float(hi.z);
+        f[k][5] = __uint_as_float(hi.w);
+      }
+    }
+    const uint32_t behind = g + gridDim.x;
+    if (behind < groups) {
+      where = tables[2 * behind];
+      what = tables[2 * behind + 1];
+      if (tid < 3) prefetch_range((tid == 0 ? a.x : tid == 1 ? a.y : a.z) + where.x, where.y * 4);
+      else if (tid < 6) prefetch_range(a.v + (tid - 3) * a.padded + where.x, where.y * 4);
+      else if (tid == 6) prefetch_range(a.keys + where.x, where.y * 4);
+      else if (tid == 7) prefetch_range(a.arrived + static_cast<size_t>(where.z) * kRecordWords, where.w * 32);
+    }
+    const int drop = drop_for<Shape>(cells_here);
+    const int hist_words = max(8, cells_here * (32 >> drop));
+    for (int i = tid; i < hist_words; i += kSettledThreads) s.hist[i] = 0;
+    __syncthreads();
+    const bool sorted = sort_placed<Shape>(s, out, places, count, begin, first_cell, cells_here, drop,
+                                           [&](int k, int r, uint2* key_index) {
+      uint32_t* to = &s.raw[r * kRecordWords];
+      if (r < home) {
+        if (key[k] == kGone) return false;
+        push_particle(a.push, f[k]);
+        *key_index = make_uint2(key[k], static_cast<uint32_t>(home_first + r));
+      } else {
+        *key_index = *reinterpret_cast<const uint2*>(to);
+      }
+      *reinterpret_cast<uint4*>(to) =
+          make_uint4(key_index->x, key_index->y, __float_as_uint(f[k][0]), __float_as_uint(f[k][1]));
+      *reinterpret_cast<uint4*>(to + 4) = make_uint4(__float_as_uint(f[k][2]), __float_as_uint(f[k][3]),
+                                                     __float_as_uint(f[k][4]), __float_as_uint(f[k][5]));
+      return true;
+    });
+    if (!sorted && tid == 0) fail_settle(a.hdr);
+  }
+}

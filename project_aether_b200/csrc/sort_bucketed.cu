@@ -59,6 +59,13 @@ namespace {
 constexpr int kRecordWords = 8;     // 32-byte record {key, index, x, y, z, vx, vy, vz}
 constexpr int kKeyRecordWords = 2;  // 8-byte record {key, index} of calls without payload
 
+// The kernels of a general call that is enqueued behind an attempt to sort a settled state
+// (`behind`, see settled_sort.cuh) have nothing to do if that succeeded.  The word they look at is
+// final before the first of them runs.
+__device__ __forceinline__ bool settled_before(const Header* hdr, bool behind) {
+  return behind && ld_relaxed(&hdr->settle_failed) == 0;
+}
+
 // ------------------------------------------------------------------------
 // Upsweep: particles per bucket.
 // ------------------------------------------------------------------------
@@ -136,8 +143,10 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountThreads ? 3 : 1)
 bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
                     PushSpec push, int64_t n, AetherGrid g, int shift, int buckets, int chunk_log,
-                    int64_t per_block, uint32_t* __restrict__ bucket_count) {
+                    int64_t per_block, uint32_t* __restrict__ bucket_count, const Header* hdr,
+                    bool behind) {
   chain_begin();
+  if (settled_before(hdr, behind)) return;
   extern __shared__ uint32_t hist[];
   const int table_words = TABLE == kTableGlobal ? 0
                           : TABLE == kTableShared16 ? (buckets + 1) / 2 : buckets;
@@ -242,8 +251,10 @@ constexpr int kRunScanPart = kRunScanThreads * 4;  // entries of a row per block
 // and after: 4 M particles in 10,000 cells 75 / 10 us, 16 M in 2 M 33 / 15, 128 M in 16 M 89 / 36.
 __global__ void __launch_bounds__(kRunScanThreads)
 run_scan_kernel(const uint32_t* __restrict__ count, int buckets, int chunk_log, uint32_t n,
-                uint32_t* __restrict__ cursor, uint32_t* __restrict__ run_begin) {
+                uint32_t* __restrict__ cursor, uint32_t* __restrict__ run_begin, const Header* hdr,
+                bool behind) {
   chain_begin();
+  if (settled_before(hdr, behind)) return;
   __shared__ uint32_t warp_sum[32];
   __shared__ uint32_t total, before_part;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -356,9 +367,10 @@ bucket_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                       const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
                       PushSpec push, int64_t n, AetherGrid g, uint32_t k0, uint32_t k1, int shift,
                       int buckets, int chunk_log, uint32_t* __restrict__ cursor,
-                      uint32_t* __restrict__ records, const Header* __restrict__ hdr) {
+                      uint32_t* __restrict__ records, const Header* __restrict__ hdr,
+                      bool behind) {
   chain_begin();
-  if (hdr->use_standard) return;
+  if (settled_before(hdr, behind) || hdr->use_standard) return;
   const int64_t groups = (n + ITEMS - 1) / ITEMS;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kScatterThreads;
   const int64_t rounds = (groups + stride - 1) / stride;
@@ -442,10 +454,11 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
                     PushSpec push, int64_t n, AetherGrid g, uint32_t k0, uint32_t k1, int shift,
                     int buckets, int chunk_log, uint32_t* __restrict__ cursor,
-                    uint32_t* __restrict__ records, const Header* __restrict__ hdr) {
+                    uint32_t* __restrict__ records, const Header* __restrict__ hdr,
+                    bool behind) {
   constexpr int kTile = kScatterThreads * ITEMS;
   chain_begin();
-  if (hdr->use_standard) return;
+  if (settled_before(hdr, behind) || hdr->use_standard) return;
   extern __shared__ uint32_t slot_of[];  // a tile's counts, then its first slots
   const int tid = threadIdx.x;
   const int64_t tiles = (n + kTile - 1) / kTile;
@@ -839,21 +852,76 @@ bucket_scatter_segments_kernel(const float* __restrict__ x, const float* __restr
 // whole 16-byte pieces (the finish kernel fetches the tables with 16-byte copies).
 __host__ __device__ inline int table_row_words(int chunks) { return (chunks + 3 + 3) / 4 * 4; }
 
-constexpr int kGroupSpan = 256;        // buckets per block of group_kernel
+constexpr int kGroupSpanLog = 8;
+constexpr int kGroupSpan = 1 << kGroupSpanLog;  // buckets per block of group_kernel
 constexpr int kGroupStagedChunks = 32; // chunks whose run starts the block keeps
+
+// What a block of group_kernel keeps while it cuts its buckets into groups.
+struct GroupCut {
+  uint32_t start[kGroupSpan + 1];  // records before each of the block's buckets
+  uint16_t link[kGroupSpan];       // where a group that began with this bucket would end
+  uint16_t group_first[kGroupSpan], jumps[kGroupSpan + 1];
+  unsigned char is_first[kGroupSpan + 1];
+  uint32_t warp_sum[32], found, list_base;
+};
+
+// Cuts every aligned block of 2^group_shift of the `here` buckets greedily into groups of at most
+// `most` consecutive buckets with at most `capacity` records (each bucket looks up where a group
+// that began with it would end, and those links are followed).  Afterwards group k of the block,
+// k < c.found, has the buckets c.group_first[k] .. c.link[c.group_first[k]], and its place in the
+// list of all groups is c.list_base + k; the list's order is of no consequence.  A bucket that
+// exceeds the capacity on its own is in no group.  Returns the largest bucket of the thread's warp.
+__device__ __forceinline__ uint32_t cut_groups_of_block(GroupCut& c, int here, int group_shift, int most,
+                                                        uint32_t capacity, uint32_t* group_count) {
+  const int tid = threadIdx.x;
+  uint32_t load = 0;
+  const bool first_of_block = tid < here && (tid & ((1 << group_shift) - 1)) == 0;
+  int jump = kGroupSpan;
+  if (tid < here) {
+    load = c.start[tid + 1] - c.start[tid];
+    const int block_end = min(here, ((tid >> group_shift) + 1) << group_shift);
+    int lo = tid + 1, hi = min(block_end, tid + most);  // the last end with start[end] - start[tid] <= capacity
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (c.start[mid] - c.start[tid] <= capacity) lo = mid; else hi = mid - 1;
+    }
+    c.link[tid] = static_cast<uint16_t>(lo);
+    jump = lo < block_end ? lo : kGroupSpan;  // leaves its aligned block: no link
+  }
+  c.is_first[tid] = first_of_block;
+  if (tid == 0) c.is_first[kGroupSpan] = 0;
+  // The groups' first buckets: those reached from the aligned blocks' first buckets along the
+  // links, 2^k links at a time in round k.
+  for (int hops = 1; hops < (1 << group_shift) && hops < kGroupSpan; hops <<= 1) {
+    c.jumps[tid] = static_cast<uint16_t>(jump);
+    if (tid == 0) c.jumps[kGroupSpan] = kGroupSpan;
+    __syncthreads();
+    const bool pass_on = c.is_first[tid];
+    const int to = jump;
+    jump = c.jumps[jump];
+    __syncthreads();
+    if (pass_on) c.is_first[to] = 1;
+  }
+  __syncthreads();
+  if (tid < here && load > capacity) c.is_first[tid] = 0;  // too large for a group
+  if (tid >= here) c.is_first[tid] = 0;
+  const uint32_t mine = c.is_first[tid];
+  const uint32_t place = block_exclusive_scan(mine, c.warp_sum, &c.found);
+  if (mine) c.group_first[place] = static_cast<uint16_t>(tid);
+  if (tid == 0) c.list_base = c.found ? atomicAdd(group_count, c.found) : 0u;
+  __syncthreads();
+  return __reduce_max_sync(0xffffffffu, load);
+}
 
 // A block takes kGroupSpan consecutive buckets.  Bucket starts: the records before bucket b are
 // the records before it in every chunk, sum over c of run_begin[c][b] - (first record of c).
-// Every aligned block of 2^group_shift buckets is then cut greedily into groups of consecutive
-// buckets with at most `capacity` records (each bucket looks up where a group that began with
-// it would end, and those links are followed), and every group gets a table
-// of where its records lie, two rows of table_row_words(chunks) words,
+// The buckets are then cut into groups, and every group gets a table of where its records lie,
+// two rows of table_row_words(chunks) words,
 //   row 0: [c] first record of the group's run in chunk c; [chunks] first output slot of the
 //          group; [chunks + 1], [chunks + 2] its buckets b0, b1
 //   row 1: [c] records of the group in chunks before c; [chunks] records of the group.
-// The order of the groups in the list is of no consequence.  A bucket that exceeds the capacity
-// on its own is not listed: finish_buckets takes it; one above `largest` cannot be
-// finished at all and hands the call over before the scatter runs.
+// A bucket that exceeds the capacity on its own is in no group: finish_buckets takes it; one above
+// `largest` cannot be finished at all and hands the call over before the scatter runs.
 // Bound by latency: with a warp per group for its table and one thread following the links it
 // took 22 us at 4 M particles (1250 buckets), with a chunk's loads one after the other 35 us at
 // 64 M (16 chunks); now 6.5 and 19.
@@ -862,15 +930,13 @@ __global__ void __launch_bounds__(kGroupSpan)
 group_kernel(const uint32_t* __restrict__ run_begin, int buckets, int chunks, int chunk_log,
              const SliceSegments* __restrict__ segments, int group_shift, uint32_t capacity,
              uint32_t largest, uint32_t* __restrict__ bucket_start, uint32_t* __restrict__ tables,
-             uint32_t* __restrict__ group_count, Header* __restrict__ hdr) {
+             uint32_t* __restrict__ group_count, Header* __restrict__ hdr, bool behind) {
   chain_begin();
+  if (settled_before(hdr, behind)) return;
   // Up to kGroupStagedChunks chunks, [chunks][kGroupSpan + 1] each: the first record of every
   // run, and the records before the bucket in the chunks before c.
   extern __shared__ uint32_t staged[];
-  __shared__ uint32_t start[kGroupSpan + 1];
-  __shared__ uint16_t link[kGroupSpan], group_first[kGroupSpan], jumps[kGroupSpan + 1];
-  __shared__ unsigned char is_first[kGroupSpan + 1];
-  __shared__ uint32_t warp_sum[32], found, list_base;
+  __shared__ GroupCut cut;
   const int tid = threadIdx.x, lane = tid & 31;
   const int b0 = blockIdx.x * kGroupSpan;
   const int here = min(kGroupSpan, buckets - b0);
@@ -899,51 +965,18 @@ group_kernel(const uint32_t* __restrict__ run_begin, int buckets, int chunks, in
         sum += s[k] - base[k];
       }
     }
-    start[i] = sum;
+    cut.start[i] = sum;
     bucket_start[b0 + i] = sum;
   }
   __syncthreads();
-  uint32_t load = 0;
-  const bool first_of_block = tid < here && (tid & ((1 << group_shift) - 1)) == 0;
-  int jump = kGroupSpan;
-  if (tid < here) {
-    load = start[tid + 1] - start[tid];
-    const int block_end = min(here, ((tid >> group_shift) + 1) << group_shift);
-    int lo = tid + 1, hi = block_end;  // the last end with start[end] - start[tid] <= capacity
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (start[mid] - start[tid] <= capacity) lo = mid; else hi = mid - 1;
-    }
-    link[tid] = static_cast<uint16_t>(lo);
-    jump = lo < block_end ? lo : kGroupSpan;  // leaves its aligned block: no link
-  }
-  is_first[tid] = first_of_block;
-  if (tid == 0) is_first[kGroupSpan] = 0;
-  const uint32_t biggest = __reduce_max_sync(0xffffffffu, load);
+  const uint32_t biggest = cut_groups_of_block(cut, here, group_shift, 1 << group_shift, capacity, group_count);
   if (lane == 0 && biggest > 0) {
     atomicMax(&hdr->max_bucket, biggest);
     if (biggest > largest) hdr->use_standard = 1;
   }
-  // The groups' first buckets: those reached from the aligned blocks' first buckets along the
-  // links, 2^k links at a time in round k.
-  for (int hops = 1; hops < (1 << group_shift) && hops < kGroupSpan; hops <<= 1) {
-    jumps[tid] = static_cast<uint16_t>(jump);
-    if (tid == 0) jumps[kGroupSpan] = kGroupSpan;
-    __syncthreads();
-    const bool pass_on = is_first[tid];
-    const int to = jump;
-    jump = jumps[jump];
-    __syncthreads();
-    if (pass_on) is_first[to] = 1;
-  }
-  __syncthreads();
-  if (tid < here && load > capacity) is_first[tid] = 0;  // too large for a group
-  if (tid >= here) is_first[tid] = 0;
-  const uint32_t mine = is_first[tid];
-  const uint32_t place = block_exclusive_scan(mine, warp_sum, &found);
-  if (mine) group_first[place] = static_cast<uint16_t>(tid);
-  if (tid == 0) list_base = found ? atomicAdd(group_count, found) : 0u;
-  __syncthreads();
+  const uint32_t found = cut.found, list_base = cut.list_base;
+  const uint32_t* start = cut.start;
+  const uint16_t *link = cut.link, *group_first = cut.group_first;
   // The block's tables are one piece of memory: written word by word in order, whatever group and
   // chunk a word belongs to.
   const int row_words = table_row_words(chunks);
@@ -1130,17 +1163,20 @@ __device__ __forceinline__ int drop_for(int cells) {
   return max(0, low_bits - Shape::kLowBits);
 }
 
-// Sorts the `count` records staged in s.raw (any order) and writes them to the
-// output from slot `begin` on.  The records belong to the cells first_cell ..
+// Sorts the records at the first `places` places of s.raw (any order) and writes them to the
+// output from slot `begin` on; `count` of the places hold a record, the others are passed over.
+// `record_at(k, r, &key_index)`, called once by the thread that has place r as its k-th, tells
+// whether there is one, and its key and index; it may first put the record there.
+// The records belong to the cells first_cell ..
 // first_cell + cells_here - 1 (at most Shape::kMaxCells).  The low key of a record is
 // its key minus the key of the first cell's first shuffle value; the counters resolve
 // all but its `drop` lowest bits, which the tie step orders together with the index.
 // s.hist must be zero over the counters used; the call leaves it overwritten.
 // Returns false if a byte counter wrapped (more than 255 records on one counter).
-template <class Shape>
-__device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOut& out, int count,
+template <class Shape, class RecordAt>
+__device__ __forceinline__ bool sort_placed(FinishSmem<Shape>& s, const FinishOut& out, int places, int count,
                                             uint32_t begin, int64_t first_cell, int cells_here,
-                                            int drop) {
+                                            int drop, RecordAt record_at) {
   constexpr int kThreads = Shape::kThreads, kItems = Shape::kItems;
   constexpr int kWordsPerThread = Shape::kWordsPerThread;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1151,6 +1187,7 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
 
   // Count the low key bits with byte-wide counters; the value an add returns
   // is the record's rank among the records of its counter.
+  constexpr uint32_t kNoRecord = 0xffffffffu;
   uint32_t packed[kItems];  // counter id | rank << 16
   // What orders the records of one counter: dropped key bits, index.  (Read again from the
   // staged record where that is free of bank conflicts, kept in a register otherwise.)
@@ -1167,11 +1204,10 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
     const int r = tid + k * kThreads;
-    packed[k] = 0;
+    packed[k] = kNoRecord;
     if (kKeep) mine[kKeep ? k : 0] = 0;
-    if (r < count) {
-      // Key and index in one access: it costs the same bank conflicts as the key alone.
-      const uint2 key_index = *reinterpret_cast<const uint2*>(&s.raw[r * Shape::kRecordWords]);
+    uint2 key_index;
+    if (r < places && record_at(k, r, &key_index)) {
       const uint32_t low = (key_index.x - key_base) >> drop;
       const int sh = 8 * (low & 3);
       const uint32_t old = atomicAdd(&s.hist[low >> 2], 1u << sh);
@@ -1250,7 +1286,7 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
   for (int k = 0; k < kItems; ++k) {
     const int r = tid + k * kThreads;
     run[k] = 0;
-    if (r < count) {
+    if (packed[k] != kNoRecord) {
       const uint32_t low = packed[k] & 0xffffu, rank = packed[k] >> 16;
       const uint32_t word = s.hist[low >> 2];
       const int sh = 8 * (low & 3);
@@ -1333,6 +1369,19 @@ __device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOu
   }
   __syncthreads();
   return true;
+}
+
+// The same for `count` records that all lie in s.raw.
+template <class Shape>
+__device__ __forceinline__ bool sort_staged(FinishSmem<Shape>& s, const FinishOut& out, int count,
+                                            uint32_t begin, int64_t first_cell, int cells_here,
+                                            int drop) {
+  return sort_placed<Shape>(s, out, count, count, begin, first_cell, cells_here, drop,
+                            [&](int, int r, uint2* key_index) {
+    // Key and index in one access: it costs the same bank conflicts as the key alone.
+    *key_index = *reinterpret_cast<const uint2*>(&s.raw[r * Shape::kRecordWords]);
+    return true;
+  });
 }
 
 // What the finish kernels need to find the records of a range of buckets.
@@ -1526,8 +1575,9 @@ __device__ __forceinline__ void touch_runs(FinishSmem<Shape>& s, int q, const Ru
 template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_device,
-                     int64_t num_cells, FinishOut out, Header* __restrict__ hdr) {
+                     int64_t num_cells, FinishOut out, Header* __restrict__ hdr, bool behind) {
   chain_begin();
+  if (settled_before(hdr, behind)) return;
   const uint32_t groups = *t.group_count;
   if (handed_over(hdr)) return;
   constexpr int kThreads = Shape::kThreads;
@@ -1603,6 +1653,8 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
   }
 }
 
+#include "settled_sort.cuh"
+
 // Buckets first, first + step, ... below `last` that hold at least `at_least` records, one by one:
 // those the kernel above skipped, with more records than its shared memory holds, and those of a
 // group whose counters wrapped.  False if one of them cannot be finished at all.
@@ -1656,8 +1708,9 @@ constexpr int kTailBlocks = Shape::kThreads <= 512 ? 2 : 1;
 template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, kTailBlocks<Shape>)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
-                   DigitPassArgs digits) {
+                   DigitPassArgs digits, bool behind) {
   chain_begin();
+  if (settled_before(hdr, behind)) return;
   const bool all_done = hdr->max_bucket <= capacity && hdr->redo_groups == 0;
   if (!handed_over(hdr) && all_done) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -2285,7 +2338,8 @@ constexpr size_t kMostScanStage = (kStagedScanMax + 2 * (kFlatScanBlock + 1)) * 
 
 cudaError_t launch_groups(cudaStream_t stream, const uint32_t* run_begin, int buckets, int chunks,
                           int chunk_log, const SliceSegments* segments, int group_shift,
-                          uint32_t capacity, uint32_t* start, uint32_t* tables, Header* hdr) {
+                          uint32_t capacity, uint32_t* start, uint32_t* tables, Header* hdr,
+                          bool behind = false) {
   const size_t staged = chunks <= kGroupStagedChunks
                             ? 2 * static_cast<size_t>(chunks) * (kGroupSpan + 1) * sizeof(uint32_t) : 0;
   if (staged > 40 * 1024) {
@@ -2295,12 +2349,16 @@ cudaError_t launch_groups(cudaStream_t stream, const uint32_t* run_begin, int bu
   return launch_chained(group_kernel, (buckets + kGroupSpan - 1) / kGroupSpan, kGroupSpan, staged,
                         stream, run_begin, buckets, chunks, chunk_log, segments, group_shift,
                         capacity, FinishLarge::kLargestBucket, start, tables,
-                        &hdr->aux_counter[1], hdr);
+                        &hdr->aux_counter[1], hdr, behind);
 }
+
+// Chained or not: the heavy kernels of a general call.  Behind a sort of a settled state they usually
+// return at once, and are short.
+bool heavy_chained(bool behind) { return chained_launches() >= (behind ? 1 : 2); }
 
 template <class Shape>
 cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                          const uint32_t* n_on_device = nullptr) {
+                          const uint32_t* n_on_device = nullptr, bool behind = false) {
   const size_t table_bytes = 3 * 2 * static_cast<size_t>(t.row_words) * sizeof(uint32_t);
   if (std::is_same_v<Shape, FinishSmall> && table_bytes > kSmallShapeTableBytes)
     return cudaErrorInvalidValue;
@@ -2308,10 +2366,9 @@ cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut&
   cudaError_t e = allow_shared(bucket_finish_kernel<Shape>,
                                sizeof(FinishSmem<Shape>) + 3 * 2 * kTableRowWords * sizeof(uint32_t));
   if (e != cudaSuccess) return e;
-  e = launch_chained<true>(bucket_finish_kernel<Shape>, std::min(t.buckets, sm_count() * Shape::kBlocks),
-                     Shape::kThreads, smem, a.stream, t, a.n, n_on_device, a.num_cells, out, hdr);
-  if (e != cudaSuccess) return e;
-  return e;
+  return launch_chained_if(heavy_chained(behind), bucket_finish_kernel<Shape>,
+                           std::min(t.buckets, sm_count() * Shape::kBlocks), Shape::kThreads, smem, a.stream,
+                           t, a.n, n_on_device, a.num_cells, out, hdr, behind);
 }
 
 // Buckets in no group (more records than a group may hold) go to the large shape whatever
@@ -2331,27 +2388,28 @@ int limited(int blocks, int most) { return most > 0 ? std::min(blocks, most) : b
 
 template <class Shape>
 cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                        uint32_t group_capacity, const DigitPassArgs& digits) {
+                        uint32_t group_capacity, const DigitPassArgs& digits, bool behind) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
   const cudaError_t e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(sm_count() * kTailBlocks<Shape>, a.n / 2048)));
-  return launch_chained<true>(bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks), Shape::kThreads,
-                              kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity, digits);
+  return launch_chained_if(heavy_chained(behind), bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks),
+                           Shape::kThreads, kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity,
+                           digits, behind);
 }
 
 template <int ITEMS>
 cudaError_t launch_tile_scatter(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, int shift,
                                 int buckets, int chunk_log, uint32_t* cursor, uint32_t* records,
-                                Header* hdr) {
+                                Header* hdr, bool behind) {
   constexpr int kTile = kScatterThreads * ITEMS;
   auto kernel = vec ? tile_scatter_kernel<true, ITEMS> : tile_scatter_kernel<false, ITEMS>;
   const int64_t blocks = std::min<int64_t>((a.n + kTile - 1) / kTile, 2 * sm_count());
-  return launch_chained<true>(kernel, static_cast<int>(blocks), kScatterThreads,
-                              static_cast<size_t>(buckets) * sizeof(uint32_t), a.stream, a.x, a.y,
-                              a.z, a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, shift, buckets,
-                              chunk_log, cursor, records, hdr);
+  return launch_chained_if(heavy_chained(behind), kernel, static_cast<int>(blocks), kScatterThreads,
+                           static_cast<size_t>(buckets) * sizeof(uint32_t), a.stream, a.x, a.y, a.z,
+                           a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, shift, buckets, chunk_log,
+                           cursor, records, hdr, behind);
 }
 
 template <int ITEMS, int THREADS>
@@ -2410,6 +2468,123 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
 }
 }  // namespace
 
+namespace {
+// From how many particles on a moved state is first tried as a settled one, where the general path
+// would reserve its slots tile by tile, and where it would not.  Per call, general / settled: re-sort
+// or step of 2.2 M particles 118 / 107 us, 4 M 184 / 163 (tiles); 8 M 287 / 288, 8 M with 4 particles
+// to a cell 256 / 262, with 40 245 / 258, 12 M 349 / 356 (its scatter is near HBM speed on input that is
+// nearly in order, and the launches count); 16 M 550 / 528, 30 M 832 / 787, 50 M 1470 / 1268, 128 M 3905 /
+// 3281 (the finish kernel's large blocks).
+constexpr int64_t kSettledLeast = int64_t{1} << 21;
+constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
+
+bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+  const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + b_bytes && y < x + a_bytes;
+}
+
+// Whether an output of the call lies over one of its inputs.  The general path reads the inputs for
+// the last time before it writes the first output, so that such calls come out as if there
+// were no overlap; the settled sort reads them while it writes.
+bool outputs_over_inputs(const SortArgs& a) {
+  const size_t row = static_cast<size_t>(a.n) * sizeof(float);
+  const void* in[6] = {a.x, a.y, a.z, a.velocity, a.velocity + a.padded, a.velocity + 2 * a.padded};
+  const void* out[8] = {a.keys_out, a.index_out, a.xs, a.ys, a.zs,
+                        a.vs, a.vs + a.padded_sorted, a.vs + 2 * a.padded_sorted};
+  for (const void* i : in) {
+    for (const void* o : out)
+      if (overlap(i, row, o, row)) return true;
+    if (overlap(i, row, a.cell_counts, static_cast<size_t>(a.num_cells) * 4) ||
+        overlap(i, row, a.cell_start, (static_cast<size_t>(a.num_cells) + 1) * 4))
+      return true;
+  }
+  return false;
+}
+
+// Lays the settled sort out in the `room` bytes at `base` (the general path's records, which that
+// path writes after this one has given up); false if the call is not one for it.
+bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, size_t room, Header* hdr,
+                  SettledArgs* out, size_t* zero_bytes) {
+  if (!a.push.enabled || p.keys_only || !a.velocity || !a.vs || a.n < (p.tiled ? kSettledLeast : kSettledLeastUntiled) ||
+      a.num_cells > (int64_t{1} << 25) - 1 || outputs_over_inputs(a))
+    return false;
+  SettledArgs s{};
+  s.shift = shift_for(a.n, a.num_cells, kSettledTarget, log2_floor(FinishSettled::kMaxCells), 1);
+  const int64_t buckets = (a.num_cells + (int64_t{1} << s.shift) - 1) >> s.shift;
+  if (a.n > kSettledMostMean * buckets || buckets > a.n) return false;
+  s.x = a.x; s.y = a.y; s.z = a.z; s.v = a.velocity;
+  s.padded = a.padded; s.num_cells = a.num_cells;
+  s.n = static_cast<int>(a.n);
+  s.push = a.push;
+  s.grid = a.grid;
+  s.k0 = static_cast<uint32_t>(a.seed);
+  s.k1 = static_cast<uint32_t>(a.seed >> 32);
+  s.buckets = static_cast<int>(buckets);
+  const int64_t most = static_cast<int64_t>(sm_count()) * 2;
+  s.per_block = static_cast<int>(((a.n + most - 1) / most + kSettledRound - 1) / kSettledRound) * kSettledRound;
+  s.scan_blocks = static_cast<int>((a.n + s.per_block - 1) / s.per_block);
+  s.capacity = static_cast<uint32_t>(group_capacity_for(a.n, FinishSettled::kCapacity, FinishSettled::kBlocks));
+  s.hdr = hdr;
+  size_t used = 0;
+  auto take = [&](int64_t words) {
+    auto* at = reinterpret_cast<uint32_t*>(base + used);
+    used = align_up(used + words * sizeof(uint32_t), 256);
+    return at;
+  };
+  s.first = take(buckets);
+  s.end = take(buckets);
+  s.leavers = take(buckets);
+  s.arrivals = take(buckets);
+  *zero_bytes = used;
+  s.keys = take(a.n);
+  s.list_count = take(s.scan_blocks);
+  s.cursor = take(buckets);
+  s.sums = take((buckets + kSettledPart - 1) / kSettledPart * 4);
+  s.tables = take(buckets * kSettledRowWords);
+  const int64_t movers = static_cast<int64_t>(s.scan_blocks) * (s.per_block / kMoverShare);
+  s.list = take(movers * kRecordWords);
+  s.arrived = take(movers * kRecordWords);
+  *out = s;
+  return used <= room;
+}
+
+// Enqueues the sort of a settled state; the general path's kernels follow it.
+cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_bytes, const FinishOut& out) {
+  constexpr int kSmem = static_cast<int>(sizeof(FinishSmem<FinishSettled>));
+  constexpr int kScanSmem = static_cast<int>(sizeof(MoverQueue)) * (kSettledThreads / 32);
+  const bool vec = aligned16(a.x) && aligned16(a.y) && aligned16(a.z) && aligned16(a.velocity) && a.padded % 4 == 0;
+  const bool whole = a.grid.ix_offset == 0 && a.grid.nx_local == a.grid.nx;
+  auto scan = vec ? (whole ? settled_scan_kernel<true, true> : settled_scan_kernel<true, false>)
+                  : (whole ? settled_scan_kernel<false, true> : settled_scan_kernel<false, false>);
+  auto finish = settled_finish_kernel;
+  cudaError_t e = allow_shared(finish, kSmem);
+  if (e == cudaSuccess) e = allow_shared(scan, kScanSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(s.first, 0, zero_bytes, a.stream);
+  if (e != cudaSuccess) return e;
+  stage_begin(kStageBucketCount, a.stream);
+  scan<<<s.scan_blocks, kSettledThreads, kScanSmem, a.stream>>>(s);
+  e = cudaGetLastError();
+  stage_end(kStageBucketCount, a.stream);
+  stage_begin(kStageBucketScan, a.stream);
+  if (e == cudaSuccess)
+    e = launch_chained(settled_sums_kernel, (s.buckets + kSettledPart - 1) / kSettledPart, 1024, 0, a.stream, s);
+  if (e == cudaSuccess)
+    e = launch_chained(settled_groups_kernel, (s.buckets + kGroupSpan - 1) / kGroupSpan, kGroupSpan, 0, a.stream, s);
+  stage_end(kStageBucketScan, a.stream);
+  stage_begin(kStageBucketScatter, a.stream);
+  if (e == cudaSuccess)
+    e = launch_chained(settled_movers_kernel, s.scan_blocks, kSettledThreads, 0, a.stream, s);
+  stage_end(kStageBucketScatter, a.stream);
+  stage_begin(kStageBucketFinish, a.stream);
+  if (e == cudaSuccess)
+    e = launch_chained<true>(finish, sm_count() * FinishSettled::kBlocks, kSettledThreads, kSmem,
+                             a.stream, s, out);
+  count_launches(5);
+  return e;
+}
+}  // namespace
+
 // Enqueues the bucketed path.  When a bucket turns out too large for the finish
 // kernel the device sets Header::use_standard, the kernels between return at once
 // and the tail kernel runs the digit passes.
@@ -2440,8 +2615,21 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   const uint32_t k0 = static_cast<uint32_t>(a.seed), k1 = static_cast<uint32_t>(a.seed >> 32);
   const bool vec = aligned16(a.x) && aligned16(a.y) && aligned16(a.z) &&
                    (!a.velocity || (aligned16(a.velocity) && a.padded % 4 == 0));
+  const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
+                      a.vs, a.padded_sorted};
 
-  stage_begin(kStageBucketCount, a.stream);
+  SettledArgs settled;
+  size_t zero_bytes = 0;
+  const bool behind = settled_args(a, p, base + l.records_off, l.total - l.records_off, hdr, &settled, &zero_bytes);
+  if (behind) {
+    e = settled_sort(a, settled, zero_bytes, out);
+    if (e != cudaSuccess) return e;
+  }
+  // Behind a sort of a settled state the stages are that sort's, and the rest counts as its finish.
+  auto begin_stage = [&](Stage stage) { if (!behind) stage_begin(stage, a.stream); };
+  auto end_stage = [&](Stage stage) { if (!behind) stage_end(stage, a.stream); };
+
+  begin_stage(kStageBucketCount);
   {
     const size_t bytes32 = static_cast<size_t>(buckets) * sizeof(uint32_t);
     const size_t bytes16 = (static_cast<size_t>(buckets) + 1) / 2 * sizeof(uint32_t);
@@ -2465,9 +2653,10 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
       e = allow_shared(kernel, kMostCountTable);                                                  \
       if (e != cudaSuccess) return e;                                                             \
     }                                                                                             \
-    kernel<<<grid, THREADS, table_bytes, a.stream>>>(a.x, a.y, a.z, a.velocity, a.padded, a.push, \
-                                                     a.n, a.grid, p.shift, buckets,               \
-                                                     l.chunk_log, per_block, count);              \
+    e = launch_chained_if(behind && chained_launches() >= 1, kernel, grid, THREADS, table_bytes,  \
+                          a.stream, a.x, a.y, a.z, a.velocity, a.padded, a.push, a.n, a.grid,     \
+                          p.shift, buckets, l.chunk_log, per_block, count, hdr, behind);          \
+    if (e != cudaSuccess) return e;                                                               \
   } while (0)
     if (table == kTableGlobal) AETHER_COUNT_LAUNCH(kTableGlobal, kCountThreads);
     else if (table == kTableShared16) AETHER_COUNT_LAUNCH(kTableShared16, kCountThreadsWide);
@@ -2475,11 +2664,11 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     else AETHER_COUNT_LAUNCH(kTableShared32, kCountThreads);
 #undef AETHER_COUNT_LAUNCH
   }
-  stage_end(kStageBucketCount, a.stream);
+  end_stage(kStageBucketCount);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
 
-  stage_begin(kStageBucketScan, a.stream);
+  begin_stage(kStageBucketScan);
   const int max_cells = p.keys_only ? FinishKeys::kMaxCells
                         : p.small_blocks ? FinishSmall::kMaxCells : FinishLarge::kMaxCells;
   const uint32_t group_capacity = bucket_group_capacity(a.n, p);
@@ -2487,17 +2676,17 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                                    std::max(0, log2_floor(max_cells) - p.shift));
   const dim3 scan_grid((buckets + kRunScanPart - 1) / kRunScanPart, l.chunks);
   e = launch_chained(run_scan_kernel, scan_grid, kRunScanThreads, 0, a.stream, count, buckets,
-                     l.chunk_log, static_cast<uint32_t>(a.n), cursor, run_begin);
+                     l.chunk_log, static_cast<uint32_t>(a.n), cursor, run_begin, hdr, behind);
   if (e == cudaSuccess)
     e = launch_groups(a.stream, run_begin, buckets, l.chunks, l.chunk_log, nullptr, group_shift,
-                      group_capacity, start, tables, hdr);
+                      group_capacity, start, tables, hdr, behind);
   if (e != cudaSuccess) return e;
   count_launches(2);
-  stage_end(kStageBucketScan, a.stream);
+  end_stage(kStageBucketScan);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
 
-  stage_begin(kStageBucketScatter, a.stream);
+  begin_stage(kStageBucketScatter);
   if (p.keys_only && buckets <= kSplitMaxBuckets) {
     // Small inputs take small tiles, so that every block gets one; with so many buckets that a
     // bucket's run in a tile of 8192 is shorter than four records (a 32-byte sector), large inputs
@@ -2514,8 +2703,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     if (e != cudaSuccess) return e;
   } else if (p.tiled) {
     e = a.n >= static_cast<int64_t>(sm_count()) * kScatterThreads * 16
-            ? launch_tile_scatter<8>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr)
-            : launch_tile_scatter<4>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr);
+            ? launch_tile_scatter<8>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind)
+            : launch_tile_scatter<4>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind);
     if (e != cudaSuccess) return e;
   } else {
     constexpr int kItems = 2;
@@ -2527,27 +2716,25 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                                      : bucket_scatter_kernel<false, kItems, kKeyRecordWords>)
                               : (vec ? bucket_scatter_kernel<true, kItems, kRecordWords>
                                      : bucket_scatter_kernel<false, kItems, kRecordWords>);
-    e = launch_chained<true>(kernel, grid, kScatterThreads, 0, a.stream, a.x, a.y, a.z, a.velocity,
-                       a.padded, a.push, a.n, a.grid, k0, k1, p.shift, buckets, l.chunk_log, cursor,
-                       records, hdr);
+    e = launch_chained_if(heavy_chained(behind), kernel, grid, kScatterThreads, 0, a.stream, a.x, a.y, a.z,
+                          a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, p.shift, buckets, l.chunk_log,
+                          cursor, records, hdr, behind);
     if (e != cudaSuccess) return e;
   }
-  stage_end(kStageBucketScatter, a.stream);
+  end_stage(kStageBucketScatter);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   count_launches(2);
 
-  stage_begin(kStageBucketFinish, a.stream);
-  const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
-                      a.vs, a.padded_sorted};
+  begin_stage(kStageBucketFinish);
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
                    table_row_words(l.chunks), l.chunks, buckets, p.shift, p.keys_only ? cursor : nullptr};
   e = p.keys_only      ? launch_finish<FinishKeys>(t, a, out, hdr)
-      : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr)
-                       : launch_finish<FinishLarge>(t, a, out, hdr);
+      : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, behind)
+                       : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, behind);
   if (e == cudaSuccess)
-    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits)
-                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits);
+    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, false)
+                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, behind);
   stage_end(kStageBucketFinish, a.stream);
   count_launches(2);
   return e;

@@ -1,0 +1,185 @@
+"""The sort of a moved state that starts cell-sorted: the settled path and the conditions under
+which it gives the call to the general path.  Against the CPU oracle, bit for bit."""
+
+import numpy as np
+import pytest
+import torch
+
+import project_aether_b200 as pa
+from oracle import sort_oracle as so
+from project_aether_b200 import particle_sort
+
+pytestmark = pytest.mark.gpu
+
+LEAST = 1 << 21  # particles from which on the settled path is tried: while slots are reserved tile by tile
+LEAST_UNTILED = 1 << 24
+SETTLE_FAILED, GROUPS = 12, 54  # words of the workspace header
+
+
+def _route(device):
+    """'settled', 'given up', or 'general' where the settled path was not tried."""
+    torch.cuda.synchronize()
+    workspace = particle_sort._workspaces[(device.index, torch.cuda.current_stream(device).cuda_stream)]
+    words = workspace[:256].view(torch.int32).cpu()
+    if words[SETTLE_FAILED]:
+        return 'given up'
+    return 'settled' if words[GROUPS] else 'general'
+
+
+def _sorted_state(n, cells, device, seed, squeeze=None, drift=0.0, drop=0):
+    """A state in cell order.  `squeeze`: (share, width) of particles pressed into a thin y-layer.
+    `drop`: leading elements cut off, so that the arrays start off 16-byte boundaries."""
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 0.7), cells)
+    gen = torch.Generator(device=device).manual_seed(seed)
+    n += drop
+    x, y, z = (torch.rand(n, device=device, generator=gen) for _ in range(3))
+    z *= 0.7
+    if squeeze:
+        layer = torch.rand(n, device=device, generator=gen) < squeeze[0]
+        y[layer] = 0.5 + squeeze[1] * (y[layer] - 0.5)
+    vel = torch.zeros((3, -(-n // 4) * 4), device=device)
+    vel[:, :n] = torch.randn((3, n), device=device, generator=gen)
+    vel[0, :n] += drift
+    state = pa.sort_and_gather_particles(x, y, z, vel, grid, seed)
+    velocity = state.velocity[:, drop:n] if drop else state.velocity
+    return grid, [t[drop:] for t in state.positions], velocity
+
+
+def _oracle(grid, pos, vel, n, dt, seed):
+    p = [np.ascontiguousarray(t.cpu().numpy()) for t in pos]
+    v = np.ascontiguousarray(vel.cpu().numpy())
+    p, rows = so.push_particles(p, [v[k, :n] for k in range(3)], dt, grid.lo, grid.hi)
+    v[:, :n] = np.stack(rows)
+    return so.c_sort_particles(*[np.ascontiguousarray(a) for a in p], v,
+                               so.Grid(grid.lo, grid.hi, grid.cells), seed)
+
+
+def _check(got, want, n):
+    order, *payload = want
+    np.testing.assert_array_equal(got.order.keys.cpu().numpy().view(np.uint32), order.keys)
+    np.testing.assert_array_equal(got.order.particle_index.cpu().numpy(), order.particle_index)
+    np.testing.assert_array_equal(got.order.cell_counts.cpu().numpy(), order.cell_counts)
+    np.testing.assert_array_equal(got.order.cell_start.cpu().numpy(), order.cell_start)
+    for g, w in zip(got.positions, payload):
+        np.testing.assert_array_equal(g.cpu().numpy(), w)
+    np.testing.assert_array_equal(got.velocity.cpu().numpy()[:, :n], payload[3][:, :n])
+
+
+def _run(grid, pos, vel, dt, device, route, out=None):
+    n, seed = pos[0].numel(), 0x9876543210 + pos[0].numel()
+    want = _oracle(grid, pos, vel, n, dt, seed)
+    got = pa.sort_and_gather_particles(*pos, vel, grid, seed, push=(dt, grid.lo, grid.hi), out=out)
+    assert pa.last_sort_status(device) == 0
+    assert not pa.last_sort_used_digit_passes(device)
+    assert _route(device) == route
+    _check(got, want, n)
+
+
+def _dt(grid, share=0.021):
+    return share / max(c / h for c, h in zip(grid.cells, grid.hi))
+
+
+# The smallest sizes, odd ones, sparse and full cells, cells of a bucket's size and more, and buckets
+# that are no multiple of the spans the tables are made in.
+@pytest.mark.parametrize('n,cells,route', [(LEAST - 1, (64, 64, 64), 'general'), (LEAST, (64, 64, 64), 'settled'),
+                                           (LEAST + 1, (101, 97, 89), 'settled'), (2_300_003, (33, 32, 31), 'settled'),
+                                           (3_000_001, (17, 16, 15), 'settled'), (2_500_000, (13, 11, 9), 'general'),
+                                           (5_000_011, (256, 128, 100), 'settled'),
+                                           (6_291_457, (107, 103, 101), 'general'),
+                                           (LEAST_UNTILED - 1, (128, 128, 128), 'general'),
+                                           (LEAST_UNTILED + 1, (131, 127, 113), 'settled')])
+def test_settled_calls(cuda, n, cells, route):
+    grid, pos, vel = _sorted_state(n, cells, cuda, n)
+    _run(grid, pos, vel, _dt(grid), cuda, route)
+
+
+@pytest.mark.parametrize('drift,share', [(0.0, 0.0), (5.0, 0.021), (-5.0, 0.05)])
+def test_no_movers_and_a_stream_against_a_wall(cuda, drift, share):
+    grid, pos, vel = _sorted_state(LEAST + 77, (80, 64, 64), cuda, 3, drift=drift)
+    _run(grid, pos, vel, _dt(grid, share), cuda, 'settled')
+
+
+@pytest.mark.parametrize('drop', [1, 2, 3])
+def test_unaligned_arrays(cuda, drop):
+    grid, pos, vel = _sorted_state(LEAST + 5, (64, 64, 64), cuda, 4, drop=drop)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+
+
+def test_dense_layer(cuda):
+    grid, pos, vel = _sorted_state(4_000_000, (128, 64, 64), cuda, 5, squeeze=(0.3, 0.1))
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+
+
+def test_buckets_that_no_block_holds(cuda):
+    grid, pos, vel = _sorted_state(4_000_000, (128, 64, 64), cuda, 6, squeeze=(0.7, 0.02))
+    _run(grid, pos, vel, _dt(grid), cuda, 'given up')
+
+
+def test_too_many_movers(cuda):
+    grid, pos, vel = _sorted_state(LEAST, (64, 64, 64), cuda, 7)
+    _run(grid, pos, vel, _dt(grid, 1.0), cuda, 'given up')
+
+
+@pytest.mark.parametrize('where', [0, 777_777, -1])
+def test_one_particle_out_of_order(cuda, where):
+    """Two particles of far-apart buckets change places; -1: the last with the first."""
+    grid, pos, vel = _sorted_state(LEAST + 3, (64, 64, 64), cuda, 8)
+    other = LEAST // 2 if where >= 0 else 0
+    for t in (*pos, *(vel[k] for k in range(3))):
+        t[where], t[other] = t[other].item(), t[where].item()
+    _run(grid, pos, vel, _dt(grid), cuda, 'given up')
+
+
+def test_random_order(cuda):
+    grid, pos, vel = _sorted_state(LEAST + 9, (64, 64, 64), cuda, 9)
+    shuffle = torch.randperm(LEAST + 9, device=cuda)
+    pos = [t[shuffle].contiguous() for t in pos]
+    vel[:, :LEAST + 9] = vel[:, shuffle]
+    _run(grid, pos, vel, _dt(grid), cuda, 'given up')
+
+
+def test_counters_that_wrap(cuda):
+    """Among 512 cells of a group every cell has 32 counters: 2400 particles of one random cell are
+    some 75 on each, but 2400 on one of two cells side by side whose shuffle bits are drawn once per
+    particle never wrap; equal low key bits do.  Here a cell holds what a block still takes."""
+    n, crowd = LEAST + 100, 2_000
+    grid, pos, vel = _sorted_state(n, (128, 128, 128), cuda, 10)
+    for t in pos:
+        t[n // 2:n // 2 + crowd] = t[n // 2].item()
+    vel[:, n // 2:n // 2 + crowd] = 0.0
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+
+
+def test_outputs_over_the_inputs(cuda):
+    n = LEAST + 4
+    grid, pos, vel = _sorted_state(n, (64, 64, 64), cuda, 11)
+    spare = pa.sort_and_gather_particles(*pos, vel, grid, 1)
+    out = particle_sort.SortedParticles(spare.order, tuple(pos), vel)
+    _run(grid, pos, vel, _dt(grid), cuda, 'general', out=out)
+
+
+def test_positions_that_are_no_numbers_and_walls_far_off(cuda):
+    grid, pos, vel = _sorted_state(LEAST, (64, 64, 64), cuda, 12)
+    vel[0, 1000] = float('inf')
+    vel[1, 2000] = float('nan')
+    vel[2, 3000] = 1e30
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+
+
+def test_capture_and_replay(cuda):
+    n = LEAST + 21
+    grid, pos, vel = _sorted_state(n, (64, 64, 64), cuda, 13)
+    dt, seed = _dt(grid), 0x9876543210 + n
+    want = _oracle(grid, pos, vel, n, dt, seed)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        out = pa.sort_and_gather_particles(*pos, vel, grid, seed, push=(dt, grid.lo, grid.hi))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        pa.sort_and_gather_particles(*pos, vel, grid, seed, push=(dt, grid.lo, grid.hi), out=out)
+    for t in (*out.order, *out.positions, out.velocity):
+        t.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    _check(out, want, n)
