@@ -228,12 +228,19 @@ void count_launches(int kernels);
 // (griddepcontrol.launch_dependents) and then waits until the grids before it are complete
 // and their memory visible (griddepcontrol.wait).  Nothing of a kernel's work moves ahead of
 // that wait, so the order of the work is that of the stream.  Launched in the ordinary way
-// the same kernels find nothing to wait for.  Measured per call with payload, ordinary launches /
-// short kernels chained / all chained: 1 M particles 66 / 61 / 56 us, 16 M 553 / 551 / 561, 64 M
-// 2225 / 2258 / 2369; without payload 1 M 57 / 53 / 52, 16 M 356 / 351 / 356, 64 M 1888 / 1884 / 1883.
-__device__ __forceinline__ void chain_begin() {
+// the same kernels find nothing to wait for.  Kernels that fill the multiprocessors for a long time
+// wait with chain_wait() and let the kernel behind them in when a block has done its work
+// (chain_release()): waiting blocks in their midst cost more than the launch.  Per call, only the short
+// kernels chained / these too: without payload 4 M particles 110.8 / 104.0 us, 16 M 348 / 343; with
+// payload 1 M 61 / 56, 16 M 556 / 557, 64 M 2241 / 2373, 256 M 10.7 / 11.0 ms.  So they are chained in
+// calls without payload and in those whose slots are reserved tile by tile.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_begin() {
+  chain_release();
+  chain_wait();
 }
 
 int chained_launches();            // process-wide: 0 none, 1 the short kernels, 2 all

@@ -369,7 +369,7 @@ bucket_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                       int buckets, int chunk_log, uint32_t* __restrict__ cursor,
                       uint32_t* __restrict__ records, const Header* __restrict__ hdr,
                       bool behind) {
-  chain_begin();
+  chain_wait();
   if (settled_before(hdr, behind) || hdr->use_standard) return;
   const int64_t groups = (n + ITEMS - 1) / ITEMS;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kScatterThreads;
@@ -429,6 +429,7 @@ bucket_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                      static_cast<uint32_t>(i0 + k), f[0][k], f[1][k], f[2][k], f[3][k], f[4][k],
                      f[5][k]);
   }
+  chain_release();
 }
 
 // Lanes of a warp that do not agree on a bucket skip the votes for the rest of a tile.
@@ -457,7 +458,7 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     uint32_t* __restrict__ records, const Header* __restrict__ hdr,
                     bool behind) {
   constexpr int kTile = kScatterThreads * ITEMS;
-  chain_begin();
+  chain_wait();
   if (settled_before(hdr, behind) || hdr->use_standard) return;
   extern __shared__ uint32_t slot_of[];  // a tile's counts, then its first slots
   const int tid = threadIdx.x;
@@ -529,6 +530,7 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
     }
     __syncthreads();  // the table is reused by the next tile
   }
+  chain_release();
 }
 
 // ------------------------------------------------------------------------
@@ -559,7 +561,7 @@ key_split_kernel(const float* __restrict__ x, const float* __restrict__ y,
                  uint2* __restrict__ records, const Header* __restrict__ hdr) {
   static_assert(ITEMS % 4 == 0, "whole 16-byte loads");
   constexpr int kTile = THREADS * ITEMS;
-  chain_begin();
+  chain_wait();
   if (hdr->use_standard) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint32_t warp_sum[2][32];
@@ -655,6 +657,7 @@ key_split_kernel(const float* __restrict__ x, const float* __restrict__ y,
     }
     __syncthreads();  // the tables and the stage are reused by the next tile
   }
+  chain_release();
 }
 
 // ------------------------------------------------------------------------
@@ -1576,7 +1579,7 @@ template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_device,
                      int64_t num_cells, FinishOut out, Header* __restrict__ hdr, bool behind) {
-  chain_begin();
+  chain_wait();
   if (settled_before(hdr, behind)) return;
   const uint32_t groups = *t.group_count;
   if (handed_over(hdr)) return;
@@ -1651,6 +1654,7 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
       if (g + 2 * stride < groups) touch_runs<Shape, false>(s, q2, t);
     }
   }
+  chain_release();
 }
 
 #include "settled_sort.cuh"
@@ -1709,7 +1713,7 @@ template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, kTailBlocks<Shape>)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
                    DigitPassArgs digits, bool behind) {
-  chain_begin();
+  chain_wait();
   if (settled_before(hdr, behind)) return;
   const bool all_done = hdr->max_bucket <= capacity && hdr->redo_groups == 0;
   if (!handed_over(hdr) && all_done) return;
@@ -2352,13 +2356,16 @@ cudaError_t launch_groups(cudaStream_t stream, const uint32_t* run_begin, int bu
                         &hdr->aux_counter[1], hdr, behind);
 }
 
-// Chained or not: the heavy kernels of a general call.  Behind a sort of a settled state they usually
-// return at once, and are short.
-bool heavy_chained(bool behind) { return chained_launches() >= (behind ? 1 : 2); }
+// Whether the kernels of a call that take long are chained (see chain_begin); those behind a sort of a
+// settled state usually return at once.
+bool heavy_chained(const BucketPlan& p, bool behind) {
+  return chained_launches() >= (behind || p.keys_only || p.tiled ? 1 : 2);
+}
 
 template <class Shape>
 cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                          const uint32_t* n_on_device = nullptr, bool behind = false) {
+                          const uint32_t* n_on_device = nullptr, bool behind = false,
+                          bool chained = false) {
   const size_t table_bytes = 3 * 2 * static_cast<size_t>(t.row_words) * sizeof(uint32_t);
   if (std::is_same_v<Shape, FinishSmall> && table_bytes > kSmallShapeTableBytes)
     return cudaErrorInvalidValue;
@@ -2366,7 +2373,7 @@ cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut&
   cudaError_t e = allow_shared(bucket_finish_kernel<Shape>,
                                sizeof(FinishSmem<Shape>) + 3 * 2 * kTableRowWords * sizeof(uint32_t));
   if (e != cudaSuccess) return e;
-  return launch_chained_if(heavy_chained(behind), bucket_finish_kernel<Shape>,
+  return launch_chained_if(chained, bucket_finish_kernel<Shape>,
                            std::min(t.buckets, sm_count() * Shape::kBlocks), Shape::kThreads, smem, a.stream,
                            t, a.n, n_on_device, a.num_cells, out, hdr, behind);
 }
@@ -2388,13 +2395,13 @@ int limited(int blocks, int most) { return most > 0 ? std::min(blocks, most) : b
 
 template <class Shape>
 cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                        uint32_t group_capacity, const DigitPassArgs& digits, bool behind) {
+                        uint32_t group_capacity, const DigitPassArgs& digits, bool behind, bool chained) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
   const cudaError_t e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(sm_count() * kTailBlocks<Shape>, a.n / 2048)));
-  return launch_chained_if(heavy_chained(behind), bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks),
+  return launch_chained_if(chained, bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks),
                            Shape::kThreads, kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity,
                            digits, behind);
 }
@@ -2402,11 +2409,11 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
 template <int ITEMS>
 cudaError_t launch_tile_scatter(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, int shift,
                                 int buckets, int chunk_log, uint32_t* cursor, uint32_t* records,
-                                Header* hdr, bool behind) {
+                                Header* hdr, bool behind, bool chained) {
   constexpr int kTile = kScatterThreads * ITEMS;
   auto kernel = vec ? tile_scatter_kernel<true, ITEMS> : tile_scatter_kernel<false, ITEMS>;
   const int64_t blocks = std::min<int64_t>((a.n + kTile - 1) / kTile, 2 * sm_count());
-  return launch_chained_if(heavy_chained(behind), kernel, static_cast<int>(blocks), kScatterThreads,
+  return launch_chained_if(chained, kernel, static_cast<int>(blocks), kScatterThreads,
                            static_cast<size_t>(buckets) * sizeof(uint32_t), a.stream, a.x, a.y, a.z,
                            a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, shift, buckets, chunk_log,
                            cursor, records, hdr, behind);
@@ -2414,7 +2421,7 @@ cudaError_t launch_tile_scatter(const SortArgs& a, bool vec, uint32_t k0, uint32
 
 template <int ITEMS, int THREADS>
 cudaError_t launch_split(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, int shift, int buckets,
-                         int chunk_log, uint32_t* cursor, uint32_t* records, Header* hdr) {
+                         int chunk_log, uint32_t* cursor, uint32_t* records, Header* hdr, bool chained) {
   constexpr int kTile = THREADS * ITEMS;
   const size_t bytes = split_smem_bytes(kTile, buckets);
   auto kernel = vec ? key_split_kernel<true, ITEMS, THREADS> : key_split_kernel<false, ITEMS, THREADS>;
@@ -2424,7 +2431,7 @@ cudaError_t launch_split(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, 
   if (e != cudaSuccess) return e;
   const int64_t blocks = std::min<int64_t>((a.n + kTile - 1) / kTile,
                                            (THREADS <= 512 ? 2 : 1) * sm_count());
-  return launch_chained<true>(kernel, static_cast<int>(blocks), THREADS, bytes, a.stream, a.x,
+  return launch_chained_if(chained, kernel, static_cast<int>(blocks), THREADS, bytes, a.stream, a.x,
                               a.y, a.z, a.n, a.grid, k0, k1, shift, buckets, chunk_log, cursor,
                               reinterpret_cast<uint2*>(records), hdr);
 }
@@ -2471,11 +2478,11 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
 namespace {
 // From how many particles on a moved state is first tried as a settled one, where the general path
 // would reserve its slots tile by tile, and where it would not.  Per call, general / settled: re-sort
-// or step of 2.2 M particles 118 / 107 us, 4 M 184 / 163 (tiles); 8 M 287 / 288, 8 M with 4 particles
+// or step of 1 M particles 70 / 73 us, 1.5 M 89 / 80, 4 M 184 / 163, 6 M 230 / 200 (tiles); 8 M 287 / 288, 8 M with 4 particles
 // to a cell 256 / 262, with 40 245 / 258, 12 M 349 / 356 (its scatter is near HBM speed on input that is
 // nearly in order, and the launches count); 16 M 550 / 528, 30 M 832 / 787, 50 M 1470 / 1268, 128 M 3905 /
 // 3281 (the finish kernel's large blocks).
-constexpr int64_t kSettledLeast = int64_t{1} << 21;
+constexpr int64_t kSettledLeast = int64_t{3} << 19;
 constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
 
 bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
@@ -2625,6 +2632,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     e = settled_sort(a, settled, zero_bytes, out);
     if (e != cudaSuccess) return e;
   }
+  const bool chained = heavy_chained(p, behind);
   // Behind a sort of a settled state the stages are that sort's, and the rest counts as its finish.
   auto begin_stage = [&](Stage stage) { if (!behind) stage_begin(stage, a.stream); };
   auto end_stage = [&](Stage stage) { if (!behind) stage_end(stage, a.stream); };
@@ -2699,12 +2707,14 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                         : a.n >= 2 * sms * kSplitThreads * 16 ? launch_split<16, kSplitThreads>
                         : a.n >= 2 * sms * kSplitThreads * 8  ? launch_split<8, kSplitThreads>
                                                               : launch_split<4, kSplitThreads>;
-    e = launch(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr);
+    e = launch(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, chained);
     if (e != cudaSuccess) return e;
   } else if (p.tiled) {
     e = a.n >= static_cast<int64_t>(sm_count()) * kScatterThreads * 16
-            ? launch_tile_scatter<8>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind)
-            : launch_tile_scatter<4>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind);
+            ? launch_tile_scatter<8>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind,
+                                     chained)
+            : launch_tile_scatter<4>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind,
+                                     chained);
     if (e != cudaSuccess) return e;
   } else {
     constexpr int kItems = 2;
@@ -2716,7 +2726,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                                      : bucket_scatter_kernel<false, kItems, kKeyRecordWords>)
                               : (vec ? bucket_scatter_kernel<true, kItems, kRecordWords>
                                      : bucket_scatter_kernel<false, kItems, kRecordWords>);
-    e = launch_chained_if(heavy_chained(behind), kernel, grid, kScatterThreads, 0, a.stream, a.x, a.y, a.z,
+    e = launch_chained_if(chained, kernel, grid, kScatterThreads, 0, a.stream, a.x, a.y, a.z,
                           a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, p.shift, buckets, l.chunk_log,
                           cursor, records, hdr, behind);
     if (e != cudaSuccess) return e;
@@ -2729,12 +2739,12 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   begin_stage(kStageBucketFinish);
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
                    table_row_words(l.chunks), l.chunks, buckets, p.shift, p.keys_only ? cursor : nullptr};
-  e = p.keys_only      ? launch_finish<FinishKeys>(t, a, out, hdr)
-      : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, behind)
-                       : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, behind);
+  e = p.keys_only      ? launch_finish<FinishKeys>(t, a, out, hdr, nullptr, behind, chained)
+      : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, behind, chained)
+                       : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, behind, chained);
   if (e == cudaSuccess)
-    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, false)
-                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, behind);
+    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, behind, chained)
+                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, behind, chained);
   stage_end(kStageBucketFinish, a.stream);
   count_launches(2);
   return e;

@@ -11,7 +11,7 @@ from project_aether_b200 import particle_sort
 
 pytestmark = pytest.mark.gpu
 
-LEAST = 1 << 21  # particles from which on the settled path is tried: while slots are reserved tile by tile
+LEAST = 3 << 19  # particles from which on the settled path is tried: while slots are reserved tile by tile
 LEAST_UNTILED = 1 << 24
 SETTLE_FAILED, GROUPS = 12, 54  # words of the workspace header
 
