@@ -433,7 +433,7 @@ settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_consta
       else if (tid == 7) prefetch_range(a.arrived + static_cast<size_t>(where.z) * kRecordWords, where.w * 32);
     }
     const int drop = drop_for<Shape>(cells_here);
-    const int hist_words = max(8, cells_here * (32 >> drop));
+    const int hist_words = counter_words(cells_here, drop);
     for (int i = tid; i < hist_words; i += kSettledThreads) s.hist[i] = 0;
     __syncthreads();
     const bool sorted = sort_placed<Shape>(s, out, places, count, begin, first_cell, cells_here, drop,
