@@ -10,6 +10,8 @@ symbol from it raises.
 import ctypes
 import os
 
+from .cell_grid import CellGrid
+
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIBRARY_PATH = os.path.join(_PKG, 'libaether_sort.so')
 
@@ -131,6 +133,11 @@ _SIGNATURES = {
 }
 
 _library = None
+binding = None        # the native binding, once the library is loaded
+bound_library = None  # the library it calls
+
+_BOUND = ('AetherSortWorkspaceBytes', 'AetherSortParticlesByCell', 'AetherSortAndGatherParticles',
+          'AetherPushSortAndGatherParticles', 'AetherDsmcCollideTma')
 
 
 def exported_symbols():
@@ -147,7 +154,7 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
     Raises:
       OSError: if the library is not built or cannot be loaded.
     """
-    global _library
+    global _library, binding, bound_library
     if _library is not None and path is None:
         return _library
     lib_path = path or os.environ.get('AETHER_SORT_LIBRARY') or LIBRARY_PATH
@@ -159,7 +166,15 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         fn.restype = restype
         fn.argtypes = argtypes
     if path is None:
-        _library = library
+        try:
+            from . import _binding
+        except ImportError as e:
+            raise OSError('the Python binding is not built or does not fit the installed PyTorch; '
+                          'run `python -m project_aether_b200.build`') from e
+        _binding.bind(CellGrid, *(ctypes.cast(getattr(library, name), ctypes.c_void_p).value
+                                  for name in _BOUND))
+        _library = bound_library = library
+        binding = _binding
     return library
 
 

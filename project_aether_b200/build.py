@@ -1,19 +1,22 @@
-"""Builds libaether_sort.so for sm_100a with nvcc, in the package folder.
+"""Builds libaether_sort.so for sm_100a with nvcc, and the Python binding, in the package folder.
 
     python -m project_aether_b200.build [--force] [--verbose]
 
 The library is a plain C-ABI shared object (see include/aether_sort.h); it is
-loaded with ctypes and needs no Python headers.
+loaded with ctypes and needs no Python headers.  The binding (csrc/binding.cpp) is a
+Python extension built against the installed PyTorch, which calls that library.
 """
 
 import argparse
 import os
 import shutil
 import subprocess
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, 'csrc')
 LIB = os.path.join(PKG, 'libaether_sort.so')
+BINDING = os.path.join(PKG, '_binding.so')
 SOURCES = ['api.cu', 'sort_standard.cu', 'sort_bucketed.cu', 'slab_partition.cu', 'particle_push.cu',
            'static_scratch.cu', 'collide.cu']
 NVCC_FLAGS = [
@@ -29,28 +32,45 @@ def _nvcc() -> str:
     raise RuntimeError('nvcc not found; the CUDA library cannot be built')
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB):
+def _stale(target: str, sources) -> bool:
+    if not os.path.exists(target):
         return True
-    built = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
-    deps.append(os.path.join(os.path.dirname(PKG), 'include', 'aether_sort.h'))
-    return any(os.path.getmtime(d) > built for d in deps)
+    built = os.path.getmtime(target)
+    return any(os.path.getmtime(d) > built for d in sources)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compiles every CUDA source into libaether_sort.so; returns its path."""
-    if not force and not _stale():
-        return LIB
-    flags = [f for f in NVCC_FLAGS if not f.startswith('--use_fast_math')]
-    if verbose:
-        flags += ['-Xptxas', '-v']
-    cmd = [_nvcc(), *flags, '-ccbin', 'g++', '-o', LIB] + [os.path.join(CSRC, s) for s in SOURCES]
+def _run(cmd, verbose: bool) -> None:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or proc.returncode != 0:
         print(proc.stdout + proc.stderr)
     if proc.returncode != 0:
-        raise RuntimeError('nvcc failed:\n' + proc.stderr[-4000:])
+        raise RuntimeError(f'{cmd[0]} failed:\n' + proc.stderr[-4000:])
+
+
+def _binding_command():
+    import torch
+    root = os.path.dirname(torch.__file__)
+    includes = [sysconfig.get_paths()['include'], os.path.join(root, 'include'),
+                os.path.join(root, 'include', 'torch', 'csrc', 'api', 'include'),
+                os.path.join(os.path.dirname(os.path.dirname(_nvcc())), 'include')]
+    return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared',
+            f'-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}',
+            *(f'-I{d}' for d in includes), '-o', BINDING, os.path.join(CSRC, 'binding.cpp'),
+            '-L' + os.path.join(root, 'lib'), '-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_python']
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compiles every CUDA source into libaether_sort.so, and the binding; returns the library's path."""
+    header = os.path.join(os.path.dirname(PKG), 'include', 'aether_sort.h')
+    binding = os.path.join(CSRC, 'binding.cpp')
+    if force or _stale(BINDING, [binding, header]):
+        _run(_binding_command(), verbose)
+    kernels = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f != 'binding.cpp']
+    if force or _stale(LIB, [*kernels, header]):
+        flags = [f for f in NVCC_FLAGS if not f.startswith('--use_fast_math')]
+        if verbose:
+            flags += ['-Xptxas', '-v']
+        _run([_nvcc(), *flags, '-ccbin', 'g++', '-o', LIB] + [os.path.join(CSRC, s) for s in SOURCES], verbose)
     return LIB
 
 

@@ -77,6 +77,10 @@ def collide(library: ctypes.CDLL, velocity: torch.Tensor, cell_start: torch.Tens
     Raises:
       RuntimeError: if the launch fails.
     """
+    if library is _native.bound_library and _native.binding.collide(
+            velocity, cell_start, sigma_g_max, collisions, num_particles, params.selection_factor,
+            params.vhs_coefficient, params.vhs_exponent, params.seed, params.step):
+        return
     if velocity.dim() != 2 or velocity.shape[0] != 3 or (
             velocity.shape[1] > 0 and (velocity.stride(1) != 1
                                        or velocity.stride(0) != velocity.shape[1])):

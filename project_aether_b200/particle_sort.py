@@ -10,6 +10,9 @@ caller gets cell-sorted positions and velocities from one call.
 
 All device work is done by libaether_sort.so (hand-written sm_100a kernels)
 through its C ABI; PyTorch only provides device memory and the current stream.
+Calls in their plain form go through the native binding (csrc/binding.cpp), which makes
+the same checks and the same call with less host time; it leaves every other call to the
+code here.
 
 Typical usage example:
 
@@ -125,6 +128,10 @@ def sort_particles_by_cell(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
         the keys would need more than 32 bits.
       RuntimeError: if a kernel launch fails.
     """
+    if _native.binding is not None and ix_offset == 0 and nx_local is None:
+        result = _native.binding.sort(x, y, z, grid, seed, _workspaces)
+        if result is not None:
+            return SortResult(*result)
     x, y, z = _check_positions(x, y, z)
     lib = _native.load_library()
     g = native_grid(grid, ix_offset, nx_local)
@@ -178,6 +185,11 @@ def sort_and_gather_particles(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor,
       SortedParticles(order, (x, y, z) sorted, velocity sorted (3, padded) with
       zero padding columns).
     """
+    if _native.binding is not None and ix_offset == 0 and nx_local is None:
+        result = _native.binding.gather(x, y, z, velocity, grid, seed, path, padded_out, out, push,
+                                        _workspaces)
+        if result is not None:
+            return SortedParticles(SortResult(*result[:4]), result[4:7], result[7])
     x, y, z = _check_positions(x, y, z)
     n, device = x.numel(), x.device
     if (not isinstance(velocity, torch.Tensor) or not velocity.is_cuda

@@ -1,0 +1,189 @@
+"""The native binding takes the plain form of a call; every other form goes through the Python code
+and comes out the same, errors included."""
+
+import numpy as np
+import pytest
+import torch
+
+import project_aether_b200 as pa
+from project_aether_b200 import _native, ntc_collide
+
+N, CELLS = 5_003, (8, 7, 6)
+GRID = pa.CellGrid((0., 0., 0.), (1., 1., 0.5), CELLS)
+
+
+@pytest.fixture(scope='module')
+def binding():
+    _native.load_library()
+    return _native.binding
+
+
+def _state(device, n=N, seed=0):
+    gen = torch.Generator().manual_seed(seed)
+    pos = [torch.rand(n, generator=gen).to(device) for _ in range(3)]
+    vel = torch.zeros((3, -(-n // 4) * 4))
+    vel[:, :n] = torch.randn((3, n), generator=gen)
+    return pos, vel.to(device)
+
+
+def test_host_tensors_and_wrong_types_are_left_to_the_python_code(binding):
+    pos, vel = _state('cpu')
+    assert binding.sort(*pos, GRID, 1, {}) is None
+    assert binding.gather(*pos, vel, GRID, 1, 0, None, None, None, {}) is None
+    assert binding.collide(vel, pos[0], pos[0], pos[0], N, 1.0, 1.0, 0.5, 1, 1) is None
+    assert binding.sort(1, None, 'x', GRID, 1, {}) is None
+    assert binding.sort(*pos, GRID, 1) is None
+    with pytest.raises(TypeError):
+        binding.bind(1, 2)
+
+
+def _flat(result):
+    if isinstance(result, pa.SortResult):
+        return list(result)
+    return [*result.order, *result.positions, result.velocity]
+
+
+def _count_plain(monkeypatch, name):
+    """How many calls of `name` the binding takes, from here on."""
+    taken = []
+    inner = getattr(_native.binding, name)
+
+    class Watched:
+        def __getattr__(self, other):
+            if other != name:
+                return getattr(real, other)
+
+            def call(*args):
+                out = inner(*args)
+                taken.append(out is not None)
+                return out
+            return call
+
+    real = _native.binding
+    monkeypatch.setattr(_native, 'binding', Watched())
+    return taken
+
+
+def _sort_forms(pos, vel):
+    """(positions, grid, seed, whether the call is a plain one)"""
+    x, y, z = pos
+    wide = torch.stack([x, x], 1)
+    yield (x, y, z), GRID, 77, True
+    yield (x, y, z), pa.CellGrid([0, 0, 0], [1, 1, 0.5], list(CELLS)), 77, True
+    yield (wide[:, 0], y, z), GRID, 77, False
+    yield (x.view(-1, 1), y.view(1, -1), z), GRID, 77, False
+    yield (x, y, z), pa.CellGrid(np.zeros(3), np.array([1., 1., 0.5]), CELLS), 77, False
+    yield (x, y, z), GRID, np.int64(77), False
+    yield (x, y, z), type('Grid', (pa.CellGrid,), {})(*GRID), 77, False
+    yield tuple(torch.nn.Parameter(t) for t in pos), GRID, 77, True
+
+
+@pytest.mark.gpu
+def test_every_form_of_the_sort_comes_out_the_same(cuda, binding, monkeypatch):
+    pos, vel = _state(cuda)
+    want = pa.sort_particles_by_cell(*pos, GRID, 77, ix_offset=0, nx_local=CELLS[0])  # not plain
+    taken = _count_plain(monkeypatch, 'sort')
+    for positions, grid, seed, plain in _sort_forms(pos, vel):
+        got = pa.sort_particles_by_cell(*positions, grid, seed)
+        assert taken.pop() is plain
+        assert isinstance(got, pa.SortResult)
+        for g, w in zip(got, want):
+            assert g.dtype == w.dtype and g.shape == w.shape and torch.equal(g, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('push', [None, (0.01, (0., 0., 0.), (1., 1., 0.5)), (0.01, [0, 0, 0], [1, 1, 0.5]),
+                                  (np.float32(0.01), (0., 0., 0.), (1., 1., 0.5))])
+def test_every_form_of_the_gather_comes_out_the_same(cuda, binding, monkeypatch, push):
+    pos, vel = _state(cuda)
+    want = pa.sort_and_gather_particles(*pos, vel, GRID, 5, push=push, ix_offset=0, nx_local=CELLS[0])
+    taken = _count_plain(monkeypatch, 'gather')
+    plain_push = push is None or isinstance(push[0], float)
+    spare = pa.sort_and_gather_particles(*pos, vel, GRID, 9)
+    taken.clear()
+    strided = torch.zeros((3, 2 * vel.shape[1]), device=cuda)
+    strided[:, ::2] = vel
+    rows = torch.zeros((3, N + 101), device=cuda)
+    rows[:, :N] = vel[:, :N]
+    for velocity, plain, extra in ((vel, True, {}), (vel, True, {'path': 2}), (vel, True, {'padded_out': N + 5}),
+                                   (vel, True, {'out': spare}), (strided[:, ::2], False, {}), (rows[:, :N], True, {})):
+        got = pa.sort_and_gather_particles(*pos, velocity, GRID, 5, push=push, **extra)
+        assert taken.pop() is (plain and plain_push)
+        flat = _flat(got)
+        for k, (g, w) in enumerate(zip(flat, _flat(want))):
+            if k == 7:
+                assert torch.equal(g[:, :N], w[:, :N]) and not g[:, N:].any()
+            else:
+                assert g.dtype == w.dtype and torch.equal(g, w)
+        if 'out' in extra:
+            assert all(g is s for g, s in zip(flat, _flat(spare)))
+        else:
+            assert not any(t._is_view() for t in flat)
+
+
+@pytest.mark.gpu
+def test_errors_are_those_of_the_python_code(cuda, binding):
+    pos, vel = _state(cuda)
+    x, y, z = pos
+    for bad in ((x.double(), y, z), (x[:-1], y, z), (x.cpu(), y, z), (x, y, None)):
+        with pytest.raises(ValueError, match='float32 CUDA'):
+            pa.sort_particles_by_cell(*bad, GRID, 1)
+    with pytest.raises(ValueError, match='32 bits|bits'):
+        pa.sort_particles_by_cell(x, y, z, pa.CellGrid((0., 0., 0.), (1., 1., 1.), (1024, 1024, 64)), 1)
+    for bad in (vel.double(), vel[:2], vel[:, :100], vel.cpu()):
+        with pytest.raises(ValueError, match='Velocity'):
+            pa.sort_and_gather_particles(x, y, z, bad, GRID, 1)
+    with pytest.raises(ValueError, match='padded_out'):
+        pa.sort_and_gather_particles(x, y, z, vel, GRID, 1, padded_out=N - 1)
+    with pytest.raises(ValueError, match='does not match'):
+        pa.sort_and_gather_particles(x, y, z, vel, GRID, 1,
+                                     out=pa.sort_and_gather_particles(x[1:], y[1:], z[1:], vel, GRID, 1))
+    with pytest.raises(AttributeError):
+        pa.sort_particles_by_cell(x, y, z, tuple(GRID), 1)
+    with pytest.raises(ZeroDivisionError):
+        pa.sort_particles_by_cell(x, y, z, pa.CellGrid((0., 0., 0.), (0., 1., 1.), CELLS), 1)
+
+
+@pytest.mark.gpu
+def test_watched_calls_are_left_to_the_python_code(cuda, binding):
+    """Modes and transforms that see the operations of a call; the workspace is there."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from project_aether_b200 import particle_sort
+    pos, vel = _state(cuda)
+    pa.sort_particles_by_cell(*pos, GRID, 1)
+    call = lambda *p: binding.sort(*p, GRID, 1, particle_sort._workspaces)
+    assert call(*pos) is not None
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    with Watch():
+        assert call(*pos) is None
+    seen = []
+    batch = torch.stack([pos[0], pos[0]])
+
+    def one(t):
+        seen.append(call(t, pos[1], pos[2]))
+        return t
+    torch.vmap(one)(batch)
+    assert seen == [None]
+    assert call(torch._neg_view(pos[0]), pos[1], pos[2]) is None
+
+
+@pytest.mark.gpu
+def test_collide_through_the_binding_equals_the_plain_call(cuda, binding):
+    pos, vel = _state(cuda)
+    order = pa.sort_particles_by_cell(*pos, GRID, 3)
+    library = ntc_collide.load_library()
+    params = ntc_collide.CollisionParams(1e-3, 1.0, 0.5, 11, 2)
+    results = []
+    for p in (params, params._replace(step=np.int64(2))):  # the second is not plain
+        v, sigma = vel.clone(), torch.ones(GRID.num_cells, device=cuda)
+        accepted = torch.zeros(GRID.num_cells, dtype=torch.int32, device=cuda)
+        plain = binding.collide(v.clone(), order.cell_start, sigma.clone(), accepted.clone(), N, *p)
+        assert plain is (True if isinstance(p.step, int) else None)
+        ntc_collide.collide(library, v, order.cell_start, sigma, accepted, N, p)
+        results.append((v, sigma, accepted))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
