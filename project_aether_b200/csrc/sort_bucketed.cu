@@ -553,7 +553,8 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
 // written out with neighbouring lanes at neighbouring addresses.  The scatter kernel above
 // instead pays one returning L2 add and one store request per particle (64 G/s at best).
 // Bound by instructions and latency (32 warps per multiprocessor between barriers): 4 M particles
-// on 1250 buckets 37 us, 16 M on 4096 155, where the 32-byte records took 93 and 241.
+// on 1250 buckets 37 us, 16 M on 4096 155, where the 32-byte records took 93 and 241 (before a tile was
+// written out beside the next one's count, see kSplitHeld).
 constexpr int kSplitThreads = 512;       // two blocks per multiprocessor
 constexpr int kSplitThreadsWide = 1024;  // one block, twice the tile
 constexpr int kSplitMaxBuckets = 16384;  // 128 KB of tables beside the stage
