@@ -4,11 +4,16 @@ The binding follows the reference's own ctypes loader for its native library
 (project_aether/src/custom_kernels/cuda/tma_collide.py:67-108): raw device
 pointers, the stream as void*, an int status that is raised as RuntimeError.
 There is no fallback: if the library is missing or fails to load, importing a
-symbol from it raises.
+symbol from it raises.  The native binding (csrc/binding.cpp) only saves host time: without
+it every call goes through ctypes.
 """
 
 import ctypes
 import os
+import sysconfig
+import warnings
+
+import torch
 
 from .cell_grid import CellGrid
 
@@ -133,7 +138,7 @@ _SIGNATURES = {
 }
 
 _library = None
-binding = None        # the native binding, once the library is loaded
+binding = None        # the native binding, once the library is loaded; None where there is none
 bound_library = None  # the library it calls
 
 _BOUND = ('AetherSortWorkspaceBytes', 'AetherSortParticlesByCell', 'AetherSortAndGatherParticles',
@@ -143,6 +148,26 @@ _BOUND = ('AetherSortWorkspaceBytes', 'AetherSortParticlesByCell', 'AetherSortAn
 def exported_symbols():
     """Names the header declares; every one must resolve in the library."""
     return tuple(_SIGNATURES)
+
+
+def binding_abi() -> str:
+    """The PyTorch build and the Python ABI whose internals the binding is compiled against."""
+    return f'torch {torch.__version__} {torch.version.git_version} {sysconfig.get_config_var("SOABI")}'
+
+
+def _load_binding():
+    """The native binding if it is built and fits this PyTorch and Python, else None with a warning.
+    One built for others may load all the same, and would read tensors by another layout."""
+    try:
+        from . import _binding
+        if _binding.built_for == binding_abi():
+            return _binding
+        why = f'it was built for {_binding.built_for}'
+    except (ImportError, AttributeError) as e:
+        why = str(e)
+    warnings.warn(f'no native binding, calls take more host time ({why}); '
+                  'run `python -m project_aether_b200.build`', RuntimeWarning)
+    return None
 
 
 def load_library(path: str | None = None) -> ctypes.CDLL:
@@ -166,15 +191,13 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         fn.restype = restype
         fn.argtypes = argtypes
     if path is None:
-        try:
-            from . import _binding
-        except ImportError as e:
-            raise OSError('the Python binding is not built or does not fit the installed PyTorch; '
-                          'run `python -m project_aether_b200.build`') from e
-        _binding.bind(CellGrid, *(ctypes.cast(getattr(library, name), ctypes.c_void_p).value
-                                  for name in _BOUND))
-        _library = bound_library = library
-        binding = _binding
+        native = _load_binding()
+        if native is not None:
+            native.bind(CellGrid, *(ctypes.cast(getattr(library, name), ctypes.c_void_p).value
+                                    for name in _BOUND))
+            bound_library = library
+            binding = native
+        _library = library
     return library
 
 

@@ -358,4 +358,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, methods, n
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__binding() { return PyModule_Create(&module); }
+// What the build compiled this against; another PyTorch or Python has other internals (see _native.py).
+PyMODINIT_FUNC PyInit__binding() {
+  PyObject* made = PyModule_Create(&module);
+  if (made && PyModule_AddStringConstant(made, "built_for", AETHER_BUILT_FOR) != 0) Py_CLEAR(made);
+  return made;
+}

@@ -1,5 +1,9 @@
 """The native binding takes the plain form of a call; every other form goes through the Python code
-and comes out the same, errors included."""
+and comes out the same, errors included.  Without a binding that fits, all calls do."""
+
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -8,6 +12,7 @@ import torch
 import project_aether_b200 as pa
 from project_aether_b200 import _native, ntc_collide
 
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 N, CELLS = 5_003, (8, 7, 6)
 GRID = pa.CellGrid((0., 0., 0.), (1., 1., 0.5), CELLS)
 
@@ -187,3 +192,36 @@ def test_collide_through_the_binding_equals_the_plain_call(cuda, binding):
         results.append((v, sigma, accepted))
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+# ---- loading: the library alone serves every call ----
+
+_LOAD = """
+import sys, types, warnings
+sys.modules['project_aether_b200._binding'] = {module}
+warnings.simplefilter('ignore')
+from project_aether_b200 import _native, ntc_collide
+library = _native.load_library()
+assert library is _native.load_library() and library is not None
+assert library.AetherSortWorkspaceBytes(1000, 100, 0) > 0
+assert _native.binding is None and _native.bound_library is None
+try:  # no binding: a call gets as far as the Python code's own checks
+    ntc_collide.collide(library, types.SimpleNamespace(dim=lambda: 1), *[None] * 4, ntc_collide.CollisionParams(*[1] * 5))
+except ValueError as e:
+    assert 'contiguous' in str(e)
+"""
+
+
+def _child(code, **env):
+    return subprocess.run([sys.executable, '-c', code], cwd=ROOT, env={**os.environ, **env}, capture_output=True,
+                          text=True)
+
+
+@pytest.mark.parametrize('module', ['None',  # none, or one that does not load
+                                    "types.SimpleNamespace(bind=None)",
+                                    "types.SimpleNamespace(bind=None, built_for='torch 1.0')"])
+@pytest.mark.parametrize('named', [False, True])
+def test_the_library_loads_without_a_binding_that_fits(module, named):
+    env = {'AETHER_SORT_LIBRARY': _native.LIBRARY_PATH} if named else {}
+    done = _child(_LOAD.format(module=module), **env)
+    assert done.returncode == 0, done.stderr
