@@ -139,7 +139,7 @@ _SIGNATURES = {
 
 _library = None
 binding = None        # the native binding, once the library is loaded; None where there is none
-bound_library = None  # the library it calls
+bound_library = None  # the library it calls; set only when `binding` is
 
 _BOUND = ('AetherSortWorkspaceBytes', 'AetherSortParticlesByCell', 'AetherSortAndGatherParticles',
           'AetherPushSortAndGatherParticles', 'AetherDsmcCollideTma')
@@ -195,8 +195,8 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         if native is not None:
             native.bind(CellGrid, *(ctypes.cast(getattr(library, name), ctypes.c_void_p).value
                                     for name in _BOUND))
+            binding = native  # before what other threads look for first
             bound_library = library
-            binding = native
         _library = library
     return library
 

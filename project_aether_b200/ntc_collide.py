@@ -77,7 +77,7 @@ def collide(library: ctypes.CDLL, velocity: torch.Tensor, cell_start: torch.Tens
     Raises:
       RuntimeError: if the launch fails.
     """
-    if library is _native.bound_library and _native.binding.collide(
+    if _native.binding is not None and library is _native.bound_library and _native.binding.collide(
             velocity, cell_start, sigma_g_max, collisions, num_particles, params.selection_factor,
             params.vhs_coefficient, params.vhs_exponent, params.seed, params.step):
         return

@@ -225,3 +225,22 @@ def test_the_library_loads_without_a_binding_that_fits(module, named):
     env = {'AETHER_SORT_LIBRARY': _native.LIBRARY_PATH} if named else {}
     done = _child(_LOAD.format(module=module), **env)
     assert done.returncode == 0, done.stderr
+
+
+def test_the_binding_is_there_before_the_library_it_is_bound_to():
+    """Another thread may call at any line of the loading: where it finds the bound library, it finds
+    the binding."""
+    done = _child("""
+import sys
+from project_aether_b200 import _native
+def look(frame, event, arg):
+    if frame.f_code is not _native.load_library.__code__:
+        return None
+    assert _native.bound_library is None or _native.binding is not None, frame.f_lineno
+    return look
+sys.settrace(look)
+_native.load_library()
+sys.settrace(None)
+assert _native.binding is not None and _native.bound_library is _native.load_library()
+""")
+    assert done.returncode == 0, done.stderr
