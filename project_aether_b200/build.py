@@ -37,6 +37,15 @@ def _nvcc() -> str:
     raise RuntimeError('nvcc not found; the CUDA library cannot be built')
 
 
+def _binding_stale(sources) -> bool:
+    """Also where the binding was built for another PyTorch or Python: its name for what it was
+    built for is a text inside it."""
+    if _stale(BINDING, sources):
+        return True
+    with open(BINDING, 'rb') as f:
+        return binding_abi().encode() not in f.read()
+
+
 def _stale(target: str, sources) -> bool:
     if not os.path.exists(target):
         return True
@@ -68,7 +77,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     """Compiles every CUDA source into libaether_sort.so, and the binding; returns the library's path."""
     header = os.path.join(os.path.dirname(PKG), 'include', 'aether_sort.h')
     binding = os.path.join(CSRC, 'binding.cpp')
-    if force or _stale(BINDING, [binding, header]):
+    if force or _binding_stale([binding, header]):
         _run(_binding_command(), verbose)
     kernels = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f != 'binding.cpp']
     if force or _stale(LIB, [*kernels, header]):

@@ -244,3 +244,15 @@ sys.settrace(None)
 assert _native.binding is not None and _native.bound_library is _native.load_library()
 """)
     assert done.returncode == 0, done.stderr
+
+
+def test_a_binding_for_another_pytorch_is_stale(tmp_path, monkeypatch):
+    build = pytest.importorskip('project_aether_b200.build')
+    source, target = tmp_path / 'binding.cpp', tmp_path / '_binding.so'
+    source.write_text('')
+    monkeypatch.setattr(build, 'BINDING', str(target))
+    assert build._binding_stale([str(source)])
+    target.write_bytes(b'\0' + build.binding_abi().encode() + b'\0')
+    assert not build._binding_stale([str(source)])
+    target.write_bytes(b'\0' + build.binding_abi().replace('torch ', 'torch 1').encode() + b'\0')
+    assert build._binding_stale([str(source)])
