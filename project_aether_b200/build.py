@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sysconfig
+import warnings
 
 import torch
 
@@ -74,17 +75,23 @@ def _binding_command():
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compiles every CUDA source into libaether_sort.so, and the binding; returns the library's path."""
+    """Compiles every CUDA source into libaether_sort.so, then the binding; returns the library's path.
+
+    A binding that cannot be built (no Python headers, say) is a warning: the library serves every call
+    without it."""
     header = os.path.join(os.path.dirname(PKG), 'include', 'aether_sort.h')
     binding = os.path.join(CSRC, 'binding.cpp')
-    if force or _binding_stale([binding, header]):
-        _run(_binding_command(), verbose)
     kernels = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f != 'binding.cpp']
     if force or _stale(LIB, [*kernels, header]):
         flags = [f for f in NVCC_FLAGS if not f.startswith('--use_fast_math')]
         if verbose:
             flags += ['-Xptxas', '-v']
         _run([_nvcc(), *flags, '-ccbin', 'g++', '-o', LIB] + [os.path.join(CSRC, s) for s in SOURCES], verbose)
+    if force or _binding_stale([binding, header]):
+        try:
+            _run(_binding_command(), verbose)
+        except (OSError, RuntimeError) as e:
+            warnings.warn(f'the Python binding was not built, calls go through ctypes: {e}', RuntimeWarning)
     return LIB
 
 

@@ -256,3 +256,18 @@ def test_a_binding_for_another_pytorch_is_stale(tmp_path, monkeypatch):
     assert not build._binding_stale([str(source)])
     target.write_bytes(b'\0' + build.binding_abi().replace('torch ', 'torch 1').encode() + b'\0')
     assert build._binding_stale([str(source)])
+
+
+def test_the_library_is_built_before_a_binding_that_cannot_be(tmp_path, monkeypatch):
+    from project_aether_b200 import build
+    ran = []
+
+    def run(cmd, verbose):
+        ran.append(cmd[0])
+        if 'binding.cpp' in ' '.join(cmd):
+            raise RuntimeError('no Python.h')
+    monkeypatch.setattr(build, '_run', run)
+    monkeypatch.setattr(build, '_nvcc', lambda: 'nvcc')
+    with pytest.warns(RuntimeWarning, match='no Python.h'):
+        assert build.build(force=True) == build.LIB
+    assert ran == ['nvcc', 'g++']
