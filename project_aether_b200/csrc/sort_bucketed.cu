@@ -561,7 +561,9 @@ constexpr int kSplitMaxBuckets = 16384;  // 128 KB of tables beside the stage
 // HELD: up to this many buckets per thread what the adds on the slot counters return stays in registers
 // until the scan is done, and the next tile's first positions are loaded while a tile is written
 // out.  Whole call, without / with: 1 M particles 43.1 / 41.1 us, 4 M 94.8 / 94.0, 8 M 172.0 / 168.0, 16 M 338.7 /
-// 333.4.  With more buckets (30 M, 8192) the registers would spill and nothing is held: 669 / 677.
+// 333.4.  With more buckets the registers would spill: nothing is held, and a tile is cleared, counted and
+// written out one after the other (8192 buckets: 30 M 661 us, 45 M 1218; with the table cleared ahead of the
+// write-out there too 666 and 1234).
 constexpr int kSplitHeld = 4;
 
 __host__ __device__ inline size_t split_smem_bytes(int tile, int buckets) {
@@ -606,12 +608,16 @@ key_split_kernel(const float* __restrict__ x, const float* __restrict__ y,
       }
     }
   };
+  auto clear_counts = [&] {
+    for (int b = tid * 4; b < table; b += THREADS * 4)
+      *reinterpret_cast<uint4*>(&place[b]) = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+  };
   int first = blockIdx.x * kTile;
   if (HELD && first < last) load_four(first, 0);
-  for (int b = tid * 4; b < table; b += THREADS * 4)
-    *reinterpret_cast<uint4*>(&place[b]) = make_uint4(0u, 0u, 0u, 0u);
-  __syncthreads();
+  if (HELD) clear_counts();
   for (; first < last; first += stride) {
+    if (!HELD) clear_counts();
     uint32_t* row = cursor + static_cast<size_t>(first >> chunk_log) * buckets;
     const bool whole = VEC && last - first >= kTile;
     uint32_t key[ITEMS], ranks[ITEMS / 2];  // two ranks of 16 bits to a word
@@ -692,17 +698,17 @@ key_split_kernel(const float* __restrict__ x, const float* __restrict__ y,
     __syncthreads();
     // The next tile's first positions are on their way while this one is written out, and the writes
     // while the next one is counted.
-    if (HELD && first + stride < last) load_four(first + stride, 0);
-    for (int b = tid * 4; b < table; b += THREADS * 4)
-      *reinterpret_cast<uint4*>(&place[b]) = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
+    if (HELD) {
+      if (first + stride < last) load_four(first + stride, 0);
+      clear_counts();
+    }
     const int here = min(kTile, last - first);
 #pragma unroll 4
     for (int j = tid; j < here; j += THREADS) {
       const uint2 r = stage[j];
       records[to_slot[r.x >> (kShuffleBits + shift)] + static_cast<uint32_t>(j)] = r;
     }
-    if (!HELD) __syncthreads();
+    if (!HELD) __syncthreads();  // the tables and the stage are reused by the next tile
   }
   chain_release();
 }

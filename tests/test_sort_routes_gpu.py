@@ -86,6 +86,13 @@ def test_middling_calls(cuda, n, cells, moved):
     _compare(n, cells, cuda, moved)
 
 
+# Tiles of 512 and of 1024 threads, with four buckets per thread of the split and with some more.
+@pytest.mark.parametrize('n,cells', [(700_001, (128, 128, 128)), (700_001, (128, 128, 129)),
+                                     (2_500_003, (256, 128, 128)), (2_500_003, (256, 128, 129))])
+def test_buckets_per_thread_of_the_split(cuda, n, cells):
+    _compare(n, cells, cuda, False)
+
+
 @pytest.mark.parametrize('n,cells', [(300_000, (64, 32, 32)), (3_000_000, (64, 64, 64))])
 def test_dense_layers_and_unaligned_arrays(cuda, n, cells):
     _compare(n, cells, cuda, False, squeeze=(0.7, 0.03))
