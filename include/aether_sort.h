@@ -70,8 +70,8 @@ int AetherSortBucketPlan(int64_t n, int64_t num_cells, int32_t* cells_per_bucket
  * after the other, with gaps between them.  mode 1 (default): the short kernels (scans,
  * tables, the digit-pass path's) are launched so that each may be set up
  * while the one before it still runs (programmatic dependent launch), and in calls without payload
- * and middling ones all of them; mode 2: the scatter, finish and tail kernels of every call
- * (measured slower on large inputs with payload); mode 0: ordinary launches.  Every
+ * (of up to some 68 million particles) and middling ones all of them; mode 2: the scatter, finish and
+ * tail kernels of every call (measured slower on larger inputs); mode 0: ordinary launches.  Every
  * kernel waits for the grids before it to complete before it touches anything, so the work
  * runs in stream order in every mode and results do not depend on it. */
 int AetherSortSetChainedLaunches(int32_t mode);

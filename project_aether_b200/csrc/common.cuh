@@ -232,8 +232,9 @@ void count_launches(int kernels);
 // wait with chain_wait() and let the kernel behind them in when a block has done its work
 // (chain_release()): waiting blocks in their midst cost more than the launch.  Per call, only the short
 // kernels chained / these too: without payload 4 M particles 110.8 / 104.0 us, 16 M 348 / 343; with
-// payload 1 M 61 / 56, 16 M 556 / 557, 64 M 2241 / 2373, 256 M 10.7 / 11.0 ms.  So they are chained in
-// calls without payload and in those whose slots are reserved tile by tile.
+// payload 1 M 61 / 56, 16 M 556 / 557, 64 M 2241 / 2373, 256 M 10.7 / 11.0 ms.  Without
+// payload and without a split, 200 M 6470 / 6810 us.  So they are chained in calls without payload whose
+// records are split tile by tile, and in those whose slots are reserved tile by tile.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
