@@ -15,13 +15,14 @@
 //   settled_finish_kernel  a block takes a group: reads its home run and keys, moves the particles once
 //                          more, leaves out those that left, adds the arrivals, and sorts and
 //                          writes the group as the general finish kernel does
+//   bucket_tail_kernel     the buckets of dense regions, which a block does not hold
 //
 // It moves 24 + 4 + 28 + 32 bytes per particle, and some 130 more per mover, where the general path moves
 // 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
 // bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3281 (941, 2157).
 //
 // Whether the input is in order is only known on the device.  Whatever speaks against it (a bucket
-// out of order, too many movers, a bucket that no block holds, a counter that wraps) sets
+// out of order, too many movers, a counter that wraps) sets
 // Header::settle_failed; the kernels above then stop, and the general path's kernels, which are
 // enqueued behind them and otherwise return at once, do the call from the start.
 
@@ -55,7 +56,7 @@ struct SettledArgs {
   uint32_t* list_count;             // [scan_blocks] movers found by each block of the scan
   uint32_t* cursor;                 // [buckets] next free place of each bucket's arrivals
   uint32_t* sums;                   // [parts][4] particles at home, arrivals, output of kSettledPart buckets
-  uint32_t* tables;                 // [groups][kSettledRowWords]
+  uint32_t* tables;                 // [buckets][kSettledRowWords]: groups, and from the end buckets in no group
   uint32_t *list, *arrived;         // records: the movers block by block, and bucket by bucket
   Header* hdr;
 };
@@ -275,7 +276,8 @@ settled_sums_kernel(const __grid_constant__ SettledArgs a) {
 // coarse sums, and the buckets between the last of those and its own).  Groups as in group_kernel; a
 // bucket needs a place for each of its particles at home and each of its arrivals.  A group's
 // table: first particle of its home run, particles in it, first of its arrivals, arrivals, first
-// output slot, records, its buckets b0, b1.
+// output slot, records, its buckets b0, b1.  A bucket that no block holds gets such a table too, for the tail
+// kernel, from the end of the array (there are no more groups and such buckets than buckets).
 __global__ void __launch_bounds__(kGroupSpan)
 settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   chain_begin();
@@ -328,17 +330,18 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   if (tid < here) a.cursor[b0 + tid] = base[1] + arrivals;
   __syncthreads();
   const int most = max(1, FinishSettled::kMaxCells >> a.shift);
-  const uint32_t biggest = cut_groups_of_block(cut, here, kGroupSpanLog, most, a.capacity, &a.hdr->aux_counter[2]);
-  if ((tid & 31) == 0 && biggest > a.capacity) fail_settle(a.hdr);
-  if (tid < static_cast<int>(cut.found)) {
-    const int first = cut.group_first[tid], end = cut.link[first];
-    uint4* table = reinterpret_cast<uint4*>(a.tables + (static_cast<size_t>(cut.list_base) + tid) * kSettledRowWords);
+  cut_groups_of_block(cut, here, kGroupSpanLog, most, a.capacity, &a.hdr->aux_counter[2]);
+  auto write_table = [&](uint32_t row, int first, int end) {
+    uint4* table = reinterpret_cast<uint4*>(a.tables + static_cast<size_t>(row) * kSettledRowWords);
     const uint32_t in_group = arrived[end] - arrived[first];
     table[0] = make_uint4(base[0] + cut.start[first] - arrived[first],
                           cut.start[end] - cut.start[first] - in_group, base[1] + arrived[first], in_group);
     table[1] = make_uint4(base[2] + output[first], output[end] - output[first],
                           static_cast<uint32_t>(b0 + first), static_cast<uint32_t>(b0 + end));
-  }
+  };
+  if (tid < static_cast<int>(cut.found)) write_table(cut.list_base + tid, cut.group_first[tid], cut.link[cut.group_first[tid]]);
+  if (tid < here && cut.start[tid + 1] - cut.start[tid] > a.capacity)
+    write_table(a.buckets - 1 - atomicAdd(&a.hdr->settle_large, 1u), tid, tid + 1);
 }
 
 // The movers' records to their buckets, with their keys.
@@ -454,4 +457,63 @@ settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_consta
     });
     if (!sorted && tid == 0) fail_settle(a.hdr);
   }
+}
+
+// The records of a bucket that no block holds: its home run in the input without those that left, and its
+// arrivals.
+template <class Shape>
+struct SettledRecords {
+  const SettledArgs& a;
+  uint32_t home_first, home, arrived_first, arrivals;
+  template <class Use>
+  __device__ __forceinline__ void keys(Use use) const {
+    for (uint32_t base = 0; base < home; base += Shape::kThreads) {
+      const uint32_t r = base + threadIdx.x;
+      const uint32_t key = r < home ? __ldcg(a.keys + home_first + r) : kGone;
+      use(key, key != kGone);
+    }
+    for (uint32_t base = 0; base < arrivals; base += Shape::kThreads) {
+      const uint32_t r = base + threadIdx.x;
+      use(r < arrivals ? __ldcg(a.arrived + static_cast<size_t>(arrived_first + r) * kRecordWords) : 0u, r < arrivals);
+    }
+  }
+  template <class Place>
+  __device__ __forceinline__ void records(Place place) const {
+    for (uint32_t r = threadIdx.x; r < home; r += Shape::kThreads) {
+      const int64_t i = home_first + r;
+      const uint32_t key = __ldcg(a.keys + i);
+      uint4* to = key != kGone ? reinterpret_cast<uint4*>(place(key)) : nullptr;
+      if (!to) continue;
+      float f[6] = {a.x[i], a.y[i], a.z[i], a.v[i], a.v[a.padded + i], a.v[2 * a.padded + i]};
+      push_particle(a.push, f);
+      to[0] = make_uint4(key, static_cast<uint32_t>(i), __float_as_uint(f[0]), __float_as_uint(f[1]));
+      to[1] = make_uint4(__float_as_uint(f[2]), __float_as_uint(f[3]), __float_as_uint(f[4]), __float_as_uint(f[5]));
+    }
+    for (uint32_t r = threadIdx.x; r < arrivals; r += Shape::kThreads) {
+      const uint4* record = reinterpret_cast<const uint4*>(a.arrived) + 2 * static_cast<size_t>(arrived_first + r);
+      const uint4 lo = __ldcg(record);
+      uint4* to = reinterpret_cast<uint4*>(place(lo.x));
+      if (!to) continue;
+      to[0] = lo;
+      to[1] = __ldcg(record + 1);
+    }
+  }
+};
+
+// Buckets first, first + step, ... of those that no block holds.  False if one of them cannot be finished.
+template <class Shape>
+__device__ bool finish_settled_large(FinishSmem<Shape>& s, const SettledArgs& a, const FinishOut& out, uint32_t first,
+                                     uint32_t step) {
+  const uint32_t large = a.hdr->settle_large;
+  for (uint32_t r = first; r < large; r += step) {
+    const uint4* table = reinterpret_cast<const uint4*>(a.tables) + 2 * static_cast<size_t>(a.buckets - 1 - r);
+    const uint4 where = table[0], what = table[1];
+    const int64_t first_cell = static_cast<int64_t>(what.z) << a.shift;
+    const int cells_here = static_cast<int>(
+        min(static_cast<long long>(1) << a.shift, static_cast<long long>(a.num_cells - first_cell)));
+    if (!finish_large_bucket<Shape>(s, out, SettledRecords<Shape>{a, where.x, where.y, where.z, where.w}, what.x,
+                                    first_cell, cells_here, [](uint32_t, int) {}))
+      return false;
+  }
+  return true;
 }

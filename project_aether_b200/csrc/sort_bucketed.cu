@@ -1512,6 +1512,45 @@ struct RunTable {
   uint32_t* redo;                // room for the groups whose counters wrapped, or null
 };
 
+// The records of one bucket, run by run.
+// `record_words`: from one record to the next; Shape's words of a record are its first.
+template <class Shape>
+struct BucketRecords {
+  const RunTable& t;
+  int b, record_words;
+  template <class Each>
+  __device__ __forceinline__ void runs(Each each) const {
+    for (int c = 0; c < t.chunks; ++c) {
+      const size_t entry = static_cast<size_t>(c) * t.buckets + b;
+      const uint32_t start = t.run_begin[entry];
+      each(start, t.run_begin[entry + 1] - start);
+    }
+  }
+  template <class Use>
+  __device__ __forceinline__ void keys(Use use) const {
+    runs([&](uint32_t start, uint32_t length) {
+      for (uint32_t base = 0; base < length; base += Shape::kThreads) {
+        const bool valid = base + threadIdx.x < length;
+        use(valid ? __ldcg(t.records + static_cast<size_t>(start + base + threadIdx.x) * record_words) : 0u, valid);
+      }
+    });
+  }
+  template <class Place>
+  __device__ __forceinline__ void records(Place place) const {
+    runs([&](uint32_t start, uint32_t length) {
+      for (uint32_t i = threadIdx.x; i < length; i += Shape::kThreads) {
+        const uint2* rec = reinterpret_cast<const uint2*>(t.records + static_cast<size_t>(start + i) * record_words);
+        const uint2 lo = __ldcg(rec);
+        uint2* to = reinterpret_cast<uint2*>(place(lo.x));
+        if (!to) continue;
+        to[0] = lo;
+#pragma unroll
+        for (int k = 1; k < Shape::kRecordWords / 2; ++k) to[k] = __ldcg(rec + k);
+      }
+    });
+  }
+};
+
 // A bucket with more records than shared memory holds (a dense region: the
 // bucket width is planned from the average load).  The block counts the
 // bucket's records per cell, cuts the cells into up to kMaxSegments runs that
@@ -1519,12 +1558,12 @@ struct RunTable {
 // reads from global memory once per run) and sorts them like a small group.
 // Returns false if it cannot (a single cell larger than shared memory, too many
 // runs, or a wrapped byte counter): the call then goes to the digit passes.
-// `record_words`: from one record to the next; Shape's words of a record are its first.
+// `source`: where the bucket's records are.  source.keys(use) calls use(key, valid) for each of them, in
+// whole warps; source.records(place) puts each record for whose key place(key) gives an address there.
 // `after(first, count)`: what is left to do for these output slots when keys and indices stand.
-template <class Shape, class After>
-__device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, const RunTable& t,
-                                    int b, uint32_t begin, int count, int64_t first_cell,
-                                    int cells_here, int record_words, After after) {
+template <class Shape, class Source, class After>
+__device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, const Source& source,
+                                    uint32_t begin, int64_t first_cell, int cells_here, After after) {
   constexpr int kThreads = Shape::kThreads, kCapacity = Shape::kCapacity;
   const int tid = threadIdx.x;
   static_assert(Shape::kMaxCells < Shape::kHistWords && Shape::kMaxCells <= 2 * kThreads, "cell counts");
@@ -1533,15 +1572,9 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
   __syncthreads();
   // Per-cell counts: one pass over the keys of the bucket's records (lanes that agree share an
   // add: a bucket that comes here is crowded).
-  for (int c = 0; c < t.chunks; ++c) {
-    const size_t entry = static_cast<size_t>(c) * t.buckets + b;
-    const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
-    for (uint32_t base = 0; base < length; base += kThreads) {
-      const bool valid = base + tid < length;
-      const uint32_t key = valid ? __ldcg(t.records + static_cast<size_t>(start + base + tid) * record_words) : 0u;
-      bin_add(cell_count, (key >> kShuffleBits) - static_cast<uint32_t>(first_cell), valid);
-    }
-  }
+  source.keys([&](uint32_t key, bool valid) {
+    bin_add(cell_count, (key >> kShuffleBits) - static_cast<uint32_t>(first_cell), valid);
+  });
   __syncthreads();
   // Exclusive scan of the counts, two cells per thread, then one thread cuts the cells into runs
   // that fit, each as long as can be.  (Walking through the counts one by one took it as long as
@@ -1588,25 +1621,12 @@ __device__ bool finish_large_bucket(FinishSmem<Shape>& s, const FinishOut& out, 
     for (int i = tid; i < words; i += kThreads) s.hist[i] = 0;
     if (tid == 0) s.fill = 0;
     __syncthreads();
-    for (int c = 0; c < t.chunks; ++c) {
-      const size_t entry = static_cast<size_t>(c) * t.buckets + b;
-      const uint32_t start = t.run_begin[entry], length = t.run_begin[entry + 1] - start;
-      for (uint32_t i = tid; i < length; i += kThreads) {
-        const uint32_t* rec = t.records + static_cast<size_t>(start + i) * record_words;
-        const uint2 lo = __ldcg(reinterpret_cast<const uint2*>(rec));
-        const int cell = static_cast<int>((lo.x >> kShuffleBits) - static_cast<uint32_t>(first_cell));
-        if (cell >= c0 && cell < c1) {
-          const uint32_t slot = atomicAdd(&s.fill, 1u);
-          if (slot < static_cast<uint32_t>(kCapacity)) {
-            uint2* to = reinterpret_cast<uint2*>(&s.raw[slot * Shape::kRecordWords]);
-            to[0] = lo;
-#pragma unroll
-            for (int k = 1; k < Shape::kRecordWords / 2; ++k)
-              to[k] = __ldcg(reinterpret_cast<const uint2*>(rec) + k);
-          }
-        }
-      }
-    }
+    source.records([&](uint32_t key) -> uint32_t* {
+      const int cell = static_cast<int>((key >> kShuffleBits) - static_cast<uint32_t>(first_cell));
+      if (cell < c0 || cell >= c1) return nullptr;
+      const uint32_t slot = atomicAdd(&s.fill, 1u);
+      return slot < static_cast<uint32_t>(kCapacity) ? &s.raw[slot * Shape::kRecordWords] : nullptr;
+    });
     __syncthreads();
     const bool consistent = s.fill == static_cast<uint32_t>(seg_count);
     __syncthreads();
@@ -1784,7 +1804,8 @@ __device__ bool finish_buckets(FinishSmem<Shape>& s, const RunTable& t, const Fi
     const int64_t first_cell = static_cast<int64_t>(b) << t.shift;
     const int cells_here = static_cast<int>(
         min(static_cast<long long>(1) << t.shift, static_cast<long long>(num_cells - first_cell)));
-    if (!finish_large_bucket<Shape>(s, out, t, b, begin, count, first_cell, cells_here, record_words, after))
+    if (!finish_large_bucket<Shape>(s, out, BucketRecords<Shape>{t, b, record_words}, begin, first_cell, cells_here,
+                                    after))
       return false;
   }
   return true;
@@ -1810,7 +1831,8 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
     hdr->use_standard = 1;
 }
 
-// Behind the finish kernel of an ordinary call: the oversized buckets and the groups whose counters
+// Behind the finish kernel of an ordinary call: the oversized buckets (also those of the sort of a settled
+// state) and the groups whose counters
 // wrapped (calls without payload, whose sparse groups have 16 counters per cell), then, when the call was
 // handed over, the whole digit-pass sort.  Usually there is nothing to do and every block returns
 // after a look at the header.  What bounds it is then the launch itself: as the separate kernels
@@ -1823,10 +1845,10 @@ constexpr int kTailBlocks = Shape::kThreads <= 512 ? 2 : 1;
 template <class Shape>
 __global__ void __launch_bounds__(Shape::kThreads, kTailBlocks<Shape>)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
-                   DigitPassArgs digits, bool behind) {
+                   DigitPassArgs digits, bool behind, const __grid_constant__ SettledArgs settled) {
   chain_wait();
-  if (settled_before(hdr, behind)) return;
-  const bool all_done = hdr->max_bucket <= capacity && hdr->redo_groups == 0;
+  const bool is_settled = Shape::kRecordWords == kRecordWords && settled_before(hdr, behind);
+  const bool all_done = is_settled ? hdr->settle_large == 0 : hdr->max_bucket <= capacity && hdr->redo_groups == 0;
   if (!handed_over(hdr) && all_done) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const uint32_t items = gridDim.x;
@@ -1839,6 +1861,13 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
     // A block that comes late may see another block's hand-over and skip its buckets: the digit
     // passes then write everything.
     FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
+    if constexpr (Shape::kRecordWords == kRecordWords) {
+      if (is_settled) {
+        if (!standard && !finish_settled_large<Shape>(s, settled, out, item, items) && threadIdx.x == 0)
+          atomicExch(&hdr->use_standard, 1);
+        return true;
+      }
+    }
     bool good = standard || finish_buckets<Shape>(s, t, out, num_cells, item, t.buckets, items, capacity + 1);
     for (uint32_t r = item; !standard && good && r < hdr->redo_groups; r += items) {
       const uint32_t* row0 = t.tables + static_cast<size_t>(t.redo[r]) * 2 * t.row_words;
@@ -2517,7 +2546,8 @@ int limited(int blocks, int most) { return most > 0 ? std::min(blocks, most) : b
 
 template <class Shape>
 cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                        uint32_t group_capacity, const DigitPassArgs& digits, bool behind, bool chained) {
+                        uint32_t group_capacity, const DigitPassArgs& digits, bool behind, bool chained,
+                        const SettledArgs& settled) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
   const cudaError_t e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
   if (e != cudaSuccess) return e;
@@ -2525,7 +2555,7 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
       1, std::min<int64_t>(sm_count() * kTailBlocks<Shape>, a.n / 2048)));
   return launch_chained_if(chained, bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks),
                            Shape::kThreads, kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity,
-                           digits, behind);
+                           digits, behind, settled);
 }
 
 template <int ITEMS>
@@ -2754,7 +2784,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
                       a.vs, a.padded_sorted, index_bits_of(a.n)};
 
-  SettledArgs settled;
+  SettledArgs settled{};
   size_t zero_bytes = 0;
   const bool behind = settled_args(a, p, base + l.records_off, l.total - l.records_off, hdr, &settled, &zero_bytes);
   if (behind) {
@@ -2874,8 +2904,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
       : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, behind, chained)
                        : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, behind, chained);
   if (e == cudaSuccess)
-    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, behind, chained)
-                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, behind, chained);
+    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, behind, chained, settled)
+                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, behind, chained, settled);
   stage_end(kStageBucketFinish, a.stream);
   count_launches(2);
   return e;

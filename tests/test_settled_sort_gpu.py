@@ -13,17 +13,21 @@ pytestmark = pytest.mark.gpu
 
 LEAST = 3 << 19  # particles from which on the settled path is tried: while slots are reserved tile by tile
 LEAST_UNTILED = 1 << 24
-SETTLE_FAILED, GROUPS = 12, 54  # words of the workspace header
+SETTLE_FAILED, LARGE, GROUPS = 12, 13, 54  # words of the workspace header
+
+
+def _words(device):
+    torch.cuda.synchronize()
+    workspace = particle_sort._workspaces[(device.index, torch.cuda.current_stream(device).cuda_stream)]
+    return workspace[:256].view(torch.int32).cpu()
 
 
 def _route(device):
     """'settled', 'given up', or 'general' where the settled path was not tried."""
-    torch.cuda.synchronize()
-    workspace = particle_sort._workspaces[(device.index, torch.cuda.current_stream(device).cuda_stream)]
-    words = workspace[:256].view(torch.int32).cpu()
+    words = _words(device)
     if words[SETTLE_FAILED]:
         return 'given up'
-    return 'settled' if words[GROUPS] else 'general'
+    return 'settled' if words[GROUPS] or words[LARGE] else 'general'  # digit passes clear the first
 
 
 def _sorted_state(n, cells, device, seed, squeeze=None, drift=0.0, drop=0):
@@ -45,13 +49,13 @@ def _sorted_state(n, cells, device, seed, squeeze=None, drift=0.0, drop=0):
     return grid, [t[drop:] for t in state.positions], velocity
 
 
-def _oracle(grid, pos, vel, n, dt, seed):
+def _oracle(grid, pos, vel, n, dt, seed, **slab):
     p = [np.ascontiguousarray(t.cpu().numpy()) for t in pos]
     v = np.ascontiguousarray(vel.cpu().numpy())
     p, rows = so.push_particles(p, [v[k, :n] for k in range(3)], dt, grid.lo, grid.hi)
     v[:, :n] = np.stack(rows)
     return so.c_sort_particles(*[np.ascontiguousarray(a) for a in p], v,
-                               so.Grid(grid.lo, grid.hi, grid.cells), seed)
+                               so.Grid(grid.lo, grid.hi, grid.cells), seed, **slab)
 
 
 def _check(got, want, n):
@@ -65,12 +69,19 @@ def _check(got, want, n):
     np.testing.assert_array_equal(got.velocity.cpu().numpy()[:, :n], payload[3][:, :n])
 
 
-def _run(grid, pos, vel, dt, device, route, out=None):
+def _crowd(pos, vel, first, count):
+    """Puts `count` particles from `first` on in one place, where they stay."""
+    for t in pos:
+        t[first:first + count] = t[first].item()
+    vel[:, first:first + count] = 0.0
+
+
+def _run(grid, pos, vel, dt, device, route, out=None, digits=False, slab={}):
     n, seed = pos[0].numel(), 0x9876543210 + pos[0].numel()
-    want = _oracle(grid, pos, vel, n, dt, seed)
-    got = pa.sort_and_gather_particles(*pos, vel, grid, seed, push=(dt, grid.lo, grid.hi), out=out)
+    want = _oracle(grid, pos, vel, n, dt, seed, **slab)
+    got = pa.sort_and_gather_particles(*pos, vel, grid, seed, push=(dt, grid.lo, grid.hi), out=out, **slab)
     assert pa.last_sort_status(device) == 0
-    assert not pa.last_sort_used_digit_passes(device)
+    assert pa.last_sort_used_digit_passes(device) == digits
     assert _route(device) == route
     _check(got, want, n)
 
@@ -112,8 +123,31 @@ def test_dense_layer(cuda):
 
 def test_buckets_that_no_block_holds(cuda):
     grid, pos, vel = _sorted_state(4_000_000, (128, 64, 64), cuda, 6, squeeze=(0.7, 0.02))
-    _run(grid, pos, vel, _dt(grid), cuda, 'given up')
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
 
+
+# A few buckets that no block holds; unaligned arrays; cells of more than 2560, the records of a block of the
+# groups; a mean of some 200 to a cell; blocks of the large finish shape behind.
+@pytest.mark.parametrize('n,cells,squeeze,drop', [(LEAST, (64, 64, 64), (0.3, 0.002), 0),
+                                                  (LEAST + 3, (101, 97, 89), (0.28, 0.03), 1),
+                                                  (2_000_001, (32, 32, 32), (0.6, 0.01), 0),
+                                                  (LEAST, (20, 21, 20), (0.7, 0.04), 0),
+                                                  (40_000_003, (180, 170, 160), (0.28, 0.02), 0)])
+def test_dense_layers_of_some_buckets(cuda, n, cells, squeeze, drop):
+    grid, pos, vel = _sorted_state(n, cells, cuda, 21, squeeze=squeeze, drop=drop)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    assert _words(cuda)[LARGE] > 0
+
+
+@pytest.mark.parametrize('crowd,digits', [(2_700, False), (5_000, False), (6_000, True)])
+def test_one_cell_of_thousands(cuda, crowd, digits):
+    """Blocks of the tail kernel hold 5120 records; a cell of more goes to the digit passes, as it does in
+    the general path."""
+    n = LEAST + 100
+    grid, pos, vel = _sorted_state(n, (64, 64, 64), cuda, 10)
+    _crowd(pos, vel, n // 2, crowd)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled', digits=digits)
+    assert _words(cuda)[LARGE] == 1
 
 def test_too_many_movers(cuda):
     grid, pos, vel = _sorted_state(LEAST, (64, 64, 64), cuda, 7)
