@@ -5,6 +5,8 @@
 // of the general path take every particle through a record in HBM; here only those that left their
 // bucket (movers) travel so, and the others are read from the input where they lie:
 //
+//   settled_probe_kernel   clears the tables, and looks at a sample of the particles: how many leave their
+//                          bucket, and whether they are in bucket order
 //   settled_scan_kernel    reads the input once and moves the particles: their keys; where every
 //                          bucket's particles lie in the input (its home run; the input must be in
 //                          bucket order, before the move); who leaves which bucket, and the movers'
@@ -21,14 +23,18 @@
 // 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
 // bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3281 (941, 2157).
 //
-// Whether the input is in order is only known on the device.  Whatever speaks against it (a bucket
-// out of order, too many movers, a counter that wraps) sets
-// Header::settle_failed; the kernels above then stop, and the general path's kernels, which are
-// enqueued behind them and otherwise return at once, do the call from the start.
+// Whether the input is in order, and how many particles move, is only known on the device.  Whatever
+// speaks against the path sets Header::settle_failed; the kernels above then stop, and the general path's
+// kernels, which are enqueued behind them and otherwise return at once, do the call from the start.  When
+// it is noticed: random order and too many movers by the probe; a particle out of order, or more movers than
+// the lists hold in one part of the input, in the round of the scan that meets it; a counter that wraps in
+// the finish.  Buckets of a dense region are no reason.
 
 constexpr int kSettledThreads = 512;
 constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round
-constexpr int kMoverShare = 4;                      // room for one mover in four particles
+constexpr int kListShare = 2;                       // a block's list has room for one mover in two particles
+constexpr int kMoverShare = 4;                      // all lists together for one in four
+constexpr int kProbeSamples = 128;                  // particles of each of the scan's blocks that the probe looks at
 constexpr int kSettledPart = 4096;                  // buckets per entry of the coarse sums
 constexpr uint32_t kGone = 0xffffffffu;             // no key: grids of 2^25 cells are left to the general path
 constexpr int kSettledRowWords = 8;                 // words of a group's table
@@ -50,6 +56,8 @@ struct SettledArgs {
   int per_block;          // particles per block of the scan, a multiple of kSettledRound
   int scan_blocks;
   uint32_t capacity;      // places of a group
+  uint32_t most_sampled;  // movers of the sample from which on the general path is faster
+  uint32_t most_movers;   // what fits `arrived`
   uint32_t *first, *end;            // [buckets] home run in the input; both zero if it is empty
   uint32_t *leavers, *arrivals;     // [buckets]
   uint32_t* keys;                   // [n] key of every particle after the move, kGone of those that left
@@ -102,12 +110,12 @@ struct MoverQueue {
 // Stores 32 (or, at the end, the last `count`) of a warp's movers in the block's list; false if
 // there is no room.
 __device__ __forceinline__ bool flush_movers(const SettledArgs& a, const MoverQueue& queue, int from, int count,
-                                             uint32_t* fill, uint32_t allowed, uint32_t* list) {
+                                             uint32_t* fill, uint32_t room, uint32_t* list) {
   const int lane = lane_id();
   uint32_t place = 0;
   if (lane == 0) place = atomicAdd(fill, static_cast<uint32_t>(count));
   place = __shfl_sync(0xffffffffu, place, 0);
-  if (place + count > allowed) return false;
+  if (place + count > room) return false;
   if (lane < count) {
     const uint4 lo = queue.record[from + lane][0], hi = queue.record[from + lane][1];
     atomicAdd(&a.arrivals[lo.x >> a.shift], 1u);
@@ -188,11 +196,50 @@ __device__ __forceinline__ bool scan_round(const SettledArgs& a, int i0, int las
   return bad;
 }
 
+// Clears the tables of the scan and takes a sample of its particles, evenly spaced, with each one's neighbour.
+// Bound by the latency of one access to HBM, which is hidden beside the kernel that zeroes the header: the inputs
+// are read before the wait.  In place of a clear of the tables alone, which took a launch too: 4 M particles
+// 143.4 -> 144.6 us per call, 1.6 M 81.5 -> 79.3.
+template <bool WHOLE>
+__global__ void __launch_bounds__(kSettledThreads)
+settled_probe_kernel(const __grid_constant__ SettledArgs a, int64_t pieces) {
+  chain_release();
+  const int tid = threadIdx.x;
+  const int i = blockIdx.x * a.per_block + tid * (a.per_block / kProbeSamples);
+  const bool sampled = tid < kProbeSamples && i < a.n;
+  float f[6] = {}, next[3] = {};
+  const int j = min(i + 1, a.n - 1);
+  if (sampled) {
+    f[0] = a.x[i];
+    f[1] = a.y[i];
+    f[2] = a.z[i];
+    f[3] = a.v[i];
+    f[4] = a.v[a.padded + i];
+    f[5] = a.v[2 * a.padded + i];
+    next[0] = a.x[j];
+    next[1] = a.y[j];
+    next[2] = a.z[j];
+  }
+  uint4* tables = reinterpret_cast<uint4*>(a.first);
+  for (int64_t p = blockIdx.x * static_cast<int64_t>(kSettledThreads) + tid; p < pieces; p += gridDim.x * kSettledThreads)
+    tables[p] = make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t home = settled_cell<WHOLE>(f[0], f[1], f[2], a.grid) >> a.shift;
+  const bool unordered = sampled && settled_cell<WHOLE>(next[0], next[1], next[2], a.grid) >> a.shift < home;
+  push_particle(a.push, f);
+  const bool moved = sampled && settled_cell<WHOLE>(f[0], f[1], f[2], a.grid) >> a.shift != home;
+  chain_wait();  // the header is zero; inputs and tables were free before the kernel that zeroes it began
+  const int movers = __syncthreads_count(moved);
+  const bool fail = __syncthreads_or(unordered) || movers > kProbeSamples / kListShare;  // more than the block's list holds
+  if (tid == 0) {
+    if (movers) atomicAdd(&a.hdr->settle_sampled, static_cast<uint32_t>(movers));
+    if (fail) fail_settle(a.hdr);
+  }
+}
+
 // Bound by instructions (73 % of the issue slots; HBM would take half the time).  The home runs are
 // written where a bucket begins and where the bucket before it ends.  A mover costs two adds and a record
 // of {cell, index, moved state}, which goes through the warp's queue so that 32 of them are
-// stored at a time: stored one by one, under a branch per particle, 128 M took 761 us without keys, now 684.  Movers are counted as they are stored, so
-// that an input with too many of them, or one that is in no order at all, is given up within the first rounds.
+// stored at a time: stored one by one, under a branch per particle, 128 M took 761 us without keys, now 684.
 template <bool VEC, bool WHOLE>
 __global__ void __launch_bounds__(kSettledThreads, 2)
 settled_scan_kernel(const __grid_constant__ SettledArgs a) {
@@ -201,11 +248,16 @@ settled_scan_kernel(const __grid_constant__ SettledArgs a) {
   extern __shared__ MoverQueue queues[];
   const int tid = threadIdx.x, lane = tid & 31;
   MoverQueue& queue = queues[tid >> 5];
-  if (tid == 0) fill = stop = 0;
-  __syncthreads();
+  // One answer for the block: others may set the word meanwhile.
+  const bool refused = a.hdr->settle_sampled > a.most_sampled;
+  if (tid == 0) {
+    fill = stop = 0;
+    if (refused && blockIdx.x == 0) fail_settle(a.hdr);
+  }
+  if (__syncthreads_or(refused || (tid == 0 && settle_failed(a.hdr)))) return;
   const int block_first = blockIdx.x * a.per_block;
   const int last = min(a.n - block_first, a.per_block) + block_first;
-  const uint32_t room = static_cast<uint32_t>(a.per_block / kMoverShare);
+  const uint32_t room = static_cast<uint32_t>(a.per_block / kListShare);
   uint32_t* list = a.list + static_cast<size_t>(blockIdx.x) * room * kRecordWords;
   // The two ends of the input; the places between are the rounds' business.
   if (tid == 0 && blockIdx.x == 0) a.first[settled_cell<WHOLE>(a.x[0], a.y[0], a.z[0], a.grid) >> a.shift] = 0;
@@ -218,12 +270,10 @@ settled_scan_kernel(const __grid_constant__ SettledArgs a) {
     const bool seen = last - i >= kSettledRound ? scan_round<VEC, WHOLE, true>(a, i0, last, queue, queued)
                                                 : scan_round<VEC, WHOLE, false>(a, i0, last, queue, queued);
     bool bad = __any_sync(0xffffffffu, seen);  // one answer for the warp, as all below
-    // What the warps of a block may have stored up to their round r, with a few rounds of slack.
-    const uint32_t allowed = min(room, static_cast<uint32_t>(r + 3) * (kSettledRound / kMoverShare));
     __syncwarp();
     while (queued >= 32 && !bad) {
       queued -= 32;
-      bad = !flush_movers(a, queue, queued, 32, &fill, allowed, list);
+      bad = !flush_movers(a, queue, queued, 32, &fill, room, list);
     }
     if (bad) {
       if (lane == 0) {
@@ -329,6 +379,7 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   if (tid == here - 1) output[here] = cut.found;
   if (tid < here) a.cursor[b0 + tid] = base[1] + arrivals;
   __syncthreads();
+  if (tid == 0 && base[1] + arrived[here] > a.most_movers) fail_settle(a.hdr);  // more than there is room for
   const int most = max(1, FinishSettled::kMaxCells >> a.shift);
   cut_groups_of_block(cut, here, kGroupSpanLog, most, a.capacity, &a.hdr->aux_counter[2]);
   auto write_table = [&](uint32_t row, int first, int end) {
@@ -349,7 +400,7 @@ __global__ void __launch_bounds__(kSettledThreads)
 settled_movers_kernel(const __grid_constant__ SettledArgs a) {
   chain_begin();
   if (settle_failed(a.hdr)) return;
-  const uint32_t room = static_cast<uint32_t>(a.per_block / kMoverShare);
+  const uint32_t room = static_cast<uint32_t>(a.per_block / kListShare);
   const uint4* list = reinterpret_cast<const uint4*>(a.list + static_cast<size_t>(blockIdx.x) * room * kRecordWords);
   const uint32_t count = a.list_count[blockIdx.x];
 #pragma unroll 2

@@ -2630,13 +2630,19 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
 
 namespace {
 // From how many particles on a moved state is first tried as a settled one, where the general path
-// would reserve its slots tile by tile, and where it would not.  Per call, general / settled: re-sort
-// or step of 1 M particles 70 / 73 us, 1.5 M 89 / 80, 4 M 184 / 163, 6 M 230 / 200 (tiles); 8 M 287 / 288, 8 M with 4 particles
-// to a cell 256 / 262, with 40 245 / 258, 12 M 349 / 356 (its scatter is near HBM speed on input that is
-// nearly in order, and the launches count); 16 M 550 / 528, 30 M 832 / 787, 50 M 1470 / 1268, 128 M 3905 /
-// 3281 (the finish kernel's large blocks).
+// would reserve its slots tile by tile, and where it would not.  Per call, general / settled, five percent leaving
+// their cell: re-sort or step of 1 M particles 70 / 73 us, 1.6 M 86 / 79, 4 M 169 / 145, 6 M 230 / 197 (tiles);
+// 8 M 287 / 288, 12.5 M 372 / 367, 14.5 M 419 / 415 (its scatter is near HBM speed on input that is nearly in
+// order, and the launches count: less gain than a call loses that gives up), 15.5 M 448 / 438; 24 M 666 / 640, 30 M
+// 820 / 780, 64 M 1850 / 1597, 128 M 3650 / 3130 (the general finish kernel's large blocks).
 constexpr int64_t kSettledLeast = int64_t{3} << 19;
 constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
+// Particles in a thousand that leave their bucket, above which the general path does the call: where the settled
+// sort takes as long as giving up and the general path (tiles; small finish blocks; large ones).  Settled / given up:
+// 1.6 M particles with 159 movers in a thousand 88.8 / 93.0 us, with 248 99.6; 4 M 153 172.8 / 177.9, 183 178.0;
+// 16.8 M 46 477 / 484, 56 483, 66 491; 24 M 66 676 / 670; 30 M 126 930 / 836; 64 M 111 1832 / 1844, 131 1893; 128 M 105
+// 3575 / 3630, 129 3751.
+constexpr int64_t kMoversTiled = 180, kMoversSmall = 60, kMoversLarge = 120;
 
 bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
   const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
@@ -2684,6 +2690,11 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
   s.per_block = static_cast<int>(((a.n + most - 1) / most + kSettledRound - 1) / kSettledRound) * kSettledRound;
   s.scan_blocks = static_cast<int>((a.n + s.per_block - 1) / s.per_block);
   s.capacity = static_cast<uint32_t>(group_capacity_for(a.n, FinishSettled::kCapacity, FinishSettled::kBlocks));
+  const int64_t in_last = a.n - static_cast<int64_t>(s.scan_blocks - 1) * s.per_block;
+  const int64_t apart = s.per_block / kProbeSamples;
+  const int64_t samples = static_cast<int64_t>(s.scan_blocks - 1) * kProbeSamples + (in_last + apart - 1) / apart;
+  s.most_sampled = static_cast<uint32_t>(samples * (p.tiled ? kMoversTiled : p.small_blocks ? kMoversSmall : kMoversLarge) / 1000);
+  s.most_movers = static_cast<uint32_t>(a.n / kMoverShare);
   s.hdr = hdr;
   size_t used = 0;
   auto take = [&](int64_t words) {
@@ -2701,9 +2712,8 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
   s.cursor = take(buckets);
   s.sums = take((buckets + kSettledPart - 1) / kSettledPart * 4);
   s.tables = take(buckets * kSettledRowWords);
-  const int64_t movers = static_cast<int64_t>(s.scan_blocks) * (s.per_block / kMoverShare);
-  s.list = take(movers * kRecordWords);
-  s.arrived = take(movers * kRecordWords);
+  s.list = take(static_cast<int64_t>(s.scan_blocks) * (s.per_block / kListShare) * kRecordWords);
+  s.arrived = take(static_cast<int64_t>(s.most_movers) * kRecordWords);
   *out = s;
   return used <= room;
 }
@@ -2720,11 +2730,10 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   cudaError_t e = allow_shared(finish, kSmem);
   if (e == cudaSuccess) e = allow_shared(scan, kScanSmem);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(s.first, 0, zero_bytes, a.stream);
-  if (e != cudaSuccess) return e;
   stage_begin(kStageBucketCount, a.stream);
-  scan<<<s.scan_blocks, kSettledThreads, kScanSmem, a.stream>>>(s);
-  e = cudaGetLastError();
+  e = launch_chained(whole ? settled_probe_kernel<true> : settled_probe_kernel<false>, s.scan_blocks, kSettledThreads, 0,
+                     a.stream, s, zero_bytes / sizeof(uint4));
+  if (e == cudaSuccess) e = launch_chained(scan, s.scan_blocks, kSettledThreads, kScanSmem, a.stream, s);
   stage_end(kStageBucketCount, a.stream);
   stage_begin(kStageBucketScan, a.stream);
   if (e == cudaSuccess)
@@ -2740,7 +2749,7 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   if (e == cudaSuccess)
     e = launch_chained<true>(finish, sm_count() * FinishSettled::kBlocks, kSettledThreads, kSmem,
                              a.stream, s, out);
-  count_launches(5);
+  count_launches(6);
   return e;
 }
 }  // namespace
@@ -2763,7 +2772,9 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   DigitPassArgs digits;  // a workspace too small for them is refused before anything is enqueued
   cudaError_t e = digit_pass_args(a, &digits);
   if (e != cudaSuccess) return e;
-  {  // header and run counts
+  // Header and run counts.  An ordinary launch, which begins when all before it in the stream is done: the
+  // kernels chained to it read the call's inputs before they wait for it.
+  {
     const int64_t pieces = static_cast<int64_t>(l.start_off / sizeof(uint4));
     const int blocks = static_cast<int>(std::min<int64_t>((pieces + 511) / 512, 2 * sm_count()));
     clear_kernel<<<blocks, 512, 0, a.stream>>>(reinterpret_cast<uint4*>(base), pieces);

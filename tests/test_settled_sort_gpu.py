@@ -154,6 +154,41 @@ def test_too_many_movers(cuda):
     _run(grid, pos, vel, _dt(grid, 1.0), cuda, 'given up')
 
 
+@pytest.mark.parametrize('some,every', [(2, 7), (3, 7)])
+def test_a_part_of_the_input_with_many_movers(cuda, some, every):
+    """Some particles of every seven of one block of the scan leave their bucket, and hardly any other."""
+    grid, pos, vel = _sorted_state(LEAST, (64, 64, 64), cuda, 14)
+    dt = _dt(grid, 0.001)
+    here = torch.arange(50 * 6144, 51 * 6144, device=cuda)
+    here = here[here % every < some]
+    vel[1, here] = (1.5 / 64 / dt) * (1 - 2 * (pos[1][here] > 0.5).float())
+    _run(grid, pos, vel, dt, cuda, 'settled')
+
+
+@pytest.mark.parametrize('most', [16, 30])
+def test_movers_that_the_sample_does_not_see(cuda, most):
+    """The sample is every 48th particle of the scan's blocks.  A third of all particles leave their bucket:
+    more than there is room for in all; five of eight: more than a block's list holds."""
+    grid, pos, vel = _sorted_state(LEAST, (64, 64, 64), cuda, 15)
+    dt = _dt(grid, 0.001)
+    at = torch.arange(LEAST, device=cuda) % 48
+    here = (at >= 1) & (at <= most)
+    vel[1, :LEAST][here] = (1.5 / 64 / dt) * (1 - 2 * (pos[1][here] > 0.5).float())
+    _run(grid, pos, vel, dt, cuda, 'given up')
+
+
+# On either side of the share from which on the general path is faster, which is another for each of its plans.
+@pytest.mark.parametrize('n,cells,share,route', [(LEAST, (64, 64, 64), 0.15, 'settled'),
+                                                 (LEAST, (64, 64, 64), 0.35, 'given up'),
+                                                 (LEAST_UNTILED + 1, (128, 128, 128), 0.06, 'settled'),
+                                                 (LEAST_UNTILED + 1, (128, 128, 128), 0.15, 'given up'),
+                                                 (40_000_003, (180, 170, 160), 0.1, 'settled'),
+                                                 (40_000_003, (180, 170, 160), 0.25, 'given up')])
+def test_shares_of_movers(cuda, n, cells, share, route):
+    """`share`: of the particles leave their cell."""
+    grid, pos, vel = _sorted_state(n, cells, cuda, 16)
+    _run(grid, pos, vel, _dt(grid, share / 2.39), cuda, route)
+
 @pytest.mark.parametrize('where', [0, 777_777, -1])
 def test_one_particle_out_of_order(cuda, where):
     """Two particles of far-apart buckets change places; -1: the last with the first."""
