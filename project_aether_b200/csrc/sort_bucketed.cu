@@ -2507,10 +2507,12 @@ cudaError_t launch_groups(cudaStream_t stream, const uint32_t* counts, int64_t n
 // Whether the kernels of a call that take long are chained (see chain_begin): without payload where tiles
 // are split, and where slots are reserved tile by tile.  Without payload but with more buckets than a split
 // takes, all chained / only the short ones: 75 M particles 2037 / 2009 us per call, 100 M 2984 / 2898, 200 M
-// 6810 / 6470.  Those behind a sort of a settled state usually return at once.
+// 6810 / 6470.  Those behind a sort of a settled state usually return at once (settled, 16.8 M
+// 467 / 473 us, 64 M 1592 / 1597), but where they do not, chained ones cost that much too (64 M in random order, given
+// up: 2357 / 2221): all are chained with small finish blocks only.
 bool heavy_chained(const BucketPlan& p, bool behind) {
   const bool split = p.keys_only && p.buckets <= kSplitMaxBuckets;
-  return chained_launches() >= (behind || split || p.tiled ? 1 : 2);
+  return chained_launches() >= ((behind && p.small_blocks) || split || p.tiled ? 1 : 2);
 }
 
 template <class Shape>
