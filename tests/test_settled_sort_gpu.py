@@ -207,10 +207,8 @@ def test_random_order(cuda):
     _run(grid, pos, vel, _dt(grid), cuda, 'given up')
 
 
-def test_counters_that_wrap(cuda):
-    """Among 512 cells of a group every cell has 32 counters: 2400 particles of one random cell are
-    some 75 on each, but 2400 on one of two cells side by side whose shuffle bits are drawn once per
-    particle never wrap; equal low key bits do.  Here a cell holds what a block still takes."""
+def test_a_crowded_cell_that_a_group_holds(cuda):
+    """Every cell of a group has 32 counters: 2000 particles of one cell are some 60 on each."""
     n, crowd = LEAST + 100, 2_000
     grid, pos, vel = _sorted_state(n, (128, 128, 128), cuda, 10)
     for t in pos:
@@ -218,6 +216,47 @@ def test_counters_that_wrap(cuda):
     vel[:, n // 2:n // 2 + crowd] = 0.0
     _run(grid, pos, vel, _dt(grid), cuda, 'settled')
 
+
+def _same_shuffle_bits(n, seed, first, last):
+    """Particles whose keys have the same shuffle bits."""
+    bits = so.shuffle_bits(n, seed)
+    return first + np.flatnonzero(bits[first:last] == bits[first])
+
+
+@pytest.mark.parametrize('crowd,route', [(0, 'given up'), (3_000, 'settled')])
+def test_counters_that_wrap(cuda, crowd, route):
+    """300 particles with equal shuffle bits meet in one cell: more than a counter of one byte counts.  Among a
+    group's records the sort is given up, after other groups have been written, and done from the start; in
+    a bucket of the tail kernel it goes to the digit passes."""
+    n, cells = LEAST + 100, (64, 64, 64)
+    grid, pos, vel = _sorted_state(n, cells, cuda, 17)
+    dt, seed = _dt(grid), 0x9876543210 + n
+    to = n // 2
+    if crowd:
+        _crowd(pos, vel, to, crowd)
+    same = _same_shuffle_bits(n, seed, 1, n - 1)
+    same = torch.from_numpy(same[np.linspace(0, same.size - 1, 300).astype(np.int64)]).to(cuda)
+    for k, h in enumerate(cells):
+        centre = ((pos[k][to] * h / grid.hi[k]).floor() + 0.5) / h * grid.hi[k]
+        vel[k, same] = (centre - pos[k][same]) / dt
+    _run(grid, pos, vel, dt, cuda, route, digits=True)
+
+
+@pytest.mark.parametrize('ix_offset,nx_local', [(0, 33), (16, 32), (43, 21)])
+@pytest.mark.parametrize('drop', [0, 1])
+def test_slabs(cuda, ix_offset, nx_local, drop):
+    """A state in the order of a slab's cells.  Particles that leave the slab are binned into its nearest column."""
+    n, cells = LEAST + 11 + drop, (64, 60, 50)
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 0.7), cells)
+    gen = torch.Generator(device=cuda).manual_seed(18)
+    x, y, z = (torch.rand(n, device=cuda, generator=gen) for _ in range(3))
+    x = (ix_offset + x * nx_local) / cells[0]
+    vel = torch.zeros((3, -(-n // 4) * 4), device=cuda)
+    vel[:, :n] = torch.randn((3, n), device=cuda, generator=gen)
+    slab = {'ix_offset': ix_offset, 'nx_local': nx_local}
+    state = pa.sort_and_gather_particles(x, y, z * 0.7, vel, grid, 3, **slab)
+    pos = [t[drop:] for t in state.positions]
+    _run(grid, pos, state.velocity[:, drop:n] if drop else state.velocity, _dt(grid), cuda, 'settled', slab=slab)
 
 def test_outputs_over_the_inputs(cuda):
     n = LEAST + 4
