@@ -29,8 +29,8 @@
 // it is noticed: random order and too many movers by the probe; a particle out of order, or more movers than
 // the lists hold in one part of the input, in the round of the scan that meets it; a counter that wraps in
 // the finish.  Buckets of a dense region are no reason.  Calls that the probe gives up, before there was this path /
-// now: 1.6 M particles 88.1 / 93.0 us, 4 M 171.5 / 177.8, 16.8 M 480 / 484, 30 M 837 / 836, 64 M 1884 / 1844; in random
-// order 1.6 M 89.4 / 94.2, 4 M 183 / 190, 16.8 M 586 / 615, 64 M 2212 / 2221.
+// now: 1.6 M particles 88.0 / 93.0 us, 4 M 171.5 / 177.8, 16.8 M 487 / 486, 30 M 854 / 837, 64 M 1874 / 1846; in random
+// order 1.6 M 92.2 / 96.4, 4 M 186 / 189, 6 M 251 / 254, 17 M 647 / 645, 24 M 840 / 830, 64 M 2290 / 2266.
 
 constexpr int kSettledThreads = 512;
 constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round

@@ -996,7 +996,10 @@ group_kernel(const uint32_t* counts, uint32_t n, uint32_t* cursor, uint32_t* run
              uint32_t capacity, uint32_t largest, uint32_t* __restrict__ bucket_start,
              uint32_t* __restrict__ tables, uint32_t* __restrict__ group_count, Header* __restrict__ hdr,
              bool behind) {
-  chain_begin();
+  // Behind a sort of a settled state the scatter kernel is chained too, and set up while these blocks hold
+  // their multiprocessors its blocks would lie unevenly (17 M particles in random order, given up: 779 -> 645 us).
+  if (!behind) chain_release();
+  chain_wait();
   if (settled_before(hdr, behind)) return;
   // Up to kGroupStagedChunks chunks, [chunks][kGroupSpan + 1] each: the first record of every
   // run, and the records before the bucket in the chunks before c.
@@ -2507,12 +2510,12 @@ cudaError_t launch_groups(cudaStream_t stream, const uint32_t* counts, int64_t n
 // Whether the kernels of a call that take long are chained (see chain_begin): without payload where tiles
 // are split, and where slots are reserved tile by tile.  Without payload but with more buckets than a split
 // takes, all chained / only the short ones: 75 M particles 2037 / 2009 us per call, 100 M 2984 / 2898, 200 M
-// 6810 / 6470.  Those behind a sort of a settled state usually return at once (settled, 16.8 M
-// 467 / 473 us, 64 M 1592 / 1597), but where they do not, chained ones cost that much too (64 M in random order, given
-// up: 2357 / 2221): all are chained with small finish blocks only.
+// 6810 / 6470.  Those behind a sort of a settled state usually return at once (16.8 M
+// 473 / 467 us, 64 M 1600 / 1593); where they do not, chaining costs nothing as long as each is let in only when
+// the one before it ends.
 bool heavy_chained(const BucketPlan& p, bool behind) {
   const bool split = p.keys_only && p.buckets <= kSplitMaxBuckets;
-  return chained_launches() >= ((behind && p.small_blocks) || split || p.tiled ? 1 : 2);
+  return chained_launches() >= (behind || split || p.tiled ? 1 : 2);
 }
 
 template <class Shape>
