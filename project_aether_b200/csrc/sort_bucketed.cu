@@ -1845,12 +1845,16 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
 // Blocks per multiprocessor, fewer of them where there is little to do.
 template <class Shape>
 constexpr int kTailBlocks = Shape::kThreads <= 512 ? 2 : 1;
-template <class Shape>
+// `settled`: what the sort of a settled state before it left, or NotSettled where there was none (with
+// the arguments of such a sort 650,000 particles took 49.1 us instead of 48.4).
+struct NotSettled {};
+template <class Shape, class Settled>
 __global__ void __launch_bounds__(Shape::kThreads, kTailBlocks<Shape>)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
-                   DigitPassArgs digits, bool behind, const __grid_constant__ SettledArgs settled) {
+                   DigitPassArgs digits, const __grid_constant__ Settled settled) {
+  constexpr bool kBehind = std::is_same_v<Settled, SettledArgs>;
   chain_wait();
-  const bool is_settled = Shape::kRecordWords == kRecordWords && settled_before(hdr, behind);
+  const bool is_settled = settled_before(hdr, kBehind);
   const bool all_done = is_settled ? hdr->settle_large == 0 : hdr->max_bucket <= capacity && hdr->redo_groups == 0;
   if (!handed_over(hdr) && all_done) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1864,7 +1868,7 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
     // A block that comes late may see another block's hand-over and skip its buckets: the digit
     // passes then write everything.
     FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
-    if constexpr (Shape::kRecordWords == kRecordWords) {
+    if constexpr (kBehind) {
       if (is_settled) {
         if (!standard && !finish_settled_large<Shape>(s, settled, out, item, items) && threadIdx.x == 0)
           atomicExch(&hdr->use_standard, 1);
@@ -2549,18 +2553,18 @@ cudaError_t launch_finish_large(const RunTable& t, const SortArgs& a, const Fini
 
 int limited(int blocks, int most) { return most > 0 ? std::min(blocks, most) : blocks; }
 
-template <class Shape>
+template <class Shape, class Settled>
 cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                        uint32_t group_capacity, const DigitPassArgs& digits, bool behind, bool chained,
-                        const SettledArgs& settled) {
+                        uint32_t group_capacity, const DigitPassArgs& digits, bool chained,
+                        const Settled& settled) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
-  const cudaError_t e = allow_shared(bucket_tail_kernel<Shape>, kSmem);
+  auto kernel = bucket_tail_kernel<Shape, Settled>;
+  const cudaError_t e = allow_shared(kernel, kSmem);
   if (e != cudaSuccess) return e;
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(sm_count() * kTailBlocks<Shape>, a.n / 2048)));
-  return launch_chained_if(chained, bucket_tail_kernel<Shape>, limited(blocks, a.most_blocks),
-                           Shape::kThreads, kSmem, a.stream, t, a.num_cells, out, hdr, group_capacity,
-                           digits, behind, settled);
+  return launch_chained_if(chained, kernel, limited(blocks, a.most_blocks), Shape::kThreads, kSmem, a.stream, t,
+                           a.num_cells, out, hdr, group_capacity, digits, settled);
 }
 
 template <int ITEMS>
@@ -2920,8 +2924,9 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
       : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, behind, chained)
                        : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, behind, chained);
   if (e == cudaSuccess)
-    e = p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, behind, chained, settled)
-                    : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, behind, chained, settled);
+    e = behind        ? launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, chained, settled)
+        : p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, chained, NotSettled{})
+                      : launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, chained, NotSettled{});
   stage_end(kStageBucketFinish, a.stream);
   count_launches(2);
   return e;
