@@ -29,8 +29,8 @@
 // it is noticed: random order and too many movers by the probe; a particle out of order, or more movers than
 // the lists hold in one part of the input, in the round of the scan that meets it; a counter that wraps in
 // the finish.  Buckets of a dense region are no reason.  Calls that the probe gives up, before there was this path /
-// now: 1.6 M particles 88.0 / 93.0 us, 4 M 171.5 / 177.8, 16.8 M 487 / 486, 30 M 854 / 837, 64 M 1874 / 1846; in random
-// order 1.6 M 92.2 / 96.4, 4 M 186 / 189, 6 M 251 / 254, 17 M 647 / 645, 24 M 840 / 830, 64 M 2290 / 2266.
+// now: 1.6 M particles 88.0 / 94.0 us, 4 M 172 / 177, 16.8 M 483 / 487, 30 M 839 / 839, 64 M 1881 / 1850; in random
+// order 1.6 M 89.0 / 92.5, 4 M 184 / 189, 6 M 251 / 252, 16.8 M 597 / 602, 64 M 2258 / 2239.
 
 constexpr int kSettledThreads = 512;
 constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round
@@ -201,7 +201,7 @@ __device__ __forceinline__ bool scan_round(const SettledArgs& a, int i0, int las
 // Clears the tables of the scan and takes a sample of its particles, evenly spaced, with each one's neighbour.
 // Bound by the latency of one access to HBM, which is hidden beside the kernel that zeroes the header: the inputs
 // are read before the wait.  In place of a clear of the tables alone, which took a launch too: 4 M particles
-// 143.4 -> 144.6 us per call, 1.6 M 81.5 -> 79.3.
+// 143.5 -> 144.5 us per call, 1.6 M 81.5 -> 79.3, 16.8 M alike.
 template <bool WHOLE>
 __global__ void __launch_bounds__(kSettledThreads)
 settled_probe_kernel(const __grid_constant__ SettledArgs a, int64_t pieces) {
@@ -245,7 +245,9 @@ settled_probe_kernel(const __grid_constant__ SettledArgs a, int64_t pieces) {
 template <bool VEC, bool WHOLE>
 __global__ void __launch_bounds__(kSettledThreads, 2)
 settled_scan_kernel(const __grid_constant__ SettledArgs a) {
-  chain_begin();
+  // No early release: the waiting blocks of the kernels behind would stand beside these (4 M particles 144.5 ->
+  // 141.9 us per call, 16.8 M 467 -> 461, 64 M 1593 -> 1583).
+  chain_wait();
   __shared__ uint32_t fill, stop;
   extern __shared__ MoverQueue queues[];
   const int tid = threadIdx.x, lane = tid & 31;

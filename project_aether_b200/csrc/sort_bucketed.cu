@@ -2640,17 +2640,18 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
 namespace {
 // From how many particles on a moved state is first tried as a settled one, where the general path
 // would reserve its slots tile by tile, and where it would not.  Per call, general / settled, five percent leaving
-// their cell: re-sort or step of 1 M particles 70 / 73 us, 1.6 M 86 / 79, 4 M 169 / 145, 6 M 230 / 197 (tiles);
+// their cell: re-sort or step of 1 M particles 70 / 73 us, 1.6 M 86 / 80, 4 M 170 / 144, 6 M 230 / 194 (tiles);
 // 8 M 287 / 288, 12.5 M 372 / 367, 14.5 M 419 / 415 (its scatter is near HBM speed on input that is nearly in
-// order, and the launches count: less gain than a call loses that gives up), 15.5 M 448 / 438; 24 M 666 / 640, 30 M
-// 820 / 780, 64 M 1850 / 1597, 128 M 3650 / 3130 (the general finish kernel's large blocks).
+// order, and the launches count), 15.5 M 448 / 438; 16.8 M 479 / 462, 24 M 663 / 632, 30 M 822 / 773, 64 M 1847 / 1585,
+// 128 M 3617 / 3115 (the general finish kernel's large blocks).  Below 2^24 the untiled gain is no more than a call
+// that gives up may lose.
 constexpr int64_t kSettledLeast = int64_t{3} << 19;
 constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
-// Particles in a thousand that leave their bucket, above which the general path does the call: where the settled
-// sort takes as long as giving up and the general path (tiles; small finish blocks; large ones).  Settled / given up:
-// 1.6 M particles with 159 movers in a thousand 88.8 / 93.0 us, with 248 99.6; 4 M 153 172.8 / 177.9, 183 178.0;
-// 16.8 M 46 477 / 484, 56 483, 66 491; 24 M 66 676 / 670; 30 M 126 930 / 836; 64 M 111 1832 / 1844, 131 1893; 128 M 105
-// 3575 / 3630, 129 3751.
+// Particles in a thousand that leave their bucket, above which the general path does the call: about where the
+// settled sort takes as long as giving up and the general path (tiles; small finish blocks; large ones).  Movers
+// in a thousand, settled / given up, us per call: 4 M 153 172.8 / 177, 183 178.0; 1.6 M 159 88.8 / 94, 248 99.6; 16.8 M
+// 56 475 / 487, 30 M 52 797 / 839, 126 930; 64 M 98 1765 / 1850, 131 1893; 128 M 98 3480 / 3631, 129 3750 (the largest of each
+// with a scan that was 1.5 % slower).
 constexpr int64_t kMoversTiled = 180, kMoversSmall = 60, kMoversLarge = 120;
 
 bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
