@@ -72,7 +72,8 @@ int AetherSortBucketPlan(int64_t n, int64_t num_cells, int32_t* cells_per_bucket
  * while the one before it still runs (programmatic dependent launch), and in calls without payload
  * (of up to some 68 million particles) and middling ones all of them; mode 2: the scatter, finish and
  * tail kernels of every call (measured slower on larger inputs); mode 0: ordinary launches.  Every
- * kernel waits for the grids before it to complete before it touches anything, so the work
+ * kernel waits for the grids before it to complete before it touches what they write, and a call's first
+ * kernel for all that is in the stream before the call, so the work
  * runs in stream order in every mode and results do not depend on it. */
 int AetherSortSetChainedLaunches(int32_t mode);
 

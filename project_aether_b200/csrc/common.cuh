@@ -225,14 +225,19 @@ void count_launches(int kernels);
 // Chained launches.  The kernels of a larger sort call (count, run scan, groups, scatter, finish,
 // tail; or the digit passes') run one after the other on one stream, and in the gaps between them
 // the next kernel's launch begins when the previous grid has drained.  A kernel launched with
-// launch_chained may be set up while its predecessor still runs: every kernel of the chain
+// launch_chained may be set up while its predecessor still runs: every short kernel of the chain
 // begins with chain_begin(), which lets the kernel behind it start its launch
 // (griddepcontrol.launch_dependents) and then waits until the grids before it are complete
-// and their memory visible (griddepcontrol.wait).  Nothing of a kernel's work moves ahead of
-// that wait, so the order of the work is that of the stream.  Launched in the ordinary way
+// and their memory visible (griddepcontrol.wait).  Nothing that an earlier kernel of the call writes is
+// touched before that wait, so the order of the work is that of the stream.  (The call's inputs, and tables that
+// no kernel before writes, may be: a call begins with clear_kernel, an ordinary launch, so that all before
+// the call is done; small_sort_kernel and settled_probe_kernel, chained to it, read their particles while
+// it runs.)  Launched in the ordinary way
 // the same kernels find nothing to wait for.  Kernels that fill the multiprocessors for a long time
 // wait with chain_wait() and let the kernel behind them in when a block has done its work
-// (chain_release()): waiting blocks in their midst cost more than the launch.  Per call, only the short
+// (chain_release()), or when they end: waiting blocks in their midst cost more than the launch, and blocks that
+// are placed while others leave lie unevenly on the multiprocessors, which a kernel whose blocks share
+// the work evenly pays for to its end.  Per call, only the short
 // kernels chained / these too: without payload 4 M particles 110.8 / 104.0 us, 16 M 348 / 343; with
 // payload 1 M 61 / 56, 16 M 556 / 557, 64 M 2241 / 2373, 256 M 10.7 / 11.0 ms.  Without
 // payload and without a split, 200 M 6470 / 6810 us.  So they are chained in calls without payload whose
@@ -249,8 +254,6 @@ __device__ __forceinline__ void chain_begin() {
 int chained_launches();            // process-wide: 0 none, 1 the short kernels, 2 all
 void set_chained_launches(int mode);
 
-// `heavy`: a kernel that fills the multiprocessors for a long time (scatter, finish); chained
-// only in mode 2.
 template <class... Params, class... Args>
 cudaError_t launch_chained_if(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block,
                               size_t shared_bytes, cudaStream_t stream, Args&&... args) {
@@ -266,6 +269,7 @@ cudaError_t launch_chained_if(bool chained, void (*kernel)(Params...), dim3 grid
   config.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
+// HEAVY: a kernel that fills the multiprocessors for a long time; chained only in mode 2.
 template <bool HEAVY = false, class... Params, class... Args>
 cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes,
                            cudaStream_t stream, Args&&... args) {

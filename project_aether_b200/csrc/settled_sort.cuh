@@ -21,7 +21,7 @@
 //
 // It moves 24 + 4 + 28 + 32 bytes per particle, and some 130 more per mover, where the general path moves
 // 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
-// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3281 (941, 2157).
+// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3255 (897, 2071).
 //
 // Whether the input is in order, and how many particles move, is only known on the device.  Whatever
 // speaks against the path sets Header::settle_failed; the kernels above then stop, and the general path's
@@ -238,7 +238,7 @@ settled_probe_kernel(const __grid_constant__ SettledArgs a, int64_t pieces) {
   }
 }
 
-// Bound by instructions (73 % of the issue slots; HBM would take half the time).  The home runs are
+// Bound by instructions (65 % of the issue slots; HBM would take half the time).  The home runs are
 // written where a bucket begins and where the bucket before it ends.  A mover costs two adds and a record
 // of {cell, index, moved state}, which goes through the warp's queue so that 32 of them are
 // stored at a time: stored one by one, under a branch per particle, 128 M took 761 us without keys, now 684.
@@ -425,7 +425,7 @@ __device__ __forceinline__ void prefetch_range(const void* from, uint32_t bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p0), "r"(static_cast<uint32_t>(p1 - p0)) : "memory");
 }
 
-// Bound by instructions: 2157 us for 128 M particles, two blocks per multiprocessor.
+// Bound by instructions and the shared-memory pipe (issue slots 55 %, pipe 55 %): 2071 us for 128 M particles, two blocks per multiprocessor.
 // The finish: groups blockIdx.x, blockIdx.x + gridDim.x, ... of the list.  A thread loads all its
 // particles of a group before the first is used; the group behind is asked into L2 meanwhile.
 __global__ void __launch_bounds__(kSettledThreads, FinishSettled::kBlocks)

@@ -1341,7 +1341,7 @@ __device__ __forceinline__ bool sort_placed(FinishSmem<Shape>& s, const FinishOu
   {
 #pragma unroll
     for (int j = 0; j < kWordsPerThread; j += 4) {
-      uint4 a = make_uint4(0u, 0u, 0u, 0u);  // hist_words is a multiple of 8
+      uint4 a = make_uint4(0u, 0u, 0u, 0u);  // hist_words is a multiple of 4
       if (tid * kWordsPerThread + j < hist_words) a = *reinterpret_cast<const uint4*>(&s.hist[tid * kWordsPerThread + j]);
       const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
@@ -1374,7 +1374,7 @@ __device__ __forceinline__ bool sort_placed(FinishSmem<Shape>& s, const FinishOu
   const uint32_t thread_base = s.warp_sum[warp] + incl - sum;
 #pragma unroll
   for (int j = 0; j < kWordsPerThread; j += 8)
-    if (tid * kWordsPerThread + j < hist_words) {  // hist_words is a multiple of 8
+    if (tid * kWordsPerThread + j < hist_words) {  // of eight words at its end four may lie past it: unused
       uint4 packed_prefix;
       packed_prefix.x = (thread_base + local[j]) | ((thread_base + local[j + 1]) << 16);
       packed_prefix.y = (thread_base + local[j + 2]) | ((thread_base + local[j + 3]) << 16);
