@@ -29,8 +29,8 @@
 // it is noticed: random order and too many movers by the probe; a particle out of order, or more movers than
 // the lists hold in one part of the input, in the round of the scan that meets it; a counter that wraps in
 // the finish.  Buckets of a dense region are no reason.  Calls that the probe gives up, before there was this path /
-// now: 1.6 M particles 88.0 / 94.0 us, 4 M 172 / 177, 16.8 M 483 / 487, 30 M 839 / 839, 64 M 1881 / 1850; in random
-// order 1.6 M 89.0 / 92.5, 4 M 184 / 189, 6 M 251 / 252, 16.8 M 597 / 602, 64 M 2258 / 2239.
+// now: 1.6 M particles 86.9 / 91.4 us, 4 M 170 / 176, 16.8 M 482 / 485, 30 M 837 / 837, 64 M 1885 / 1849; in random
+// order 1.6 M 87.3 / 90.9, 4 M 184 / 187, 6 M 250.5 / 251, 16.8 M 599 / 602, 64 M 2266 / 2246.
 
 constexpr int kSettledThreads = 512;
 constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round
@@ -402,7 +402,10 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
 // The movers' records to their buckets, with their keys.
 __global__ void __launch_bounds__(kSettledThreads)
 settled_movers_kernel(const __grid_constant__ SettledArgs a) {
-  chain_begin();
+  // No early release, so that the finish is placed on free multiprocessors (chained to this and let in at once /
+  // at its end: 16.8 M particles 464 / 460 us per call, 64 M 1592 / 1580; an ordinary launch 463 / 1582, 2.6 M 106.2
+  // against 103.8).
+  chain_wait();
   if (settle_failed(a.hdr)) return;
   const uint32_t room = static_cast<uint32_t>(a.per_block / kListShare);
   const uint4* list = reinterpret_cast<const uint4*>(a.list + static_cast<size_t>(blockIdx.x) * room * kRecordWords);

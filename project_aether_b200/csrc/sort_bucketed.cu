@@ -2640,10 +2640,10 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
 namespace {
 // From how many particles on a moved state is first tried as a settled one, where the general path
 // would reserve its slots tile by tile, and where it would not.  Per call, general / settled, five percent leaving
-// their cell: re-sort or step of 1 M particles 70 / 73 us, 1.6 M 86 / 80, 4 M 170 / 144, 6 M 230 / 194 (tiles);
+// their cell: re-sort or step of 1 M particles 70 / 73 us, 1.6 M 84 / 78, 4 M 168 / 142, 6 M 229 / 191 (tiles);
 // 8 M 287 / 288, 12.5 M 372 / 367, 14.5 M 419 / 415 (its scatter is near HBM speed on input that is nearly in
-// order, and the launches count), 15.5 M 448 / 438; 16.8 M 479 / 462, 24 M 663 / 632, 30 M 822 / 773, 64 M 1847 / 1585,
-// 128 M 3617 / 3115 (the general finish kernel's large blocks).  Below 2^24 the untiled gain is no more than a call
+// order, and the launches count), 15.5 M 448 / 438; 16.8 M 479 / 460, 24 M 662 / 627, 30 M 822 / 770, 64 M 1852 / 1581,
+// 128 M 3625 / 3107 (the general finish kernel's large blocks).  Below 2^24 the untiled gain is no more than a call
 // that gives up may lose.
 constexpr int64_t kSettledLeast = int64_t{3} << 19;
 constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
@@ -2757,8 +2757,7 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   stage_end(kStageBucketScatter, a.stream);
   stage_begin(kStageBucketFinish, a.stream);
   if (e == cudaSuccess)
-    e = launch_chained<true>(finish, sm_count() * FinishSettled::kBlocks, kSettledThreads, kSmem,
-                             a.stream, s, out);
+    e = launch_chained(finish, sm_count() * FinishSettled::kBlocks, kSettledThreads, kSmem, a.stream, s, out);
   count_launches(6);
   return e;
 }
