@@ -21,7 +21,7 @@
 //
 // It moves 24 + 4 + 28 + 32 bytes per particle, and some 130 more per mover, where the general path moves
 // 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
-// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3255 (897, 2071).
+// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3248 (897, 2071).
 //
 // Whether the input is in order, and how many particles move, is only known on the device.  Whatever
 // speaks against the path sets Header::settle_failed; the kernels above then stop, and the general path's
