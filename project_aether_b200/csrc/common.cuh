@@ -63,7 +63,7 @@ struct alignas(16) Header {
   // groups cut, next task and tasks done of the finish.
   uint32_t tiles_counted, tiles_stored, help_next, groups, task_next, tasks_done;
   uint32_t settle_failed;     // the sort of a settled state gave the call to the general path
-  uint32_t settle_large;      // buckets of the sort of a settled state that no block holds
+  uint32_t settle_large;      // buckets of the sort of a settled state that a block of its finish does not hold
   uint32_t settle_sampled;    // movers among the particles that its probe looked at
   uint32_t kept_pad[1];
   uint32_t tile_claimed[kMaxTiles / 32], tile_loose[kMaxTiles / 32];  // one bit per tile

@@ -15,13 +15,13 @@
 //   settled_groups_kernel
 //   settled_movers_kernel  the lists' records to their buckets' arrivals
 //   settled_finish_kernel  a block takes a group: reads its home run and keys, moves the particles once
-//                          more, leaves out those that left, adds the arrivals, and sorts and
-//                          writes the group as the general finish kernel does
-//   bucket_tail_kernel     the buckets of dense regions, which a block does not hold
+//                          more, leaves out those that left, adds the arrivals, sorts and writes the group
+//   bucket_tail_kernel     the same for dense regions, whose buckets those blocks do not hold
 //
 // It moves 24 + 4 + 28 + 32 bytes per particle, and some 130 more per mover, where the general path moves
 // 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
-// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where they now take 3248 (897, 2071).
+// bytes, 128 M particles took 3499 us (scan 684, finish 2649) where with keys from the scan they took 3248 (897, 2071;
+// the finish now 1560).
 //
 // Whether the input is in order, and how many particles move, is only known on the device.  Whatever
 // speaks against the path sets Header::settle_failed; the kernels above then stop, and the general path's
@@ -38,12 +38,37 @@ constexpr int kListShare = 2;                       // a block's list has room f
 constexpr int kMoverShare = 4;                      // all lists together for one in four
 constexpr int kProbeSamples = 128;                  // particles of each of the scan's blocks that the probe looks at
 constexpr int kSettledPart = 4096;                  // buckets per entry of the coarse sums
+constexpr int kSettledSums = 4 * (1 + kSettledPart / kGroupSpan);  // words of such an entry: of the part, of its kGroupSpan buckets each
 constexpr uint32_t kGone = 0xffffffffu;             // no key: grids of 2^25 cells are left to the general path
 constexpr int kSettledRowWords = 8;                 // words of a group's table
-using FinishSettled = FinishSmall;
+// What sorts a group in the finish: THREADS threads that hold ITEMS records each, move and all, in registers.
+template <int THREADS, int ITEMS, int LOW_BITS>
+struct SettledShape {
+  static constexpr int kThreads = THREADS, kItems = ITEMS, kLowBits = LOW_BITS;
+  static constexpr int kBlocks = 1024 / THREADS;          // per multiprocessor, 64 registers a thread
+  static constexpr int kCapacity = THREADS * ITEMS;
+  static constexpr int kHistWords = (1 << LOW_BITS) / 4;  // byte counters, four to a word
+  static constexpr int kWordsPerThread = kHistWords / THREADS;
+  static constexpr int kMaxDrop = 2, kMostIndexBits = 0;  // see FinishShape
+  static constexpr int kMaxCells = 1 << (LOW_BITS + kMaxDrop - kShuffleBits);
+  static_assert(kWordsPerThread % 4 == 0 && THREADS <= 1024, "the counter scan reads four words at a time");
+};
+// Teams are the usual shape: a group's barriers hold up four warps only, and eight groups share a
+// multiprocessor (finish of 16.8 M particles, 8 to a cell: 199 us; 256 threads that hold 1024 records 213, 512 that
+// hold 2048 242, 64 that hold 256 214; three items a thread 217, six 220, eight 279, which leave fewer threads).  Their
+// groups span 64 cells at most, so that sparse grids do not fill them, and a cell may have some 400 particles: beyond
+// either limit the groups are blocks' (20 M particles, 4 / 5 / 6 to a cell: teams 351 / 300 / 253 us, blocks 285 /
+// 286 / 286).  Where the density differs from place to place, buckets above the shape's capacity, and what
+// lies near them, go to wide groups, which the tail kernel sorts.
+using SettledTeam = SettledShape<128, 4, 11>;
+using SettledBlock = SettledShape<512, 4, 14>;
+using SettledWide = SettledShape<1024, 4, 15>;
+constexpr int64_t kSettledTeamLeast = 352;     // particles on a team's most cells, on average at least
+constexpr int64_t kSettledTeamMostMean = 384;  // particles of a cell, on average at most
 // Records per bucket, on average at most.  Buckets cost this path little (a few words each), and with
-// eight or more to a group the groups fill a block whatever the density.
-constexpr int64_t kSettledTarget = 320;
+// five or more to a group the groups fill a team, or a block (teams, 16.8 M particles: 64 to a bucket 443 us per
+// call, 128 450).
+constexpr int64_t kSettledTeamTarget = 104, kSettledBlockTarget = 320;
 // Where single cells hold more than this on average, the buckets of the path would not fit a block.
 constexpr int64_t kSettledMostMean = 1024;
 
@@ -57,7 +82,7 @@ struct SettledArgs {
   int shift, buckets;
   int per_block;          // particles per block of the scan, a multiple of kSettledRound
   int scan_blocks;
-  uint32_t capacity;      // places of a group
+  int teams;              // whether groups of a few hundred places pay
   uint32_t most_sampled;  // movers of the sample from which on the general path is faster
   uint32_t most_movers;   // what fits `arrived`
   uint32_t *first, *end;            // [buckets] home run in the input; both zero if it is empty
@@ -65,9 +90,11 @@ struct SettledArgs {
   uint32_t* keys;                   // [n] key of every particle after the move, kGone of those that left
   uint32_t* list_count;             // [scan_blocks] movers found by each block of the scan
   uint32_t* cursor;                 // [buckets] next free place of each bucket's arrivals
-  uint32_t* sums;                   // [parts][4] particles at home, arrivals, output of kSettledPart buckets
-  uint32_t* tables;                 // [buckets][kSettledRowWords]: groups, and from the end buckets in no group
+  uint32_t* sums;                   // [parts][kSettledSums] particles at home, arrivals, output of kSettledPart buckets
+  uint32_t* tables;                 // [buckets][kSettledRowWords]: groups of teams, and from the end buckets in no group
+  uint32_t* wide_tables;            // [buckets][kSettledRowWords]: groups of dense regions
   uint32_t *list, *arrived;         // records: the movers block by block, and bucket by bucket
+  int vec_out;            // the outputs take 16-byte stores where the place is a multiple of four
   Header* hdr;
 };
 
@@ -295,43 +322,45 @@ settled_scan_kernel(const __grid_constant__ SettledArgs a) {
   if (tid == 0) a.list_count[blockIdx.x] = min(fill, room);
 }
 
-// Particles at home before the move, arrivals and output of every kSettledPart buckets.
+// Particles at home before the move, arrivals and output of every kSettledPart buckets, and of every kGroupSpan.
 __global__ void __launch_bounds__(1024)
 settled_sums_kernel(const __grid_constant__ SettledArgs a) {
   chain_begin();
   if (settle_failed(a.hdr)) return;
-  __shared__ uint32_t sum[3];
-  if (threadIdx.x < 3) sum[threadIdx.x] = 0;
+  __shared__ uint32_t sum[kSettledSums];
+  for (int i = threadIdx.x; i < kSettledSums; i += 1024) sum[i] = 0;
   __syncthreads();
-  uint32_t home = 0, arrivals = 0, left = 0;
   const int b0 = blockIdx.x * kSettledPart;
 #pragma unroll
   for (int k = 0; k < kSettledPart / 1024; ++k) {
-    const int b = b0 + k * 1024 + threadIdx.x;
+    const int at = k * 1024 + threadIdx.x, b = b0 + at;
+    uint32_t home = 0, arrivals = 0, left = 0;
     if (b < a.buckets) {
-      home += a.end[b] - a.first[b];
-      arrivals += a.arrivals[b];
-      left += a.leavers[b];
+      home = a.end[b] - a.first[b];
+      arrivals = a.arrivals[b];
+      left = a.leavers[b];
+    }
+    home = __reduce_add_sync(0xffffffffu, home);
+    arrivals = __reduce_add_sync(0xffffffffu, arrivals);
+    left = __reduce_add_sync(0xffffffffu, left);
+    if ((threadIdx.x & 31) < 2) {  // lane 0 adds to the part's sums, lane 1 to its kGroupSpan buckets'
+      uint32_t* to = sum + ((threadIdx.x & 31) == 0 ? 0 : 4 * (1 + at / kGroupSpan));
+      atomicAdd(to, home);
+      atomicAdd(to + 1, arrivals);
+      atomicAdd(to + 2, home + arrivals - left);
     }
   }
-  home = __reduce_add_sync(0xffffffffu, home);
-  arrivals = __reduce_add_sync(0xffffffffu, arrivals);
-  left = __reduce_add_sync(0xffffffffu, left);
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&sum[0], home);
-    atomicAdd(&sum[1], arrivals);
-    atomicAdd(&sum[2], home + arrivals - left);
-  }
   __syncthreads();
-  if (threadIdx.x < 3) a.sums[blockIdx.x * 4 + threadIdx.x] = sum[threadIdx.x];
+  for (int i = threadIdx.x; i < kSettledSums; i += 1024) a.sums[blockIdx.x * kSettledSums + i] = sum[i];
 }
 
-// A block takes kGroupSpan consecutive buckets; it adds up what lies before them for itself (the
-// coarse sums, and the buckets between the last of those and its own).  Groups as in group_kernel; a
-// bucket needs a place for each of its particles at home and each of its arrivals.  A group's
-// table: first particle of its home run, particles in it, first of its arrivals, arrivals, first
-// output slot, records, its buckets b0, b1.  A bucket that no block holds gets such a table too, for the tail
-// kernel, from the end of the array (there are no more groups and such buckets than buckets).
+// A block takes kGroupSpan consecutive buckets; it adds up what lies before them for itself, from the sums.
+// Groups as in group_kernel; a bucket needs a place for each of its particles at home and each of its arrivals.
+// A group's table: first particle of its home run, particles in it, first of its arrivals, arrivals, first
+// output slot, records, its buckets b0, b1.  Where one of the block's buckets is more than the finish kernel
+// holds, all are cut into wide groups, for the tail kernel; so is, with a table from the end of the first array (there
+// are no more groups and such buckets than buckets), a bucket that a wide group does not hold.  aux_counter[2], [3], [4]:
+// the three kinds.
 __global__ void __launch_bounds__(kGroupSpan)
 settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   chain_begin();
@@ -346,17 +375,11 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   if (tid < 3) base[tid] = 0;
   __syncthreads();
   uint32_t before[3] = {0, 0, 0};
-  const int part = b0 / kSettledPart;
-  for (int p = tid; p < part; p += kGroupSpan) {
+  const int part = b0 / kSettledPart, spans = (b0 - part * kSettledPart) / kGroupSpan;
+  for (int p = tid; p < part + spans; p += kGroupSpan) {
+    const uint32_t* sums = a.sums + (p < part ? p * kSettledSums : part * kSettledSums + 4 * (1 + p - part));
 #pragma unroll
-    for (int c = 0; c < 3; ++c) before[c] += a.sums[p * 4 + c];
-  }
-#pragma unroll 4
-  for (int b = part * kSettledPart + tid; b < b0; b += kGroupSpan) {
-    const uint32_t home = a.end[b] - a.first[b], in = a.arrivals[b];
-    before[0] += home;
-    before[1] += in;
-    before[2] += home + in - a.leavers[b];
+    for (int c = 0; c < 3; ++c) before[c] += sums[c];
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -384,19 +407,28 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   if (tid < here) a.cursor[b0 + tid] = base[1] + arrivals;
   __syncthreads();
   if (tid == 0 && base[1] + arrived[here] > a.most_movers) fail_settle(a.hdr);  // more than there is room for
-  const int most = max(1, FinishSettled::kMaxCells >> a.shift);
-  cut_groups_of_block(cut, here, kGroupSpanLog, most, a.capacity, &a.hdr->aux_counter[2]);
-  auto write_table = [&](uint32_t row, int first, int end) {
-    uint4* table = reinterpret_cast<uint4*>(a.tables + static_cast<size_t>(row) * kSettledRowWords);
+  const uint32_t mine = tid < here ? cut.start[tid + 1] - cut.start[tid] : 0u;
+  uint32_t capacity = a.teams ? SettledTeam::kCapacity : SettledBlock::kCapacity;
+  int cells = a.teams ? SettledTeam::kMaxCells : SettledBlock::kMaxCells;
+  const int crowded = __syncthreads_count(mine > capacity);
+  const bool wide = crowded > 0;
+  if (wide) {
+    if (tid == 0) atomicAdd(&a.hdr->settle_large, static_cast<uint32_t>(crowded));
+    capacity = SettledWide::kCapacity;
+    cells = SettledWide::kMaxCells;
+  }
+  cut_groups_of_block(cut, here, kGroupSpanLog, cells >> a.shift, capacity, &a.hdr->aux_counter[wide ? 3 : 2]);
+  auto write_table = [&](uint32_t* tables, uint32_t row, int first, int end) {
+    uint4* table = reinterpret_cast<uint4*>(tables + static_cast<size_t>(row) * kSettledRowWords);
     const uint32_t in_group = arrived[end] - arrived[first];
     table[0] = make_uint4(base[0] + cut.start[first] - arrived[first],
                           cut.start[end] - cut.start[first] - in_group, base[1] + arrived[first], in_group);
     table[1] = make_uint4(base[2] + output[first], output[end] - output[first],
                           static_cast<uint32_t>(b0 + first), static_cast<uint32_t>(b0 + end));
   };
-  if (tid < static_cast<int>(cut.found)) write_table(cut.list_base + tid, cut.group_first[tid], cut.link[cut.group_first[tid]]);
-  if (tid < here && cut.start[tid + 1] - cut.start[tid] > a.capacity)
-    write_table(a.buckets - 1 - atomicAdd(&a.hdr->settle_large, 1u), tid, tid + 1);
+  if (tid < static_cast<int>(cut.found))
+    write_table(wide ? a.wide_tables : a.tables, cut.list_base + tid, cut.group_first[tid], cut.link[cut.group_first[tid]]);
+  if (mine > capacity) write_table(a.tables, a.buckets - 1 - atomicAdd(&a.hdr->aux_counter[4], 1u), tid, tid + 1);
 }
 
 // The movers' records to their buckets, with their keys.
@@ -428,65 +460,74 @@ __device__ __forceinline__ void prefetch_range(const void* from, uint32_t bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p0), "r"(static_cast<uint32_t>(p1 - p0)) : "memory");
 }
 
-// Bound by instructions and the shared-memory pipe (issue slots 55 %, pipe 55 %): 2071 us for 128 M particles, two blocks per multiprocessor.
-// The finish: groups blockIdx.x, blockIdx.x + gridDim.x, ... of the list.  A thread loads all its
-// particles of a group before the first is used; the group behind is asked into L2 meanwhile.
-__global__ void __launch_bounds__(kSettledThreads, FinishSettled::kBlocks)
-settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_constant__ FinishOut out) {
-  // No early release: the count kernel of the general path, set up while these blocks still hold their
-  // multiprocessors, would lie unevenly on them (16.8 M particles given up: 72 -> 88 us).
-  chain_wait();
-  using Shape = FinishSettled;
-  constexpr int kItems = Shape::kItems;
-  const uint32_t groups = a.hdr->aux_counter[2];
-  const int tid = threadIdx.x;
-  // One answer for the block: others may set the word meanwhile.
-  if (__syncthreads_or(tid == 0 && settle_failed(a.hdr))) return;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
-  if (blockIdx.x == 0 && tid == 0) out.cell_start[a.num_cells] = a.n;
-  const uint4* tables = reinterpret_cast<const uint4*>(a.tables);
-  uint32_t g = blockIdx.x;
+template <class Shape>
+struct __align__(16) SettledSmem {
+  static constexpr int kRow = Shape::kCapacity + 4;
+  uint32_t hist[Shape::kHistWords];
+  union {
+    struct {
+      uint32_t tie[Shape::kCapacity + 4];  // the last words are read, but not used, behind the last run
+      uint16_t word_prefix[Shape::kHistWords];
+    };
+    uint32_t stage[kRecordWords][kRow];  // the output, array by array
+  };
+  uint32_t warp_sum[32];
+};
+
+// Groups g, g + step, ... of a list, one after the other; false if a counter wrapped.  The sort is that of
+// sort_placed: byte counters of the low key, whose returned value is the rank on a counter, their scan, and a compare
+// of the records that share one.  But a thread keeps its records in registers from load to store, and puts them in
+// output order in shared memory array by array, so that the output goes out 16 bytes at a time: a record costs eight
+// stores of a word at one address with constant offsets and a quarter of eight loads and stores of 16 bytes, where
+// whole records, pulled out of shared memory by sorted place, cost four accesses of 16 bytes, eight stores of a word and
+// their addresses.  The bodies of the item loops are written so that the compiler predicates single accesses
+// instead of branching around them (258 -> 220 instructions a record).  Bound by instructions and the
+// shared-memory pipe (issue slots 49 %, pipe 66 %).  16.8 M particles, 8 to a cell, 285 -> 199 us, 20 M with 64
+// 344 -> 253, 128 M 2168 -> 1560 (60 bytes a particle: 5.2 TB/s).  Stored to the output straight from the
+// registers, neighbouring lanes to places a few cells wide, 16.8 M took 221 us in groups of 1024, and 64 to a cell
+// 372, in parts of sectors; read by sorted place instead, 250 and 299.
+template <class Shape>
+__device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, const SettledArgs& a, const FinishOut& out,
+                                                      const uint32_t* list, uint32_t g, uint32_t groups, uint32_t step) {
+  constexpr int kThreads = Shape::kThreads, kItems = Shape::kItems, kWarps = kThreads / 32;
+  constexpr int kWordsPerThread = Shape::kWordsPerThread;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < Shape::kHistWords; i += kThreads) s.hist[i] = 0;
+  const uint4* tables = reinterpret_cast<const uint4*>(list);  // two to a group
   uint4 where{}, what{};
   if (g < groups) {
     where = tables[2 * g];
     what = tables[2 * g + 1];
   }
-  for (; g < groups; g += gridDim.x) {
-    const int home_first = static_cast<int>(where.x), home = static_cast<int>(where.y);
-    const int places = home + static_cast<int>(where.w);
-    const uint4* arrived = reinterpret_cast<const uint4*>(a.arrived) + 2 * static_cast<size_t>(where.z);
-    const uint32_t begin = what.x;
-    const int count = static_cast<int>(what.y);
-    const int64_t first_cell = static_cast<int64_t>(what.z) << a.shift;
-    const int cells_here = static_cast<int>(
-        min(static_cast<long long>(what.w - what.z) << a.shift, static_cast<long long>(a.num_cells - first_cell)));
+  for (; g < groups; g += step) {
+    const uint32_t home_first = where.x, home = where.y, places = home + where.w, first_arrived = where.z;
+    const uint32_t begin = what.x, count = what.y;
+    const uint32_t first_cell = what.z << a.shift;
+    const int cells_here = min(static_cast<int>((what.w << a.shift) - first_cell),
+                               static_cast<int>(a.num_cells - first_cell));
     float f[kItems][6];
-    uint32_t key[kItems];
+    uint32_t key[kItems], word[kItems];
+    {
+      const uint32_t mine = home_first + tid;
+      const uint32_t* keys = a.keys + mine;
+      const float *x = a.x + mine, *y = a.y + mine, *z = a.z + mine;
+      const float *vx = a.v + mine, *vy = a.v + a.padded + mine, *vz = a.v + 2 * a.padded + mine;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const int r = tid + k * kSettledThreads;
-      if (r < home) {
-        const int i = home_first + r;
-        key[k] = __ldcs(a.keys + i);
-        f[k][0] = __ldcs(a.x + i);
-        f[k][1] = __ldcs(a.y + i);
-        f[k][2] = __ldcs(a.z + i);
-        f[k][3] = __ldcs(a.v + i);
-        f[k][4] = __ldcs(a.v + a.padded + i);
-        f[k][5] = __ldcs(a.v + 2 * a.padded + i);
-      } else if (r < places) {
-        const uint4 lo = __ldcg(arrived + 2 * (r - home)), hi = __ldcg(arrived + 2 * (r - home) + 1);
-        *reinterpret_cast<uint2*>(&s.raw[r * kRecordWords]) = make_uint2(lo.x, lo.y);
-        f[k][0] = __uint_as_float(lo.z);
-        f[k][1] = __uint_as_float(lo.w);
-        f[k][2] = __uint_as_float(hi.x);
-        f[k][3] = __uint_as_float(hi.y);
-        f[k][4] = __uint_as_float(hi.z);
-        f[k][5] = __uint_as_float(hi.w);
+      for (int k = 0; k < kItems; ++k) {
+        key[k] = kGone;
+        word[k] = mine + k * kThreads;
+        if (static_cast<uint32_t>(tid + k * kThreads) < home) {
+          key[k] = __ldcs(keys + k * kThreads);
+          f[k][0] = __ldcs(x + k * kThreads);
+          f[k][1] = __ldcs(y + k * kThreads);
+          f[k][2] = __ldcs(z + k * kThreads);
+          f[k][3] = __ldcs(vx + k * kThreads);
+          f[k][4] = __ldcs(vy + k * kThreads);
+          f[k][5] = __ldcs(vz + k * kThreads);
+        }
       }
     }
-    const uint32_t behind = g + gridDim.x;
+    const uint32_t behind = g + step;
     if (behind < groups) {
       where = tables[2 * behind];
       what = tables[2 * behind + 1];
@@ -496,27 +537,167 @@ settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_consta
       else if (tid == 7) prefetch_range(a.arrived + static_cast<size_t>(where.z) * kRecordWords, where.w * 32);
     }
     const int drop = drop_for<Shape>(cells_here);
-    const int hist_words = counter_words(cells_here, drop);
-    for (int i = tid; i < hist_words; i += kSettledThreads) s.hist[i] = 0;
-    __syncthreads();
-    const bool sorted = sort_placed<Shape>(s, out, places, count, begin, first_cell, cells_here, drop,
-                                           [&](int k, int r, uint2* key_index) {
-      uint32_t* to = &s.raw[r * kRecordWords];
-      if (r < home) {
-        if (key[k] == kGone) return false;
-        push_particle(a.push, f[k]);
-        *key_index = make_uint2(key[k], static_cast<uint32_t>(home_first + r));
-      } else {
-        *key_index = *reinterpret_cast<const uint2*>(to);
+    const int dropped = max(drop, 0);
+    const uint32_t drop_mask = (1u << dropped) - 1;
+    const uint32_t key_base = first_cell << kShuffleBits;
+    // The move; then the arrivals, which have moved already (few warps have any).
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      if (__any_sync(0xffffffffu, static_cast<uint32_t>(tid + k * kThreads) < home)) push_particle(a.push, f[k]);
+      const uint32_t r = tid + k * kThreads;
+      if (r >= home && r < places) {
+        const uint4* arrived = reinterpret_cast<const uint4*>(a.arrived) + 2 * static_cast<size_t>(first_arrived + (r - home));
+        const uint4 lo = __ldcg(arrived), hi = __ldcg(arrived + 1);
+        key[k] = lo.x;
+        word[k] = lo.y;
+        f[k][0] = __uint_as_float(lo.z);
+        f[k][1] = __uint_as_float(lo.w);
+        f[k][2] = __uint_as_float(hi.x);
+        f[k][3] = __uint_as_float(hi.y);
+        f[k][4] = __uint_as_float(hi.z);
+        f[k][5] = __uint_as_float(hi.w);
       }
-      *reinterpret_cast<uint4*>(to) =
-          make_uint4(key_index->x, key_index->y, __float_as_uint(f[k][0]), __float_as_uint(f[k][1]));
-      *reinterpret_cast<uint4*>(to + 4) = make_uint4(__float_as_uint(f[k][2]), __float_as_uint(f[k][3]),
-                                                     __float_as_uint(f[k][4]), __float_as_uint(f[k][5]));
-      return true;
-    });
-    if (!sorted && tid == 0) fail_settle(a.hdr);
+    }
+    __syncthreads();  // the counters are zero
+
+    // Written without branches around more than one access, so that the compiler predicates them.
+    uint32_t run[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const uint32_t low = (key[k] - key_base) >> dropped, sh = (low << 3) & 31u;
+      uint32_t old = 0;
+      if (key[k] != kGone) old = atomicAdd(&s.hist[low >> 2], 1u << sh);
+      run[k] = (old >> sh) & 0xffu;
+      word[k] |= (key[k] & drop_mask) << (32 - Shape::kMaxDrop);
+    }
+    __syncthreads();
+
+    // Exclusive scan of the counters.
+    uint32_t local[kWordsPerThread];
+    uint32_t sum = 0;
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; j += 4) {
+      const uint4 w = *reinterpret_cast<const uint4*>(&s.hist[tid * kWordsPerThread + j]);
+      local[j] = sum;
+      sum = __dp4a(w.x, 0x01010101u, sum);
+      local[j + 1] = sum;
+      sum = __dp4a(w.y, 0x01010101u, sum);
+      local[j + 2] = sum;
+      sum = __dp4a(w.z, 0x01010101u, sum);
+      local[j + 3] = sum;
+      sum = __dp4a(w.w, 0x01010101u, sum);
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) s.warp_sum[warp] = incl;
+    __syncthreads();
+    // Every warp adds up the warps' sums for itself.
+    const uint32_t warps = lane < kWarps ? s.warp_sum[lane] : 0u;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, warps);
+    const uint32_t thread_base = __reduce_add_sync(0xffffffffu, lane < warp ? warps : 0u) + incl - sum;
+    const uint32_t both = thread_base * 0x10001u;
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; j += 4) {
+      uint2 prefix;  // no carry between the halves: all below 2^16
+      prefix.x = both + (local[j] + (local[j + 1] << 16));
+      prefix.y = both + (local[j + 2] + (local[j + 3] << 16));
+      *reinterpret_cast<uint2*>(&s.word_prefix[tid * kWordsPerThread + j]) = prefix;
+    }
+    if (total != count) return false;  // a counter wrapped (the same answer everywhere)
+    __syncthreads();
+
+    const int cell_words = cell_words_for(drop);
+    const int hist_words = counter_words(cells_here, drop);
+    for (int c = tid; c < cells_here; c += kThreads) {
+      const uint32_t lo = s.word_prefix[c * cell_words];
+      const uint32_t hi = (c + 1) * cell_words < hist_words ? s.word_prefix[(c + 1) * cell_words] : count;
+      out.cell_start[first_cell + c] = static_cast<int32_t>(begin + lo);
+      out.cell_counts[first_cell + c] = static_cast<int32_t>(hi - lo);
+    }
+    uint32_t longest = 0;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const uint32_t low = (key[k] != kGone ? key[k] - key_base : 0u) >> dropped, sh = (low << 3) & 31u;
+      const uint32_t counters = s.hist[low >> 2];
+      const uint32_t start = __dp4a(counters & ((1u << sh) - 1u), 0x01010101u, static_cast<uint32_t>(s.word_prefix[low >> 2]));
+      const uint32_t length = (counters >> sh) & 0xffu;
+      if (key[k] != kGone) s.tie[start + run[k]] = word[k];
+      longest = max(longest, length);
+      run[k] = start | length << 16;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kWordsPerThread; j += 4)
+      *reinterpret_cast<uint4*>(&s.hist[tid * kWordsPerThread + j]) = make_uint4(0u, 0u, 0u, 0u);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const uint32_t length = run[k] >> 16, start = run[k] & 0xffffu;
+      const uint32_t* others = &s.tie[start];
+      uint32_t slot = start;
+      const uint32_t o0 = others[0], o1 = others[1], o2 = others[2];
+      slot += o0 < word[k];
+      slot += 1 < length && o1 < word[k];
+      slot += 2 < length && o2 < word[k];
+      if (longest > 3)
+        for (uint32_t j = 3; j < longest; ++j)
+          if (j < length) slot += others[j] < word[k];
+      run[k] = slot;
+    }
+    __syncthreads();
+    // The places of the stage are those of the output, from the 16 bytes on in which it begins.
+    const uint32_t lead = begin & 3u;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      uint32_t* to = &s.stage[0][lead + run[k]];
+      if (key[k] != kGone) {
+        to[0] = key[k];
+        to[SettledSmem<Shape>::kRow] = word[k] & ((1u << (32 - Shape::kMaxDrop)) - 1);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) to[(2 + c) * SettledSmem<Shape>::kRow] = __float_as_uint(f[k][c]);
+      }
+    }
+    __syncthreads();
+    const uint32_t base = begin - lead, last = lead + count;
+    for (uint32_t p = tid * 4; p < last; p += kThreads * 4) {
+      uint32_t* const rows[kRecordWords] = {
+          out.keys, reinterpret_cast<uint32_t*>(out.index), reinterpret_cast<uint32_t*>(out.xs),
+          reinterpret_cast<uint32_t*>(out.ys), reinterpret_cast<uint32_t*>(out.zs), reinterpret_cast<uint32_t*>(out.vs),
+          reinterpret_cast<uint32_t*>(out.vs + out.padded_sorted), reinterpret_cast<uint32_t*>(out.vs + 2 * out.padded_sorted)};
+      if (a.vec_out && p >= lead && p + 4 <= last) {
+#pragma unroll
+        for (int c = 0; c < kRecordWords; ++c)
+          __stcs(reinterpret_cast<uint4*>(rows[c] + (base + p)), *reinterpret_cast<const uint4*>(&s.stage[c][p]));
+      } else {
+#pragma unroll 1
+        for (uint32_t e = max(p, lead); e < min(p + 4, last); ++e)
+#pragma unroll
+          for (int c = 0; c < kRecordWords; ++c) __stcs(rows[c] + (base + e), s.stage[c][e]);
+      }
+    }
   }
+  return true;
+}
+
+template <class Shape>
+__global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
+settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_constant__ FinishOut out) {
+  // No early release: the count kernel of the general path, set up while these blocks still hold their
+  // multiprocessors, would lie unevenly on them (16.8 M particles given up: 72 -> 88 us).
+  chain_wait();
+  const uint32_t groups = a.hdr->aux_counter[2];
+  // One answer for the block: others may set the word meanwhile.
+  if (__syncthreads_or(threadIdx.x == 0 && settle_failed(a.hdr))) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) out.cell_start[a.num_cells] = a.n;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  if (!finish_settled_groups<Shape>(*reinterpret_cast<SettledSmem<Shape>*>(smem_raw), a, out, a.tables, blockIdx.x,
+                                    groups, gridDim.x) &&
+      threadIdx.x == 0)
+    fail_settle(a.hdr);
 }
 
 // The records of a bucket that no block holds: its home run in the input without those that left, and its
@@ -564,7 +745,7 @@ struct SettledRecords {
 template <class Shape>
 __device__ bool finish_settled_large(FinishSmem<Shape>& s, const SettledArgs& a, const FinishOut& out, uint32_t first,
                                      uint32_t step) {
-  const uint32_t large = a.hdr->settle_large;
+  const uint32_t large = a.hdr->aux_counter[4];
   for (uint32_t r = first; r < large; r += step) {
     const uint4* table = reinterpret_cast<const uint4*>(a.tables) + 2 * static_cast<size_t>(a.buckets - 1 - r);
     const uint4 where = table[0], what = table[1];

@@ -1834,8 +1834,8 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
     hdr->use_standard = 1;
 }
 
-// Behind the finish kernel of an ordinary call: the oversized buckets (also those of the sort of a settled
-// state) and the groups whose counters
+// Behind the finish kernel of an ordinary call: the oversized buckets (of the sort of a settled state the wide
+// groups and what those do not hold) and the groups whose counters
 // wrapped (calls without payload, whose sparse groups have 16 counters per cell), then, when the call was
 // handed over, the whole digit-pass sort.  Usually there is nothing to do and every block returns
 // after a look at the header.  What bounds it is then the launch itself: as the separate kernels
@@ -1870,8 +1870,13 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
     FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
     if constexpr (kBehind) {
       if (is_settled) {
-        if (!standard && !finish_settled_large<Shape>(s, settled, out, item, items) && threadIdx.x == 0)
-          atomicExch(&hdr->use_standard, 1);
+        static_assert(Shape::kThreads == SettledWide::kThreads, "one block size");
+        auto& wide = *reinterpret_cast<SettledSmem<SettledWide>*>(smem_raw);
+        bool good = standard || finish_settled_groups<SettledWide>(wide, settled, out, settled.wide_tables, item,
+                                                                   hdr->aux_counter[3], items);
+        __syncthreads();
+        good = good && (standard || finish_settled_large<Shape>(s, settled, out, item, items));
+        if (!good && threadIdx.x == 0) atomicExch(&hdr->use_standard, 1);
         return true;
       }
     }
@@ -2558,6 +2563,8 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
                         uint32_t group_capacity, const DigitPassArgs& digits, bool chained,
                         const Settled& settled) {
   constexpr int kSmem = static_cast<int>(std::max(sizeof(FinishSmem<Shape>), sizeof(PassSmem<Shape::kThreads>)));
+  static_assert(std::is_same_v<Settled, NotSettled> ||
+                    sizeof(SettledSmem<SettledWide>) <= kSmem, "shared memory");
   auto kernel = bucket_tail_kernel<Shape, Settled>;
   const cudaError_t e = allow_shared(kernel, kSmem);
   if (e != cudaSuccess) return e;
@@ -2685,7 +2692,9 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
       a.num_cells > (int64_t{1} << 25) - 1 || outputs_over_inputs(a))
     return false;
   SettledArgs s{};
-  s.shift = shift_for(a.n, a.num_cells, kSettledTarget, log2_floor(FinishSettled::kMaxCells), 1);
+  s.teams = a.n * SettledTeam::kMaxCells >= kSettledTeamLeast * a.num_cells && a.n <= kSettledTeamMostMean * a.num_cells;
+  s.shift = shift_for(a.n, a.num_cells, s.teams ? kSettledTeamTarget : kSettledBlockTarget,
+                      log2_floor(s.teams ? SettledTeam::kMaxCells : SettledBlock::kMaxCells), 1);
   const int64_t buckets = (a.num_cells + (int64_t{1} << s.shift) - 1) >> s.shift;
   if (a.n > kSettledMostMean * buckets || buckets > a.n) return false;
   s.x = a.x; s.y = a.y; s.z = a.z; s.v = a.velocity;
@@ -2699,13 +2708,14 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
   const int64_t most = static_cast<int64_t>(sm_count()) * 2;
   s.per_block = static_cast<int>(((a.n + most - 1) / most + kSettledRound - 1) / kSettledRound) * kSettledRound;
   s.scan_blocks = static_cast<int>((a.n + s.per_block - 1) / s.per_block);
-  s.capacity = static_cast<uint32_t>(group_capacity_for(a.n, FinishSettled::kCapacity, FinishSettled::kBlocks));
   const int64_t in_last = a.n - static_cast<int64_t>(s.scan_blocks - 1) * s.per_block;
   const int64_t apart = s.per_block / kProbeSamples;
   const int64_t samples = static_cast<int64_t>(s.scan_blocks - 1) * kProbeSamples + (in_last + apart - 1) / apart;
   s.most_sampled = static_cast<uint32_t>(samples * (p.tiled ? kMoversTiled : p.small_blocks ? kMoversSmall : kMoversLarge) / 1000);
   s.most_movers = static_cast<uint32_t>(a.n / kMoverShare);
   s.hdr = hdr;
+  s.vec_out = aligned16(a.keys_out) && aligned16(a.index_out) && aligned16(a.xs) && aligned16(a.ys) && aligned16(a.zs) &&
+              aligned16(a.vs) && a.padded_sorted % 4 == 0;
   size_t used = 0;
   auto take = [&](int64_t words) {
     auto* at = reinterpret_cast<uint32_t*>(base + used);
@@ -2720,8 +2730,9 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
   s.keys = take(a.n);
   s.list_count = take(s.scan_blocks);
   s.cursor = take(buckets);
-  s.sums = take((buckets + kSettledPart - 1) / kSettledPart * 4);
+  s.sums = take((buckets + kSettledPart - 1) / kSettledPart * kSettledSums);
   s.tables = take(buckets * kSettledRowWords);
+  s.wide_tables = take(buckets * kSettledRowWords);
   s.list = take(static_cast<int64_t>(s.scan_blocks) * (s.per_block / kListShare) * kRecordWords);
   s.arrived = take(static_cast<int64_t>(s.most_movers) * kRecordWords);
   *out = s;
@@ -2730,14 +2741,14 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
 
 // Enqueues the sort of a settled state; the general path's kernels follow it.
 cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_bytes, const FinishOut& out) {
-  constexpr int kSmem = static_cast<int>(sizeof(FinishSmem<FinishSettled>));
   constexpr int kScanSmem = static_cast<int>(sizeof(MoverQueue)) * (kSettledThreads / 32);
   const bool vec = aligned16(a.x) && aligned16(a.y) && aligned16(a.z) && aligned16(a.velocity) && a.padded % 4 == 0;
   const bool whole = a.grid.ix_offset == 0 && a.grid.nx_local == a.grid.nx;
   auto scan = vec ? (whole ? settled_scan_kernel<true, true> : settled_scan_kernel<true, false>)
                   : (whole ? settled_scan_kernel<false, true> : settled_scan_kernel<false, false>);
-  auto finish = settled_finish_kernel;
-  cudaError_t e = allow_shared(finish, kSmem);
+  auto finish = s.teams ? settled_finish_kernel<SettledTeam> : settled_finish_kernel<SettledBlock>;
+  const int finish_smem = static_cast<int>(s.teams ? sizeof(SettledSmem<SettledTeam>) : sizeof(SettledSmem<SettledBlock>));
+  cudaError_t e = allow_shared(finish, finish_smem);
   if (e == cudaSuccess) e = allow_shared(scan, kScanSmem);
   if (e != cudaSuccess) return e;
   stage_begin(kStageBucketCount, a.stream);
@@ -2757,7 +2768,8 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   stage_end(kStageBucketScatter, a.stream);
   stage_begin(kStageBucketFinish, a.stream);
   if (e == cudaSuccess)
-    e = launch_chained(finish, sm_count() * FinishSettled::kBlocks, kSettledThreads, kSmem, a.stream, s, out);
+    e = launch_chained(finish, sm_count() * (s.teams ? SettledTeam::kBlocks : SettledBlock::kBlocks),
+                       s.teams ? SettledTeam::kThreads : SettledBlock::kThreads, finish_smem, a.stream, s, out);
   count_launches(6);
   return e;
 }

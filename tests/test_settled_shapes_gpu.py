@@ -1,0 +1,56 @@
+"""What sorts a group of a settled state: teams, blocks, wide groups in the tail kernel, and its large buckets.
+At the edges of their capacities, against the CPU oracle, bit for bit."""
+
+import pytest
+import torch
+
+import project_aether_b200 as pa
+from project_aether_b200 import particle_sort
+from test_settled_sort_gpu import LARGE, LEAST, _crowd, _dt, _run, _sorted_state, _words
+
+pytestmark = pytest.mark.gpu
+
+TEAM_GROUPS, WIDE_GROUPS, LARGE_BUCKETS = 54, 55, 56  # words of the workspace header
+TEAM_TARGET = 104                                     # records of a team's bucket, on average at most
+
+
+@pytest.mark.parametrize('records,wide,large', [(511, 0, 0), (512, 0, 0), (513, 1, 0), (4095, 1, 0), (4096, 1, 0),
+                                                (4097, 1, 1)])
+def test_a_bucket_at_a_capacity(cuda, records, wide, large):
+    """One bucket has exactly `records`, most of them in one cell; nothing moves."""
+    n, cells = LEAST + 100, (64, 64, 64)
+    grid, pos, vel = _sorted_state(n, cells, cuda, 31)
+    vel.zero_()
+    shift = max(s for s in range(7) if n <= TEAM_TARGET * (64 ** 3 >> s))
+    here = n // 2
+    bucket = sum((pos[k][here].item() * cells[k] / grid.hi[k]) // 1 * 64 ** k for k in range(3)) // 2 ** shift
+    own = [(p * (c / h)).floor() for p, c, h in zip(pos, cells, grid.hi)]
+    in_bucket = ((own[0] + 64 * own[1] + 4096 * own[2]) // 2 ** shift == bucket).nonzero().flatten()
+    first, last = in_bucket[0].item(), in_bucket[-1].item()
+    assert last - first + 1 == in_bucket.numel() < records
+    _crowd(pos, vel, first, records)  # so many from the bucket's first on
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    words = _words(cuda)
+    assert words[LARGE] == wide and words[LARGE_BUCKETS] == large and (words[WIDE_GROUPS] > 0) == wide
+    assert words[TEAM_GROUPS] > 0
+
+
+# Sparse grids and full cells (blocks), either side of the lines between teams and blocks.
+@pytest.mark.parametrize('n,cells', [(LEAST + 7, (96, 100, 90)), (LEAST + 1, (66, 66, 66)), (LEAST + 1, (64, 66, 66)),
+                                     (2_000_003, (17, 17, 18)), (2_000_003, (17, 17, 17)), (2_100_001, (13, 13, 13))])
+def test_sparse_and_full_cells(cuda, n, cells):
+    grid, pos, vel = _sorted_state(n, cells, cuda, 32)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+
+
+@pytest.mark.parametrize('off', [(1, 0), (0, 2), (3, 3)])
+@pytest.mark.parametrize('squeeze', [None, (0.3, 0.01)])
+def test_outputs_off_16_byte_boundaries(cuda, off, squeeze):
+    """`off`: elements by which positions, and keys and indices, start behind a boundary."""
+    n = LEAST + 3
+    grid, pos, vel = _sorted_state(n, (64, 64, 64), cuda, 33, squeeze=squeeze)
+    plain = pa.sort_and_gather_particles(*pos, vel, grid, 1)
+    move = lambda t, k: torch.cat([t.new_zeros(k), t])[k:]
+    order = plain.order._replace(keys=move(plain.order.keys, off[1]), particle_index=move(plain.order.particle_index, off[1]))
+    out = particle_sort.SortedParticles(order, tuple(move(t, off[0]) for t in plain.positions), plain.velocity)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled', out=out)
