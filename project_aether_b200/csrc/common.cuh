@@ -65,7 +65,7 @@ struct alignas(16) Header {
   uint32_t settle_failed;     // the sort of a settled state gave the call to the general path
   uint32_t settle_large;      // buckets of the sort of a settled state that a block of its finish does not hold
   uint32_t settle_sampled;    // movers among the particles that its probe looked at
-  uint32_t kept_pad[1];
+  uint32_t shared_rounds;     // rounds in which the count kernel has seen neighbours in one bucket
   uint32_t tile_claimed[kMaxTiles / 32], tile_loose[kMaxTiles / 32];  // one bit per tile
   uint32_t tile_counter[kMaxPasses];  // ticket dispenser of each digit pass
   uint32_t aux_counter[8];

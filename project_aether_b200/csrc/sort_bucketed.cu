@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kCountThreads ? 3 : 1)
 bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
                     PushSpec push, int64_t n, AetherGrid g, int shift, int buckets, int chunk_log,
-                    int64_t per_block, uint32_t* __restrict__ bucket_count, const Header* hdr,
+                    int64_t per_block, uint32_t* __restrict__ bucket_count, Header* hdr,
                     bool behind) {
   chain_begin();
   if (settled_before(hdr, behind)) return;
@@ -164,6 +164,7 @@ bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
   // Particle numbers fit 30 bits: index arithmetic in 32.
   int first = static_cast<int>(blockIdx.x * per_block);
   const int block_last = static_cast<int>(min(static_cast<long long>(n), static_cast<long long>(first) + per_block));
+  uint32_t shared_rounds = 0;
   while (first < block_last) {
     const int chunk = first >> chunk_log;
     const int last = static_cast<int>(min(static_cast<long long>(block_last),
@@ -220,6 +221,7 @@ bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
         if (sharing) sharing = count_add<TABLE>(target, row, bin, valid);
         else if (valid) table_add<TABLE>(target, row, bin, 1u);
       }
+      shared_rounds += sharing;
       if (TABLE == kTableShared16 && (r + 1) % kRoundsPerBarrier == 0) __syncthreads();
     }
     if (TABLE != kTableGlobal) {
@@ -240,6 +242,8 @@ bucket_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
     }
     first = last;
   }
+  // What the block's first warp has seen tells the scatter whether the input is in some order.
+  if (threadIdx.x == 0 && shared_rounds) atomicAdd(&hdr->shared_rounds, shared_rounds);
 }
 
 // ------------------------------------------------------------------------
@@ -361,6 +365,7 @@ __device__ __forceinline__ uint32_t reserve_slot(uint32_t* cursor, uint32_t b, b
 // loads with twice the resident threads to keep more slot reservations in flight).
 template <int ITEMS>
 __device__ __forceinline__ void load_items(const float* p, float* out) {
+  static_assert(ITEMS == 4 || ITEMS == 2, "one access");
   if (ITEMS == 4) {
     const float4 a = ldcs4(p);
     out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
@@ -370,6 +375,10 @@ __device__ __forceinline__ void load_items(const float* p, float* out) {
   }
 }
 
+// Input in some order (the count kernel's first warps have seen neighbours in one bucket in `some_order` rounds), input
+// in none, or any.
+enum ScatterOnly { kScatterAny, kScatterOrdered, kScatterRandom };
+
 template <bool VEC, int ITEMS, int RECORD_WORDS>
 __global__ void __launch_bounds__(kScatterThreads, 8 / ITEMS)
 bucket_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
@@ -377,9 +386,10 @@ bucket_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                       PushSpec push, int64_t n, AetherGrid g, uint32_t k0, uint32_t k1, int shift,
                       int buckets, int chunk_log, uint32_t* __restrict__ cursor,
                       uint32_t* __restrict__ records, const Header* __restrict__ hdr,
-                      bool behind) {
+                      ScatterOnly only, uint32_t some_order, bool behind) {
   chain_wait();
   if (settled_before(hdr, behind) || hdr->use_standard) return;
+  if (only != kScatterAny && (hdr->shared_rounds >= some_order) != (only == kScatterOrdered)) return;
   const int64_t groups = (n + ITEMS - 1) / ITEMS;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kScatterThreads;
   const int64_t rounds = (groups + stride - 1) / stride;
@@ -2288,21 +2298,38 @@ inline int index_bits_of(int64_t n) {
 }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// Above this many particles input in random order is scattered window by window, see scatter_span (20 M 649 -> 684 us per
+// call, 33 M 1162 -> 1143, 50 M 1698 -> 1687, 64 M 2171 -> 2168, 75 M 2707 -> 2519, 100 M 3359 -> 3200).
+constexpr int64_t kScatterWindowsFrom = int64_t{1} << 26;
+
 // The chunk-major record layout: while a chunk is scattered its stores stay inside the
 // chunk's region, which L2 serves faster than the whole record array; but every bucket gets
 // one run per chunk, and short runs cost the scatter (partial lines) and the finish kernel
-// (many small copies) more than the window saves.  Measured optimum on random input: runs of
-// about 256 records, i.e. 2^22 particles per chunk with 16 K buckets (64 M particles: 2.50 ms
-// against 2.63 at 2^23), 2^23 with 32 K buckets (128 M: 5.15 against 5.66 at 2^22 and 5.50 at
-// 2^24), 2^24 with 64 K buckets (256 M: 11.8 against 14.7 at 2^22, 12.8 at 2^23, 12.0 at
-// 2^25).  Smaller inputs take smaller chunks (fewer particles contend for a slot counter):
-// best 2^20 at 4 M particles, 2^21 at 16 M.
+// (many small copies) more than the window saves.  Measured optimum on random input (us per call): 2^22 particles per chunk
+// with 16 K buckets (64 M 2164 against 2271 with 2^23), 2^23 with 32 K or 64 K (100 M 3185 against 3298 with 2^22 and
+// 3457 with 2^24, 128 M 4306 / 4486 / 4598, 256 M 9006 against 9422 with 2^24), 2^24 beyond.  Smaller inputs take
+// smaller chunks (fewer particles contend for a slot counter): best 2^20 at 4 M particles, 2^21 at 16 M.
 inline int chunk_log_for(int64_t buckets, int64_t n) {
   if (n <= (int64_t{1} << 22)) return kChunkLog - 2;
   if (n <= (int64_t{1} << 24)) return kChunkLog - 1;
-  int bucket_log = 0;
-  while ((int64_t{1} << bucket_log) < buckets) ++bucket_log;
-  return std::min(kChunkLog + 2, std::max(kChunkLog, bucket_log + 8));
+  return buckets <= (1 << 14) ? kChunkLog : buckets <= (1 << 16) ? kChunkLog + 1 : kChunkLog + 2;
+}
+
+// Particles from one round of a scatter block to its next (a power of two), where the input is in random order.  n / span
+// windows of the record array are then written at a time, by blocks that started at different times: the slot counters
+// they contend for are as many times as many.  With too many windows the lines that every bucket has open in each no
+// longer stay in L2 until they are full: 128 bytes a bucket and window, best at 32 MB in all.  Every block has few
+// rounds, and the next takes its place when it ends, which evens out that multiprocessors differ in speed (blocks that
+// stay, and walk through the input in such an order: 128 M 4949 us per call, 256 M 11198; warps that draw their
+// particles by ticket 4405, 9069).  us per call at log2 span: 100 M 22 3302, 23 3185, 24 3238; 128 M 22 4557, 24 4306, 25 4460; 256 M 24.6 10524, 25 9907, 26 9006,
+// 27 9055.  (Before, two particles a thread and a span of 2.4 M whatever the size: 100 M 3359, 128 M 4695, 256 M 10392.)  Input
+// in some order is better off that way: scattered window by window, 134 M moved by two cells take 4067 us against 3777.  Without payload a line takes sixteen records, and few windows are best: 100 M 24 2704, 25 2566,
+// 26 2540, 27 2589; 150 M 25 4352, 26 4162, 27 4040; 200 M 25 6078, 26 5528, 27 5275 (before 2860, 4516, 6400).
+int64_t scatter_span(int64_t n, int64_t buckets, bool keys_only) {
+  const int64_t want = keys_only ? n / 2 : (n >> 9) * buckets / (1 << 9);
+  int64_t span = int64_t{1} << 23;
+  while (4 * span < want * 3) span *= 2;
+  return span;
 }
 
 constexpr int kKeyChunkLog = 24;  // particles per chunk of a call without payload
@@ -2334,9 +2361,9 @@ BucketLayout bucket_layout_of(int64_t n, int64_t buckets, int chunk_log, int chu
 
 BucketLayout bucket_layout(int64_t n, const BucketPlan& p) {
   const int64_t buckets = p.buckets;
-  // Tiles split in shared memory write whole runs: no window has to be kept small for them.
-  const int chunk_log = p.one_launch || p.tiled || (p.keys_only && buckets <= kSplitMaxBuckets)
-                            ? kKeyChunkLog : chunk_log_for(buckets, n);
+  // Tiles split in shared memory write whole runs: no window has to be kept small for them.  Nor for 8-byte records
+  // (scattered, 100 M particles 2540 us per call against 2682 with 2^23 particles to a chunk, 2622 with 2^25).
+  const int chunk_log = p.one_launch || p.tiled || p.keys_only ? kKeyChunkLog : chunk_log_for(buckets, n);
   const int chunks = static_cast<int>(
       std::max<int64_t>(1, (n + (int64_t{1} << chunk_log) - 1) >> chunk_log));
   return bucket_layout_of(n, buckets, chunk_log, chunks,
@@ -2828,6 +2855,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   auto begin_stage = [&](Stage stage) { if (!behind) stage_begin(stage, a.stream); };
   auto end_stage = [&](Stage stage) { if (!behind) stage_end(stage, a.stream); };
 
+  uint32_t some_order;  // rounds of the count kernel's first warps that have seen neighbours in one bucket
   begin_stage(kStageBucketCount);
   {
     const size_t bytes32 = static_cast<size_t>(buckets) * sizeof(uint32_t);
@@ -2844,6 +2872,7 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     const int64_t most = static_cast<int64_t>(sm_count()) * blocks_per_sm;
     const int64_t per_block = std::max<int64_t>(kCountRounds, ((a.n + most - 1) / most + round - 1) / round) * round;
     const int grid = static_cast<int>((a.n + per_block - 1) / per_block);
+    some_order = static_cast<uint32_t>(std::max<int64_t>(1, a.n / round / 2));
 #define AETHER_COUNT_LAUNCH(TABLE, THREADS)                                                      \
   do {                                                                                            \
     auto kernel = vec ? bucket_count_kernel<TABLE, true, THREADS>                                 \
@@ -2910,18 +2939,26 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
                                      chained);
     if (e != cudaSuccess) return e;
   } else {
-    constexpr int kItems = 2;
-    const int64_t groups = (a.n + kItems - 1) / kItems;
-    const int grid = static_cast<int>(std::max<int64_t>(
-        1, std::min<int64_t>((groups + kScatterThreads - 1) / kScatterThreads,
-                             sm_count() * (8 / kItems) * 4)));
-    auto kernel = p.keys_only ? (vec ? bucket_scatter_kernel<true, kItems, kKeyRecordWords>
-                                     : bucket_scatter_kernel<false, kItems, kKeyRecordWords>)
-                              : (vec ? bucket_scatter_kernel<true, kItems, kRecordWords>
-                                     : bucket_scatter_kernel<false, kItems, kRecordWords>);
-    e = launch_chained_if(chained, kernel, grid, kScatterThreads, 0, a.stream, a.x, a.y, a.z,
-                          a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, p.shift, buckets, l.chunk_log,
-                          cursor, records, hdr, behind);
+    auto launch = [&](auto items, int64_t blocks, ScatterOnly only) {
+      constexpr int kItems = decltype(items)::value;
+      constexpr int kRound = kScatterThreads * kItems;
+      auto kernel = p.keys_only ? (vec ? bucket_scatter_kernel<true, kItems, kKeyRecordWords>
+                                       : bucket_scatter_kernel<false, kItems, kKeyRecordWords>)
+                                : (vec ? bucket_scatter_kernel<true, kItems, kRecordWords>
+                                       : bucket_scatter_kernel<false, kItems, kRecordWords>);
+      const int grid = static_cast<int>(std::max<int64_t>(1, std::min((a.n + kRound - 1) / kRound, blocks)));
+      return launch_chained_if(chained, kernel, grid, kScatterThreads, 0, a.stream, a.x, a.y, a.z,
+                               a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, p.shift, buckets, l.chunk_log,
+                               cursor, records, hdr, only, some_order, behind);
+    };
+    using Two = std::integral_constant<int, 2>;
+    using Four = std::integral_constant<int, 4>;
+    const bool windows = !behind && a.n > kScatterWindowsFrom;
+    e = launch(Two(), sm_count() * 16, windows ? kScatterOrdered : kScatterAny);
+    if (e == cudaSuccess && windows) {
+      e = launch(Four(), scatter_span(a.n, buckets, p.keys_only) / (kScatterThreads * 4), kScatterRandom);
+      count_launches(1);
+    }
     if (e != cudaSuccess) return e;
   }
   end_stage(kStageBucketScatter);
