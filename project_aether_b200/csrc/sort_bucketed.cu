@@ -468,15 +468,20 @@ __device__ __forceinline__ uint32_t rank_in_tile(uint32_t* table, uint32_t b, bo
 // consecutive threads on consecutive counters: 17 us, the rate of scattered 32-byte stores
 // (62 G/s).  It pays while a tile has about as many particles as there are buckets.  Staging the
 // tile in shared memory, so that a bucket's records leave side by side, took 23 us.
-template <bool VEC, int ITEMS>
-__global__ void __launch_bounds__(kScatterThreads, ITEMS <= 4 ? 2 : 1)
+// us per call as blocks of 512 threads, two per multiprocessor, that stay and take tiles in turn / one tile each, the next
+// block placed as one ends / 1024 threads, one tile each: 650,000 particles 47.0 / 45.1 / 47.1, 1 M 53.7 / 51.3 / 51.4,
+// 2 M 95.2 / 90.9 / 90.5, 4 M 158.5 / 157.1 / 153.5, 6 M 216 / 216 / 210; 512 threads with eight
+// particles each, one block per multiprocessor (as it was from 1.2 M on) 2 M 97, 4 M 167, 6 M 231.  Behind a sort of a
+// settled state, where the kernel usually returns at once, blocks stay.
+template <bool VEC, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     const float* __restrict__ z, const float* __restrict__ v, int64_t padded,
                     PushSpec push, int64_t n, AetherGrid g, uint32_t k0, uint32_t k1, int shift,
                     int buckets, int chunk_log, uint32_t* __restrict__ cursor,
                     uint32_t* __restrict__ records, const Header* __restrict__ hdr,
                     bool behind) {
-  constexpr int kTile = kScatterThreads * ITEMS;
+  constexpr int ITEMS = 4, kTile = THREADS * ITEMS;
   chain_wait();
   if (settled_before(hdr, behind) || hdr->use_standard) return;
   extern __shared__ uint32_t slot_of[];  // a tile's counts, then its first slots
@@ -485,14 +490,14 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t first = tile * kTile;
     uint32_t* row = cursor + static_cast<size_t>(first >> chunk_log) * buckets;
-    for (int b = tid; b < buckets; b += kScatterThreads) slot_of[b] = 0;
+    for (int b = tid; b < buckets; b += THREADS) slot_of[b] = 0;
     __syncthreads();
     float f[6][ITEMS];
     uint32_t key[ITEMS], rank[ITEMS];
     bool sharing = true;
 #pragma unroll
     for (int q = 0; q < ITEMS; q += 4) {
-      const int64_t i0 = first + (q / 4 * kScatterThreads + tid) * 4;
+      const int64_t i0 = first + (q / 4 * THREADS + tid) * 4;
       if (VEC && i0 + 4 <= n) {
         load_items<4>(x + i0, f[0] + q);
         load_items<4>(y + i0, f[1] + q);
@@ -521,7 +526,7 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
     }
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
-      const int64_t i = first + (k / 4 * kScatterThreads + tid) * 4 + k % 4;
+      const int64_t i = first + (k / 4 * THREADS + tid) * 4 + k % 4;
       if (push.enabled) {  // the fused move stage: the record carries the moved particle
         push_axis(f[0][k], f[3][k], push.dt, push.lo[0], push.hi[0]);
         push_axis(f[1][k], f[4][k], push.dt, push.lo[1], push.hi[1]);
@@ -533,14 +538,14 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
     }
     __syncthreads();
 #pragma unroll 4
-    for (int b = tid; b < buckets; b += kScatterThreads) {
+    for (int b = tid; b < buckets; b += THREADS) {
       const uint32_t c = slot_of[b];
       if (c) slot_of[b] = atomicAdd(&row[b], c);
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
-      const int64_t i = first + (k / 4 * kScatterThreads + tid) * 4 + k % 4;
+      const int64_t i = first + (k / 4 * THREADS + tid) * 4 + k % 4;
       if (i < n)
         store_record(records + static_cast<size_t>(slot_of[key[k] >> (kShuffleBits + shift)] + rank[k]) *
                                    kRecordWords,
@@ -2392,6 +2397,10 @@ int small_call_blocks(int64_t n, int64_t buckets) {
 // Up to where slots are reserved tile by tile.
 constexpr int64_t kTiledMostParticles = 6 << 20;
 constexpr int64_t kTiledMostBuckets = 8192;
+// From here on tiles of 4096 particles, 1024 threads (against 2048, 512 threads: 2 M particles with 20 to a cell 86.9 / 85.8
+// us per call, 2.4 M 102.2 / 106.8, 3 M 121.1 / 128.4, 4 M 153.8 / 170.9; with 8 to a cell 90.3 / 91.5, 92.8 / 94.9, 109.6 /
+// 112.3, 150.8 / 158.1, but 3.2 M 128.0 / 122.3).
+constexpr int64_t kWideTilesFrom = 2300000;
 
 // Largest bucket width 2^s, s <= max_shift, whose average load stays at or below `target`,
 // with at least 2048 buckets (fewer make the slot counters of the scatter contend: measured
@@ -2601,14 +2610,15 @@ cudaError_t launch_tail(const RunTable& t, const SortArgs& a, const FinishOut& o
                            a.num_cells, out, hdr, group_capacity, digits, settled);
 }
 
-template <int ITEMS>
+template <int THREADS>
 cudaError_t launch_tile_scatter(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, int shift,
                                 int buckets, int chunk_log, uint32_t* cursor, uint32_t* records,
                                 Header* hdr, bool behind, bool chained) {
-  constexpr int kTile = kScatterThreads * ITEMS;
-  auto kernel = vec ? tile_scatter_kernel<true, ITEMS> : tile_scatter_kernel<false, ITEMS>;
-  const int64_t blocks = std::min<int64_t>((a.n + kTile - 1) / kTile, 2 * sm_count());
-  return launch_chained_if(chained, kernel, static_cast<int>(blocks), kScatterThreads,
+  constexpr int kTile = THREADS * 4;
+  auto kernel = vec ? tile_scatter_kernel<true, THREADS> : tile_scatter_kernel<false, THREADS>;
+  const int64_t tiles = (a.n + kTile - 1) / kTile;
+  const int64_t blocks = behind ? std::min<int64_t>(tiles, sm_count() * (1024 / THREADS)) : tiles;
+  return launch_chained_if(chained, kernel, static_cast<int>(blocks), THREADS,
                            static_cast<size_t>(buckets) * sizeof(uint32_t), a.stream, a.x, a.y, a.z,
                            a.velocity, a.padded, a.push, a.n, a.grid, k0, k1, shift, buckets, chunk_log,
                            cursor, records, hdr, behind);
@@ -2932,11 +2942,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     e = launch(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, chained);
     if (e != cudaSuccess) return e;
   } else if (p.tiled) {
-    e = a.n >= static_cast<int64_t>(sm_count()) * kScatterThreads * 16
-            ? launch_tile_scatter<8>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind,
-                                     chained)
-            : launch_tile_scatter<4>(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind,
-                                     chained);
+    const auto launch = a.n >= kWideTilesFrom ? launch_tile_scatter<1024> : launch_tile_scatter<512>;
+    e = launch(a, vec, k0, k1, p.shift, buckets, l.chunk_log, cursor, records, hdr, behind, chained);
     if (e != cudaSuccess) return e;
   } else {
     auto launch = [&](auto items, int64_t blocks, ScatterOnly only) {
