@@ -106,6 +106,16 @@ int AetherSortAndGatherParticles(const float* x, const float* y, const float* z,
                                  float* velocity_sorted, int64_t padded_sorted, int path,
                                  void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same, and columns [n, padded_sorted) of velocity_sorted become zero, before anything is read. */
+int AetherSortAndGatherParticlesZeroPadded(
+    const float* x, const float* y, const float* z,
+    const float* velocity, int64_t padded, int64_t n,
+    const AetherGrid* grid, uint64_t seed, uint32_t* keys_out,
+    int32_t* index_out, int32_t* cell_counts, int32_t* cell_start,
+    float* x_sorted, float* y_sorted, float* z_sorted,
+    float* velocity_sorted, int64_t padded_sorted, int path,
+    void* workspace, size_t workspace_bytes, void* stream);
+
 /* The payload gather alone (dsmc_gpu_pipeline.py:107-109): out[r] = in[index[r]]. */
 int AetherGatherParticles(const int32_t* index, int64_t n, const float* x, const float* y,
                           const float* z, const float* velocity, int64_t padded,
@@ -297,6 +307,14 @@ int AetherParticlePush(float* x, float* y, float* z, float* vx, float* vy, float
  * three floats each; velocity is required; the workspace must have the size
  * AetherSortWorkspaceBytes(n, num_cells, 1) reports. */
 int AetherPushSortAndGatherParticles(
+    const float* x, const float* y, const float* z, const float* velocity, int64_t padded,
+    int64_t n, float dt, const float* lo, const float* hi, const AetherGrid* grid, uint64_t seed,
+    uint32_t* keys_out, int32_t* index_out, int32_t* cell_counts, int32_t* cell_start,
+    float* x_sorted, float* y_sorted, float* z_sorted, float* velocity_sorted,
+    int64_t padded_sorted, int path, void* workspace, size_t workspace_bytes, void* stream);
+
+/* The same, and columns [n, padded_sorted) of velocity_sorted become zero, before anything is read. */
+int AetherPushSortAndGatherParticlesZeroPadded(
     const float* x, const float* y, const float* z, const float* velocity, int64_t padded,
     int64_t n, float dt, const float* lo, const float* hi, const AetherGrid* grid, uint64_t seed,
     uint32_t* keys_out, int32_t* index_out, int32_t* cell_counts, int32_t* cell_start,

@@ -46,12 +46,22 @@ _SIGNATURES = {
                                                     ctypes.POINTER(AetherGrid), ctypes.c_uint64,
                                                     _P, _P, _P, _P, _P, _P, _P, _P, _I64,
                                                     ctypes.c_int, _P, ctypes.c_size_t, _P]),
+    'AetherSortAndGatherParticlesZeroPadded': (ctypes.c_int, [_P, _P, _P, _P, _I64, _I64,
+                                                              ctypes.POINTER(AetherGrid), ctypes.c_uint64,
+                                                              _P, _P, _P, _P, _P, _P, _P, _P, _I64,
+                                                              ctypes.c_int, _P, ctypes.c_size_t, _P]),
     'AetherPushSortAndGatherParticles': (ctypes.c_int, [_P, _P, _P, _P, _I64, _I64, ctypes.c_float,
                                                         ctypes.POINTER(ctypes.c_float),
                                                         ctypes.POINTER(ctypes.c_float),
                                                         ctypes.POINTER(AetherGrid), ctypes.c_uint64,
                                                         _P, _P, _P, _P, _P, _P, _P, _P, _I64,
                                                         ctypes.c_int, _P, ctypes.c_size_t, _P]),
+    'AetherPushSortAndGatherParticlesZeroPadded': (ctypes.c_int, [_P, _P, _P, _P, _I64, _I64, ctypes.c_float,
+                                                                  ctypes.POINTER(ctypes.c_float),
+                                                                  ctypes.POINTER(ctypes.c_float),
+                                                                  ctypes.POINTER(AetherGrid), ctypes.c_uint64,
+                                                                  _P, _P, _P, _P, _P, _P, _P, _P, _I64,
+                                                                  ctypes.c_int, _P, ctypes.c_size_t, _P]),
     'AetherGatherParticles': (ctypes.c_int, [_P, _I64, _P, _P, _P, _P, _I64, _P, _P, _P, _P,
                                              _I64, _P]),
     'AetherMakeKeys': (ctypes.c_int, [_P, _P, _P, _I64, ctypes.POINTER(AetherGrid),
@@ -141,8 +151,8 @@ _library = None
 binding = None        # the native binding, once the library is loaded; None where there is none
 bound_library = None  # the library it calls; set only when `binding` is
 
-_BOUND = ('AetherSortWorkspaceBytes', 'AetherSortParticlesByCell', 'AetherSortAndGatherParticles',
-          'AetherPushSortAndGatherParticles', 'AetherDsmcCollideTma')
+_BOUND = ('AetherSortWorkspaceBytes', 'AetherSortParticlesByCell', 'AetherSortAndGatherParticlesZeroPadded',
+          'AetherPushSortAndGatherParticlesZeroPadded', 'AetherDsmcCollideTma')
 
 
 def exported_symbols():

@@ -31,6 +31,20 @@ bool grid_ok(const AetherGrid* g) {
 
 bool count_ok(int64_t n) { return n >= 0 && n < (int64_t{1} << 30); }
 
+// Whether the padding columns of the sorted velocities lie over an input.
+bool padding_over_inputs(const SortArgs& a) {
+  const size_t row = static_cast<size_t>(a.n) * sizeof(float), pad = static_cast<size_t>(a.padded_sorted - a.n) * sizeof(float);
+  const float* in[6] = {a.x, a.y, a.z, a.velocity, a.velocity + a.padded, a.velocity + 2 * a.padded};
+  for (int r = 0; r < 3; ++r) {
+    const auto to = reinterpret_cast<uintptr_t>(a.vs + r * a.padded_sorted + a.n);
+    for (const float* i : in) {
+      const auto from = reinterpret_cast<uintptr_t>(i);
+      if (to < from + row && from < to + pad) return true;
+    }
+  }
+  return false;
+}
+
 int run_sort(SortArgs& a, int path) {
   if (!count_ok(a.n) || !grid_ok(&a.grid)) return cudaErrorInvalidValue;
   if (!a.cell_counts || !a.cell_start || !a.workspace) return cudaErrorInvalidValue;
@@ -49,6 +63,14 @@ int run_sort(SortArgs& a, int path) {
   const bool roomy = a.workspace_bytes >= bucketed_workspace_bytes(a.n, a.num_cells, keys_only);
   const bool bucketed = plan.usable && path != 1 && (roomy || path == 2);
   if (path == 2 && (!plan.usable || !roomy)) return cudaErrorInvalidValue;
+  a.zero_padding = a.zero_padding && a.vs && a.padded_sorted > a.n;
+  // The bucketed path's clearing kernel zeroes the padding, but kernels behind it read the inputs while it runs.
+  if (a.zero_padding && (!bucketed || padding_over_inputs(a))) {
+    const cudaError_t e = cudaMemset2DAsync(a.vs + a.n, a.padded_sorted * sizeof(float), 0,
+                                            (a.padded_sorted - a.n) * sizeof(float), 3, a.stream);
+    if (e != cudaSuccess) return e;
+    a.zero_padding = false;
+  }
   return bucketed ? bucketed_sort(a, plan) : standard_sort(a);
 }
 
@@ -273,7 +295,8 @@ int sort_and_gather(const float* x, const float* y, const float* z, const float*
                     uint32_t* keys_out, int32_t* index_out, int32_t* cell_counts,
                     int32_t* cell_start, float* x_sorted, float* y_sorted, float* z_sorted,
                     float* velocity_sorted, int64_t padded_sorted, int path, void* workspace,
-                    size_t workspace_bytes, void* stream, const PushSpec& push, int most_blocks = 0) {
+                    size_t workspace_bytes, void* stream, const PushSpec& push, int most_blocks = 0,
+                    bool zero_padding = false) {
   if (!grid) return cudaErrorInvalidValue;
   if (n > 0 && !most_blocks && (!x_sorted || !y_sorted || !z_sorted)) return cudaErrorInvalidValue;
   if ((velocity == nullptr) != (velocity_sorted == nullptr)) return cudaErrorInvalidValue;
@@ -291,6 +314,7 @@ int sort_and_gather(const float* x, const float* y, const float* z, const float*
   a.stream = static_cast<cudaStream_t>(stream);
   a.push = push;
   a.most_blocks = most_blocks;
+  a.zero_padding = zero_padding;
   return run_sort(a, path);
 }
 }  // namespace
@@ -305,6 +329,17 @@ extern "C" int AetherSortAndGatherParticles(
   return sort_and_gather(x, y, z, velocity, padded, n, grid, seed, keys_out, index_out,
                          cell_counts, cell_start, x_sorted, y_sorted, z_sorted, velocity_sorted,
                          padded_sorted, path, workspace, workspace_bytes, stream, PushSpec{});
+}
+
+extern "C" int AetherSortAndGatherParticlesZeroPadded(
+    const float* x, const float* y, const float* z, const float* velocity, int64_t padded,
+    int64_t n, const AetherGrid* grid, uint64_t seed, uint32_t* keys_out, int32_t* index_out,
+    int32_t* cell_counts, int32_t* cell_start, float* x_sorted, float* y_sorted, float* z_sorted,
+    float* velocity_sorted, int64_t padded_sorted, int path, void* workspace,
+    size_t workspace_bytes, void* stream) {
+  return sort_and_gather(x, y, z, velocity, padded, n, grid, seed, keys_out, index_out,
+                         cell_counts, cell_start, x_sorted, y_sorted, z_sorted, velocity_sorted,
+                         padded_sorted, path, workspace, workspace_bytes, stream, PushSpec{}, 0, true);
 }
 
 extern "C" int AetherSortProbeFewBlocks(
@@ -340,6 +375,25 @@ extern "C" int AetherPushSortAndGatherParticles(
   return sort_and_gather(x, y, z, velocity, padded, n, grid, seed, keys_out, index_out,
                          cell_counts, cell_start, x_sorted, y_sorted, z_sorted, velocity_sorted,
                          padded_sorted, path, workspace, workspace_bytes, stream, push);
+}
+
+extern "C" int AetherPushSortAndGatherParticlesZeroPadded(
+    const float* x, const float* y, const float* z, const float* velocity, int64_t padded,
+    int64_t n, float dt, const float* lo, const float* hi, const AetherGrid* grid, uint64_t seed,
+    uint32_t* keys_out, int32_t* index_out, int32_t* cell_counts, int32_t* cell_start,
+    float* x_sorted, float* y_sorted, float* z_sorted, float* velocity_sorted,
+    int64_t padded_sorted, int path, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!lo || !hi) return cudaErrorInvalidValue;
+  PushSpec push{};
+  push.enabled = 1;
+  push.dt = dt;
+  for (int c = 0; c < 3; ++c) {
+    push.lo[c] = lo[c];
+    push.hi[c] = hi[c];
+  }
+  return sort_and_gather(x, y, z, velocity, padded, n, grid, seed, keys_out, index_out,
+                         cell_counts, cell_start, x_sorted, y_sorted, z_sorted, velocity_sorted,
+                         padded_sorted, path, workspace, workspace_bytes, stream, push, 0, true);
 }
 
 extern "C" int AetherGatherParticles(const int32_t* index, int64_t n, const float* x,

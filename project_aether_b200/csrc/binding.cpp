@@ -27,8 +27,8 @@ namespace {
 // Entry points of the library that ctypes loaded (bind).
 decltype(&AetherSortWorkspaceBytes) workspace_bytes = nullptr;
 decltype(&AetherSortParticlesByCell) sort_entry = nullptr;
-decltype(&AetherSortAndGatherParticles) gather_entry = nullptr;
-decltype(&AetherPushSortAndGatherParticles) push_entry = nullptr;
+decltype(&AetherSortAndGatherParticlesZeroPadded) gather_entry = nullptr;
+decltype(&AetherPushSortAndGatherParticlesZeroPadded) push_entry = nullptr;
 decltype(&AetherDsmcCollideTma) collide_entry = nullptr;
 PyTypeObject* grid_type = nullptr;  // CellGrid
 
@@ -258,7 +258,12 @@ PyObject* gather(PyObject*, PyObject* const* args, Py_ssize_t count) {
     for (int k = 4; k < 7; ++k) out[k] = fresh({s.n}, at::kFloat, s.device);
     out[7] = fresh({3, padded_sorted}, at::kFloat, s.device);
   }
-  if (padded_sorted > s.n) out[7].narrow(1, s.n, padded_sorted - s.n).zero_();
+  // The library zeroes the padding columns.  A given tensor that PyTorch would not let be written to, or that it counts
+  // the writes to, is treated as by its own operation.
+  if (padded_sorted > s.n && given[7]) {
+    if (out[7].requires_grad() || out[7].is_inference()) out[7].narrow(1, s.n, padded_sorted - s.n).zero_();
+    else out[7].unsafeGetTensorImpl()->bump_version();
+  }
   const float flo[3] = {static_cast<float>(lo[0]), static_cast<float>(lo[1]), static_cast<float>(lo[2])};
   const float fhi[3] = {static_cast<float>(hi[0]), static_cast<float>(hi[1]), static_cast<float>(hi[2])};
   const float *x = at_start<float>(*s.c[0]), *y = at_start<float>(*s.c[1]), *z = at_start<float>(*s.c[2]),

@@ -316,6 +316,7 @@ struct SortArgs {
   cudaStream_t stream;
   PushSpec push;
   int most_blocks;  // 0, or a limit on the blocks of the kernels that work in phases (probe)
+  bool zero_padding;  // columns n and on of the sorted velocities become zero
 };
 
 size_t standard_workspace_bytes(int64_t n, int64_t num_cells);

@@ -1,0 +1,61 @@
+"""The padding columns of the sorted velocities become zero, whatever kernel does it."""
+
+import pytest
+import torch
+
+import project_aether_b200 as pa
+from project_aether_b200 import particle_sort
+
+pytestmark = pytest.mark.gpu
+
+GRID = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (12, 11, 10))
+
+
+def _state(device, n):
+    gen = torch.Generator(device=device).manual_seed(n)
+    pos = tuple(torch.rand(n, device=device, generator=gen) for _ in range(3))
+    return pos, torch.randn((3, n), device=device, generator=gen)
+
+
+# One launch, tiles, digit passes; columns for a few, many, and none.
+@pytest.mark.parametrize('n,path', [(1, 0), (5001, 0), (5001, 1), (700_001, 0), (2_000_003, 0)])
+@pytest.mark.parametrize('extra', [0, 1, 70_000])
+@pytest.mark.parametrize('given', [False, True])
+@pytest.mark.parametrize('push', [None, (1e-3, (0., 0., 0.), (1., 1., 1.))])
+def test_columns_behind_the_particles(cuda, n, path, extra, given, push):
+    pos, vel = _state(cuda, n)
+    plain = pa.sort_and_gather_particles(*pos, vel, GRID, 9, path=path, push=push)
+    out = None
+    if given:
+        out = particle_sort.SortedParticles(plain.order, plain.positions, torch.full((3, n + extra), 7., device=cuda))
+        version = out.velocity._version
+    got = pa.sort_and_gather_particles(*pos, vel, GRID, 9, path=path, push=push, padded_out=n + extra, out=out)
+    assert got.velocity.shape == (3, n + extra)
+    assert torch.equal(got.velocity[:, :n], plain.velocity) and not got.velocity[:, n:].any()
+    if given and extra:
+        assert out.velocity._version > version
+
+
+@pytest.mark.parametrize('n', [5001, 700_001])
+def test_padding_over_an_input(cuda, n):
+    """The columns become zero before anything is read."""
+    pos, vel = _state(cuda, n)
+    buffer = torch.empty(3 * (2 * n + 4), device=cuda)
+    velocity = buffer.view(3, 2 * n + 4)
+    x = velocity[0, n:2 * n]
+    x.copy_(pos[0])
+    plain = pa.sort_and_gather_particles(torch.zeros_like(pos[0]), *pos[1:], vel, GRID, 9)
+    out = particle_sort.SortedParticles(plain.order._replace(keys=plain.order.keys.clone()),
+                                        tuple(t.clone() for t in plain.positions), velocity)
+    got = pa.sort_and_gather_particles(x, *pos[1:], vel, GRID, 9, padded_out=2 * n + 4, out=out)
+    assert torch.equal(got.order.keys, plain.order.keys) and torch.equal(got.velocity[:, :n], plain.velocity)
+    assert not got.velocity[:, n:].any()
+
+
+def test_an_output_that_wants_gradients_is_refused(cuda):
+    pos, vel = _state(cuda, 5001)
+    plain = pa.sort_and_gather_particles(*pos, vel, GRID, 9)
+    wants = torch.zeros((3, 5004), device=cuda, requires_grad=True)
+    out = particle_sort.SortedParticles(plain.order, plain.positions, wants)
+    with pytest.raises(RuntimeError):
+        pa.sort_and_gather_particles(*pos, vel, GRID, 9, padded_out=5004, out=out)
