@@ -63,13 +63,16 @@ constexpr int kKeyRecordWords = 2;  // 8-byte record {key, index} of calls witho
 // one behind it can be chained to it and is set up, and has loaded its particles, by the time this is
 // done.  Per call, memset / this: sort of 5000 particles 19.7 / 18.0 us, gather of 500,000 37.6 / 34.9, of
 // 1 M 54.3 / 52.3, step of 200,003 38.5 / 36.0.
-// Also zeroes `columns` columns of three rows `row` apart, from `padding` on: as a launch of its own that cost a step of
-// 200,003 particles 2.6 us and the host 4.
+// PADDED: also zeroes `columns` columns of three rows `row` apart, from `padding` on (as a launch of its own that cost a
+// step of 200,003 particles 2.6 us).  Apart, so that the usual kernel holds few registers: with them the count kernel chained
+// to it lay unevenly on the multiprocessors, and a sort of 4 M or 16 M particles took 1 to 2 us more.
+template <bool PADDED>
 __global__ void __launch_bounds__(512) clear_kernel(uint4* words, int64_t n, float* padding, int64_t row, int64_t columns) {
   chain_release();
-  for (int64_t i = blockIdx.x * 512ll + threadIdx.x; i < 3 * columns; i += gridDim.x * 512ll)
-    padding[i / columns * row + i % columns] = 0.f;
   for (int64_t i = blockIdx.x * 512ll + threadIdx.x; i < n; i += gridDim.x * 512ll) words[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (PADDED)
+    for (int64_t i = blockIdx.x * 512ll + threadIdx.x; i < columns; i += gridDim.x * 512ll)
+      padding[i] = padding[row + i] = padding[2 * row + i] = 0.f;
 }
 
 // The kernels of a general call that is enqueued behind an attempt to sort a settled state
@@ -2846,8 +2849,9 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   {
     const int64_t pieces = static_cast<int64_t>(l.start_off / sizeof(uint4));
     const int blocks = static_cast<int>(std::min<int64_t>((pieces + 511) / 512, 2 * sm_count()));
-    clear_kernel<<<blocks, 512, 0, a.stream>>>(reinterpret_cast<uint4*>(base), pieces, a.vs + a.n, a.padded_sorted,
-                                               a.zero_padding ? a.padded_sorted - a.n : 0);
+    auto clear = a.zero_padding ? clear_kernel<true> : clear_kernel<false>;
+    clear<<<blocks, 512, 0, a.stream>>>(reinterpret_cast<uint4*>(base), pieces, a.vs + a.n, a.padded_sorted,
+                                        a.padded_sorted - a.n);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     count_launches(1);
