@@ -2292,6 +2292,7 @@ small_sort_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ F
     __syncthreads();
   }
   if (done >= kFailedTask && tid == 0) atomicExch(&hdr->use_standard, 1);
+  chain_release();  // all blocks run by now: what is enqueued behind (the collisions of a step) may be set up
   arrive(&hdr->tasks_done, done);
   uint32_t seen = 0;
   if (!wait_for(&hdr->tasks_done, tasks, &hdr->error, kWaitLimitNs, kFailedTask - 1, &seen)) return;
