@@ -29,8 +29,8 @@
 // it is noticed: random order and too many movers by the probe; a particle out of order, or more movers than
 // the lists hold in one part of the input, in the round of the scan that meets it; a counter that wraps in
 // the finish.  Buckets of a dense region are no reason.  Calls that the probe gives up, before there was this path /
-// now: 1.6 M particles 86.9 / 91.4 us, 4 M 170 / 176, 16.8 M 482 / 485, 30 M 837 / 837, 64 M 1885 / 1849; in random
-// order 1.6 M 87.3 / 90.9, 4 M 184 / 187, 6 M 250.5 / 251, 16.8 M 599 / 602, 64 M 2266 / 2246.
+// now: 1.6 M particles 86.9 / 83.9 us, 4 M 170 / 167, 16.8 M 482 / 490, 30 M 837 / 833, 64 M 1885 / 1843; in random
+// order 1.6 M 87.3 / 88.0, 4 M 184 / 174, 6 M 250 / 234, 16.8 M 599 / 604, 64 M 2266 / 2238.
 
 constexpr int kSettledThreads = 512;
 constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round

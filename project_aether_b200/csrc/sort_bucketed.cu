@@ -2706,12 +2706,11 @@ namespace {
 // that gives up may lose.
 constexpr int64_t kSettledLeast = int64_t{3} << 19;
 constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
-// Particles in a thousand that leave their bucket, above which the general path does the call: about where the
-// settled sort takes as long as giving up and the general path (tiles; small finish blocks; large ones).  Movers
-// in a thousand, settled / given up, us per call: 4 M 153 172.8 / 177, 183 178.0; 1.6 M 159 88.8 / 94, 248 99.6; 16.8 M
-// 56 475 / 487, 30 M 52 797 / 839, 126 930; 64 M 98 1765 / 1850, 131 1893; 128 M 98 3480 / 3631, 129 3750 (the largest of each
-// with a scan that was 1.5 % slower).
-constexpr int64_t kMoversTiled = 180, kMoversSmall = 60, kMoversLarge = 120;
+// Particles in a thousand that leave their bucket, above which the general path does the call (tiles; small finish blocks;
+// large ones).  Up to there the settled sort is faster: us per call, movers in a thousand, settled / given up, 16.8 M 76 407 / 488;
+// 64 M 129 1525 / 1835, 98 1475 / 1850; 128 M 98 2912 / 3631.  It would be beyond too; a call that fails late, when the
+// lists of the scan are full, costs most.
+constexpr int64_t kMoversTiled = 180, kMoversSmall = 80, kMoversLarge = 140;
 
 bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
   const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
