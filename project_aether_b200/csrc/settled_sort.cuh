@@ -481,8 +481,8 @@ struct __align__(16) SettledSmem {
 // stores of a word at one address with constant offsets and a quarter of eight loads and stores of 16 bytes, where
 // whole records, pulled out of shared memory by sorted place, cost four accesses of 16 bytes, eight stores of a word and
 // their addresses.  The bodies of the item loops are written so that the compiler predicates single accesses
-// instead of branching around them (258 -> 220 instructions a record).  Bound by instructions and the
-// shared-memory pipe (issue slots 49 %, pipe 66 %).  16.8 M particles, 8 to a cell, 285 -> 199 us, 20 M with 64
+// instead of branching around them (325 -> 229 instructions a record).  Bound by instructions and the
+// shared-memory pipe (issue slots 54 %, pipe 74 %).  16.8 M particles, 8 to a cell, 285 -> 199 us, 20 M with 64
 // 344 -> 253, 128 M 2168 -> 1560 (60 bytes a particle: 5.2 TB/s).  Stored to the output straight from the
 // registers, neighbouring lanes to places a few cells wide, 16.8 M took 221 us in groups of 1024, and 64 to a cell
 // 372, in parts of sectors; read by sorted place instead, 250 and 299.
