@@ -2824,6 +2824,19 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   count_launches(6);
   return e;
 }
+
+// Clears `bytes` at `base`, and the padding columns where they are the kernel's.  As many blocks as either takes: with
+// those of the header and counts alone, two or three, 5001 particles with a million columns took 299 us (now 22), 1 M
+// particles with a million 136 (60).
+cudaError_t launch_clear(const SortArgs& a, void* base, size_t bytes) {
+  const auto pieces = static_cast<int64_t>(bytes / sizeof(uint4));
+  const int64_t columns = a.zero_padding ? a.padded_sorted - a.n : 0;
+  const int blocks = static_cast<int>(std::min<int64_t>((std::max(pieces, columns) + 511) / 512, 2 * sm_count()));
+  auto clear = a.zero_padding ? clear_kernel<true> : clear_kernel<false>;
+  clear<<<blocks, 512, 0, a.stream>>>(static_cast<uint4*>(base), pieces, a.vs + a.n, a.padded_sorted, columns);
+  count_launches(1);
+  return cudaGetLastError();
+}
 }  // namespace
 
 // Enqueues the bucketed path.  When a bucket turns out too large for the finish
@@ -2846,16 +2859,8 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   if (e != cudaSuccess) return e;
   // Header and run counts.  An ordinary launch, which begins when all before it in the stream is done: the
   // kernels chained to it read the call's inputs before they wait for it.
-  {
-    const int64_t pieces = static_cast<int64_t>(l.start_off / sizeof(uint4));
-    const int blocks = static_cast<int>(std::min<int64_t>((pieces + 511) / 512, 2 * sm_count()));
-    auto clear = a.zero_padding ? clear_kernel<true> : clear_kernel<false>;
-    clear<<<blocks, 512, 0, a.stream>>>(reinterpret_cast<uint4*>(base), pieces, a.vs + a.n, a.padded_sorted,
-                                        a.padded_sorted - a.n);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    count_launches(1);
-  }
+  e = launch_clear(a, base, l.start_off);
+  if (e != cudaSuccess) return e;
   if (p.one_launch) {
     stage_begin(kStageBucketFinish, a.stream);
     e = p.keys_only ? launch_small<FinishKeys>(a, p, l, digits) : launch_small<FinishSmall>(a, p, l, digits);
