@@ -64,10 +64,10 @@ int run_sort(SortArgs& a, int path) {
   const bool bucketed = plan.usable && path != 1 && (roomy || path == 2);
   if (path == 2 && (!plan.usable || !roomy)) return cudaErrorInvalidValue;
   a.zero_padding = a.zero_padding && a.vs && a.padded_sorted > a.n;
-  // The bucketed path's clearing kernel zeroes the padding, but kernels behind it read the inputs while it runs.
+  // The bucketed path's clearing kernel zeroes the padding, but kernels behind it read the inputs while it runs.  (Not
+  // cudaMemset2D: rows of 2^29 floats and more are above the largest pitch that devices state, 2^31 - 1 bytes.)
   if (a.zero_padding && (!bucketed || padding_over_inputs(a))) {
-    const cudaError_t e = cudaMemset2DAsync(a.vs + a.n, a.padded_sorted * sizeof(float), 0,
-                                            (a.padded_sorted - a.n) * sizeof(float), 3, a.stream);
+    const cudaError_t e = zero_padding_first(a);
     if (e != cudaSuccess) return e;
     a.zero_padding = false;
   }

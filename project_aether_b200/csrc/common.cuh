@@ -359,6 +359,8 @@ void set_small_shape_buckets(int64_t buckets);
 uint32_t bucket_group_capacity(int64_t n, const BucketPlan& p);
 size_t bucketed_workspace_bytes(int64_t n, int64_t num_cells, bool keys_only);
 cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p);
+// Zeroes the padding columns of the sorted velocities in a launch of its own, ahead of all that the call does.
+cudaError_t zero_padding_first(const SortArgs& a);
 
 // The bucketed sort of a segmented input, slice by slice (the local sort of the sliced
 // multi-GPU exchange): a.n is the CAPACITY of the input arrays, the particle count and the

@@ -2839,6 +2839,10 @@ cudaError_t launch_clear(const SortArgs& a, void* base, size_t bytes) {
 }
 }  // namespace
 
+// What comes behind it is launched in the ordinary way (the memset of the digit passes, another clearing kernel), so that
+// it is complete by then although it lets chained kernels in at once.
+cudaError_t zero_padding_first(const SortArgs& a) { return launch_clear(a, nullptr, 0); }
+
 // Enqueues the bucketed path.  When a bucket turns out too large for the finish
 // kernel the device sets Header::use_standard, the kernels between return at once
 // and the tail kernel runs the digit passes.

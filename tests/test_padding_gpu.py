@@ -78,3 +78,15 @@ def test_wide_padding_is_zeroed_by_all_multiprocessors(cuda, n):
         took.append(begin.elapsed_time(end))
     assert not out.velocity[:, n:].any()
     assert min(took) < 1.0
+
+
+@pytest.mark.parametrize('n,path', [(0, 0), (5001, 0), (5001, 1)])
+def test_rows_of_more_than_2_to_the_31_bytes(cuda, n, path):
+    """A row of the sorted velocities may be longer than the largest pitch of a 2D copy."""
+    pos, vel = _state(cuda, n + 1)
+    plain = pa.sort_and_gather_particles(*(p[:n] for p in pos), vel, GRID, 9, path=path)
+    rows = torch.full((3, (1 << 29) + 8), 7., device=cuda)
+    out = particle_sort.SortedParticles(plain.order, plain.positions, rows)
+    got = pa.sort_and_gather_particles(*(p[:n] for p in pos), vel, GRID, 9, path=path, padded_out=rows.shape[1], out=out)
+    assert torch.equal(got.velocity[:, :n], plain.velocity[:, :n])
+    assert not any(row[n:].any() for row in got.velocity)
