@@ -16,7 +16,8 @@
 //   settled_movers_kernel  the lists' records to their buckets' arrivals
 //   settled_finish_kernel  a block takes a group: reads its home run and keys, moves the particles once
 //                          more, leaves out those that left, adds the arrivals, sorts and writes the group
-//   bucket_tail_kernel     the same for dense regions, whose buckets those blocks do not hold
+//   bucket_finish_kernel   (of the general path) the same for dense regions, whose buckets those blocks do not hold
+//   bucket_tail_kernel     the same for single buckets that the kernel before does not hold
 //
 // It moves 24 + 4 + 28 + 32 bytes per particle, and some 130 more per mover, where the general path moves
 // 24 + 24 + 32 + 32 + 32.  Bound by instructions: with the keys made in the finish kernel, 24 + 24 + 32
@@ -39,6 +40,8 @@ constexpr int kMoverShare = 4;                      // all lists together for on
 constexpr int kProbeSamples = 128;                  // particles of each of the scan's blocks that the probe looks at
 constexpr int kSettledPart = 4096;                  // buckets per entry of the coarse sums
 constexpr int kSettledSums = 4 * (1 + kSettledPart / kGroupSpan);  // words of such an entry: of the part, of its kGroupSpan buckets each
+constexpr int kDenseSpanLog = 3;                    // buckets that are dense or not together
+constexpr int kSettledWideShare = 1024;             // particles to a bucket above a dense group's capacity, at least
 constexpr uint32_t kGone = 0xffffffffu;             // no key: grids of 2^25 cells are left to the general path
 constexpr int kSettledRowWords = 8;                 // words of a group's table
 // What sorts a group in the finish: THREADS threads that hold ITEMS records each, move and all, in registers.
@@ -58,10 +61,18 @@ struct SettledShape {
 // hold 2048 242, 64 that hold 256 214; three items a thread 217, six 220, eight 279, which leave fewer threads).  Their
 // groups span 64 cells at most, so that sparse grids do not fill them, and a cell may have some 400 particles: beyond
 // either limit the groups are blocks' (20 M particles, 4 / 5 / 6 to a cell: teams 351 / 300 / 253 us, blocks 285 /
-// 286 / 286).  Where the density differs from place to place, buckets above the shape's capacity, and what
-// lies near them, go to wide groups, which the tail kernel sorts.
+// 286 / 286).  Where the density differs from place to place, spans of 2^kDenseSpanLog buckets with one above a
+// team's capacity are cut into groups of SettledDense, which the general path's finish kernel sorts, otherwise idle then; a
+// bucket that those do not hold is a whole block's of the tail kernel, SettledWide, up to its capacity.
+// us per call before teams / with all 256 buckets around such a bucket in groups of 4096 places, one to a multiprocessor, in the tail
+// kernel / this, share of the particles in a share of the space: 4 M in 79^3 cells, 0.1 in 0.01 142 / 159 / 134, 0.28 in 0.03
+// 162 / 157 / 141; 16.8 M in 112^3, 0.5 in 0.05 476 / 543 / 477, 0.5 in 0.1 466 / 525 / 453; 64 M in 175^3 1638 / 1804 / 1644, 1609 / 1752 / 1550.
+// Worst where a bucket is just above half of a dense group: 2.5 M in 59^3, 0.5 in 0.05 105 / 133 / 115; 30 M in 67^3
+// 868 / 966 / 918.  (Dense groups of 2560 places, five records a thread: 110, 874, but 5 to 7 percent more elsewhere.  Two parts of a block of the
+// tail kernel instead of the finish kernel: 130, 1060.  Buckets half as wide: 2 percent more where the density is even.)
 using SettledTeam = SettledShape<128, 4, 11>;
 using SettledBlock = SettledShape<512, 4, 14>;
+using SettledDense = SettledBlock;
 using SettledWide = SettledShape<1024, 4, 15>;
 constexpr int64_t kSettledTeamLeast = 352;     // particles on a team's most cells, on average at least
 constexpr int64_t kSettledTeamMostMean = 384;  // particles of a cell, on average at most
@@ -82,7 +93,8 @@ struct SettledArgs {
   int shift, buckets;
   int per_block;          // particles per block of the scan, a multiple of kSettledRound
   int scan_blocks;
-  int teams;              // whether groups of a few hundred places pay
+  uint32_t capacity;      // of the shape that sorts the usual groups
+  int most_cells;
   uint32_t most_sampled;  // movers of the sample from which on the general path is faster
   uint32_t most_movers;   // what fits `arrived`
   uint32_t *first, *end;            // [buckets] home run in the input; both zero if it is empty
@@ -92,7 +104,8 @@ struct SettledArgs {
   uint32_t* cursor;                 // [buckets] next free place of each bucket's arrivals
   uint32_t* sums;                   // [parts][kSettledSums] particles at home, arrivals, output of kSettledPart buckets
   uint32_t* tables;                 // [buckets][kSettledRowWords]: groups of teams, and from the end buckets in no group
-  uint32_t* wide_tables;            // [buckets][kSettledRowWords]: groups of dense regions
+  uint32_t* dense_tables;           // [buckets][kSettledRowWords]: groups of dense regions
+  uint32_t* wide_tables;            // [n / kSettledWideShare + 1][kSettledRowWords]: buckets that those do not hold
   uint32_t *list, *arrived;         // records: the movers block by block, and bucket by bucket
   int vec_out;            // the outputs take 16-byte stores where the place is a multiple of four
   Header* hdr;
@@ -357,10 +370,9 @@ settled_sums_kernel(const __grid_constant__ SettledArgs a) {
 // A block takes kGroupSpan consecutive buckets; it adds up what lies before them for itself, from the sums.
 // Groups as in group_kernel; a bucket needs a place for each of its particles at home and each of its arrivals.
 // A group's table: first particle of its home run, particles in it, first of its arrivals, arrivals, first
-// output slot, records, its buckets b0, b1.  Where one of the block's buckets is more than the finish kernel
-// holds, all are cut into wide groups, for the tail kernel; so is, with a table from the end of the first array (there
-// are no more groups and such buckets than buckets), a bucket that a wide group does not hold.  aux_counter[2], [3], [4]:
-// the three kinds.
+// output slot, records, its buckets b0, b1.  Runs of spans with a bucket that is more than a team holds have lists of their own,
+// of dense groups and of single buckets that no such group holds; a bucket that no block holds gets a table from the end of
+// the first array (there are no more groups and such buckets than buckets).  aux_counter[2], [3], [5], [4]: the four kinds.
 __global__ void __launch_bounds__(kGroupSpan)
 settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   chain_begin();
@@ -408,16 +420,23 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
   __syncthreads();
   if (tid == 0 && base[1] + arrived[here] > a.most_movers) fail_settle(a.hdr);  // more than there is room for
   const uint32_t mine = tid < here ? cut.start[tid + 1] - cut.start[tid] : 0u;
-  uint32_t capacity = a.teams ? SettledTeam::kCapacity : SettledBlock::kCapacity;
-  int cells = a.teams ? SettledTeam::kMaxCells : SettledBlock::kMaxCells;
-  const int crowded = __syncthreads_count(mine > capacity);
-  const bool wide = crowded > 0;
-  if (wide) {
-    if (tid == 0) atomicAdd(&a.hdr->settle_large, static_cast<uint32_t>(crowded));
-    capacity = SettledWide::kCapacity;
-    cells = SettledWide::kMaxCells;
-  }
-  cut_groups_of_block(cut, here, kGroupSpanLog, cells >> a.shift, capacity, &a.hdr->aux_counter[wide ? 3 : 2]);
+  const int crowded = __syncthreads_count(mine > a.capacity);
+  if (crowded && tid == 0) atomicAdd(&a.hdr->settle_large, static_cast<uint32_t>(crowded));
+  // Dense spans, a bit each: a run of such, or of others, is cut into groups by itself.
+  __shared__ uint32_t dense_spans;
+  if (tid == 0) dense_spans = 0;
+  __syncthreads();
+  if (crowded && a.capacity < SettledDense::kCapacity && mine > a.capacity) atomicOr(&dense_spans, 1u << (tid >> kDenseSpanLog));
+  __syncthreads();
+  const int span = tid >> kDenseSpanLog;
+  const bool dense = (dense_spans >> span) & 1u;
+  const uint32_t unlike = dense ? ~dense_spans : dense_spans;
+  const bool begins = tid == 0 || ((tid & ((1 << kDenseSpanLog) - 1)) == 0 && ((unlike >> (span - 1)) & 1u));
+  const int next = __ffs(static_cast<int>(unlike & ~((2u << span) - 1)));  // one more than the next unlike span, or 0
+  const uint32_t capacity = dense ? SettledDense::kCapacity : a.capacity;
+  cut_groups_of_block(cut, here, begins, next ? (next - 1) << kDenseSpanLog : kGroupSpan, kGroupSpan,
+                      (dense ? SettledDense::kMaxCells : a.most_cells) >> a.shift, capacity, &a.hdr->aux_counter[2],
+                      &a.hdr->aux_counter[3], dense);
   auto write_table = [&](uint32_t* tables, uint32_t row, int first, int end) {
     uint4* table = reinterpret_cast<uint4*>(tables + static_cast<size_t>(row) * kSettledRowWords);
     const uint32_t in_group = arrived[end] - arrived[first];
@@ -426,9 +445,12 @@ settled_groups_kernel(const __grid_constant__ SettledArgs a) {
     table[1] = make_uint4(base[2] + output[first], output[end] - output[first],
                           static_cast<uint32_t>(b0 + first), static_cast<uint32_t>(b0 + end));
   };
-  if (tid < static_cast<int>(cut.found))
-    write_table(wide ? a.wide_tables : a.tables, cut.list_base + tid, cut.group_first[tid], cut.link[cut.group_first[tid]]);
-  if (mine > capacity) write_table(a.tables, a.buckets - 1 - atomicAdd(&a.hdr->aux_counter[4], 1u), tid, tid + 1);
+  const int found = static_cast<int>(cut.found), all = found + static_cast<int>(cut.found_other);
+  if (tid < all)
+    write_table(tid < found ? a.tables : a.dense_tables, tid < found ? cut.list_base + tid : cut.other_base + tid - found,
+                cut.group_first[tid], cut.link[cut.group_first[tid]]);
+  if (mine > SettledWide::kCapacity) write_table(a.tables, a.buckets - 1 - atomicAdd(&a.hdr->aux_counter[4], 1u), tid, tid + 1);
+  else if (mine > capacity) write_table(a.wide_tables, atomicAdd(&a.hdr->aux_counter[5], 1u), tid, tid + 1);
 }
 
 // The movers' records to their buckets, with their keys.
@@ -474,6 +496,24 @@ struct __align__(16) SettledSmem {
   uint32_t warp_sum[32];
 };
 
+// What the kernels behind the sort of a settled state know of it.
+struct SettledCall {
+  SettledArgs args;
+  FinishOut out;
+};
+
+struct BlockBarrier {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+// Of the THREADS threads of a part of a block.
+template <int THREADS>
+struct PartBarrier {
+  int part;
+  __device__ __forceinline__ void operator()() const {
+    asm volatile("bar.sync %0, %1;" ::"r"(part + 1), "n"(THREADS) : "memory");
+  }
+};
+
 // Groups g, g + step, ... of a list, one after the other; false if a counter wrapped.  The sort is that of
 // sort_placed: byte counters of the low key, whose returned value is the rank on a counter, their scan, and a compare
 // of the records that share one.  But a thread keeps its records in registers from load to store, and puts them in
@@ -486,12 +526,13 @@ struct __align__(16) SettledSmem {
 // 344 -> 253, 128 M 2168 -> 1560 (60 bytes a particle: 5.2 TB/s).  Stored to the output straight from the
 // registers, neighbouring lanes to places a few cells wide, 16.8 M took 221 us in groups of 1024, and 64 to a cell
 // 372, in parts of sectors; read by sorted place instead, 250 and 299.
-template <class Shape>
+template <class Shape, class Barrier>
 __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, const SettledArgs& a, const FinishOut& out,
-                                                      const uint32_t* list, uint32_t g, uint32_t groups, uint32_t step) {
+                                                      const uint32_t* list, uint32_t g, uint32_t groups, uint32_t step,
+                                                      int tid, Barrier barrier) {
   constexpr int kThreads = Shape::kThreads, kItems = Shape::kItems, kWarps = kThreads / 32;
   constexpr int kWordsPerThread = Shape::kWordsPerThread;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < Shape::kHistWords; i += kThreads) s.hist[i] = 0;
   const uint4* tables = reinterpret_cast<const uint4*>(list);  // two to a group
   uint4 where{}, what{};
@@ -558,7 +599,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
         f[k][5] = __uint_as_float(hi.w);
       }
     }
-    __syncthreads();  // the counters are zero
+    barrier();  // the counters are zero
 
     // Written without branches around more than one access, so that the compiler predicates them.
     uint32_t run[kItems];
@@ -570,7 +611,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
       run[k] = (old >> sh) & 0xffu;
       word[k] |= (key[k] & drop_mask) << (32 - Shape::kMaxDrop);
     }
-    __syncthreads();
+    barrier();
 
     // Exclusive scan of the counters.
     uint32_t local[kWordsPerThread];
@@ -594,7 +635,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
       if (lane >= o) incl += t;
     }
     if (lane == 31) s.warp_sum[warp] = incl;
-    __syncthreads();
+    barrier();
     // Every warp adds up the warps' sums for itself.
     const uint32_t warps = lane < kWarps ? s.warp_sum[lane] : 0u;
     const uint32_t total = __reduce_add_sync(0xffffffffu, warps);
@@ -608,7 +649,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
       *reinterpret_cast<uint2*>(&s.word_prefix[tid * kWordsPerThread + j]) = prefix;
     }
     if (total != count) return false;  // a counter wrapped (the same answer everywhere)
-    __syncthreads();
+    barrier();
 
     const int cell_words = cell_words_for(drop);
     const int hist_words = counter_words(cells_here, drop);
@@ -629,7 +670,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
       longest = max(longest, length);
       run[k] = start | length << 16;
     }
-    __syncthreads();
+    barrier();
 #pragma unroll
     for (int j = 0; j < kWordsPerThread; j += 4)
       *reinterpret_cast<uint4*>(&s.hist[tid * kWordsPerThread + j]) = make_uint4(0u, 0u, 0u, 0u);
@@ -648,7 +689,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
           if (j < length) slot += others[j] < word[k];
       run[k] = slot;
     }
-    __syncthreads();
+    barrier();
     // The places of the stage are those of the output, from the 16 bytes on in which it begins.
     const uint32_t lead = begin & 3u;
 #pragma unroll
@@ -661,7 +702,7 @@ __device__ __forceinline__ bool finish_settled_groups(SettledSmem<Shape>& s, con
         for (int c = 0; c < 6; ++c) to[(2 + c) * SettledSmem<Shape>::kRow] = __float_as_uint(f[k][c]);
       }
     }
-    __syncthreads();
+    barrier();
     const uint32_t base = begin - lead, last = lead + count;
     for (uint32_t p = tid * 4; p < last; p += kThreads * 4) {
       uint32_t* const rows[kRecordWords] = {
@@ -694,10 +735,30 @@ settled_finish_kernel(const __grid_constant__ SettledArgs a, const __grid_consta
   if (__syncthreads_or(threadIdx.x == 0 && settle_failed(a.hdr))) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) out.cell_start[a.num_cells] = a.n;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  if (!finish_settled_groups<Shape>(*reinterpret_cast<SettledSmem<Shape>*>(smem_raw), a, out, a.tables, blockIdx.x,
-                                    groups, gridDim.x) &&
+  if (!finish_settled_groups(*reinterpret_cast<SettledSmem<Shape>*>(smem_raw), a, out, a.tables, blockIdx.x, groups,
+                             gridDim.x, threadIdx.x, BlockBarrier{}) &&
       threadIdx.x == 0)
     fail_settle(a.hdr);
+}
+
+// The groups of dense regions, by the THREADS of the general path's finish kernel, which has nothing else to do behind a
+// sort that succeeds: block `block` of `blocks`.  False if a counter wrapped.  A thread's registers are full: with two or
+// three records a thread for groups of fewer, picked group by group, the compiler spilled 350 to 850 bytes and 16.8 M particles, half
+// of them in a twentieth of the space, took 533 us instead of 504.
+template <int THREADS>
+__device__ __forceinline__ bool finish_settled_dense(unsigned char* smem, const SettledCall& call, uint32_t block,
+                                                     uint32_t blocks) {
+  constexpr int kPart = SettledDense::kThreads, kParts = THREADS / kPart;
+  static_assert(THREADS == kParts * kPart, "whole parts");
+  auto* s = reinterpret_cast<SettledSmem<SettledDense>*>(smem);
+  const uint32_t* list = call.args.dense_tables;
+  const uint32_t groups = call.args.hdr->aux_counter[3];
+  if (block * kParts >= groups) return true;
+  if constexpr (kParts == 1)
+    return finish_settled_groups(*s, call.args, call.out, list, block, groups, blocks, threadIdx.x, BlockBarrier{});
+  const int part = threadIdx.x / kPart;
+  return finish_settled_groups(s[part], call.args, call.out, list, block * kParts + part, groups, blocks * kParts,
+                               threadIdx.x % kPart, PartBarrier<kPart>{part});
 }
 
 // The records of a bucket that no block holds: its home run in the input without those that left, and its

@@ -943,24 +943,27 @@ struct GroupCut {
   uint16_t link[kGroupSpan];       // where a group that began with this bucket would end
   uint16_t group_first[kGroupSpan], jumps[kGroupSpan + 1];
   unsigned char is_first[kGroupSpan + 1];
-  uint32_t warp_sum[32], found, list_base;
+  uint32_t warp_sum[32], found, list_base, found_other, other_base;
 };
 
-// Cuts every aligned block of 2^group_shift of the `here` buckets greedily into groups of at most
-// `most` consecutive buckets with at most `capacity` records (each bucket looks up where a group
+// Cuts every block of the `here` buckets (from one that is `first_of_block` to its `block_end`, `longest` buckets at most) greedily
+// into groups of at most `most` consecutive buckets with at most `capacity` records (each bucket looks up where a group
 // that began with it would end, and those links are followed).  Afterwards group k of the block,
 // k < c.found, has the buckets c.group_first[k] .. c.link[c.group_first[k]], and its place in the
 // list of all groups is c.list_base + k; the list's order is of no consequence.  A bucket that
 // exceeds the capacity on its own is in no group.  Returns the largest bucket of the thread's warp.
-__device__ __forceinline__ uint32_t cut_groups_of_block(GroupCut& c, int here, int group_shift, int most,
-                                                        uint32_t capacity, uint32_t* group_count) {
+// `most` and `capacity` may differ from one block to another, and with `other_count` groups of blocks that
+// are `other` have a list of their own: group c.found + k of the block, k < c.found_other, is at c.other_base + k there.
+__device__ __forceinline__ uint32_t cut_groups_of_block(GroupCut& c, int here, bool first_of_block, int block_end,
+                                                        int longest, int most, uint32_t capacity, uint32_t* group_count,
+                                                        uint32_t* other_count = nullptr, bool other = false) {
   const int tid = threadIdx.x;
   uint32_t load = 0;
-  const bool first_of_block = tid < here && (tid & ((1 << group_shift) - 1)) == 0;
+  first_of_block = first_of_block && tid < here;
+  block_end = min(here, block_end);
   int jump = kGroupSpan;
   if (tid < here) {
     load = c.start[tid + 1] - c.start[tid];
-    const int block_end = min(here, ((tid >> group_shift) + 1) << group_shift);
     int lo = tid + 1, hi = min(block_end, tid + most);  // the last end with start[end] - start[tid] <= capacity
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -971,9 +974,9 @@ __device__ __forceinline__ uint32_t cut_groups_of_block(GroupCut& c, int here, i
   }
   c.is_first[tid] = first_of_block;
   if (tid == 0) c.is_first[kGroupSpan] = 0;
-  // The groups' first buckets: those reached from the aligned blocks' first buckets along the
+  // The groups' first buckets: those reached from the blocks' first buckets along the
   // links, 2^k links at a time in round k.
-  for (int hops = 1; hops < (1 << group_shift) && hops < kGroupSpan; hops <<= 1) {
+  for (int hops = 1; hops < longest; hops <<= 1) {
     c.jumps[tid] = static_cast<uint16_t>(jump);
     if (tid == 0) c.jumps[kGroupSpan] = kGroupSpan;
     __syncthreads();
@@ -987,9 +990,17 @@ __device__ __forceinline__ uint32_t cut_groups_of_block(GroupCut& c, int here, i
   if (tid < here && load > capacity) c.is_first[tid] = 0;  // too large for a group
   if (tid >= here) c.is_first[tid] = 0;
   const uint32_t mine = c.is_first[tid];
-  const uint32_t place = block_exclusive_scan(mine, c.warp_sum, &c.found);
-  if (mine) c.group_first[place] = static_cast<uint16_t>(tid);
-  if (tid == 0) c.list_base = c.found ? atomicAdd(group_count, c.found) : 0u;
+  // Both kinds in one scan, half a word each.
+  const uint32_t place = block_exclusive_scan(mine << (other ? 16 : 0), c.warp_sum, &c.found);
+  const uint32_t found = c.found & 0xffffu, found_other = c.found >> 16;
+  if (mine) c.group_first[other ? found + (place >> 16) : place & 0xffffu] = static_cast<uint16_t>(tid);
+  __syncthreads();
+  if (tid == 0) {
+    c.found = found;
+    c.list_base = found ? atomicAdd(group_count, found) : 0u;
+    c.found_other = found_other;
+    if (found_other) c.other_base = atomicAdd(other_count, found_other);
+  }
   __syncthreads();
   return __reduce_max_sync(0xffffffffu, load);
 }
@@ -1087,7 +1098,8 @@ group_kernel(const uint32_t* counts, uint32_t n, uint32_t* cursor, uint32_t* run
     bucket_start[b0 + i] = sum;
   }
   __syncthreads();
-  const uint32_t biggest = cut_groups_of_block(cut, here, group_shift, 1 << group_shift, capacity, group_count);
+  const uint32_t biggest = cut_groups_of_block(cut, here, (tid & ((1 << group_shift) - 1)) == 0, ((tid >> group_shift) + 1) << group_shift,
+                                               1 << group_shift, 1 << group_shift, capacity, group_count);
   if (lane == 0 && biggest > 0) {
     atomicMax(&hdr->max_bucket, biggest);
     if (biggest > largest) hdr->use_standard = 1;
@@ -1727,20 +1739,32 @@ __device__ __forceinline__ void touch_runs(FinishSmem<Shape>& s, int q, const Ru
   }
 }
 
+#include "settled_sort.cuh"
+
+// `settled`: what the sort of a settled state before the kernel left, or NotSettled where there was none (in the tail kernel,
+// with the arguments of such a sort 650,000 particles took 49.1 us instead of 48.4).
+struct NotSettled {};
+
 // A block works through groups blockIdx.x, blockIdx.x + gridDim.x, ... of the group list.
 // What it needs to know about a group (where its runs lie) arrives two groups ahead by
 // asynchronous copies; a group's records are asked into L2 while the group before it is
 // sorted, and copied into shared memory as soon as that one's output is written.
-template <class Shape>
+// Behind a sort of a settled state it takes that sort's groups of dense regions.
+template <class Shape, class Settled>
 __global__ void __launch_bounds__(Shape::kThreads, Shape::kBlocks)
 bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_device,
-                     int64_t num_cells, FinishOut out, Header* __restrict__ hdr, bool behind) {
-  chain_wait();
-  if (settled_before(hdr, behind)) return;
-  const uint32_t groups = *t.group_count;
-  if (handed_over(hdr)) return;
+                     int64_t num_cells, FinishOut out, Header* __restrict__ hdr, const __grid_constant__ Settled settled) {
   constexpr int kThreads = Shape::kThreads;
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  chain_wait();
+  if constexpr (std::is_same_v<Settled, SettledCall>) {
+    if (settled_before(hdr, true)) {
+      if (!finish_settled_dense<kThreads>(smem_raw, settled, blockIdx.x, gridDim.x)) hdr->use_standard = 1;
+      return;
+    }
+  }
+  const uint32_t groups = *t.group_count;
+  if (handed_over(hdr)) return;
   FinishSmem<Shape>& s = *reinterpret_cast<FinishSmem<Shape>*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5;
   if (blockIdx.x == 0 && tid == 0)
@@ -1813,8 +1837,6 @@ bucket_finish_kernel(RunTable t, int64_t n, const uint32_t* __restrict__ n_on_de
   chain_release();
 }
 
-#include "settled_sort.cuh"
-
 // Buckets first, first + step, ... below `last` that hold at least `at_least` records, one by one:
 // those the kernel above skipped, with more records than its shared memory holds, and those of a
 // group whose counters wrapped.  False if one of them cannot be finished at all.
@@ -1856,8 +1878,8 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
     hdr->use_standard = 1;
 }
 
-// Behind the finish kernel of an ordinary call: the oversized buckets (of the sort of a settled state the wide
-// groups and what those do not hold) and the groups whose counters
+// Behind the finish kernel of an ordinary call: the oversized buckets (of the sort of a settled state those that its
+// dense groups do not hold) and the groups whose counters
 // wrapped (calls without payload, whose sparse groups have 16 counters per cell), then, when the call was
 // handed over, the whole digit-pass sort.  Usually there is nothing to do and every block returns
 // after a look at the header.  What bounds it is then the launch itself: as the separate kernels
@@ -1867,14 +1889,11 @@ bucket_finish_large_kernel(RunTable t, int64_t num_cells, FinishOut out,
 // Blocks per multiprocessor, fewer of them where there is little to do.
 template <class Shape>
 constexpr int kTailBlocks = Shape::kThreads <= 512 ? 2 : 1;
-// `settled`: what the sort of a settled state before it left, or NotSettled where there was none (with
-// the arguments of such a sort 650,000 particles took 49.1 us instead of 48.4).
-struct NotSettled {};
 template <class Shape, class Settled>
 __global__ void __launch_bounds__(Shape::kThreads, kTailBlocks<Shape>)
 bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, uint32_t capacity,
                    DigitPassArgs digits, const __grid_constant__ Settled settled) {
-  constexpr bool kBehind = std::is_same_v<Settled, SettledArgs>;
+  constexpr bool kBehind = std::is_same_v<Settled, SettledCall>;
   chain_wait();
   const bool is_settled = settled_before(hdr, kBehind);
   const bool all_done = is_settled ? hdr->settle_large == 0 : hdr->max_bucket <= capacity && hdr->redo_groups == 0;
@@ -1893,11 +1912,11 @@ bucket_tail_kernel(RunTable t, int64_t num_cells, FinishOut out, Header* hdr, ui
     if constexpr (kBehind) {
       if (is_settled) {
         static_assert(Shape::kThreads == SettledWide::kThreads, "one block size");
-        auto& wide = *reinterpret_cast<SettledSmem<SettledWide>*>(smem_raw);
-        bool good = standard || finish_settled_groups<SettledWide>(wide, settled, out, settled.wide_tables, item,
-                                                                   hdr->aux_counter[3], items);
+        bool good = standard || finish_settled_groups(*reinterpret_cast<SettledSmem<SettledWide>*>(smem_raw), settled.args,
+                                                      settled.out, settled.args.wide_tables, item, hdr->aux_counter[5], items,
+                                                      threadIdx.x, BlockBarrier{});
         __syncthreads();
-        good = good && (standard || finish_settled_large<Shape>(s, settled, out, item, items));
+        good = good && (standard || finish_settled_large<Shape>(s, settled.args, settled.out, item, items));
         if (!good && threadIdx.x == 0) atomicExch(&hdr->use_standard, 1);
         return true;
       }
@@ -2571,20 +2590,21 @@ bool heavy_chained(const BucketPlan& p, bool behind) {
   return chained_launches() >= (behind || split || p.tiled ? 1 : 2);
 }
 
-template <class Shape>
+template <class Shape, class Settled = NotSettled>
 cudaError_t launch_finish(const RunTable& t, const SortArgs& a, const FinishOut& out, Header* hdr,
-                          const uint32_t* n_on_device = nullptr, bool behind = false,
-                          bool chained = false) {
+                          const uint32_t* n_on_device = nullptr, bool chained = false, const Settled& settled = {}) {
   const size_t table_bytes = 3 * 2 * static_cast<size_t>(t.row_words) * sizeof(uint32_t);
   if (std::is_same_v<Shape, FinishSmall> && table_bytes > kSmallShapeTableBytes)
     return cudaErrorInvalidValue;
+  static_assert(std::is_same_v<Settled, NotSettled> ||
+                    sizeof(SettledSmem<SettledDense>) * Shape::kThreads / SettledDense::kThreads <= sizeof(FinishSmem<Shape>),
+                "shared memory");
   const int smem = static_cast<int>(sizeof(FinishSmem<Shape>) + table_bytes);
-  cudaError_t e = allow_shared(bucket_finish_kernel<Shape>,
-                               sizeof(FinishSmem<Shape>) + 3 * 2 * kTableRowWords * sizeof(uint32_t));
+  auto kernel = bucket_finish_kernel<Shape, Settled>;
+  cudaError_t e = allow_shared(kernel, sizeof(FinishSmem<Shape>) + 3 * 2 * kTableRowWords * sizeof(uint32_t));
   if (e != cudaSuccess) return e;
-  return launch_chained_if(chained, bucket_finish_kernel<Shape>,
-                           std::min(t.buckets, sm_count() * Shape::kBlocks), Shape::kThreads, smem, a.stream,
-                           t, a.n, n_on_device, a.num_cells, out, hdr, behind);
+  return launch_chained_if(chained, kernel, std::min(t.buckets, sm_count() * Shape::kBlocks), Shape::kThreads, smem, a.stream,
+                           t, a.n, n_on_device, a.num_cells, out, hdr, settled);
 }
 
 // Buckets in no group (more records than a group may hold) go to the large shape whatever
@@ -2735,6 +2755,12 @@ bool outputs_over_inputs(const SortArgs& a) {
   return false;
 }
 
+enum SettledKind { kSettledTeams, kSettledBlocks };  // the shape that sorts the usual groups
+SettledKind settled_kind(int64_t n, int64_t num_cells) {
+  return n * SettledTeam::kMaxCells >= kSettledTeamLeast * num_cells && n <= kSettledTeamMostMean * num_cells ? kSettledTeams
+                                                                                                              : kSettledBlocks;
+}
+
 // Lays the settled sort out in the `room` bytes at `base` (the general path's records, which that
 // path writes after this one has given up); false if the call is not one for it.
 bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, size_t room, Header* hdr,
@@ -2743,9 +2769,10 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
       a.num_cells > (int64_t{1} << 25) - 1 || outputs_over_inputs(a))
     return false;
   SettledArgs s{};
-  s.teams = a.n * SettledTeam::kMaxCells >= kSettledTeamLeast * a.num_cells && a.n <= kSettledTeamMostMean * a.num_cells;
-  s.shift = shift_for(a.n, a.num_cells, s.teams ? kSettledTeamTarget : kSettledBlockTarget,
-                      log2_floor(s.teams ? SettledTeam::kMaxCells : SettledBlock::kMaxCells), 1);
+  const SettledKind kind = settled_kind(a.n, a.num_cells);
+  s.capacity = static_cast<uint32_t>(kind == kSettledTeams ? SettledTeam::kCapacity : SettledBlock::kCapacity);
+  s.most_cells = kind == kSettledTeams ? SettledTeam::kMaxCells : SettledBlock::kMaxCells;
+  s.shift = shift_for(a.n, a.num_cells, kind == kSettledTeams ? kSettledTeamTarget : kSettledBlockTarget, log2_floor(s.most_cells), 1);
   const int64_t buckets = (a.num_cells + (int64_t{1} << s.shift) - 1) >> s.shift;
   if (a.n > kSettledMostMean * buckets || buckets > a.n) return false;
   s.x = a.x; s.y = a.y; s.z = a.z; s.v = a.velocity;
@@ -2783,11 +2810,20 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
   s.cursor = take(buckets);
   s.sums = take((buckets + kSettledPart - 1) / kSettledPart * kSettledSums);
   s.tables = take(buckets * kSettledRowWords);
-  s.wide_tables = take(buckets * kSettledRowWords);
+  s.dense_tables = take(buckets * kSettledRowWords);
+  s.wide_tables = take((a.n / kSettledWideShare + 1) * kSettledRowWords);
   s.list = take(static_cast<int64_t>(s.scan_blocks) * (s.per_block / kListShare) * kRecordWords);
   s.arrived = take(static_cast<int64_t>(s.most_movers) * kRecordWords);
   *out = s;
   return used <= room;
+}
+
+template <class Shape>
+cudaError_t launch_settled_finish(const SettledArgs& s, const FinishOut& out, cudaStream_t stream) {
+  constexpr int kSmem = static_cast<int>(sizeof(SettledSmem<Shape>));
+  const cudaError_t e = allow_shared(settled_finish_kernel<Shape>, kSmem);
+  if (e != cudaSuccess) return e;
+  return launch_chained(settled_finish_kernel<Shape>, sm_count() * Shape::kBlocks, Shape::kThreads, kSmem, stream, s, out);
 }
 
 // Enqueues the sort of a settled state; the general path's kernels follow it.
@@ -2797,10 +2833,7 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   const bool whole = a.grid.ix_offset == 0 && a.grid.nx_local == a.grid.nx;
   auto scan = vec ? (whole ? settled_scan_kernel<true, true> : settled_scan_kernel<true, false>)
                   : (whole ? settled_scan_kernel<false, true> : settled_scan_kernel<false, false>);
-  auto finish = s.teams ? settled_finish_kernel<SettledTeam> : settled_finish_kernel<SettledBlock>;
-  const int finish_smem = static_cast<int>(s.teams ? sizeof(SettledSmem<SettledTeam>) : sizeof(SettledSmem<SettledBlock>));
-  cudaError_t e = allow_shared(finish, finish_smem);
-  if (e == cudaSuccess) e = allow_shared(scan, kScanSmem);
+  cudaError_t e = allow_shared(scan, kScanSmem);
   if (e != cudaSuccess) return e;
   stage_begin(kStageBucketCount, a.stream);
   e = launch_chained(whole ? settled_probe_kernel<true> : settled_probe_kernel<false>, s.scan_blocks, kSettledThreads, 0,
@@ -2818,9 +2851,9 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
     e = launch_chained(settled_movers_kernel, s.scan_blocks, kSettledThreads, 0, a.stream, s);
   stage_end(kStageBucketScatter, a.stream);
   stage_begin(kStageBucketFinish, a.stream);
-  if (e == cudaSuccess)
-    e = launch_chained(finish, sm_count() * (s.teams ? SettledTeam::kBlocks : SettledBlock::kBlocks),
-                       s.teams ? SettledTeam::kThreads : SettledBlock::kThreads, finish_smem, a.stream, s, out);
+  const SettledKind kind = settled_kind(a.n, a.num_cells);
+  const auto finish = kind == kSettledTeams ? launch_settled_finish<SettledTeam> : launch_settled_finish<SettledBlock>;
+  if (e == cudaSuccess) e = finish(s, out, a.stream);
   count_launches(6);
   return e;
 }
@@ -2878,11 +2911,11 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   const FinishOut out{a.keys_out, a.index_out, a.cell_counts, a.cell_start, a.xs, a.ys, a.zs,
                       a.vs, a.padded_sorted, index_bits_of(a.n)};
 
-  SettledArgs settled{};
+  SettledCall settled{SettledArgs{}, out};
   size_t zero_bytes = 0;
-  const bool behind = settled_args(a, p, base + l.records_off, l.total - l.records_off, hdr, &settled, &zero_bytes);
+  const bool behind = settled_args(a, p, base + l.records_off, l.total - l.records_off, hdr, &settled.args, &zero_bytes);
   if (behind) {
-    e = settled_sort(a, settled, zero_bytes, out);
+    e = settled_sort(a, settled.args, zero_bytes, out);
     if (e != cudaSuccess) return e;
   }
   const bool chained = heavy_chained(p, behind);
@@ -3001,9 +3034,11 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
   begin_stage(kStageBucketFinish);
   const RunTable t{records, start, run_begin, tables, &hdr->aux_counter[1],
                    table_row_words(l.chunks), l.chunks, buckets, p.shift, p.keys_only ? cursor : nullptr};
-  e = p.keys_only      ? launch_finish<FinishKeys>(t, a, out, hdr, nullptr, behind, chained)
-      : p.small_blocks ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, behind, chained)
-                       : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, behind, chained);
+  e = p.keys_only      ? launch_finish<FinishKeys>(t, a, out, hdr, nullptr, chained)
+      : p.small_blocks ? (behind ? launch_finish<FinishSmall>(t, a, out, hdr, nullptr, chained, settled)
+                                 : launch_finish<FinishSmall>(t, a, out, hdr, nullptr, chained))
+      : behind         ? launch_finish<FinishLarge>(t, a, out, hdr, nullptr, chained, settled)
+                       : launch_finish<FinishLarge>(t, a, out, hdr, nullptr, chained);
   if (e == cudaSuccess)
     e = behind        ? launch_tail<FinishLarge>(t, a, out, hdr, group_capacity, digits, chained, settled)
         : p.keys_only ? launch_tail<FinishKeys>(t, a, out, hdr, group_capacity, digits, chained, NotSettled{})

@@ -6,11 +6,13 @@ import torch
 
 import project_aether_b200 as pa
 from project_aether_b200 import particle_sort
+import test_settled_sort_gpu
 from test_settled_sort_gpu import LARGE, LEAST, _crowd, _dt, _run, _sorted_state, _words
 
 pytestmark = pytest.mark.gpu
 
-TEAM_GROUPS, WIDE_GROUPS, LARGE_BUCKETS = 54, 55, 56  # words of the workspace header
+# Words of the workspace header; the second: groups of dense spans, wider than a team's.
+TEAM_GROUPS, WIDE_GROUPS, LARGE_BUCKETS, WIDE_BUCKETS = 54, 55, 56, 57
 TEAM_TARGET = 104                                     # records of a team's bucket, on average at most
 
 
@@ -54,3 +56,51 @@ def test_outputs_off_16_byte_boundaries(cuda, off, squeeze):
     order = plain.order._replace(keys=move(plain.order.keys, off[1]), particle_index=move(plain.order.particle_index, off[1]))
     out = particle_sort.SortedParticles(order, tuple(move(t, off[0]) for t in plain.positions), plain.velocity)
     _run(grid, pos, vel, _dt(grid), cuda, 'settled', out=out)
+
+
+def _bucket_of(n, cells, records, device, drop=0):
+    """A state with one bucket of exactly `records`, most of them in one cell; nothing moves."""
+    grid, pos, vel = _sorted_state(n, cells, device, 31, drop=drop)
+    vel.zero_()
+    total = cells[0] * cells[1] * cells[2]
+    shift = max(s for s in range(7) if n <= TEAM_TARGET * (total >> s))
+    own = [(p * (c / h)).floor().clamp(max=c - 1) for p, c, h in zip(pos, cells, grid.hi)]
+    bucket = ((own[0] + cells[0] * (own[1] + cells[1] * own[2])) // 2 ** shift)
+    first = (bucket == bucket[n // 2]).nonzero()[0].item()
+    _crowd(pos, vel, first, records)
+    return grid, pos, vel
+
+
+@pytest.mark.parametrize('drop', [0, 1])
+@pytest.mark.parametrize('records,wide', [(2047, 0), (2048, 0), (2049, 1)])
+def test_a_bucket_at_the_capacity_of_a_dense_group(cuda, records, wide, drop):
+    grid, pos, vel = _bucket_of(LEAST + 100, (64, 64, 64), records, cuda, drop)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    words = _words(cuda)
+    assert words[WIDE_GROUPS] > 0 and words[WIDE_BUCKETS] == wide and words[LARGE_BUCKETS] == 0
+
+
+# Layers of other widths, small and large blocks of the general path's finish kernel, aligned and not.
+@pytest.mark.parametrize('n,cells,squeeze,drop', [(LEAST + 2, (60, 64, 61), (0.5, 0.05), 0), (LEAST + 5, (60, 64, 61), (0.5, 0.05), 3),
+                                                  (2_500_001, (29, 29, 29), (0.28, 0.03), 1), (2_500_001, (29, 29, 29), (0.5, 0.1), 0),
+                                                  (40_000_001, (170, 170, 170), (0.5, 0.05), 0),
+                                                  (40_000_003, (170, 170, 170), (0.2, 0.02), 1)])
+def test_dense_spans(cuda, n, cells, squeeze, drop):
+    grid, pos, vel = _sorted_state(n, cells, cuda, 34, squeeze=squeeze, drop=drop)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    words = _words(cuda)
+    assert words[TEAM_GROUPS] > 0 and words[WIDE_GROUPS] > 1
+
+
+def test_what_lies_near_a_dense_layer_stays_with_the_teams(cuda):
+    """A tenth of the particles in a layer one cell thick: four of five particles at least are sorted by teams, 512 places each."""
+    n = 4_000_000
+    grid, pos, vel = _sorted_state(n, (79, 79, 79), cuda, 35, squeeze=(0.1, 0.01))
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    words = _words(cuda)
+    assert words[WIDE_GROUPS] > 0 and words[TEAM_GROUPS].item() * 512 > 0.8 * n
+
+
+def test_a_counter_that_wraps_in_a_dense_group(cuda):
+    """300 particles with equal shuffle bits meet in a cell of some 800: the dense group gives the call to the digit passes."""
+    test_settled_sort_gpu.test_counters_that_wrap(cuda, 800, 'settled')
