@@ -72,8 +72,15 @@ struct SettledShape {
 // tail kernel instead of the finish kernel: 130, 1060.  Buckets half as wide: 2 percent more where the density is even.)
 using SettledTeam = SettledShape<128, 4, 11>;
 using SettledBlock = SettledShape<512, 4, 14>;
+// Below some four fifths of a particle to a cell a group is short of records, not of cells, and what it costs is its 2^14
+// counters and the places that stay empty: few records a thread, four groups to a multiprocessor.  us per call before groups were
+// sorted from registers / by SettledBlock / by this: 1.6 M in 160^3 cells 155 / 165 / 117, in 140^3 124 / 128 / 98, 17 M
+// in 320^3 1068 / 1115 / 758, in 290^3 880 / 891 / 627 (512 threads with one record each 126, 102, 817, 678; with two 141, 111,
+// 923, 749; 256 with four 130, 107, 855, 699; 128 with four 168, 138, 1173, 953).
+using SettledSparse = SettledShape<256, 2, 14>;
 using SettledDense = SettledBlock;
 using SettledWide = SettledShape<1024, 4, 15>;
+constexpr int64_t kSettledSparseMost = 400;    // particles on its most cells, on average at most: of 512 places
 constexpr int64_t kSettledTeamLeast = 352;     // particles on a team's most cells, on average at least
 constexpr int64_t kSettledTeamMostMean = 384;  // particles of a cell, on average at most
 // Records per bucket, on average at most.  Buckets cost this path little (a few words each), and with

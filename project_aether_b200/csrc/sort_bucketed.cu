@@ -2755,8 +2755,9 @@ bool outputs_over_inputs(const SortArgs& a) {
   return false;
 }
 
-enum SettledKind { kSettledTeams, kSettledBlocks };  // the shape that sorts the usual groups
+enum SettledKind { kSettledTeams, kSettledBlocks, kSettledSparse };  // the shape that sorts the usual groups
 SettledKind settled_kind(int64_t n, int64_t num_cells) {
+  if (n * SettledSparse::kMaxCells <= kSettledSparseMost * num_cells) return kSettledSparse;
   return n * SettledTeam::kMaxCells >= kSettledTeamLeast * num_cells && n <= kSettledTeamMostMean * num_cells ? kSettledTeams
                                                                                                               : kSettledBlocks;
 }
@@ -2770,8 +2771,10 @@ bool settled_args(const SortArgs& a, const BucketPlan& p, unsigned char* base, s
     return false;
   SettledArgs s{};
   const SettledKind kind = settled_kind(a.n, a.num_cells);
-  s.capacity = static_cast<uint32_t>(kind == kSettledTeams ? SettledTeam::kCapacity : SettledBlock::kCapacity);
-  s.most_cells = kind == kSettledTeams ? SettledTeam::kMaxCells : SettledBlock::kMaxCells;
+  s.capacity = static_cast<uint32_t>(kind == kSettledTeams    ? SettledTeam::kCapacity
+                                     : kind == kSettledBlocks ? SettledBlock::kCapacity : SettledSparse::kCapacity);
+  s.most_cells = kind == kSettledTeams    ? SettledTeam::kMaxCells
+                 : kind == kSettledBlocks ? SettledBlock::kMaxCells : SettledSparse::kMaxCells;
   s.shift = shift_for(a.n, a.num_cells, kind == kSettledTeams ? kSettledTeamTarget : kSettledBlockTarget, log2_floor(s.most_cells), 1);
   const int64_t buckets = (a.num_cells + (int64_t{1} << s.shift) - 1) >> s.shift;
   if (a.n > kSettledMostMean * buckets || buckets > a.n) return false;
@@ -2852,7 +2855,8 @@ cudaError_t settled_sort(const SortArgs& a, const SettledArgs& s, size_t zero_by
   stage_end(kStageBucketScatter, a.stream);
   stage_begin(kStageBucketFinish, a.stream);
   const SettledKind kind = settled_kind(a.n, a.num_cells);
-  const auto finish = kind == kSettledTeams ? launch_settled_finish<SettledTeam> : launch_settled_finish<SettledBlock>;
+  const auto finish = kind == kSettledTeams    ? launch_settled_finish<SettledTeam>
+                      : kind == kSettledBlocks ? launch_settled_finish<SettledBlock> : launch_settled_finish<SettledSparse>;
   if (e == cudaSuccess) e = finish(s, out, a.stream);
   count_launches(6);
   return e;

@@ -104,3 +104,37 @@ def test_what_lies_near_a_dense_layer_stays_with_the_teams(cuda):
 def test_a_counter_that_wraps_in_a_dense_group(cuda):
     """300 particles with equal shuffle bits meet in a cell of some 800: the dense group gives the call to the digit passes."""
     test_settled_sort_gpu.test_counters_that_wrap(cuda, 800, 'settled')
+
+
+# Either side of the line below which grids are sparse, with and without dense layers; the fewest particles to a cell that such a call has.
+@pytest.mark.parametrize('n,cells,squeeze,drop', [(1_600_000, (128, 125, 128), None, 0), (1_600_001, (128, 125, 128), None, 1),
+                                                  (LEAST, (160, 160, 160), (0.3, 0.1), 2), (LEAST + 1, (160, 160, 160), (0.1, 0.01), 0),
+                                                  (LEAST + 3, (200, 160, 131), (0.7, 0.02), 3), ((1 << 24) + 3, (322, 322, 322), (0.5, 0.3), 1)])
+def test_sparse_grids(cuda, n, cells, squeeze, drop):
+    grid, pos, vel = _sorted_state(n, cells, cuda, 36, squeeze=squeeze, drop=drop)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    assert _words(cuda)[TEAM_GROUPS] >= n // 512
+
+
+def test_groups_of_a_sparse_grid_are_short(cuda):
+    """By a block of 512 threads with four records each, groups of some 400 records, 1.6 M particles in 160^3 cells took more than
+    without such groups."""
+    n = 1_600_000
+    grid, pos, vel = _sorted_state(n, (160, 160, 160), cuda, 37)
+    push = (_dt(grid), grid.lo, grid.hi)
+    out = pa.sort_and_gather_particles(*pos, vel, grid, 1, push=push)
+
+    def took(share):
+        times = []
+        for _ in range(6):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for k in range(5):
+                pa.sort_and_gather_particles(*pos, vel, grid, k, push=(_dt(grid, share), grid.lo, grid.hi), out=out)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end) / 5)
+        return min(times)
+
+    settled, given_up = took(0.021), took(1.0)
+    assert settled < 0.85 * given_up, (settled, given_up)
