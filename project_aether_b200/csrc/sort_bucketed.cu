@@ -488,7 +488,7 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
                     int buckets, int chunk_log, uint32_t* __restrict__ cursor,
                     uint32_t* __restrict__ records, const Header* __restrict__ hdr,
                     bool behind) {
-  constexpr int ITEMS = 4, kTile = THREADS * ITEMS;
+  constexpr int kItems = 4, kTile = THREADS * kItems;
   chain_wait();
   if (settled_before(hdr, behind) || hdr->use_standard) return;
   extern __shared__ uint32_t slot_of[];  // a tile's counts, then its first slots
@@ -499,41 +499,38 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
     uint32_t* row = cursor + static_cast<size_t>(first >> chunk_log) * buckets;
     for (int b = tid; b < buckets; b += THREADS) slot_of[b] = 0;
     __syncthreads();
-    float f[6][ITEMS];
-    uint32_t key[ITEMS], rank[ITEMS];
+    float f[6][kItems];
+    uint32_t key[kItems], rank[kItems];
     bool sharing = true;
-#pragma unroll
-    for (int q = 0; q < ITEMS; q += 4) {
-      const int64_t i0 = first + (q / 4 * THREADS + tid) * 4;
-      if (VEC && i0 + 4 <= n) {
-        load_items<4>(x + i0, f[0] + q);
-        load_items<4>(y + i0, f[1] + q);
-        load_items<4>(z + i0, f[2] + q);
-        if (v) {
-          load_items<4>(v + i0, f[3] + q);
-          load_items<4>(v + padded + i0, f[4] + q);
-          load_items<4>(v + 2 * padded + i0, f[5] + q);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const bool ok = i0 + k < n;
-          f[0][q + k] = ok ? x[i0 + k] : 0.f;
-          f[1][q + k] = ok ? y[i0 + k] : 0.f;
-          f[2][q + k] = ok ? z[i0 + k] : 0.f;
-          f[3][q + k] = ok && v ? v[i0 + k] : 0.f;
-          f[4][q + k] = ok && v ? v[padded + i0 + k] : 0.f;
-          f[5][q + k] = ok && v ? v[2 * padded + i0 + k] : 0.f;
-        }
+    const int64_t i0 = first + tid * 4;
+    if (VEC && i0 + 4 <= n) {
+      load_items<4>(x + i0, f[0]);
+      load_items<4>(y + i0, f[1]);
+      load_items<4>(z + i0, f[2]);
+      if (v) {
+        load_items<4>(v + i0, f[3]);
+        load_items<4>(v + padded + i0, f[4]);
+        load_items<4>(v + 2 * padded + i0, f[5]);
       }
-      if (!v) {
+    } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) f[3][q + k] = f[4][q + k] = f[5][q + k] = 0.f;
+      for (int k = 0; k < 4; ++k) {
+        const bool ok = i0 + k < n;
+        f[0][k] = ok ? x[i0 + k] : 0.f;
+        f[1][k] = ok ? y[i0 + k] : 0.f;
+        f[2][k] = ok ? z[i0 + k] : 0.f;
+        f[3][k] = ok && v ? v[i0 + k] : 0.f;
+        f[4][k] = ok && v ? v[padded + i0 + k] : 0.f;
+        f[5][k] = ok && v ? v[2 * padded + i0 + k] : 0.f;
       }
     }
+    if (!v) {
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      const int64_t i = first + (k / 4 * THREADS + tid) * 4 + k % 4;
+      for (int k = 0; k < 4; ++k) f[3][k] = f[4][k] = f[5][k] = 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const int64_t i = i0 + k;
       if (push.enabled) {  // the fused move stage: the record carries the moved particle
         push_axis(f[0][k], f[3][k], push.dt, push.lo[0], push.hi[0]);
         push_axis(f[1][k], f[4][k], push.dt, push.lo[1], push.hi[1]);
@@ -551,8 +548,8 @@ tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < ITEMS; ++k) {
-      const int64_t i = first + (k / 4 * THREADS + tid) * 4 + k % 4;
+    for (int k = 0; k < kItems; ++k) {
+      const int64_t i = i0 + k;
       if (i < n)
         store_record(records + static_cast<size_t>(slot_of[key[k] >> (kShuffleBits + shift)] + rank[k]) *
                                    kRecordWords,
