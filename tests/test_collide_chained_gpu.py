@@ -79,3 +79,48 @@ def test_captured_behind_another_stream(cuda):
         graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(g, w) for g, w in zip((*out[:1], out[2], accepted), want))
+
+
+# Kernels that let the collisions in before they end: the sort in one launch does so when all its blocks run, and writes on.
+# `crowd`: in one cell, so many that the call ends in the digit passes, behind that point.
+@pytest.mark.parametrize('n,crowd', [(5001, 0), (20_003, 6000), (100_003, 0), (200_003, 6000), (500_001, 0), (500_001, 6000)])
+@pytest.mark.parametrize('captured', [False, True])
+def test_behind_a_sort_in_one_launch(cuda, n, crowd, captured):
+    grid = pa.CellGrid((0., 0., 0.), (1., 1., 1.), (20, 20, 10))
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    pos = [torch.rand(n, device=cuda, generator=gen) for _ in range(3)]
+    for t in pos:
+        t[:crowd] = 0.5
+    vel = torch.randn((3, n), device=cuda, generator=gen)
+    library = ntc_collide.load_library()
+    sigma, accepted = torch.empty(CELLS, device=cuda), torch.empty(CELLS, dtype=torch.int32, device=cuda)
+    stream = torch.cuda.Stream()
+
+    def step(out, between):
+        out = pa.sort_and_gather_particles(*pos, vel, grid, 5, padded_out=-(-n // 4) * 4, out=out)
+        between()
+        pa.collide(library, out.velocity, out.order.cell_start, sigma, accepted, n, PARAMS)
+        return out
+
+    def outputs(out):
+        return [t.clone() for t in (*out.order, *out.positions, out.velocity, sigma, accepted)]
+
+    with torch.cuda.stream(stream):
+        sigma.fill_(4.0)
+        out = step(None, torch.cuda.synchronize)
+        want = outputs(out)
+        assert pa.last_sort_used_digit_passes(cuda) == bool(crowd) and want[-1].sum() > 0
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    if captured:
+        with torch.cuda.graph(graph, stream=stream):
+            step(out, lambda: None)
+    for _ in range(5):
+        with torch.cuda.stream(stream):
+            for t in (*out.order, *out.positions, out.velocity):
+                t.zero_()
+            sigma.fill_(4.0)
+            graph.replay() if captured else step(out, lambda: None)
+            got = outputs(out)
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, w) for g, w in zip(got, want))

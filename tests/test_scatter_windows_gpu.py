@@ -36,7 +36,9 @@ def test_either_kernel(cuda, ordered, payload):
     assert pa.last_sort_status(cuda) == 0 and not pa.last_sort_used_digit_passes(cuda)
     torch.cuda.synchronize()
     workspace = particle_sort._workspaces[(cuda.index, torch.cuda.current_stream(cuda).cuda_stream)]
-    assert (workspace[:256].view(torch.int32)[SHARED_ROUNDS].item() >= N // 4096 // 2) == ordered
+    # Of the count kernel's rounds, 2048 particles each with so many buckets, nearly all or hardly any: the line is half of them.
+    shared, rounds = workspace[:256].view(torch.int32)[SHARED_ROUNDS].item(), N // 2048
+    assert 0.9 * rounds < shared <= rounds + 1000 if ordered else shared < 0.1 * rounds
     host = [np.ascontiguousarray(t.cpu().numpy()) for t in (x, y, z)]
     want, *rest = so.c_sort_particles(*host, np.ascontiguousarray(vel.cpu().numpy()),
                                       so.Grid(grid.lo, grid.hi, grid.cells), seed)

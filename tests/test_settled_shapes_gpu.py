@@ -1,5 +1,5 @@
-"""What sorts a group of a settled state: teams, blocks, wide groups in the tail kernel, and its large buckets.
-At the edges of their capacities, against the CPU oracle, bit for bit."""
+"""What sorts a group of a settled state: teams, blocks, sparse groups, dense groups in the general path's finish kernel, wide
+and large buckets in the tail kernel.  At the edges of their capacities, against the CPU oracle, bit for bit."""
 
 import pytest
 import torch
@@ -37,7 +37,7 @@ def test_a_bucket_at_a_capacity(cuda, records, wide, large):
     assert words[TEAM_GROUPS] > 0
 
 
-# Sparse grids and full cells (blocks), either side of the lines between teams and blocks.
+# Sparse grids and full cells (blocks), either side of the lower line between teams and blocks.  (The upper one is below.)
 @pytest.mark.parametrize('n,cells', [(LEAST + 7, (96, 100, 90)), (LEAST + 1, (66, 66, 66)), (LEAST + 1, (64, 66, 66)),
                                      (2_000_003, (17, 17, 18)), (2_000_003, (17, 17, 17)), (2_100_001, (13, 13, 13))])
 def test_sparse_and_full_cells(cuda, n, cells):
@@ -138,3 +138,32 @@ def test_groups_of_a_sparse_grid_are_short(cuda):
 
     settled, given_up = took(0.021), took(1.0)
     assert settled < 0.85 * given_up, (settled, given_up)
+
+
+# The upper line between teams and blocks, 384 to a cell: groups of one cell each, or of five.
+@pytest.mark.parametrize('n,teams', [(384 * 5202, True), (384 * 5202 + 1, False)])
+def test_full_cells_either_side_of_the_line(cuda, n, teams):
+    grid, pos, vel = _sorted_state(n, (17, 17, 18), cuda, 38)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    words = _words(cuda)
+    assert words[WIDE_GROUPS] == 0 and words[LARGE] == 0
+    assert words[TEAM_GROUPS] == 5202 if teams else words[TEAM_GROUPS] < 5202 // 4
+
+
+@pytest.mark.parametrize('drop', [0, 1])
+def test_full_cells_of_teams_some_above_their_capacity(cuda, drop):
+    """Half of the space with some 465 to a cell, the other with 307: cells above 512 here and there."""
+    grid, pos, vel = _sorted_state(384 * 5202 - 4, (17, 17, 18), cuda, 39, squeeze=(0.205, 0.5), drop=drop)
+    _run(grid, pos, vel, _dt(grid), cuda, 'settled')
+    words = _words(cuda)
+    assert words[TEAM_GROUPS] > 2000 and words[WIDE_GROUPS] > 10 and words[WIDE_BUCKETS] == 0
+
+
+# More buckets above all shapes' capacities than the tail kernel has blocks: of several cells, and of one.
+@pytest.mark.parametrize('drop', [0, 1])
+@pytest.mark.parametrize('n,cells,squeeze', [(LEAST + 4, (64, 63, 64), (0.72, 0.01)), (2_000_000, (16, 63, 16), (0.58, 0.01))])
+def test_many_buckets_that_no_block_holds(cuda, n, cells, squeeze, drop):
+    grid, pos, vel = _sorted_state(n, cells, cuda, 40, squeeze=squeeze, drop=drop)
+    _run(grid, pos, vel, _dt(grid, 0.002), cuda, 'settled')
+    blocks = torch.cuda.get_device_properties(cuda).multi_processor_count
+    assert _words(cuda)[LARGE_BUCKETS] > blocks

@@ -122,12 +122,13 @@ def test_dense_layer(cuda):
 
 
 def test_buckets_that_no_block_holds(cuda):
+    """Most of the particles in a thin layer: most buckets there are above a team's capacity, many above a dense group's."""
     grid, pos, vel = _sorted_state(4_000_000, (128, 64, 64), cuda, 6, squeeze=(0.7, 0.02))
     _run(grid, pos, vel, _dt(grid), cuda, 'settled')
 
 
-# A few buckets that no block holds; unaligned arrays; cells of more than 2560, the records of a block of the
-# groups; a mean of some 200 to a cell; blocks of the large finish shape behind.
+# Some buckets that no team holds (those that no block holds, in numbers: test_settled_shapes_gpu.py); unaligned arrays; cells
+# above the capacity of a dense group; a mean of some 200 to a cell; blocks of the large finish shape behind.
 @pytest.mark.parametrize('n,cells,squeeze,drop', [(LEAST, (64, 64, 64), (0.3, 0.002), 0),
                                                   (LEAST + 3, (101, 97, 89), (0.28, 0.03), 1),
                                                   (2_000_001, (32, 32, 32), (0.6, 0.01), 0),
