@@ -64,8 +64,8 @@ int run_sort(SortArgs& a, int path) {
   const bool bucketed = plan.usable && path != 1 && (roomy || path == 2);
   if (path == 2 && (!plan.usable || !roomy)) return cudaErrorInvalidValue;
   a.zero_padding = a.zero_padding && a.vs && a.padded_sorted > a.n;
-  // The bucketed path's clearing kernel zeroes the padding, but kernels behind it read the inputs while it runs.  (Not
-  // cudaMemset2D: rows of 2^29 floats and more are above the largest pitch that devices state, 2^31 - 1 bytes.)
+  // The bucketed path's clearing kernel zeroes the padding, but kernels behind it read the inputs while it runs: where the
+  // padding lies over one, and for the digit passes, the same kernel goes ahead in a launch of its own.
   if (a.zero_padding && (!bucketed || padding_over_inputs(a))) {
     const cudaError_t e = zero_padding_first(a);
     if (e != cudaSuccess) return e;

@@ -108,7 +108,8 @@ __device__ __forceinline__ bool collide_pair(float* a, float* b, float majorant,
 // registers) per multiprocessor.  A first design staged every particle of the block's cells in
 // shared memory, four blocks per multiprocessor, and wrote the stage back: 16 M particles in 2 M
 // cells took it 123 us, this kernel 61 (436 MB if every velocity is read and written once).  Chained to the kernel before
-// it, the sort's last in a step: step of 200,003 particles 33.6 -> 33.2 us, of 100,000 30.0 -> 27.4, of 1 M 57.7 -> 54.9.
+// it, the sort's last in a step: step of 100,000 particles 30.2 -> 27.4 us, of 200,003 33.3 -> 31.7, of 1 M 57.8 -> 55.5,
+// of 16.8 M 441 -> 438.
 __global__ void __launch_bounds__(kCollideThreads, kCollideBlocks)
 collide_kernel(CollideArgs a) {
   __shared__ int start[kCollideThreads];

@@ -29,9 +29,9 @@
 // kernels, which are enqueued behind them and otherwise return at once, do the call from the start.  When
 // it is noticed: random order and too many movers by the probe; a particle out of order, or more movers than
 // the lists hold in one part of the input, in the round of the scan that meets it; a counter that wraps in
-// the finish.  Buckets of a dense region are no reason.  Calls that the probe gives up, before there was this path /
-// now: 1.6 M particles 86.9 / 83.9 us, 4 M 170 / 167, 16.8 M 482 / 490, 30 M 837 / 833, 64 M 1885 / 1843; in random
-// order 1.6 M 87.3 / 88.0, 4 M 184 / 174, 6 M 250 / 234, 16.8 M 599 / 604, 64 M 2266 / 2238.
+// the finish.  Buckets of a dense region are no reason.  Calls that the probe gives up, without the attempt / with
+// it, particles that have all left their cell: 1.6 M 74 / 91 us, 4 M 162 / 176, 6 M 225 / 240, 16.8 M 551 / 567, 30 M 909 / 925, 64 M
+// 1951 / 1965, 128 M 3848 / 3890; in random order 1.6 M 77 / 91, 4 M 164 / 176, 16.8 M 599 / 614, 64 M 2239 / 2252.
 
 constexpr int kSettledThreads = 512;
 constexpr int kSettledRound = kSettledThreads * 4;  // particles of a block per round

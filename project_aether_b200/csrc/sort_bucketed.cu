@@ -2336,7 +2336,8 @@ constexpr int64_t kScatterWindowsFrom = int64_t{1} << 26;
 // one run per chunk, and short runs cost the scatter (partial lines) and the finish kernel
 // (many small copies) more than the window saves.  Measured optimum on random input (us per call): 2^22 particles per chunk
 // with 16 K buckets (64 M 2164 against 2271 with 2^23), 2^23 with 32 K or 64 K (100 M 3185 against 3298 with 2^22 and
-// 3457 with 2^24, 128 M 4306 / 4486 / 4598, 256 M 9006 against 9422 with 2^24), 2^24 beyond.  Smaller inputs take
+// 3457 with 2^24, 128 M 4306 / 4486 / 4598, 256 M 9006 against 9422 with 2^24; also with 33 chunks, one more than the groups kernel
+// keeps, 268,435,461 particles 9125 against 9535, 271 M 9225 against 9627), 2^24 beyond.  Smaller inputs take
 // smaller chunks (fewer particles contend for a slot counter): best 2^20 at 4 M particles, 2^21 at 16 M.
 inline int chunk_log_for(int64_t buckets, int64_t n) {
   if (n <= (int64_t{1} << 22)) return kChunkLog - 2;
@@ -2391,7 +2392,9 @@ BucketLayout bucket_layout_of(int64_t n, int64_t buckets, int chunk_log, int chu
 BucketLayout bucket_layout(int64_t n, const BucketPlan& p) {
   const int64_t buckets = p.buckets;
   // Tiles split in shared memory write whole runs: no window has to be kept small for them.  Nor for 8-byte records
-  // (scattered, 100 M particles 2540 us per call against 2682 with 2^23 particles to a chunk, 2622 with 2^25).
+  // (scattered, with 2^24 particles to a chunk / 2^23, us per call: 32 K buckets 28 M 1029 / 1046, 50 M 1504 / 1568, 67 M 1915 / 2039, 101 M
+  // 2629 / 2780, 135 M 3388 / 3630; 17 K buckets 20 M 673 / 687, 52 M 1424 / 1409, 101 M 2588 / 2809.  Below 2^26 either is ahead by up to 5 percent
+  // at single sizes, 32 K buckets 16.9 M 818 / 784, 17 K buckets 36 M 1088 / 1034; 2^24 by one or two on average.)
   const int chunk_log = p.one_launch || p.tiled || p.keys_only ? kKeyChunkLog : chunk_log_for(buckets, n);
   const int chunks = static_cast<int>(
       std::max<int64_t>(1, (n + (int64_t{1} << chunk_log) - 1) >> chunk_log));
@@ -2421,9 +2424,10 @@ int small_call_blocks(int64_t n, int64_t buckets) {
 // Up to where slots are reserved tile by tile.
 constexpr int64_t kTiledMostParticles = 6 << 20;
 constexpr int64_t kTiledMostBuckets = 8192;
-// From here on tiles of 4096 particles, 1024 threads (against 2048, 512 threads: 2 M particles with 20 to a cell 86.9 / 85.8
-// us per call, 2.4 M 102.2 / 106.8, 3 M 121.1 / 128.4, 4 M 153.8 / 170.9; with 8 to a cell 90.3 / 91.5, 92.8 / 94.9, 109.6 /
-// 112.3, 150.8 / 158.1, but 3.2 M 128.0 / 122.3).
+// From here on tiles of 4096 particles, 1024 threads (against 2048, 512 threads, us per call: 2 M particles with 20 to a cell
+// 86.1 / 85.6, 2.3 M 102.1 / 107.8, 3 M 119.5 / 123.1, 4 M 152.4 / 166.9; with 8 to a cell 91.1 / 93.4, 91.3 / 91.6, 110.1 / 113.4,
+// 149.0 / 164.1).  Of nine sizes from 1.5 to 4 M at 4, 8, 20, 64 and 300 to a cell 3.2 M alone is slower for it, 4 percent
+// at 4, 8 and 64 to a cell (126.6 / 121.7): not the number of rounds, which is the same either way.
 constexpr int64_t kWideTilesFrom = 2300000;
 
 // Largest bucket width 2^s, s <= max_shift, whose average load stays at or below `target`,
@@ -2662,8 +2666,8 @@ cudaError_t launch_split(const SortArgs& a, bool vec, uint32_t k0, uint32_t k1, 
   const cudaError_t e = allow_shared(kernel, kMostSplitShared);
   if (e != cudaSuccess) return e;
   // All blocks, and tiles as even as their rounds are (4 M particles: two of 6784 a block in place of two of 8192 for
-  // some and one for the others); in one chunk, which a tile may not leave.  us per call 1 M particles 41.6 -> 39.0, 1.6 M
-  // 53.6 -> 51.6, 2.5 M 80.4 -> 74, 3 M 84.0 -> 77.0, 4 M 94.8 -> 92.7, 5 M 122.0 -> 113.7, 8 M 170 -> 167, 15 M 327 -> 319.
+  // some and one for the others); in one chunk, which a tile may not leave.  us per call, 8 to a cell, 1 M particles 41.8 -> 39.6, 1.6 M
+  // 51.0 -> 45.9, 2.5 M 80.7 -> 74.3, 3 M 84.8 -> 77.7, 4 M 89.3 -> 87.3, 5 M 122.3 -> 114.1, 8 M 167 -> 163, 15 M 309 -> 304.
   const int64_t most = (THREADS <= 512 ? 2 : 1) * sm_count();
   const bool one_chunk = a.n <= int64_t{1} << chunk_log;
   const int64_t blocks = std::min<int64_t>(one_chunk ? (a.n + THREADS * 4 - 1) / (THREADS * 4) : (a.n + kTile - 1) / kTile, most);
@@ -2715,18 +2719,20 @@ cudaError_t launch_small(const SortArgs& a, const BucketPlan& p, const BucketLay
 
 namespace {
 // From how many particles on a moved state is first tried as a settled one, where the general path
-// would reserve its slots tile by tile, and where it would not.  Per call, general / settled, five percent leaving
-// their cell: re-sort or step of 1 M particles 70 / 73 us, 1.6 M 84 / 78, 4 M 168 / 142, 6 M 229 / 191 (tiles);
-// 8 M 287 / 288, 12.5 M 372 / 367, 14.5 M 419 / 415 (its scatter is near HBM speed on input that is nearly in
-// order, and the launches count), 15.5 M 448 / 438; 16.8 M 479 / 460, 24 M 662 / 627, 30 M 822 / 770, 64 M 1852 / 1581,
-// 128 M 3625 / 3107 (the general finish kernel's large blocks).  Below 2^24 the untiled gain is no more than a call
-// that gives up may lose.
+// would reserve its slots tile by tile, and where it would not.  us per call, general / settled / given up, five percent leaving
+// their cell, or all: 1.6 M particles 72 / 68 / 91, 4 M 157 / 119 / 176, 6 M 216 / 159 / 240 (tiles); 8 M 253 / 208 / 286,
+// 12.5 M 370 / 297 / 405, 15.5 M 448 / 358 / 490; 16.8 M 467 / 382 / 567, 30 M 805 / 637 / 925, 64 M 1794 / 1294 / 1965, 128 M
+// 3555 / 2573 / 3890.  The second line was drawn with a finish that sorted whole records in shared memory (12.5 M 372 /
+// 367, 16.8 M 479 / 460), where up to there a call had no more to gain than to lose by giving up (3 to 5 percent).  With the present finish it
+// would gain 18 percent from 6.3 M on; the line has not been moved.
 constexpr int64_t kSettledLeast = int64_t{3} << 19;
 constexpr int64_t kSettledLeastUntiled = int64_t{1} << 24;
 // Particles in a thousand that leave their bucket, above which the general path does the call (tiles; small finish blocks;
 // large ones).  Up to there the settled sort is faster: us per call, movers in a thousand, settled / given up, 16.8 M 76 407 / 488;
-// 64 M 129 1525 / 1835, 98 1475 / 1850; 128 M 98 2912 / 3631.  It would be beyond too; a call that fails late, when the
-// lists of the scan are full, costs most.
+// 64 M 129 1525 / 1835, 98 1475 / 1850; 128 M 98 2912 / 3631.  It would be beyond: without a limit, at 20 / 30 percent out of their cell 4 M
+// 131 / 138 us against 168 given up, 16.8 M 447 / 484 against 494, 64 M 1536 / 1704 against 1841.  What the limits keep off is a call
+// that fails late, when all the scan's lists are full (40 percent out of their cell: 209, 661, 2444 against 166, 504, 1888); from the
+// limits to there is room for a sample that sees too few.  One block whose list is full costs nothing: 16.8 M 484 either way.
 constexpr int64_t kMoversTiled = 180, kMoversSmall = 80, kMoversLarge = 140;
 
 bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
@@ -3019,6 +3025,9 @@ cudaError_t bucketed_sort(const SortArgs& a, const BucketPlan& p) {
     };
     using Two = std::integral_constant<int, 2>;
     using Four = std::integral_constant<int, 4>;
+    // Behind a settled attempt one kernel for any order: a second that returns at once, too, costs settled states more than
+    // windows gain those in random order (us per call without / with windows behind, settled 128 M 2680 / 2729, 256 M 7597 / 7732; random
+    // 128 M 4900 / 4630, 256 M 9253 / 9385).
     const bool windows = !behind && a.n > kScatterWindowsFrom;
     e = launch(Two(), sm_count() * 16, windows ? kScatterOrdered : kScatterAny);
     if (e == cudaSuccess && windows) {
